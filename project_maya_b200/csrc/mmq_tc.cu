@@ -34,6 +34,7 @@
 
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 #include "maya_internal.cuh"
 #include "maya_tcgen05.cuh"
@@ -67,9 +68,12 @@ template<int T> constexpr int kUnitBytes = kUnitRows * kRawRow<T>;
 template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 10 : T == MAYA_Q8_0 ? 8 : T == MAYA_IQ2_S ? 14 : 12;   // raw units in flight
 template<int T> constexpr int kBStages = T == MAYA_Q4_K ? 6 : 4;            // activation tiles (64 K-values) in flight
 template<int T> constexpr int kBRing = kBStages<T> * kBStage;
-// i-quants: the codebook as f16 (IQ2_S 1024 x 8 values, IQ3_S 512 x 4 values) and the 256 sign patterns as f16 sign masks
-template<int T> constexpr int kGridBytes = T == MAYA_IQ2_S ? 1024 * 16 : T == MAYA_IQ3_S ? 512 * 8 : 0;
-template<int T> constexpr int kTabBytes = kIq<T> ? kGridBytes<T> + 256 * 16 : 0;
+// i-quants: the codebook's bytes (IQ2_S 1024 x 8, IQ3_S 512 x 4), kept in kCopies copies that lie side by side in every
+// entry - lane l reads copy l % kCopies - so that a warp's 32 random entries spread over the banks: four 8-byte copies cost
+// about 5 wavefronts a lookup, sixteen 4-byte copies 2 (one copy: 6 and 3.5).  The first form of this expansion looked
+// f16 entries and f16 sign masks up 16 bytes at a time, 11 wavefronts each: 1400 of the 2000 cycles a pair of K steps took.
+template<int T> constexpr int kCopies = T == MAYA_IQ2_S ? 4 : T == MAYA_IQ3_S ? 16 : 0;
+template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 8 * kCopies<T> : T == MAYA_IQ3_S ? 512 * 4 * kCopies<T> : 0;
 template<int T> constexpr int kTabOff = kBRing<T> + kUnits<T> * kUnitBytes<T>;
 template<int T> constexpr size_t kSmemBytes = (size_t) kTabOff<T> + kTabBytes<T>;
 static_assert(kUnits<MAYA_Q4_K> <= kMaxUnits && kUnits<MAYA_Q8_0> <= kMaxUnits && kUnits<MAYA_IQ2_S> <= kMaxUnits &&
@@ -211,74 +215,102 @@ __device__ __forceinline__ void q80_stage(const uint8_t* rrow, uint32_t* r) {
 }
 
 // ---- i-quants.  `w` = the row's window as 32-bit words; the block starts OFF bytes into it (OFF is even and the same
-// for all rows of a K block: every field position is a compile-time constant).
+// for all rows of a K block).  Only the FIELDS are taken apart by code that knows OFF (eight small variants, every position a
+// compile-time constant); the expansion works on the taken-out fields, so there is one copy of it.  Expanding straight from
+// the window in eight variants made the loop too long for the instruction cache: half of all warp cycles waited for a fetch.
 template<int BYTE> __device__ __forceinline__ uint32_t win_u32(const uint32_t* w) {
     constexpr int i = BYTE / 4, r = BYTE % 4;
+    static_assert(r % 2 == 0, "fields start on even bytes");
     if constexpr (r == 0) return w[i];
-    else if constexpr (r == 1) return __byte_perm(w[i], w[i + 1], 0x4321);
-    else if constexpr (r == 2) return __byte_perm(w[i], w[i + 1], 0x5432);
-    else return __byte_perm(w[i], w[i + 1], 0x6543);
+    else return __byte_perm(w[i], w[i + 1], 0x5432);
 }
-template<int BYTE> __device__ __forceinline__ uint32_t win_u8(const uint32_t* w) { return (w[BYTE / 4] >> (8 * (BYTE % 4))) & 0xFF; }
+// bytes {B, B + 1, C, C + 1} (B and C even)
+template<int B, int C> __device__ __forceinline__ uint32_t win_two16(const uint32_t* w) {
+    return __byte_perm(w[B / 4], w[C / 4], (B % 4) | (B % 4 + 1) << 4 | (C % 4 + 4) << 8 | (C % 4 + 5) << 12);
+}
 template<int BYTE> __device__ __forceinline__ float win_f16(const uint32_t* w) {
     return __half2float(__ushort_as_half((unsigned short) ((w[BYTE / 4] >> (8 * (BYTE % 4))) & 0xFFFF)));
 }
-// IQ2_S (ggml dequantize_row_iq2_s): sub-block ib32 of 32 values: y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign;
-// here dl = f16(d (2 ls + 1) / 8) and w = dl * grid (one more f16 rounding), the sign XOR-ed into dl.
-template<int OFF, int PP>
-__device__ __forceinline__ void iq2s_pair(const uint32_t* w, const uint4* grid, const uint4* sgn, uint32_t* o) {
-    const float d = win_f16<OFF>(w);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int ib = 2 * PP + h;
-        const uint32_t qs4 = h ? win_u32<OFF + 2 + 4 * (2 * PP + 1)>(w) : win_u32<OFF + 2 + 4 * (2 * PP)>(w);
-        const uint32_t sg4 = h ? win_u32<OFF + 34 + 4 * (2 * PP + 1)>(w) : win_u32<OFF + 34 + 4 * (2 * PP)>(w);
-        const uint32_t qh = h ? win_u8<OFF + 66 + 2 * PP + 1>(w) : win_u8<OFF + 66 + 2 * PP>(w);
-        const uint32_t sc = h ? win_u8<OFF + 74 + 2 * PP + 1>(w) : win_u8<OFF + 74 + 2 * PP>(w);
-        (void) ib;
-        const uint32_t dl0 = h2_bits(__float2half2_rn(d * (float) (2 * (sc & 15) + 1) * 0.125f));
-        const uint32_t dl1 = h2_bits(__float2half2_rn(d * (float) (2 * (sc >> 4) + 1) * 0.125f));
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const uint32_t idx = ((qs4 >> (8 * l)) & 0xFF) | ((qh << (8 - 2 * l)) & 0x300);
-            const uint4 G = grid[idx], M = sgn[(sg4 >> (8 * l)) & 0xFF];
-            const uint32_t dl = l < 2 ? dl0 : dl1;
-            uint32_t* r = o + 16 * h + 4 * l;
-            r[0] = h2_bits(__hmul2(bits_h2(G.x), bits_h2(dl ^ M.x)));
-            r[1] = h2_bits(__hmul2(bits_h2(G.y), bits_h2(dl ^ M.y)));
-            r[2] = h2_bits(__hmul2(bits_h2(G.z), bits_h2(dl ^ M.z)));
-            r[3] = h2_bits(__hmul2(bits_h2(G.w), bits_h2(dl ^ M.w)));
-        }
+// The fields of the four sub-blocks of 32 values a team expands of a block: pairs TEAM and TEAM + 2, i.e. sub-blocks
+// 2 TEAM + {0, 1, 4, 5}.  q: codebook index bytes (one word a sub-block for IQ2_S, two for IQ3_S); sg: sign bytes; byte j of
+// qh: sub-block j's high index bits; sc: scale bytes, IQ2_S byte j = sub-block j's, IQ3_S byte j = pair j's.
+template<int T> struct IqFields {
+    uint32_t q[T == MAYA_IQ2_S ? 4 : 8], sg[4], qh, sc;
+    float d;
+};
+template<int T, int OFF, int TEAM> __device__ __forceinline__ void iq_fields(const uint32_t* w, IqFields<T>& F) {
+    constexpr int a = 2 * TEAM, c = a + 4;
+    F.d = win_f16<OFF>(w);
+    F.qh = win_two16<OFF + 66 + a, OFF + 66 + c>(w);
+    if constexpr (T == MAYA_IQ2_S) {
+        F.q[0] = win_u32<OFF + 2 + 4 * a>(w); F.q[1] = win_u32<OFF + 6 + 4 * a>(w);
+        F.q[2] = win_u32<OFF + 2 + 4 * c>(w); F.q[3] = win_u32<OFF + 6 + 4 * c>(w);
+        F.sg[0] = win_u32<OFF + 34 + 4 * a>(w); F.sg[1] = win_u32<OFF + 38 + 4 * a>(w);
+        F.sg[2] = win_u32<OFF + 34 + 4 * c>(w); F.sg[3] = win_u32<OFF + 38 + 4 * c>(w);
+        F.sc = win_two16<OFF + 74 + a, OFF + 74 + c>(w);
+    } else {
+        F.q[0] = win_u32<OFF + 2 + 8 * a>(w); F.q[1] = win_u32<OFF + 6 + 8 * a>(w);
+        F.q[2] = win_u32<OFF + 10 + 8 * a>(w); F.q[3] = win_u32<OFF + 14 + 8 * a>(w);
+        F.q[4] = win_u32<OFF + 2 + 8 * c>(w); F.q[5] = win_u32<OFF + 6 + 8 * c>(w);
+        F.q[6] = win_u32<OFF + 10 + 8 * c>(w); F.q[7] = win_u32<OFF + 14 + 8 * c>(w);
+        F.sg[0] = win_u32<OFF + 74 + 4 * a>(w); F.sg[1] = win_u32<OFF + 78 + 4 * a>(w);
+        F.sg[2] = win_u32<OFF + 74 + 4 * c>(w); F.sg[3] = win_u32<OFF + 78 + 4 * c>(w);
+        // the block's four scale bytes lie side by side: pair TEAM's and pair TEAM + 2's
+        F.sc = __byte_perm(win_u32<OFF + 106>(w), 0, TEAM == 0 ? 0x4420 : 0x4431);
     }
 }
-// IQ3_S (ggml dequantize_row_iq3_s): y = d (1 + 2 scale) * grid[qs | qh bit] * sign; 4 values per codebook entry.
-template<int OFF, int PP>
-__device__ __forceinline__ void iq3s_pair(const uint32_t* w, const uint2* grid, const uint4* sgn, uint32_t* o) {
-    const float d = win_f16<OFF>(w);
-    const uint32_t scb = win_u8<OFF + 106 + PP>(w);                    // scales[ib32 / 2]: low nibble ib32 even, high odd
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t q0 = h ? win_u32<OFF + 2 + 8 * (2 * PP + 1)>(w) : win_u32<OFF + 2 + 8 * (2 * PP)>(w);
-        const uint32_t q1 = h ? win_u32<OFF + 6 + 8 * (2 * PP + 1)>(w) : win_u32<OFF + 6 + 8 * (2 * PP)>(w);
-        const uint32_t qh = h ? win_u8<OFF + 66 + 2 * PP + 1>(w) : win_u8<OFF + 66 + 2 * PP>(w);
-        const uint32_t sg4 = h ? win_u32<OFF + 74 + 4 * (2 * PP + 1)>(w) : win_u32<OFF + 74 + 4 * (2 * PP)>(w);
-        const uint32_t nib = h ? (scb >> 4) : (scb & 15);
-        const uint32_t db = h2_bits(__float2half2_rn(d * (float) (1 + 2 * nib)));
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const uint32_t q = l < 2 ? q0 : q1;
-            const uint32_t i1 = ((q >> (16 * (l & 1))) & 0xFF) | ((qh << (8 - 2 * l)) & 256);
-            const uint32_t i2 = ((q >> (16 * (l & 1) + 8)) & 0xFF) | ((qh << (7 - 2 * l)) & 256);
-            const uint2 G1 = grid[i1], G2 = grid[i2];
-            const uint4 M = sgn[(sg4 >> (8 * l)) & 0xFF];
-            uint32_t* r = o + 16 * h + 4 * l;
-            r[0] = h2_bits(__hmul2(bits_h2(G1.x), bits_h2(db ^ M.x)));
-            r[1] = h2_bits(__hmul2(bits_h2(G1.y), bits_h2(db ^ M.y)));
-            r[2] = h2_bits(__hmul2(bits_h2(G2.x), bits_h2(db ^ M.z)));
-            r[3] = h2_bits(__hmul2(bits_h2(G2.y), bits_h2(db ^ M.w)));
-        }
-    }
+// Two codebook bytes -> two weights: `x` = (1024 + v) pairs, ndl = -1024 dl, so the fma is dl * v rounded once; then the
+// signs of values 2 P and 2 P + 1 from sign byte s: s * (2^(15 - 2P) + 2^(30 - 2P)) has them at bits 15 and 31 (the two
+// shifted copies of the 8 bits do not meet), and one three-input operation masks them out and flips the signs.
+template<int P> __device__ __forceinline__ uint32_t iq_two(__half2 x, uint32_t s, __half2 dl, __half2 ndl) {
+    const uint32_t v = h2_bits(__hfma2(x, dl, ndl));
+    return v ^ ((s * ((1u << (15 - 2 * P)) + (1u << (30 - 2 * P)))) & 0x80008000u);
 }
+__device__ __forceinline__ __half2 neg1024(__half2 dl) { return __hmul2(dl, __float2half2_rn(-1024.0f)); }
+// eight values of one sign byte: bytes ga (values 0..3) and gb (4..7)
+__device__ __forceinline__ void iq_eight(uint32_t ga, uint32_t gb, uint32_t s, __half2 dl, __half2 ndl, uint32_t* r) {
+    r[0] = iq_two<0>(bytes01_plus1024(ga), s, dl, ndl);
+    r[1] = iq_two<1>(bytes23_plus1024(ga), s, dl, ndl);
+    r[2] = iq_two<2>(bytes01_plus1024(gb), s, dl, ndl);
+    r[3] = iq_two<3>(bytes23_plus1024(gb), s, dl, ndl);
+}
+// Sub-block J of the fields -> 32 weights.  `tab`: this lane's copy of the codebook.
+// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; here dl = f16(d (2 ls + 1) / 8) and
+// w = dl * grid (one more f16 rounding).
+template<int J> __device__ __forceinline__ void iq_half(const IqFields<MAYA_IQ2_S>& F, float d, const uint2* tab, uint32_t* o) {
+    constexpr int C = kCopies<MAYA_IQ2_S>;
+    const uint32_t qh = byte_of(F.qh, J), sc = byte_of(F.sc, J), sg4 = F.sg[J];
+    // byte l of hw = bits 2l, 2l + 1 of qh: an entry's index is one byte permute {qs byte l, hw byte l, 0, 0}
+    const uint32_t hw = ((qh & 0x33u) * 0x1001u + (qh & 0xCCu) * 0x40040u) & 0x03030303u;
+    const __half2 dl0 = __float2half2_rn(d * (float) (2 * (sc & 15) + 1) * 0.125f), dl1 = __float2half2_rn(d * (float) (2 * (sc >> 4) + 1) * 0.125f);
+    const __half2 nd0 = neg1024(dl0), nd1 = neg1024(dl1);
+    const uint2 g0 = tab[prmt_raw(F.q[J], hw, 0xCC40u) * C], g1 = tab[prmt_raw(F.q[J], hw, 0xCC51u) * C];
+    const uint2 g2 = tab[prmt_raw(F.q[J], hw, 0xCC62u) * C], g3 = tab[prmt_raw(F.q[J], hw, 0xCC73u) * C];
+    iq_eight(g0.x, g0.y, byte_of(sg4, 0), dl0, nd0, o);
+    iq_eight(g1.x, g1.y, byte_of(sg4, 1), dl0, nd0, o + 4);
+    iq_eight(g2.x, g2.y, byte_of(sg4, 2), dl1, nd1, o + 8);
+    iq_eight(g3.x, g3.y, byte_of(sg4, 3), dl1, nd1, o + 12);
+}
+// IQ3_S (ggml dequantize_row_iq3_s): y = d (1 + 2 scale) * grid[qs | qh bit] * sign; 4 values per entry.
+template<int J> __device__ __forceinline__ void iq_half(const IqFields<MAYA_IQ3_S>& F, float d, const uint32_t* tab, uint32_t* o) {
+    const uint32_t qh = byte_of(F.qh, J), sg4 = F.sg[J], nib = (F.sc >> (8 * (J / 2) + 4 * (J % 2))) & 15u;
+    // byte l of h0 / h1 = bit l / 4 + l of qh, the ninth index bit of entry l / 4 + l
+    const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
+    const __half2 db = __float2half2_rn(d * (float) (1 + 2 * nib)), nd = neg1024(db);
+    uint32_t g[8];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        g[l] = tab[prmt_raw(F.q[2 * J], h0, 0xCC00u + ((4 + l) << 4) + l) * kCopies<MAYA_IQ3_S>];
+        g[4 + l] = tab[prmt_raw(F.q[2 * J + 1], h1, 0xCC00u + ((4 + l) << 4) + l) * kCopies<MAYA_IQ3_S>];
+    }
+    iq_eight(g[0], g[1], byte_of(sg4, 0), db, nd, o);
+    iq_eight(g[2], g[3], byte_of(sg4, 1), db, nd, o + 4);
+    iq_eight(g[4], g[5], byte_of(sg4, 2), db, nd, o + 8);
+    iq_eight(g[6], g[7], byte_of(sg4, 3), db, nd, o + 12);
+}
+// The super-scale at which -1024 dl would leave f16's range (d x 31 / 8 or d x 31 at or above 63): such a block is expanded
+// at a 64th of it and its weights are multiplied by 64 afterwards, both exact.
+template<int T> constexpr float kIqBigScale = T == MAYA_IQ2_S ? 16.0f : 2.0f;
 
 struct Pipe {                       // static shared memory of a block
     uint64_t a_full[kSt], b_full[6];
@@ -384,36 +416,13 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         mbar_init(&P.final, 2);
         P.fail = 0;
     }
-    if constexpr (kIq<T>) {                         // the codebook as f16 and the sign masks, once per block
-        uint4* sgn = (uint4*) (smem + kTabOff<T> + kGridBytes<T>);
-        for (int i = tid; i < 256; i += kMmqThreads) {
-            uint4 m;
-            const uint32_t b = (uint32_t) i;       // bit j of the pattern: value j is negative; two values per f16 pair
-            m.x = ((b & 1u) << 15) | ((b & 2u) << 30);
-            m.y = ((b & 4u) << 13) | ((b & 8u) << 28);
-            m.z = ((b & 16u) << 11) | ((b & 32u) << 26);
-            m.w = ((b & 64u) << 9) | ((b & 128u) << 24);
-            sgn[i] = m;
-        }
-        const __half2 k1024 = __float2half2_rn(1024.0f);
-        if constexpr (T == MAYA_IQ2_S) {
-            uint4* grid = (uint4*) (smem + kTabOff<T>);
-            for (int i = tid; i < 1024; i += kMmqThreads) {
-                const uint2 g = ((const uint2*) g_iq2s_grid)[i];
-                uint4 v;
-                v.x = h2_bits(__hsub2(bytes01_plus1024(g.x), k1024)); v.y = h2_bits(__hsub2(bytes23_plus1024(g.x), k1024));
-                v.z = h2_bits(__hsub2(bytes01_plus1024(g.y), k1024)); v.w = h2_bits(__hsub2(bytes23_plus1024(g.y), k1024));
-                grid[i] = v;
-            }
-        } else {
-            uint2* grid = (uint2*) (smem + kTabOff<T>);
-            for (int i = tid; i < 512; i += kMmqThreads) {
-                const uint32_t g = g_iq3s_grid[i];
-                uint2 v;
-                v.x = h2_bits(__hsub2(bytes01_plus1024(g), k1024)); v.y = h2_bits(__hsub2(bytes23_plus1024(g), k1024));
-                grid[i] = v;
-            }
-        }
+    if constexpr (T == MAYA_IQ2_S) {                // the codebook's copies, once per block
+        uint2* grid = (uint2*) (smem + kTabOff<T>);
+        for (int i = tid; i < 1024 * kCopies<T>; i += kMmqThreads) grid[i] = ((const uint2*) g_iq2s_grid)[i / kCopies<T>];
+    }
+    if constexpr (T == MAYA_IQ3_S) {
+        uint32_t* grid = (uint32_t*) (smem + kTabOff<T>);
+        for (int i = tid; i < 512 * kCopies<T>; i += kMmqThreads) grid[i] = g_iq3s_grid[i / kCopies<T>];
     }
     mbar_fence_init();
     if (warp == 0) tmem_alloc(&P.tmem, 512);
@@ -448,6 +457,9 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             if (lane == 0) mbar_arrive(&P.a_full[s]);
             return true;
         };
+        // i-quants: this lane's copy of the codebook
+        using Entry = std::conditional_t<T == MAYA_IQ2_S, uint2, uint32_t>;
+        [[maybe_unused]] const Entry* const tab = (const Entry*) (smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) : 0);
         [[maybe_unused]] uint4 corr[8];      // Q4_K: the constant terms of the current 8-block chunk (indexed by kb: local memory)
         // The same in two halves of 32 K-values: the first half's tensor-memory store is under way while the second half
         // is expanded (the store, its wait and the hand-off were a serial tail of every pair).
@@ -481,33 +493,35 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     const uint4 v = *(const uint4*) (rrow + 16 * i);
                     wv[4 * i] = v.x; wv[4 * i + 1] = v.y; wv[4 * i + 2] = v.z; wv[4 * i + 3] = v.w;
                 }
-                const uint4* sgn = (const uint4*) (smem + kTabOff<T> + kGridBytes<T>);
-                // the block's offset in its window, (kb * block bytes) % 16, has period 8 in kb: 8 unrolled variants
-#define MAYA_IQ_PAIRS(OFF)                                                                                          \
-    if constexpr (T == MAYA_IQ2_S) {                                                                               \
-        const uint4* grid = (const uint4*) (smem + kTabOff<T>);                                                    \
-        if (team == 0) { iq2s_pair<OFF, 0>(wv, grid, sgn, o); ok = put(kb * 4 + 0, o);                             \
-                         if (ok) { iq2s_pair<OFF, 2>(wv, grid, sgn, o); ok = put(kb * 4 + 2, o); } }              \
-        else { iq2s_pair<OFF, 1>(wv, grid, sgn, o); ok = put(kb * 4 + 1, o);                                       \
-               if (ok) { iq2s_pair<OFF, 3>(wv, grid, sgn, o); ok = put(kb * 4 + 3, o); } }                        \
-    } else {                                                                                                       \
-        const uint2* grid = (const uint2*) (smem + kTabOff<T>);                                                    \
-        if (team == 0) { iq3s_pair<OFF, 0>(wv, grid, sgn, o); ok = put(kb * 4 + 0, o);                             \
-                         if (ok) { iq3s_pair<OFF, 2>(wv, grid, sgn, o); ok = put(kb * 4 + 2, o); } }              \
-        else { iq3s_pair<OFF, 1>(wv, grid, sgn, o); ok = put(kb * 4 + 1, o);                                       \
-               if (ok) { iq3s_pair<OFF, 3>(wv, grid, sgn, o); ok = put(kb * 4 + 3, o); } }                        \
-    }
-                switch ((kb * kBlkBytes<T>) & 15) {
-                    case 0: MAYA_IQ_PAIRS(0) break;
-                    case 2: MAYA_IQ_PAIRS(2) break;
-                    case 4: MAYA_IQ_PAIRS(4) break;
-                    case 6: MAYA_IQ_PAIRS(6) break;
-                    case 8: MAYA_IQ_PAIRS(8) break;
-                    case 10: MAYA_IQ_PAIRS(10) break;
-                    case 12: MAYA_IQ_PAIRS(12) break;
-                    default: MAYA_IQ_PAIRS(14) break;
+                IqFields<T> F;
+#define MAYA_IQ_FIELDS(OFF) case OFF: if (team == 0) iq_fields<T, OFF, 0>(wv, F); else iq_fields<T, OFF, 1>(wv, F); break;
+                switch ((kb * kBlkBytes<T>) & 15) {      // where the block starts in its window: period 8 in kb
+                    MAYA_IQ_FIELDS(0) MAYA_IQ_FIELDS(2) MAYA_IQ_FIELDS(4) MAYA_IQ_FIELDS(6)
+                    MAYA_IQ_FIELDS(8) MAYA_IQ_FIELDS(10) MAYA_IQ_FIELDS(12)
+                    default: if (team == 0) iq_fields<T, 14, 0>(wv, F); else iq_fields<T, 14, 1>(wv, F); break;
                 }
-#undef MAYA_IQ_PAIRS
+#undef MAYA_IQ_FIELDS
+                const bool big = fabsf(F.d) >= kIqBigScale<T>, any_big = __any_sync(0xFFFFFFFFu, big);
+                const float ds = big ? F.d * 0.015625f : F.d;
+                auto half_block = [&](auto j, uint32_t* v) {
+                    iq_half<decltype(j)::value>(F, ds, tab, v);
+                    if (any_big) {
+                        const __half2 up = __float2half2_rn(big ? 64.0f : 1.0f);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i] = h2_bits(__hmul2(bits_h2(v[i]), up));
+                    }
+                };
+                auto pair = [&](auto i, int kp) {        // a pair of sub-blocks leaves in two halves, as the other types'
+                    constexpr int J = 2 * decltype(i)::value;
+                    half_block(std::integral_constant<int, J>{}, o);
+                    if (!acquire(kp)) return false;
+                    st_half(kp, 0, o);
+                    half_block(std::integral_constant<int, J + 1>{}, o + 16);
+                    st_half(kp, 1, o + 16);
+                    release(kp);
+                    return true;
+                };
+                ok = pair(std::integral_constant<int, 0>{}, kb * 4 + team) && pair(std::integral_constant<int, 1>{}, kb * 4 + team + 2);
             } else if constexpr (T == MAYA_Q4_K) {
                 Q4Scales S;
                 q4k_scales(*(const uint4*) rrow, S);
