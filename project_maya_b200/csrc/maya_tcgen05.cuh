@@ -108,23 +108,26 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
-// The products of 64 K-values (four K = 16 steps) into one accumulator and the commit that follows them, as one block of
-// instructions for a lean issuing thread.  The four B descriptors (already assembled: address word + 2 per step, 32 bytes
-// inside the 128-byte swizzle row) and the A column (8 per step) are computed by the caller BEFORE it waits for the
-// operands, so that nothing but the products stands between the wait and the tensor core.  `first` = 0 makes the first
-// product overwrite the accumulator.
-__device__ __forceinline__ void mma_f16_ts_x4_commit(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint64_t b1, uint64_t b2,
-                                                     uint64_t b3, uint32_t idesc, uint32_t first, uint32_t bar_smem) {
+// The products of 64 K-values (four K = 16 steps) into one accumulator and the commit that follows them, issued by one elected
+// lane of a CONVERGED warp.  Every operand must be warp-uniform and the caller's control flow too: then the operands live in
+// uniform registers, where the instruction wants them.  The four B descriptors are the address word `b_lo`, + 2 per step (32
+// bytes inside the 128-byte swizzle row), under the constant upper word `b_hi`; the A column advances 8 per step.
+// `first` = 0 makes the first product overwrite the accumulator.
+__device__ __forceinline__ void mma_f16_ts_x4_commit(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                                     uint32_t first, uint32_t bar_smem) {
     asm volatile(
-        "{\n\t.reg .pred p, t;\n\t.reg .b32 a1, a2, a3;\n\t"
-        "setp.ne.b32 p, %7, 0;\n\tsetp.eq.b32 t, %9, 0;\n\t"
+        "{\n\t.reg .pred e, p, t;\n\t.reg .b32 a1, a2, a3, b1, b2, b3;\n\t.reg .b64 d0, d1, d2, d3;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
         "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %6, {%9, %9, %9, %9}, p;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], %3, %6, {%9, %9, %9, %9}, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], %4, %6, {%9, %9, %9, %9}, t;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], %5, %6, {%9, %9, %9, %9}, t;\n\t"
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%8];\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b0), "l"(b1), "l"(b2), "l"(b3), "r"(idesc), "r"(first), "r"(bar_smem), "r"(0u)
+        "add.u32 b1, %2, 2;\n\tadd.u32 b2, %2, 4;\n\tadd.u32 b3, %2, 6;\n\t"
+        "mov.b64 d0, {%2, %3};\n\tmov.b64 d1, {b1, %3};\n\tmov.b64 d2, {b2, %3};\n\tmov.b64 d3, {b3, %3};\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d0, %4, p;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], d1, %4, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], d2, %4, t;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], d3, %4, t;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(bar_smem)
         : "memory");
 }
 // one look at the barrier at shared address `bar_smem`
@@ -160,6 +163,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// arrive on `bar` when every tcgen05.mma the elected lane of this (converged) warp issued so far has completed
+__device__ __forceinline__ void mma_commit_elect(uint32_t bar_smem) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar_smem) : "memory");
+}
 // arrive on `bar` when every tcgen05.mma this thread issued so far has completed
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -20,9 +20,9 @@
 //   warps 0..15 two teams of 8 warps that take alternate K steps; in a team one thread per weight row expands 32
 //               K-values of the row per step (packed half2 arithmetic: Q8_0 w = q * d; Q4_K w = fma(q, d * sc,
 //               -(dmin * m))) and tcgen05.st-s them into the row's lane;
-//   warps 17,19 one lane each, one accumulator each: two tcgen05.mma per step (2 K = 16 halves, A from tensor memory,
-//               B from shared memory), one commit per two steps -> the steps' buffers are free (a single thread
-//               cannot issue products as fast as the tensor core retires them unless its loop is a few instructions);
+//   warps 17,19 one accumulator each: two tcgen05.mma per step (2 K = 16 halves, A from tensor memory, B from shared
+//               memory), one commit per two steps -> the steps' buffers are free (the warp cannot issue products as fast as
+//               the tensor core retires them unless their operands stay in uniform registers: see there);
 //   warps 0..15 afterwards: the epilogue - tcgen05.ld (lane = weight row, column = activation row), SwiGLU, optional
 //               q8_1 rounding of h for the next product, then through shared memory: one bulk copy per activation row.
 // Which expert and which 160-row group of it a block handles is found on the device from `bounds`; no count travels
@@ -686,44 +686,44 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 for (int u = max(0, issued - NU); u < issued; ++u) wait_or_fail(P, &P.raw_full[u % NU], (u / NU) & 1);
         }
     } else if (warp == kDqWarps + 1 || warp == kDqWarps + 3) {
-        // ------------------------------------------------------------ tensor-core issue (one lane of two warps: one
-        //                                                              accumulator each, on different schedulers)
-        if (lane == 0) {
-            const int my = warp == kDqWarps + 1 ? 0 : 1;
-            // One product of N = rows rounded up to 16 per accumulator and K = 16: an M = 128 product occupies the
-            // tensor core for N / 2 cycles, but only if this thread can issue one that often - a single thread's
-            // instruction stream is the limit, so everything here is precomputed or kept incrementally (no divisions,
-            // no descriptor construction, the ready barrier tested once before falling into the bounded wait).
-            const int n_mma = max(16, (nrows + 15) & ~15);
-            const uint32_t idesc = (1u << 4) | ((uint32_t) (n_mma >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
-            const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem));
-            const uint32_t b_hi = (uint32_t) (bdesc0 >> 32), b_lo0 = (uint32_t) bdesc0, b_lo_end = b_lo0 + NB * (kBStage >> 4);
-            const uint32_t a0 = tmem + kACol + my * 32, a_end = a0 + kSt * 64, d0 = tmem + my * kAccCols;
-            const uint32_t bfull0 = smem_u32(&P.b_full[0]), afull0 = smem_u32(&P.a_full[0]), done0 = smem_u32(&P.done[0]);
-            uint32_t b_lo = b_lo0, at = a0, bfull = bfull0, afull = afull0;   // of the next pair of K steps
-            uint32_t ph_a = 0, ph_b = 0, first = 0;  // the barriers' phases; first = 0: the first product overwrites
-            const int npairs = nkt / 2 + ntp;
-            bool ok = true;
-            for (int kp = 0; kp < npairs; ++kp) {
-                // everything the products need, before the waits
-                const uint64_t hi = (uint64_t) b_hi << 32;
-                const uint64_t d0b = hi | b_lo, d1b = hi | (b_lo + 2), d2b = hi | (b_lo + 4), d3b = hi | (b_lo + 6);
-                const uint32_t done_bar = done0 + ((kp & (kDone - 1)) << 3);
-                const bool rb = mbar_test_wait_addr(bfull, ph_b), ra = mbar_test_wait_addr(afull, ph_a);
-                if (!rb && !wait_or_fail(P, &P.b_full[(bfull - bfull0) >> 3], ph_b)) { ok = false; break; }   // not there yet: the bounded wait
-                if (!ra && !wait_or_fail(P, &P.a_full[(afull - afull0) >> 3], ph_a)) { ok = false; break; }
-                tc_fence_after();
-                if (my == 0 && kp == 0) MAYA_STAMP(2);       // the first product
-                mma_f16_ts_x4_commit(d0, at, d0b, d1b, d2b, d3b, idesc, first, done_bar);
-                first = 1;
-                at += 64; afull += 8;
-                if (at == a_end) { at = a0; afull = afull0; ph_a ^= 1; }
-                b_lo += kBStage >> 4; bfull += 8;
-                if (b_lo == b_lo_end) { b_lo = b_lo0; bfull = bfull0; ph_b ^= 1; }
+        // ------------------------------------------------------------ tensor-core issue (two warps, one accumulator each, on
+        //                                                              different schedulers)
+        // One product of N = rows rounded up to 16 per accumulator and K = 16: an M = 128 product occupies the tensor core
+        // for N / 2 cycles, but only if this warp can issue one that often.  The whole warp walks the loop, converged, and
+        // one elected lane issues: everything the products take is warp-uniform and stays in uniform registers.  (With a
+        // single lane inside a divergent branch every operand of every product crossed from a vector register - 31 such
+        // moves and 430-550 cycles a pair of K steps, the longest stage of the whole pipeline.)
+        const int my = warp == kDqWarps + 1 ? 0 : 1;
+        const int n_rows = __shfl_sync(0xFFFFFFFFu, nrows, 0);
+        const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
+        const int n_mma = max(16, (n_rows + 15) & ~15);
+        const uint32_t idesc = (1u << 4) | ((uint32_t) (n_mma >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+        const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem));
+        const uint32_t b_hi = (uint32_t) (bdesc0 >> 32), b_lo0 = (uint32_t) bdesc0, b_lo_end = b_lo0 + NB * (kBStage >> 4);
+        const uint32_t a0 = tm + kACol + my * 32, a_end = a0 + kSt * 64, d0 = tm + my * kAccCols;
+        const uint32_t bfull0 = smem_u32(&P.b_full[0]), afull0 = smem_u32(&P.a_full[0]), done0 = smem_u32(&P.done[0]);
+        uint32_t b_lo = b_lo0, at = a0, bfull = bfull0, afull = afull0;   // of the next pair of K steps
+        uint32_t ph_a = 0, ph_b = 0, first = 0;      // the barriers' phases; first = 0: the first product overwrites
+        const int npairs = nkt / 2 + ntp;
+        bool ok = true;
+        for (int kp = 0; kp < npairs; ++kp) {
+            const uint32_t done_bar = done0 + ((kp & (kDone - 1)) << 3);
+            const bool rb = mbar_test_wait_addr(bfull, ph_b), ra = mbar_test_wait_addr(afull, ph_a);
+            if (!__all_sync(0xFFFFFFFFu, rb && ra)) {            // not there yet: the bounded waits
+                const bool got = wait_or_fail(P, &P.b_full[(bfull - bfull0) >> 3], ph_b) && wait_or_fail(P, &P.a_full[(afull - afull0) >> 3], ph_a);
+                if (!__all_sync(0xFFFFFFFFu, got)) { ok = false; break; }
             }
-            if (my == 0) MAYA_STAMP(3);                      // the last product issued
-            if (ok) mma_commit(&P.final);
+            tc_fence_after();
+            if (my == 0 && kp == 0 && lane == 0) MAYA_STAMP(2);  // the first product
+            mma_f16_ts_x4_commit(d0, at, b_lo, b_hi, idesc, first, done_bar);
+            first = 1;
+            at += 64; afull += 8;
+            if (at == a_end) { at = a0; afull = afull0; ph_a ^= 1; }
+            b_lo += kBStage >> 4; bfull += 8;
+            if (b_lo == b_lo_end) { b_lo = b_lo0; bfull = bfull0; ph_b ^= 1; }
         }
+        if (my == 0 && lane == 0) MAYA_STAMP(3);                 // the last product issued
+        if (ok) mma_commit_elect(smem_u32(&P.final));
     } else if (warp == kDqWarps + 2) {
         // ------------------------------------------------------------ activation tiles (one lane)
         if (lane == 0) {
