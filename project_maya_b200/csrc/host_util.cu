@@ -22,6 +22,19 @@ int refuse(int status) {
     return status;
 }
 
+int sm_count() {
+    static std::atomic<int> cached_dev{-1}, cached_n{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cached_dev.load() != dev) {
+        int n = 0;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        cached_n.store(n);
+        cached_dev.store(dev);
+    }
+    return cached_n.load();
+}
+
 }  // namespace maya
 
 using namespace maya;

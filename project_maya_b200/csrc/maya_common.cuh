@@ -12,6 +12,7 @@ namespace maya {
 // ---------------------------------------------------------------- launch bookkeeping (host)
 int note_launch(const char* what);          // cudaGetLastError -> status; counts failures
 int refuse(int status);                     // counts a refused call, returns status
+int sm_count();                             // multiprocessors of the current device
 inline cudaStream_t as_stream(void* s) { return (cudaStream_t) s; }
 inline bool aligned16(const void* p) { return (((uintptr_t) p) & 15u) == 0; }
 

@@ -88,9 +88,6 @@ static_assert(kUnits<MAYA_Q4_K> <= kMaxUnits && kUnits<MAYA_Q8_0> <= kMaxUnits &
 // mmq_tile_phases.py): 16 slots per tile for the first 4096 tiles of each of the four (type class, fused) kernels.
 #ifdef MAYA_MMQ_STAMPS
 __device__ long long g_stamps[4 * 4096 * 16];
-#define MAYA_STAMP(i) do { if (stamp_id >= 0) stamps[(i)] = clock64(); } while (0)
-#else
-#define MAYA_STAMP(i) do { } while (0)
 #endif
 __host__ __device__ constexpr int64_t xq_tail(int64_t cols) { return ((cols / 32) + 63) & ~(int64_t) 63; }
 __host__ __device__ constexpr int64_t xq_ld(int64_t cols) { return cols + xq_tail(cols); }
@@ -312,14 +309,22 @@ template<int J> __device__ __forceinline__ void iq_half(const IqFields<MAYA_IQ3_
 // at a 64th of it and its weights are multiplied by 64 afterwards, both exact.
 template<int T> constexpr float kIqBigScale = T == MAYA_IQ2_S ? 16.0f : 2.0f;
 
+// A block works on tile after tile (see mmq_kernel): what the roles share of one of them.  e < 0: no tile left.
+struct TileInfo { int e, row0, nrows, m0; };
+constexpr int kTiles = 8;            // ring of tile entries: the raw-unit loader, which makes them, is at most kMaxUnits / 4 + 1
+                                     // tiles ahead of the slowest reader (it waits for every unit to be read)
+
 struct Pipe {                       // static shared memory of a block
     uint64_t a_full[kSt], b_full[6];
     uint64_t done[kDone];            // done[p % kDone]: the products of K-step pair p (64 K-values) have completed
     uint64_t raw_full[kMaxUnits], raw_empty[kMaxUnits];
-    uint64_t final;
+    uint64_t tile_full[kTiles];      // tile entry written
+    uint64_t final;                  // a tile's products have completed
+    uint64_t acc_free;               // its accumulators have been read: the next tile's products may overwrite them
+    uint64_t stg_free[2];            // the write-back of an even / odd tile has left shared memory: loads may overwrite it
+    TileInfo tile[kTiles];
     uint32_t tmem;
     int fail;
-    int scan[2];                     // the block's (matrix, row group), found by warp 0
 };
 
 __device__ __forceinline__ bool failed(const Pipe& P) { return *(volatile const int*) &P.fail != 0; }
@@ -338,6 +343,16 @@ __device__ __forceinline__ bool wait_or_fail(Pipe& P, uint64_t* bar, uint32_t pa
     return false;
 }
 
+// A group's activation rows as the write-back leaves them in shared memory: rows rounded up to 8, and the bytes of the whole
+__device__ __forceinline__ int rows_up8(int nrows) { return (nrows + 7) & ~7; }
+template<bool GLU> __device__ __forceinline__ int staging_bytes(int nrows) { return rows_up8(nrows) * (GLU ? 128 * 6 + 8 : TM * 4); }
+
+// Persistent: one block an SM takes tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the list (group-major, a group's slabs
+// of weight rows side by side, so that the blocks at work share its activation rows in L2).  How many groups there are is
+// known only on the device; a grid sized for the most there can be cost 20 to 30 us a launch in blocks that found no tile
+// (64 tokens over 256 experts: 259 group rows launched, 55 in use), and every tile paid the block's set-up - tensor-memory
+// allocation, codebook, barriers - and its first loads' latency behind the previous block's write-back.  Here the barriers'
+// phases run on from tile to tile, and the raw loader starts the next tile's units while the last one is written back.
 template<int T, bool GLU>
 __global__ void __launch_bounds__(kMmqThreads, 1)
 mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -346,65 +361,20 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
     __shared__ Pipe P;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int NU = kUnits<T>, NB = kBStages<T>;
-
-    // ---- which (matrix, 160-row group) is blockIdx.y: ONE warp scans the per-matrix group counts (each lane the counts
-    //      of a run of consecutive matrices, an exclusive warp scan of the runs' sums, then the lane whose run holds the
-    //      wanted group walks it), 1024 matrices a round, and leaves the answer in shared memory - one block barrier
-    //      instead of the twenty a block-wide scan needs, on a path every tile and every surplus block of the grid takes
-    if (warp == 0) {
-        int found_e = -1, found_g = 0, base = 0;
-        const int want_all = (int) blockIdx.y;
-        for (int e0 = 0; e0 < A.n && found_e < 0; e0 += 1024) {
-            const int per = (min(A.n - e0, 1024) + 31) >> 5;          // matrices a lane (<= 32)
-            const int lo = e0 + lane * per, hi = min(lo + per, min(A.n, e0 + 1024));
-            int mine = 0;
-            for (int e = lo; e < hi; ++e) {
-                const int be = A.expert_map ? A.expert_map[e] : e;
-                mine += (A.bounds[be + 1] - A.bounds[be] + TN - 1) / TN;
-            }
-            int incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            const int want = want_all - base;
-            const unsigned holds = __ballot_sync(0xFFFFFFFFu, want >= incl - mine && want < incl);
-            if (want < total && holds != 0u && lane == __ffs(holds) - 1) {
-                int g = want - (incl - mine);
-                for (int e = lo; e < hi; ++e) {
-                    const int be = A.expert_map ? A.expert_map[e] : e;
-                    const int cnt = (A.bounds[be + 1] - A.bounds[be] + TN - 1) / TN;
-                    if (g < cnt) { found_e = e; found_g = g; break; }
-                    g -= cnt;
-                }
-                P.scan[0] = found_e;
-                P.scan[1] = found_g;
-            }
-            found_e = __shfl_sync(0xFFFFFFFFu, found_e, holds != 0u && want < total ? __ffs(holds) - 1 : 0);
-            base += total;
-        }
-        if (found_e < 0 && lane == 0) P.scan[0] = -1;
-    }
-    __syncthreads();
-    const int found_e = P.scan[0], found_g = P.scan[1];
-    if (found_e < 0) return;                        // beyond the last group: uniform for the whole block
-    const int be = A.expert_map ? A.expert_map[found_e] : found_e;
-    const int row0 = A.bounds[be] + found_g * TN;
-    const int nrows = min(TN, A.bounds[be + 1] - row0);
-    const bool big = nrows > 128;                   // the activation tile is a 128-row box and a 32-row box
-    const int m0 = (int) blockIdx.x * (GLU ? 128 : TM);
     const int nkt = A.w_cols / BK, nkb = A.w_cols / 256;
     // Q4_K: after every 8 blocks of K (32 pairs of K steps) one more pair carries the sum correction of those blocks' 64
     // groups - A = the groups' constant terms -dmin * m, B = the tail of the activation image (see xq_tail); the last pair
     // of a K that is not a multiple of 2048 is padded with zeros.  ntp = how many such pairs.
     const int ntp = T == MAYA_Q4_K ? (nkb + 7) / 8 : 0;
+    const int npairs = nkt / 2 + ntp;               // pairs of K steps of a tile
+    constexpr int kSlab = GLU ? 128 : TM;
+    const int nslab = (A.w_rows + kSlab - 1) / kSlab;
 #ifdef MAYA_MMQ_STAMPS
-    const int stamp_lin = (int) (blockIdx.y * gridDim.x + blockIdx.x);
-    const int stamp_id = stamp_lin < 4096 ? stamp_lin : -1;
-    long long* const stamps = g_stamps + ((size_t) ((T == MAYA_Q4_K || T == MAYA_IQ3_S ? 2 : 0) + (GLU ? 1 : 0)) * 4096 + max(stamp_id, 0)) * 16;
-    if (tid == 0 && stamp_id >= 0) { stamps[0] = clock64(); stamps[14] = nrows; stamps[15] = nkt / 2 + ntp; }
+    // stamps of tile t of this block: the tile's place in the list is blockIdx.x + t * gridDim.x
+    auto stamps_of = [&](int t) -> long long* {
+        const int lin = (int) blockIdx.x + t * (int) gridDim.x;
+        return lin < 4096 ? g_stamps + ((size_t) ((T == MAYA_Q4_K || T == MAYA_IQ3_S ? 2 : 0) + (GLU ? 1 : 0)) * 4096 + lin) * 16 : nullptr;
+    };
 #endif
 
     uint8_t* const raw = smem + kBRing<T>;
@@ -413,56 +383,49 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         for (int s = 0; s < NB; ++s) mbar_init(&P.b_full[s], 1);
         for (int s = 0; s < kDone; ++s) mbar_init(&P.done[s], 2);      // both issuers commit
         for (int u = 0; u < NU; ++u) { mbar_init(&P.raw_full[u], 1); mbar_init(&P.raw_empty[u], 4); }
+        for (int i = 0; i < kTiles; ++i) mbar_init(&P.tile_full[i], 1);
         mbar_init(&P.final, 2);
+        mbar_init(&P.acc_free, kDqWarps);
+        mbar_init(&P.stg_free[0], kDqWarps);
+        mbar_init(&P.stg_free[1], kDqWarps);
         P.fail = 0;
+        mbar_fence_init();
     }
-    if constexpr (T == MAYA_IQ2_S) {                // the codebook's copies, once per block
-        uint2* grid = (uint2*) (smem + kTabOff<T>);
-        for (int i = tid; i < 1024 * kCopies<T>; i += kMmqThreads) grid[i] = ((const uint2*) g_iq2s_grid)[i / kCopies<T>];
-    }
-    if constexpr (T == MAYA_IQ3_S) {
-        uint32_t* grid = (uint32_t*) (smem + kTabOff<T>);
-        for (int i = tid; i < 512 * kCopies<T>; i += kMmqThreads) grid[i] = g_iq3s_grid[i / kCopies<T>];
-    }
-    mbar_fence_init();
+    if (warp == kDqWarps && lane < 3)
+        asm volatile("prefetch.tensormap [%0];" ::"l"(lane == 0 ? &tm_w : lane == 1 ? &tm_x : &tm_x32) : "memory");
     if (warp == 0) tmem_alloc(&P.tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = P.tmem;
-    if (tid == 0) MAYA_STAMP(1);                    // set-up done
+    // the block's t-th tile, for a role that waits for its entry; false: the wait ran out or another role has failed
+    auto tile_of = [&](int t, TileInfo& ti) -> bool {
+        if (!wait_or_fail(P, &P.tile_full[t % kTiles], (t / kTiles) & 1)) return false;
+        ti = P.tile[t % kTiles];
+        return true;
+    };
 
     if (warp < kDqWarps) {
         // ------------------------------------------------------------ weight expansion
         // Two teams of 8 warps; in each, thread = one of the slab's 256 rows.  Team t expands the K steps kt with
         // kt % 2 == t, so that a step's latency (shared-memory reads, the packed-half chain, the tensor-memory store
         // and its wait) overlaps the other team's step.
+        if constexpr (T == MAYA_IQ2_S) {            // the codebook's copies, once per block, under the first loads' latency
+            uint2* grid = (uint2*) (smem + kTabOff<T>);
+            for (int i = tid; i < 1024 * kCopies<T>; i += kDqWarps * 32) grid[i] = ((const uint2*) g_iq2s_grid)[i / kCopies<T>];
+            named_bar_sync(2, kDqWarps * 32);
+        }
+        if constexpr (T == MAYA_IQ3_S) {
+            uint32_t* grid = (uint32_t*) (smem + kTabOff<T>);
+            for (int i = tid; i < 512 * kCopies<T>; i += kDqWarps * 32) grid[i] = g_iq3s_grid[i / kCopies<T>];
+            named_bar_sync(2, kDqWarps * 32);
+        }
         const int team = warp >> 3, row = tid & 255, w8 = warp & 7;
         const int slab = row >> 6;
         const uint8_t* const rbase = raw + (size_t) (row & 63) * kRawRow<T>;
         // rows 0..127 feed accumulator 0, rows 128..255 accumulator 1; a warp reaches the 32 lanes of its quadrant
         const uint32_t a_lane = tmem + ((uint32_t) (32 * (w8 & 3)) << 16) + kACol + (w8 >> 2) * 32;
-        bool ok = true;
-        auto put = [&](int kp, const uint32_t (&o)[32]) -> bool {   // the row's 64 values of pair kp -> its lane
-            const int s = kp % kSt;
-            if (kp >= kSt) {                     // the stage was last read by pair kp - kSt
-                const int pp = kp - kSt;
-                if (!wait_or_fail(P, &P.done[pp & (kDone - 1)], (pp / kDone) & 1)) return false;
-                tc_fence_after();
-            }
-            tmem_st32(a_lane + s * 64, o);
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&P.a_full[s]);
-            return true;
-        };
-        // i-quants: this lane's copy of the codebook
-        using Entry = std::conditional_t<T == MAYA_IQ2_S, uint2, uint32_t>;
-        [[maybe_unused]] const Entry* const tab = (const Entry*) (smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) : 0);
-        [[maybe_unused]] uint4 corr[8];      // Q4_K: the constant terms of the current 8-block chunk (indexed by kb: local memory)
-        // The same in two halves of 32 K-values: the first half's tensor-memory store is under way while the second half
-        // is expanded (the store, its wait and the hand-off were a serial tail of every pair).
+        // the stage of pair kp (counted over the block's tiles) is free: it was last read by pair kp - kSt
         auto acquire = [&](int kp) -> bool {
             if (kp >= kSt) {
                 const int pp = kp - kSt;
@@ -471,17 +434,39 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             }
             return true;
         };
-        auto st_half = [&](int kp, int h, const uint32_t* o16) {
-            tmem_st16(a_lane + (kp % kSt) * 64 + 16 * h, *(const uint32_t(*)[16]) o16);
-        };
         auto release = [&](int kp) {
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&P.a_full[kp % kSt]);
         };
+        auto put = [&](int kp, const uint32_t (&o)[32]) -> bool {   // the row's 64 values of pair kp -> its lane
+            if (!acquire(kp)) return false;
+            tmem_st32(a_lane + (kp % kSt) * 64, o);
+            release(kp);
+            return true;
+        };
+        // i-quants: this lane's copy of the codebook
+        using Entry = std::conditional_t<T == MAYA_IQ2_S, uint2, uint32_t>;
+        [[maybe_unused]] const Entry* const tab = (const Entry*) (smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) : 0);
+        [[maybe_unused]] uint4 corr[8];      // Q4_K: the constant terms of the current 8-block chunk (indexed by kb: local memory)
+        // A pair's two halves of 32 K-values: the first half's tensor-memory store is under way while the second half is
+        // expanded (the store, its wait and the hand-off were a serial tail of every pair).
+        auto st_half = [&](int kp, int h, const uint32_t* o16) {
+            tmem_st16(a_lane + (kp % kSt) * 64 + 16 * h, *(const uint32_t(*)[16]) o16);
+        };
+        int kp0 = 0, u0 = 0;                 // pairs and raw units of the tiles before this one
+        for (int t = 0;; ++t, kp0 += npairs, u0 += 4 * nkb) {
+        TileInfo ti;
+        bool ok = tile_of(t, ti);
+        if (named_bar_or(3, kDqWarps * 32, !ok) || ti.e < 0) break;      // the same for every expanding warp
+        const int nrows = ti.nrows, row0 = ti.row0, m0 = ti.m0;
+#ifdef MAYA_MMQ_STAMPS
+        long long* const stamps = tid == 0 && ok ? stamps_of(t) : nullptr;
+        if (stamps) { stamps[0] = stamps[1] = clock64(); stamps[14] = nrows; stamps[15] = npairs; }
+#endif
         for (int kb = 0; kb < nkb && ok; ++kb) {
-            const int u = kb * 4 + slab, slot = u % NU;
+            const int u = u0 + kb * 4 + slab, slot = u % NU;
             if (!wait_or_fail(P, &P.raw_full[slot], (u / NU) & 1)) { ok = false; break; }
             const uint8_t* rrow = rbase + (size_t) slot * kUnitBytes<T>;
             uint32_t o[32];
@@ -521,7 +506,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     release(kp);
                     return true;
                 };
-                ok = pair(std::integral_constant<int, 0>{}, kb * 4 + team) && pair(std::integral_constant<int, 1>{}, kb * 4 + team + 2);
+                ok = pair(std::integral_constant<int, 0>{}, kp0 + kb * 4 + team) && pair(std::integral_constant<int, 1>{}, kp0 + kb * 4 + team + 2);
             } else if constexpr (T == MAYA_Q4_K) {
                 Q4Scales S;
                 q4k_scales(*(const uint4*) rrow, S);
@@ -533,7 +518,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 for (int i = 0; i < 2; ++i) {        // the 64 values of quant pair p: low nibbles, then high nibbles
                     const int p = 2 * i + team;
                     const uint4 qa = *(const uint4*) (rrow + 16 + 32 * p), qb = *(const uint4*) (rrow + 32 + 32 * p);
-                    const int kp = kb * 4 + chunk + p, sb0 = 4 * i + 2 * team;
+                    const int kp = kp0 + kb * 4 + chunk + p, sb0 = 4 * i + 2 * team;
                     q4k_stage(qa, qb, 0, S.dl[sb0], S.nml[sb0], o);
                     if (!acquire(kp)) { ok = false; break; }
                     st_half(kp, 0, o);
@@ -547,18 +532,18 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                         const uint4 c = b <= (kb & 7) ? corr[b] : make_uint4(0u, 0u, 0u, 0u);
                         o[4 * b] = c.x; o[4 * b + 1] = c.y; o[4 * b + 2] = c.z; o[4 * b + 3] = c.w;
                     }
-                    ok = put(kb * 4 + chunk + 4, o);
+                    ok = put(kp0 + kb * 4 + chunk + 4, o);
                 }
             } else {
 #define MAYA_Q80_PAIR(PP)                                                                      \
     if (ok) {                                                                                  \
         q80_stage<2 * (PP)>(rrow, o);                                                          \
-        ok = acquire(kb * 4 + (PP));                                                           \
+        ok = acquire(kp0 + kb * 4 + (PP));                                                           \
         if (ok) {                                                                              \
-            st_half(kb * 4 + (PP), 0, o);                                                      \
+            st_half(kp0 + kb * 4 + (PP), 0, o);                                                      \
             q80_stage<2 * (PP) + 1>(rrow, o + 16);                                             \
-            st_half(kb * 4 + (PP), 1, o + 16);                                                 \
-            release(kb * 4 + (PP));                                                            \
+            st_half(kp0 + kb * 4 + (PP), 1, o + 16);                                                 \
+            release(kp0 + kb * 4 + (PP));                                                            \
         }                                                                                      \
     }
                 if (team == 0) { MAYA_Q80_PAIR(0) MAYA_Q80_PAIR(2) }
@@ -569,29 +554,37 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             __syncwarp();
             if (lane == 0) mbar_arrive(&P.raw_empty[slot]);      // 4 warps read a unit; after the 4th it may be overwritten
         }
-        // ------------------------------------------------------------ epilogue
-        if (ok && !wait_or_fail(P, &P.final, 0)) ok = false;
+        // ------------------------------------------------------------ write-back
+        if (ok && !wait_or_fail(P, &P.final, t & 1)) ok = false;
         tc_fence_after();
-        named_bar_sync(3, kDqWarps * 32);            // every expansion warp gets here (all waits are bounded) ...
-        ok = !failed(P);                             // ... and they agree: the epilogue's barriers need all of them
-        if (tid == 0) MAYA_STAMP(4);                 // accumulators complete, expanding warps met
-        if (ok) {
-            // The tile leaves through shared memory (both rings are free now: every load was consumed): the warps drop
-            // their lanes' values into [activation row][weight row] order, then one bulk copy per activation row
-            // writes it out.
+        // every expansion warp gets here (all waits are bounded) and they agree: what follows has barriers that need them all
+        if (named_bar_or(3, kDqWarps * 32, !ok)) break;
+#ifdef MAYA_MMQ_STAMPS
+        if (stamps) stamps[4] = clock64();               // accumulators complete, expanding warps met
+#endif
+        {
+            // The tile leaves through shared memory (the activation ring, and the raw ring behind it where the group is large:
+            // the loaders know, and wait for stg_free before they write there): the warps drop their lanes' values into
+            // [activation row][weight row] order, then one bulk copy per activation row writes it out.
             const int q = warp & 3, hs = warp >> 2;                      // hs = 0..3
             const uint32_t lane_base = tmem + ((uint32_t) (32 * q) << 16);
             uint8_t* const stg = smem;
             constexpr int kThreadsEpi = kDqWarps * 32;
+            auto accumulators_read = [&] {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&P.acc_free);
+            };
             if constexpr (GLU) {
                 // Two passes.  First the tile goes from tensor memory to shared memory as h = SwiGLU(gate, up) in f32,
                 // [activation row][128]: 16 warps = 4 lane quadrants x 4 groups, a group takes every 4th chunk of 8
                 // activation rows.  Then, for the f16 image, every thread rounds 8 consecutive values of a row at a time
                 // (4 threads a 32-value group, as maya_mmq_quantize does: the same function, the same bytes) - the
                 // groups' amax and sums cost two shuffles each instead of a warp-wide reduction per value.
+                const int r8 = rows_up8(nrows);
                 __half* b16 = (__half*) stg;                             // [rows][128] f16 image of h
-                float* b32 = (float*) (stg + TN * 128 * 2);              // [rows][128] h
-                __half* bxa = (__half*) (stg + TN * 128 * 6);            // [rows][4] sum corrections of the row's four 32-value groups
+                float* b32 = (float*) (stg + r8 * 128 * 2);              // [rows][128] h
+                __half* bxa = (__half*) (stg + r8 * 128 * 6);            // [rows][4] sum corrections of the row's four 32-value groups
                 const int nchunk = (nrows + 7) >> 3;
                 const int mcol = 32 * q + lane;
                 for (int c = hs; c < nchunk; c += 4) {
@@ -603,7 +596,10 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     for (int j = 0; j < 8; ++j)
                         if (col0 + j < nrows) b32[(col0 + j) * 128 + mcol] = swiglu(v[j], up[j], A.limit);   // uniform in the warp
                 }
-                if (tid == 0) MAYA_STAMP(5);             // SwiGLU tile in shared memory
+                accumulators_read();
+#ifdef MAYA_MMQ_STAMPS
+                if (stamps) stamps[5] = clock64();       // SwiGLU tile in shared memory
+#endif
                 if (A.xq_out) {
                     named_bar_sync(2, kThreadsEpi);
                     const int ch = tid & 15;                             // the row's 8-value chunk; a warp covers two rows
@@ -621,7 +617,9 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                         }
                     }
                 }
-                if (tid == 0) MAYA_STAMP(6);             // tile rounded
+#ifdef MAYA_MMQ_STAMPS
+                if (stamps) stamps[6] = clock64();       // tile rounded
+#endif
                 fence_proxy_async();
                 named_bar_sync(1, kThreadsEpi);
                 if (tid < nrows) {                                       // one activation row each
@@ -630,7 +628,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                         const int64_t ldq = xq_ld(A.w_rows);
                         bulk_store(A.xq_out + row_g * ldq + m0, b16 + tid * 128, 128 * 2);
                         *(uint2*) (A.xq_out + row_g * ldq + A.w_rows + (m0 >> 5)) = *(const uint2*) (bxa + tid * 4);
-                        if (blockIdx.x == 0)                             // the zero padding behind the row's corrections
+                        if (m0 == 0)                                     // the zero padding behind the row's corrections
                             for (int64_t c = A.w_rows + A.w_rows / 32; c < ldq; ++c) A.xq_out[row_g * ldq + c] = __float2half_rn(0.0f);
                     }
                     if (A.dst) bulk_store(A.dst + (int64_t) (A.ids ? A.ids[row_g] : row_g) * A.ld_dst + m0, b32 + tid * 128, 128 * 4);
@@ -654,6 +652,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                             if (col0 + j < nrows) buf[(col0 + j) * TM + mcol] = v[j];
                     }
                 }
+                accumulators_read();
                 fence_proxy_async();
                 named_bar_sync(1, kThreadsEpi);
                 if (tid < nrows) {
@@ -662,28 +661,92 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     bulk_commit();
                 }
             }
-            if (tid < nrows) bulk_wait_read<0>();                        // the copies have read shared memory: the block may end
+            if (tid < nrows) bulk_wait_read<0>();                        // the copies have read shared memory ...
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&P.stg_free[t & 1]);              // ... which the next tile's loads may overwrite
+        }
+#ifdef MAYA_MMQ_STAMPS
+        if (stamps) stamps[7] = clock64();               // written back
+#endif
         }
     } else if (warp == kDqWarps) {
-        // ------------------------------------------------------------ raw weight units (one lane)
-        if (lane == 0) {
-            int issued = 0;
+        // ------------------------------------------------------------ the tile list, and raw weight units (one lane)
+        int u0 = 0, prev_rows = 0;           // raw units of the tiles before this one; rows of the tile before this one
+        for (int t = 0;; ++t, u0 += 4 * nkb) {
+            // Which (matrix, 160-row group) is this tile's: the warp scans the per-matrix group counts - each lane the counts
+            // of a run of consecutive matrices, an exclusive warp scan of the runs' sums, then the lane whose run holds the
+            // wanted group walks it - 1024 matrices a round.
+            const int lin = (int) blockIdx.x + t * (int) gridDim.x, want_all = lin / nslab;
+            int found_e = -1, row0 = 0, nrows = 0, base = 0;
+            for (int e0 = 0; e0 < A.n; e0 += 1024) {
+                const int per = (min(A.n - e0, 1024) + 31) >> 5;          // matrices a lane (<= 32)
+                const int lo = e0 + lane * per, hi = min(lo + per, min(A.n, e0 + 1024));
+                int mine = 0;
+                for (int e = lo; e < hi; ++e) {
+                    const int be = A.expert_map ? A.expert_map[e] : e;
+                    mine += (A.bounds[be + 1] - A.bounds[be] + TN - 1) / TN;
+                }
+                int incl = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+                const int want = want_all - base;
+                const bool mine_is_it = want >= incl - mine && want < incl;
+                if (mine_is_it) {
+                    int g = want - (incl - mine);
+                    for (int e = lo; e < hi; ++e) {
+                        const int be = A.expert_map ? A.expert_map[e] : e;
+                        const int b0 = A.bounds[be], b1 = A.bounds[be + 1], cnt = (b1 - b0 + TN - 1) / TN;
+                        if (g < cnt) { found_e = e; row0 = b0 + g * TN; nrows = min(TN, b1 - row0); break; }
+                        g -= cnt;
+                    }
+                }
+                const unsigned holds = __ballot_sync(0xFFFFFFFFu, mine_is_it);
+                if (holds != 0u) {
+                    const int src = __ffs(holds) - 1;
+                    found_e = __shfl_sync(0xFFFFFFFFu, found_e, src);
+                    row0 = __shfl_sync(0xFFFFFFFFu, row0, src);
+                    nrows = __shfl_sync(0xFFFFFFFFu, nrows, src);
+                    break;
+                }
+                base += total;
+            }
+            const int m0 = (lin % nslab) * kSlab;
             bool ok = true;
-            for (int kb = 0; kb < nkb && ok; ++kb) {
-                for (int sl = 0; sl < 4; ++sl) {
-                    const int u = kb * 4 + sl, slot = u % NU;
-                    if (u >= NU && !wait_or_fail(P, &P.raw_empty[slot], ((u / NU) - 1) & 1)) { ok = false; break; }
-                    const int wrow = GLU ? (sl < 2 ? m0 + 64 * sl : A.w_rows + m0 + 64 * (sl - 2)) : m0 + 64 * sl;
-                    mbar_expect_tx(&P.raw_full[slot], kUnitBytes<T>);
-                    // x: the block's 32-bit words (k-quants), or the 16-byte aligned byte offset of the window around the
-                    // i-quant block (the box is then 112 / 144 bytes of each row; past the row's end it reads as zeros)
-                    const int x0 = kIq<T> ? (int) (((size_t) kb * kBlkBytes<T>) & ~(size_t) 15) : kb * (kRawRow<T> / 4);
-                    tma_load_3d(raw + (size_t) slot * kUnitBytes<T>, &tm_w, &P.raw_full[slot], x0, wrow, found_e);
-                    issued = u + 1;
+            if (lane == 0) {
+                // Entry t % kTiles was read by every role before tile t - kTiles ended.  The write-back of the tile two before
+                // this one has to be over in any case (so that a barrier's phase is never two behind), that of the tile before
+                // only where it stretches into the raw ring.
+                if (t >= 2) ok = wait_or_fail(P, &P.stg_free[t & 1], ((t - 2) >> 1) & 1);
+                P.tile[t % kTiles] = TileInfo{found_e, row0, nrows, m0};
+                mbar_arrive(&P.tile_full[t % kTiles]);
+                if (found_e >= 0) {
+                    if (ok && t >= 1 && staging_bytes<GLU>(prev_rows) > kBRing<T>)
+                        ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
+                    int issued = u0;
+                    for (int kb = 0; kb < nkb && ok; ++kb) {
+                        for (int sl = 0; sl < 4; ++sl) {
+                            const int u = u0 + kb * 4 + sl, slot = u % NU;
+                            if (u >= NU && !wait_or_fail(P, &P.raw_empty[slot], ((u / NU) - 1) & 1)) { ok = false; break; }
+                            const int wrow = GLU ? (sl < 2 ? m0 + 64 * sl : A.w_rows + m0 + 64 * (sl - 2)) : m0 + 64 * sl;
+                            mbar_expect_tx(&P.raw_full[slot], kUnitBytes<T>);
+                            // x: the block's 32-bit words (k-quants), or the 16-byte aligned byte offset of the window around the
+                            // i-quant block (the box is then 112 / 144 bytes of each row; past the row's end it reads as zeros)
+                            const int x0 = kIq<T> ? (int) (((size_t) kb * kBlkBytes<T>) & ~(size_t) 15) : kb * (kRawRow<T> / 4);
+                            tma_load_3d(raw + (size_t) slot * kUnitBytes<T>, &tm_w, &P.raw_full[slot], x0, wrow, found_e);
+                            issued = u + 1;
+                        }
+                    }
+                    if (!ok)                                     // let the copies in flight land before the block ends
+                        for (int u = max(0, issued - NU); u < issued; ++u) wait_or_fail(P, &P.raw_full[u % NU], (u / NU) & 1);
                 }
             }
-            if (!ok)                                             // let the copies in flight land before the block ends
-                for (int u = max(0, issued - NU); u < issued; ++u) wait_or_fail(P, &P.raw_full[u % NU], (u / NU) & 1);
+            ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
+            if (!ok || found_e < 0) break;
+            prev_rows = nrows;
         }
     } else if (warp == kDqWarps + 1 || warp == kDqWarps + 3) {
         // ------------------------------------------------------------ tensor-core issue (two warps, one accumulator each, on
@@ -694,69 +757,92 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         // single lane inside a divergent branch every operand of every product crossed from a vector register - 31 such
         // moves and 430-550 cycles a pair of K steps, the longest stage of the whole pipeline.)
         const int my = warp == kDqWarps + 1 ? 0 : 1;
-        const int n_rows = __shfl_sync(0xFFFFFFFFu, nrows, 0);
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
-        const int n_mma = max(16, (n_rows + 15) & ~15);
-        const uint32_t idesc = (1u << 4) | ((uint32_t) (n_mma >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
         const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem));
         const uint32_t b_hi = (uint32_t) (bdesc0 >> 32), b_lo0 = (uint32_t) bdesc0, b_lo_end = b_lo0 + NB * (kBStage >> 4);
         const uint32_t a0 = tm + kACol + my * 32, a_end = a0 + kSt * 64, d0 = tm + my * kAccCols;
         const uint32_t bfull0 = smem_u32(&P.b_full[0]), afull0 = smem_u32(&P.a_full[0]), done0 = smem_u32(&P.done[0]);
         uint32_t b_lo = b_lo0, at = a0, bfull = bfull0, afull = afull0;   // of the next pair of K steps
-        uint32_t ph_a = 0, ph_b = 0, first = 0;      // the barriers' phases; first = 0: the first product overwrites
-        const int npairs = nkt / 2 + ntp;
-        bool ok = true;
-        for (int kp = 0; kp < npairs; ++kp) {
-            const uint32_t done_bar = done0 + ((kp & (kDone - 1)) << 3);
-            const bool rb = mbar_test_wait_addr(bfull, ph_b), ra = mbar_test_wait_addr(afull, ph_a);
-            if (!__all_sync(0xFFFFFFFFu, rb && ra)) {            // not there yet: the bounded waits
-                const bool got = wait_or_fail(P, &P.b_full[(bfull - bfull0) >> 3], ph_b) && wait_or_fail(P, &P.a_full[(afull - afull0) >> 3], ph_a);
-                if (!__all_sync(0xFFFFFFFFu, got)) { ok = false; break; }
+        uint32_t ph_a = 0, ph_b = 0, done_at = 0;    // the barriers' phases; the next pair's place in the ring of done barriers
+        for (int t = 0;; ++t) {
+            TileInfo ti;
+            bool ok = tile_of(t, ti);
+            if (!__all_sync(0xFFFFFFFFu, ok)) break;
+            const int n_rows = __shfl_sync(0xFFFFFFFFu, ti.nrows, 0);
+            if (__shfl_sync(0xFFFFFFFFu, ti.e, 0) < 0) break;
+            if (t > 0) {                             // the accumulators still hold the tile before until its write-back has read them
+                ok = wait_or_fail(P, &P.acc_free, (t - 1) & 1);
+                if (!__all_sync(0xFFFFFFFFu, ok)) break;
+                tc_fence_after();
             }
-            tc_fence_after();
-            if (my == 0 && kp == 0 && lane == 0) MAYA_STAMP(2);  // the first product
-            mma_f16_ts_x4_commit(d0, at, b_lo, b_hi, idesc, first, done_bar);
-            first = 1;
-            at += 64; afull += 8;
-            if (at == a_end) { at = a0; afull = afull0; ph_a ^= 1; }
-            b_lo += kBStage >> 4; bfull += 8;
-            if (b_lo == b_lo_end) { b_lo = b_lo0; bfull = bfull0; ph_b ^= 1; }
+            const int n_mma = max(16, (n_rows + 15) & ~15);
+            const uint32_t idesc = (1u << 4) | ((uint32_t) (n_mma >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+            uint32_t first = 0;                      // 0: the first product overwrites
+            for (int kp = 0; kp < npairs; ++kp) {
+                const bool rb = mbar_test_wait_addr(bfull, ph_b), ra = mbar_test_wait_addr(afull, ph_a);
+                if (!__all_sync(0xFFFFFFFFu, rb && ra)) {        // not there yet: the bounded waits
+                    const bool got = wait_or_fail(P, &P.b_full[(bfull - bfull0) >> 3], ph_b) && wait_or_fail(P, &P.a_full[(afull - afull0) >> 3], ph_a);
+                    if (!__all_sync(0xFFFFFFFFu, got)) { ok = false; break; }
+                }
+                tc_fence_after();
+#ifdef MAYA_MMQ_STAMPS
+                if (my == 0 && kp == 0 && lane == 0 && stamps_of(t)) stamps_of(t)[2] = clock64();       // the first product
+#endif
+                mma_f16_ts_x4_commit(d0, at, b_lo, b_hi, idesc, first, done0 + done_at);
+                first = 1;
+                done_at = (done_at + 8) & (8 * kDone - 1);
+                at += 64; afull += 8;
+                if (at == a_end) { at = a0; afull = afull0; ph_a ^= 1; }
+                b_lo += kBStage >> 4; bfull += 8;
+                if (b_lo == b_lo_end) { b_lo = b_lo0; bfull = bfull0; ph_b ^= 1; }
+            }
+#ifdef MAYA_MMQ_STAMPS
+            if (my == 0 && lane == 0 && stamps_of(t)) stamps_of(t)[3] = clock64();                      // the last product issued
+#endif
+            if (!ok) break;
+            mma_commit_elect(smem_u32(&P.final));
         }
-        if (my == 0 && lane == 0) MAYA_STAMP(3);                 // the last product issued
-        if (ok) mma_commit_elect(smem_u32(&P.final));
     } else if (warp == kDqWarps + 2) {
         // ------------------------------------------------------------ activation tiles (one lane)
         if (lane == 0) {
-            int issued = 0;
-            bool ok = true;
-            const uint32_t tx_bytes = big ? kBStage : kBBox;
             const int nmain = nkt / 2;
-            for (int kb2 = 0; kb2 < nmain + ntp; ++kb2) {
-                const int sb = kb2 % NB;
-                // the pair's 64 K-values in the image: K values in order, and after every 32 pairs (or at the end) the
-                // chunk's 64 corrections from the tail behind the row's K values
-                int xcol;
-                if (ntp == 0) xcol = kb2 * 64;
-                else {
-                    const int c = kb2 / 33, r = kb2 - c * 33;
-                    const bool is_corr = r == 32 || kb2 == nmain + ntp - 1;
-                    xcol = is_corr ? A.w_cols + 64 * c : (kb2 - c) * 64;
+            int p0 = 0, issued = 0;                  // pairs of the tiles before this one; tiles of activations asked for
+            bool ok = true;
+            for (int t = 0;; ++t, p0 += npairs) {
+                TileInfo ti;
+                ok = tile_of(t, ti);
+                if (!ok || ti.e < 0) break;
+                // the write-back of the tile before uses the activation ring
+                if (t > 0) ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
+                const bool big = ti.nrows > 128;     // the activation tile is a 128-row box and a 32-row box
+                const uint32_t tx_bytes = big ? kBStage : kBBox;
+                for (int kb2 = 0; kb2 < npairs && ok; ++kb2) {
+                    const int pg = p0 + kb2, sb = pg % NB;
+                    // the pair's 64 K-values in the image: K values in order, and after every 32 pairs (or at the end) the
+                    // chunk's 64 corrections from the tail behind the row's K values
+                    int xcol;
+                    if (ntp == 0) xcol = kb2 * 64;
+                    else {
+                        const int c = kb2 / 33, r = kb2 - c * 33;
+                        const bool is_corr = r == 32 || kb2 == nmain + ntp - 1;
+                        xcol = is_corr ? A.w_cols + 64 * c : (kb2 - c) * 64;
+                    }
+                    if (pg >= NB) {                          // the slot was last read by pair pg - NB
+                        const int pp = pg - NB;
+                        if (!wait_or_fail(P, &P.done[pp % kDone], (pp / kDone) & 1)) { ok = false; break; }
+                    }
+                    uint8_t* bt = smem + (size_t) sb * kBStage;
+                    mbar_expect_tx(&P.b_full[sb], tx_bytes);
+                    tma_load_2d(bt, &tm_x, &P.b_full[sb], xcol, ti.row0);
+                    if (big) tma_load_2d(bt + kBBox, &tm_x32, &P.b_full[sb], xcol, ti.row0 + 128);
+                    issued = pg + 1;
                 }
-                if (kb2 >= NB) {                             // the slot was last read by pair kb2 - NB
-                    const int pp = kb2 - NB;
-                    if (!wait_or_fail(P, &P.done[pp % kDone], (pp / kDone) & 1)) { ok = false; break; }
-                }
-                uint8_t* bt = smem + (size_t) sb * kBStage;
-                mbar_expect_tx(&P.b_full[sb], tx_bytes);
-                tma_load_2d(bt, &tm_x, &P.b_full[sb], xcol, row0);
-                if (big) tma_load_2d(bt + kBBox, &tm_x32, &P.b_full[sb], xcol, row0 + 128);
-                issued = kb2 + 1;
+                if (!ok) break;
             }
-            if (!ok)
-                for (int kb2 = max(0, issued - NB); kb2 < issued; ++kb2) wait_or_fail(P, &P.b_full[kb2 % NB], (kb2 / NB) & 1);
+            if (!ok)                                         // let the copies in flight land before the block ends
+                for (int pg = max(0, issued - NB); pg < issued; ++pg) wait_or_fail(P, &P.b_full[pg % NB], (pg / NB) & 1);
         }
     }
-    if (tid == 0) MAYA_STAMP(7);                    // written back
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
@@ -883,9 +969,10 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
         return note_launch("mmq smem attribute");
     const int64_t groups = p->total_rows / TN + p->n;   // an upper bound of sum(ceil(rows_e / 160)), known without the counts
     if (groups > 65535) return refuse(MAYA_ERR_LIMIT);
-    const int slab = GLU ? 128 : TM;
-    const dim3 grid((unsigned) ((A.w_rows + slab - 1) / slab), (unsigned) groups);
-    mmq_kernel<T, GLU><<<grid, kMmqThreads, smem, s>>>(tw, tx, tx32, A);
+    const int slab = GLU ? 128 : TM, sms = sm_count();
+    if (sms <= 0) return refuse(MAYA_ERR_DEVICE);
+    const int64_t most = (int64_t) ((A.w_rows + slab - 1) / slab) * groups;      // tiles there can be
+    mmq_kernel<T, GLU><<<(unsigned) (most < sms ? most : sms), kMmqThreads, smem, s>>>(tw, tx, tx32, A);
     return note_launch("mmq");
 }
 

@@ -178,19 +178,6 @@ template<int T> size_t stream_smem(int n_ff) {
     return 2 * stage + (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_ff / 32, kWNC);
 }
 
-int sm_count() {
-    static std::atomic<int> cached_dev{-1}, cached_n{0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cached_dev.load() != dev) {
-        int n = 0;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        cached_n.store(n);
-        cached_dev.store(dev);
-    }
-    return cached_n.load();
-}
-
 template<int T>
 int launch_stream(const WGroups& G, int n_embd, int n_ff, size_t down_off, const void* hq, float* part, cudaStream_t s) {
     const size_t smem = stream_smem<T>(n_ff);
