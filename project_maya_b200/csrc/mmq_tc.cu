@@ -65,15 +65,16 @@ template<int T> constexpr int kBlkBytes = T == MAYA_IQ2_S ? 82 : T == MAYA_IQ3_S
 template<int T> constexpr int kWin = T == MAYA_IQ2_S ? 96 : 128;
 template<int T> constexpr int kRawRow = T == MAYA_Q4_K ? 144 : T == MAYA_Q8_0 ? 272 : T == MAYA_IQ2_S ? 112 : 144;
 template<int T> constexpr int kUnitBytes = kUnitRows * kRawRow<T>;
-template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 10 : T == MAYA_Q8_0 ? 8 : T == MAYA_IQ2_S ? 14 : 12;   // raw units in flight
+template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 10 : T == MAYA_Q8_0 ? 8 : T == MAYA_IQ2_S ? 11 : 9;   // raw units in flight
 template<int T> constexpr int kBStages = T == MAYA_Q4_K ? 6 : 4;            // activation tiles (64 K-values) in flight
 template<int T> constexpr int kBRing = kBStages<T> * kBStage;
-// i-quants: the codebook's bytes (IQ2_S 1024 x 8, IQ3_S 512 x 4), kept in kCopies copies that lie side by side in every
-// entry - lane l reads copy l % kCopies - so that a warp's 32 random entries spread over the banks: four 8-byte copies cost
-// about 5 wavefronts a lookup, sixteen 4-byte copies 2 (one copy: 6 and 3.5).  The first form of this expansion looked
-// f16 entries and f16 sign masks up 16 bytes at a time, 11 wavefronts each: 1400 of the 2000 cycles a pair of K steps took.
+// i-quants: the codebook as f16 (IQ2_S 1024 entries of 8 values, IQ3_S 512 of 4), kept in kCopies copies that lie side by
+// side in every entry - lane l reads copy l % kCopies - so that a warp's 32 random entries spread over the banks: sixteen
+// 8-byte copies are free of conflicts, four 16-byte copies cost about 8 wavefronts a look-up where one costs 11.  (The
+// codebook as bytes takes a quarter of the wavefronts' width but one byte permute more for every two weights; the expansion
+// is bound by those instructions: 64 tokens of IQ3_S 553 -> 475 us, 777 of IQ2_S 1436 -> 1316.)
 template<int T> constexpr int kCopies = T == MAYA_IQ2_S ? 4 : T == MAYA_IQ3_S ? 16 : 0;
-template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 8 * kCopies<T> : T == MAYA_IQ3_S ? 512 * 4 * kCopies<T> : 0;
+template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 16 * kCopies<T> : T == MAYA_IQ3_S ? 512 * 8 * kCopies<T> : 0;
 template<int T> constexpr int kTabOff = kBRing<T> + kUnits<T> * kUnitBytes<T>;
 template<int T> constexpr size_t kSmemBytes = (size_t) kTabOff<T> + kTabBytes<T>;
 static_assert(kUnits<MAYA_Q4_K> <= kMaxUnits && kUnits<MAYA_Q8_0> <= kMaxUnits && kUnits<MAYA_IQ2_S> <= kMaxUnits &&
@@ -256,58 +257,50 @@ template<int T, int OFF, int TEAM> __device__ __forceinline__ void iq_fields(con
         F.sc = __byte_perm(win_u32<OFF + 106>(w), 0, TEAM == 0 ? 0x4420 : 0x4431);
     }
 }
-// Two codebook bytes -> two weights: `x` = (1024 + v) pairs, ndl = -1024 dl, so the fma is dl * v rounded once; then the
-// signs of values 2 P and 2 P + 1 from sign byte s: s * (2^(15 - 2P) + 2^(30 - 2P)) has them at bits 15 and 31 (the two
-// shifted copies of the 8 bits do not meet), and one three-input operation masks them out and flips the signs.
-template<int P> __device__ __forceinline__ uint32_t iq_two(__half2 x, uint32_t s, __half2 dl, __half2 ndl) {
-    const uint32_t v = h2_bits(__hfma2(x, dl, ndl));
-    return v ^ ((s * ((1u << (15 - 2 * P)) + (1u << (30 - 2 * P)))) & 0x80008000u);
-}
-__device__ __forceinline__ __half2 neg1024(__half2 dl) { return __hmul2(dl, __float2half2_rn(-1024.0f)); }
-// eight values of one sign byte: bytes ga (values 0..3) and gb (4..7)
-__device__ __forceinline__ void iq_eight(uint32_t ga, uint32_t gb, uint32_t s, __half2 dl, __half2 ndl, uint32_t* r) {
-    r[0] = iq_two<0>(bytes01_plus1024(ga), s, dl, ndl);
-    r[1] = iq_two<1>(bytes23_plus1024(ga), s, dl, ndl);
-    r[2] = iq_two<2>(bytes01_plus1024(gb), s, dl, ndl);
-    r[3] = iq_two<3>(bytes23_plus1024(gb), s, dl, ndl);
-}
-// Sub-block J of the fields -> 32 weights.  `tab`: this lane's copy of the codebook.
-// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; here dl = f16(d (2 ls + 1) / 8) and
-// w = dl * grid (one more f16 rounding).
-template<int J> __device__ __forceinline__ void iq_half(const IqFields<MAYA_IQ2_S>& F, float d, const uint2* tab, uint32_t* o) {
-    constexpr int C = kCopies<MAYA_IQ2_S>;
-    const uint32_t qh = byte_of(F.qh, J), sc = byte_of(F.sc, J), sg4 = F.sg[J];
+// Sub-block J's codebook values, unsigned f16 pairs -> o[16].  `tab`: this lane's copy of the codebook.
+template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ2_S>& F, const uint4* tab, uint32_t* o) {
+    const uint32_t qh = byte_of(F.qh, J);
     // byte l of hw = bits 2l, 2l + 1 of qh: an entry's index is one byte permute {qs byte l, hw byte l, 0, 0}
     const uint32_t hw = ((qh & 0x33u) * 0x1001u + (qh & 0xCCu) * 0x40040u) & 0x03030303u;
-    const __half2 dl0 = __float2half2_rn(d * (float) (2 * (sc & 15) + 1) * 0.125f), dl1 = __float2half2_rn(d * (float) (2 * (sc >> 4) + 1) * 0.125f);
-    const __half2 nd0 = neg1024(dl0), nd1 = neg1024(dl1);
-    const uint2 g0 = tab[prmt_raw(F.q[J], hw, 0xCC40u) * C], g1 = tab[prmt_raw(F.q[J], hw, 0xCC51u) * C];
-    const uint2 g2 = tab[prmt_raw(F.q[J], hw, 0xCC62u) * C], g3 = tab[prmt_raw(F.q[J], hw, 0xCC73u) * C];
-    iq_eight(g0.x, g0.y, byte_of(sg4, 0), dl0, nd0, o);
-    iq_eight(g1.x, g1.y, byte_of(sg4, 1), dl0, nd0, o + 4);
-    iq_eight(g2.x, g2.y, byte_of(sg4, 2), dl1, nd1, o + 8);
-    iq_eight(g3.x, g3.y, byte_of(sg4, 3), dl1, nd1, o + 12);
-}
-// IQ3_S (ggml dequantize_row_iq3_s): y = d (1 + 2 scale) * grid[qs | qh bit] * sign; 4 values per entry.
-template<int J> __device__ __forceinline__ void iq_half(const IqFields<MAYA_IQ3_S>& F, float d, const uint32_t* tab, uint32_t* o) {
-    const uint32_t qh = byte_of(F.qh, J), sg4 = F.sg[J], nib = (F.sc >> (8 * (J / 2) + 4 * (J % 2))) & 15u;
-    // byte l of h0 / h1 = bit l / 4 + l of qh, the ninth index bit of entry l / 4 + l
-    const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
-    const __half2 db = __float2half2_rn(d * (float) (1 + 2 * nib)), nd = neg1024(db);
-    uint32_t g[8];
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-        g[l] = tab[prmt_raw(F.q[2 * J], h0, 0xCC00u + ((4 + l) << 4) + l) * kCopies<MAYA_IQ3_S>];
-        g[4 + l] = tab[prmt_raw(F.q[2 * J + 1], h1, 0xCC00u + ((4 + l) << 4) + l) * kCopies<MAYA_IQ3_S>];
+        const uint4 g = tab[prmt_raw(F.q[J], hw, 0xCC00u + ((4 + l) << 4) + l) * kCopies<MAYA_IQ2_S>];
+        o[4 * l] = g.x; o[4 * l + 1] = g.y; o[4 * l + 2] = g.z; o[4 * l + 3] = g.w;
     }
-    iq_eight(g[0], g[1], byte_of(sg4, 0), db, nd, o);
-    iq_eight(g[2], g[3], byte_of(sg4, 1), db, nd, o + 4);
-    iq_eight(g[4], g[5], byte_of(sg4, 2), db, nd, o + 8);
-    iq_eight(g[6], g[7], byte_of(sg4, 3), db, nd, o + 12);
 }
-// The super-scale at which -1024 dl would leave f16's range (d x 31 / 8 or d x 31 at or above 63): such a block is expanded
-// at a 64th of it and its weights are multiplied by 64 afterwards, both exact.
-template<int T> constexpr float kIqBigScale = T == MAYA_IQ2_S ? 16.0f : 2.0f;
+template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ3_S>& F, const uint2* tab, uint32_t* o) {
+    const uint32_t qh = byte_of(F.qh, J);
+    // byte l of h0 / h1 = bit l / 4 + l of qh, the ninth index bit of entry l / 4 + l
+    const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
+#pragma unroll
+    for (int l = 0; l < 8; ++l) {
+        const uint2 g = tab[prmt_raw(F.q[2 * J + l / 4], l < 4 ? h0 : h1, 0xCC00u + ((4 + l % 4) << 4) + l % 4) * kCopies<MAYA_IQ3_S>];
+        o[2 * l] = g.x; o[2 * l + 1] = g.y;
+    }
+}
+// Eight values in place: times dl (one f16 rounding), then the signs.  Pair p's signs from sign byte s: s * (2^(15 - 2p) +
+// 2^(30 - 2p)) has them at bits 15 and 31 (the two shifted copies of the 8 bits do not meet), and one three-input operation
+// masks them out and flips the signs.
+__device__ __forceinline__ void iq_eight(uint32_t s, __half2 dl, uint32_t* r) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+        r[p] = h2_bits(__hmul2(bits_h2(r[p]), dl)) ^ ((s * ((1u << (15 - 2 * p)) + (1u << (30 - 2 * p)))) & 0x80008000u);
+}
+// Sub-block J's values -> weights, in place.
+// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; dl = f16(d (2 ls + 1) / 8).
+template<int J> __device__ __forceinline__ void iq_finish(const IqFields<MAYA_IQ2_S>& F, uint32_t* o) {
+    const uint32_t sc = byte_of(F.sc, J);
+    const __half2 dl0 = __float2half2_rn(F.d * (float) (2 * (sc & 15) + 1) * 0.125f), dl1 = __float2half2_rn(F.d * (float) (2 * (sc >> 4) + 1) * 0.125f);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J], l), l < 2 ? dl0 : dl1, o + 4 * l);
+}
+// IQ3_S (ggml dequantize_row_iq3_s): y = d (1 + 2 scale) * grid[qs | qh bit] * sign.
+template<int J> __device__ __forceinline__ void iq_finish(const IqFields<MAYA_IQ3_S>& F, uint32_t* o) {
+    const uint32_t nib = (F.sc >> (8 * (J / 2) + 4 * (J % 2))) & 15u;
+    const __half2 db = __float2half2_rn(F.d * (float) (1 + 2 * nib));
+#pragma unroll
+    for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J], l), db, o + 4 * l);
+}
 
 // A block works on tile after tile (see mmq_kernel): what the roles share of one of them.  e < 0: no tile left.
 struct TileInfo { int e, row0, nrows, m0; };
@@ -410,14 +403,17 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         // Two teams of 8 warps; in each, thread = one of the slab's 256 rows.  Team t expands the K steps kt with
         // kt % 2 == t, so that a step's latency (shared-memory reads, the packed-half chain, the tensor-memory store
         // and its wait) overlaps the other team's step.
-        if constexpr (T == MAYA_IQ2_S) {            // the codebook's copies, once per block, under the first loads' latency
-            uint2* grid = (uint2*) (smem + kTabOff<T>);
-            for (int i = tid; i < 1024 * kCopies<T>; i += kDqWarps * 32) grid[i] = ((const uint2*) g_iq2s_grid)[i / kCopies<T>];
-            named_bar_sync(2, kDqWarps * 32);
-        }
-        if constexpr (T == MAYA_IQ3_S) {
-            uint32_t* grid = (uint32_t*) (smem + kTabOff<T>);
-            for (int i = tid; i < 512 * kCopies<T>; i += kDqWarps * 32) grid[i] = g_iq3s_grid[i / kCopies<T>];
+        if constexpr (kIq<T>) {                     // the codebook's copies, once per block, under the first loads' latency
+            const __half2 k1024 = __float2half2_rn(1024.0f);
+            auto wide = [&](uint32_t g) {           // four codebook bytes as f16
+                return make_uint2(h2_bits(__hsub2(bytes01_plus1024(g), k1024)), h2_bits(__hsub2(bytes23_plus1024(g), k1024)));
+            };
+            uint2* const grid = (uint2*) (smem + kTabOff<T>);
+            constexpr int W = T == MAYA_IQ2_S ? 2 : 1;                   // four-value words of an entry
+            for (int i = tid; i < kTabBytes<T> / 8; i += kDqWarps * 32) {
+                const int e = i / (W * kCopies<T>), h = i % W;
+                grid[i] = wide(T == MAYA_IQ2_S ? ((const uint32_t*) g_iq2s_grid)[2 * e + h] : g_iq3s_grid[e]);
+            }
             named_bar_sync(2, kDqWarps * 32);
         }
         const int team = warp >> 3, row = tid & 255, w8 = warp & 7;
@@ -447,7 +443,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             return true;
         };
         // i-quants: this lane's copy of the codebook
-        using Entry = std::conditional_t<T == MAYA_IQ2_S, uint2, uint32_t>;
+        using Entry = std::conditional_t<T == MAYA_IQ2_S, uint4, uint2>;
         [[maybe_unused]] const Entry* const tab = (const Entry*) (smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) : 0);
         [[maybe_unused]] uint4 corr[8];      // Q4_K: the constant terms of the current 8-block chunk (indexed by kb: local memory)
         // A pair's two halves of 32 K-values: the first half's tensor-memory store is under way while the second half is
@@ -486,22 +482,14 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     default: if (team == 0) iq_fields<T, 14, 0>(wv, F); else iq_fields<T, 14, 1>(wv, F); break;
                 }
 #undef MAYA_IQ_FIELDS
-                const bool big = fabsf(F.d) >= kIqBigScale<T>, any_big = __any_sync(0xFFFFFFFFu, big);
-                const float ds = big ? F.d * 0.015625f : F.d;
-                auto half_block = [&](auto j, uint32_t* v) {
-                    iq_half<decltype(j)::value>(F, ds, tab, v);
-                    if (any_big) {
-                        const __half2 up = __float2half2_rn(big ? 64.0f : 1.0f);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = h2_bits(__hmul2(bits_h2(v[i]), up));
-                    }
-                };
-                auto pair = [&](auto i, int kp) {        // a pair of sub-blocks leaves in two halves, as the other types'
+                auto pair = [&](auto i, int kp) {        // both sub-blocks' look-ups are under way before the first is finished
                     constexpr int J = 2 * decltype(i)::value;
-                    half_block(std::integral_constant<int, J>{}, o);
+                    iq_lookup<J>(F, tab, o);
+                    iq_lookup<J + 1>(F, tab, o + 16);
+                    iq_finish<J>(F, o);
                     if (!acquire(kp)) return false;
                     st_half(kp, 0, o);
-                    half_block(std::integral_constant<int, J + 1>{}, o + 16);
+                    iq_finish<J + 1>(F, o + 16);
                     st_half(kp, 1, o + 16);
                     release(kp);
                     return true;
