@@ -466,11 +466,14 @@ template<> struct Dec<MAYA_IQ1_S> {
 #undef MAYA_IQ3XXS_GRID
 #undef MAYA_GRID_QUAL
 
+template<int T> __device__ __forceinline__ const uint32_t* tab_source() {
+    return T == MAYA_IQ2_S ? (const uint32_t*) g_iq2s_grid : T == MAYA_IQ3_S ? (const uint32_t*) g_iq3s_grid
+           : T == MAYA_IQ2_XXS ? (const uint32_t*) g_iq2xxs_grid : T == MAYA_IQ1_S ? (const uint32_t*) g_iq1s_grid
+           : (const uint32_t*) g_iq3xxs_grid;
+}
 template<int T> __device__ __forceinline__ void load_tab(uint32_t* s_tab) {
     if constexpr (Fmt<T>::tab_words > 0) {
-        const uint32_t* src = T == MAYA_IQ2_S ? (const uint32_t*) g_iq2s_grid : T == MAYA_IQ3_S ? (const uint32_t*) g_iq3s_grid
-                              : T == MAYA_IQ2_XXS ? (const uint32_t*) g_iq2xxs_grid : T == MAYA_IQ1_S ? (const uint32_t*) g_iq1s_grid
-                              : (const uint32_t*) g_iq3xxs_grid;
+        const uint32_t* src = tab_source<T>();
         for (int i = threadIdx.x; i < Fmt<T>::tab_words; i += blockDim.x) s_tab[i] = src[i];
     }
 }

@@ -27,6 +27,12 @@ int down_groups(int d_type, const GroupArgs& A, int n_groups_grid, int n_embd, i
                 float* part, cudaStream_t s);
 int down_plan(int d_type, const maya_moe_plan& P, int k, int n_embd, int n_ff, size_t down_off, const void* hq,
               const float* sh_out, float* out, cudaStream_t s);
+// The streamed forms (moe_window.cu), for up to 128 groups; kWindowTooWide: the shapes do not fit them, nothing launched.
+constexpr int kWindowTooWide = 1;
+int window_gate_up(int gu_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t up_off, float limit, const void* xq,
+                   size_t xq_stride, void* hq, cudaStream_t s);
+int window_down(int d_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t down_off, const void* hq, float* part,
+                cudaStream_t s);
 int win_combine(const unsigned long long* plan_ptr, const float* plan_w, int T, int k, int n_embd, const float* part,
                 const float* cpu_part, const int* cpu_flag, const float* sh_out, float* out, size_t out_stride,
                 cudaStream_t s);

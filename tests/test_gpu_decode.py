@@ -335,6 +335,25 @@ def test_window_equals_token_by_token_bitwise(T, api, oracle, t, n_tok):
     assert H.rel_err(out[0].cpu().numpy(), want) <= TIGHT
 
 
+@pytest.mark.parametrize("t,n_embd,n_ff,n_tok", [
+    (H.IQ2_S, 4096, 256, 5), (H.IQ2_S, 4352, 768, 7), (H.IQ2_S, 8448, 256, 3),     # column capacities 128, 256 and none; 5 and 7 columns
+    (H.IQ3_S, 6144, 256, 16), (H.IQ3_S, 2304, 1280, 7), (H.IQ3_XXS, 4352, 768, 5),  # two jobs of one expert; rows off a 16-byte boundary
+    (H.Q4_K, 7168, 256, 9), (H.Q5_K, 6400, 512, 4), (H.Q8_0, 2880, 1056, 6), (H.Q6_K, 3328, 768, 8), (H.IQ2_XXS, 2048, 256, 2)])
+def test_window_edges_bitwise(T, api, t, n_embd, n_ff, n_tok):
+    """Every token shares its experts with every other one, so the jobs are as wide as the shared memory lets them be: each
+    token's output equals its single-token window's, in which every job has one column, bit for bit."""
+    E, k = 3, 2
+    store = dev(T, np.stack([H.constructed_expert(t, t, n_embd, n_ff, H.rng_for("win-edge", t, n_embd, e)) for e in range(E)]))
+    rng = H.rng_for("win-edge", t, n_embd, n_tok)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(n_tok)]).astype(np.int64)
+    w = rng.random((n_tok, k)).astype(np.float32)
+    x = rng.standard_normal((n_tok, n_embd)).astype(np.float32)
+    out = run_window(T, api, t, n_embd, n_ff, store, ids, w, x, H.INF)[0]
+    for i in range(n_tok):
+        one = run_window(T, api, t, n_embd, n_ff, store, ids[i:i + 1], w[i:i + 1], x[i:i + 1], H.INF)[0]
+        assert T.isfinite(one).all() and T.equal(out[i], one[0]), f"token {i}"
+
+
 # ------------------------------------------------------------------------------------------------ grouped (native) form
 @pytest.mark.parametrize("t", [H.Q4_K, H.IQ2_S, H.Q6_K, H.IQ4_XS, H.IQ3_XXS])
 def test_expert_grouped(T, api, oracle, t):
