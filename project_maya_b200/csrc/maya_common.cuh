@@ -14,6 +14,24 @@ int note_launch(const char* what);          // cudaGetLastError -> status; count
 int refuse(int status);                     // counts a refused call, returns status
 int sm_count();                             // multiprocessors of the current device
 inline cudaStream_t as_stream(void* s) { return (cudaStream_t) s; }
+// A launch whose set-up may overlap the tail of the launch in front of it (programmatic dependent launch): the kernel must call
+// grid_dependency_wait() before it reads or writes anything that launch could touch.
+template<class... KArgs, class... Args>
+inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, (KArgs) args...);
+}
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 inline bool aligned16(const void* p) { return (((uintptr_t) p) & 15u) == 0; }
 
 // ---------------------------------------------------------------- GGUF block geometry

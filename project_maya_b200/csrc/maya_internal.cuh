@@ -27,17 +27,27 @@ int down_groups(int d_type, const GroupArgs& A, int n_groups_grid, int n_embd, i
                 float* part, cudaStream_t s);
 int down_plan(int d_type, const maya_moe_plan& P, int k, int n_embd, int n_ff, size_t down_off, const void* hq,
               const float* sh_out, float* out, cudaStream_t s);
-// The streamed forms (moe_window.cu), for up to 128 groups; kWindowTooWide: the shapes do not fit them, nothing launched.
+// The streamed forms (moe_window.cuh), for up to 128 groups.  kWindowTooWide: the shapes do not fit them, nothing launched.
+// sh: a Q8_0 shared expert every one of n_tok tokens (whose columns are xq, xq_stride apart) uses, in the same launches: gate/up
+// leaves its h in sh->hq [n_tok][n_ff / 32], down its output in sh->out [n_tok][n_embd].
 constexpr int kWindowTooWide = 1;
+struct SharedArgs {
+    const uint8_t* blob;         // [gate rows | up rows | down rows]
+    int n_ff, n_tok;
+    void* hq;
+    float* out;
+};
+inline bool window_fits(int n_embd, int n_ff, int n_ff_sh) { return n_embd <= 8192 && n_ff <= 8192 && n_ff_sh <= 8192; }
 int window_gate_up(int gu_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t up_off, float limit, const void* xq,
-                   size_t xq_stride, void* hq, cudaStream_t s);
+                   size_t xq_stride, void* hq, const SharedArgs* sh, cudaStream_t s);
 int window_down(int d_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t down_off, const void* hq, float* part,
-                cudaStream_t s);
+                const SharedArgs* sh, cudaStream_t s);
 int win_combine(const unsigned long long* plan_ptr, const float* plan_w, int T, int k, int n_embd, const float* part,
                 const float* cpu_part, const int* cpu_flag, const float* sh_out, float* out, size_t out_stride,
                 cudaStream_t s);
 
-int win_experts(int gu_type, int d_type, const maya_moe_win* w, const maya_peer_ar* ar, int mi, unsigned seq, cudaStream_t s);
+int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, const maya_peer_ar* ar, int mi,
+                unsigned seq, cudaStream_t s);
 
 // The fused single-token layer kernel (moe_fused.cu).
 bool fused_t1_supported(const maya_moe_layer& L);

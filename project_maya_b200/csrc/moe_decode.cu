@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "maya_dots.cuh"
+#include "maya_group.cuh"
 #include "maya_internal.cuh"
 #include "maya_peer_ar.cuh"
 #include "maya_stream.cuh"
@@ -358,56 +359,13 @@ __global__ void __launch_bounds__(kDownWarps * 32, 4) down_groups_kernel(Groups 
 }
 
 // ------------------------------------------------------------------------------------------------ window grouping
-// Entries i = t * 8 + j (token t, plan slot j) with a non-zero blob address are grouped by address: groups in order of
-// first appearance, members in ascending i.  One block; T * 8 <= 128 entries.
-__global__ void __launch_bounds__(128) win_group_kernel(const unsigned long long* __restrict__ plan_ptr, int T, int k,
-                                                        unsigned long long* __restrict__ grp_ptr,
-                                                        int* __restrict__ grp_start, int* __restrict__ grp_ent,
-                                                        int* __restrict__ n_groups) {
-    __shared__ unsigned long long s_ptr[128];
-    __shared__ int s_leader[128], s_gidx[128], s_cnt[129];
-    const int i = threadIdx.x, n = T * 8;
-    const int t = i >> 3, j = i & 7;
-    s_ptr[i] = (i < n && j < k) ? plan_ptr[i] : 0ull;
-    __syncthreads();
-    const unsigned long long p = s_ptr[i];
-    int leader = -1;
-    if (p != 0ull) {
-        leader = i;
-        for (int f = 0; f < i; ++f)
-            if (s_ptr[f] == p) { leader = f; break; }
-    }
-    s_leader[i] = leader;
-    __syncthreads();
-    // group index of a leader = leaders before it
-    int gi = 0;
-    if (leader == i)
-        for (int f = 0; f < i; ++f) gi += (s_leader[f] == f);
-    s_gidx[i] = gi;
-    s_cnt[i] = 0;
-    if (i == 0) s_cnt[128] = 0;
-    __syncthreads();
-    const int my_group = leader >= 0 ? s_gidx[leader] : -1;
-    int rank = 0;   // members of my group before me
-    if (leader >= 0)
-        for (int f = 0; f < i; ++f) rank += (s_leader[f] == leader);
-    if (leader >= 0) atomicAdd(&s_cnt[my_group], 1);
-    __syncthreads();
-    // exclusive scan of the counts by every thread for its own group (<= 128 groups)
-    int ng = 0;
-    for (int f = 0; f < 128; ++f) ng += (s_leader[f] == f);
-    int start = 0;
-    if (leader >= 0)
-        for (int f = 0; f < my_group; ++f) start += s_cnt[f];
-    if (leader >= 0) grp_ent[start + rank] = i;
-    if (leader == i) { grp_ptr[my_group] = p; grp_start[my_group] = start; }
-    if (i == 0) {
-        int total = 0;
-        for (int f = 0; f < ng; ++f) total += s_cnt[f];
-        grp_start[ng] = total;
-        *n_groups = ng;
-    }
-    (void) t;
+// Entries i = t * 8 + j (token t, plan slot j): see group_entries.
+__global__ void __launch_bounds__(128) win_group_kernel(const unsigned long long* __restrict__ plan_ptr, int T, int k, GroupOut G) {
+    __shared__ GroupShared sh;
+    const int i = threadIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    group_entries(i < T * 8 && (i & 7) < k ? plan_ptr[i] : 0ull, T * 8, G, sh);
 }
 
 // out[t][r] = fma chain over the token's plan slots in plan order (a skipped slot contributes w * 0, as the plan
@@ -420,8 +378,11 @@ __global__ void __launch_bounds__(256) win_combine_kernel(const unsigned long lo
                                                           const float* __restrict__ sh_out, float* __restrict__ out,
                                                           size_t out_stride) {
     const int t = blockIdx.y, r = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
     if (r >= n_embd) return;
     float m = 0.0f;
+#pragma unroll 8
     for (int j = 0; j < k; ++j) {
         const float pv = plan_ptr[t * 8 + j] != 0ull ? part[((size_t) t * 8 + j) * n_embd + r] : 0.0f;
         m = __fmaf_rn(plan_w[t * 8 + j], pv, m);
@@ -619,7 +580,7 @@ int win_combine(const unsigned long long* plan_ptr, const float* plan_w, int T, 
                 const float* cpu_part, const int* cpu_flag, const float* sh_out, float* out, size_t out_stride,
                 cudaStream_t s) {
     const dim3 grid((unsigned) ((n_embd + 255) / 256), (unsigned) T);
-    win_combine_kernel<<<grid, 256, 0, s>>>(plan_ptr, plan_w, k, n_embd, part, cpu_part, cpu_flag, sh_out, out, out_stride);
+    launch_dependent(win_combine_kernel, grid, dim3(256), 0, s, plan_ptr, plan_w, k, n_embd, part, cpu_part, cpu_flag, sh_out, out, out_stride);
     return note_launch("moe_win_combine");
 }
 
@@ -633,8 +594,11 @@ int win_combine_ar(const unsigned long long* plan_ptr, const float* plan_w, int 
     return note_launch("moe_win_combine_ar");
 }
 
-// moe_win_experts; with `ar` the cross-rank sum of out[T][n_embd] (contiguous) runs inside the combine launch.
-int win_experts(int gu_type, int d_type, const maya_moe_win* w, const maya_peer_ar* ar, int mi, unsigned seq, cudaStream_t s) {
+// moe_win_experts; with `ar` the cross-rank sum of out[T][n_embd] (contiguous) runs inside the combine launch.  grouped: the
+// group arrays are filled already.  sh: the shared expert in the same launches (w->sh_out == sh->out); the caller has asked
+// window_fits.
+int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, const maya_peer_ar* ar, int mi,
+                unsigned seq, cudaStream_t s) {
     if (!w || !w->plan_w || !w->xq || !w->hq || !w->part || !w->out) return refuse(MAYA_ERR_ARG);
     if (w->cpu_flag != nullptr && w->cpu_part == nullptr) return refuse(MAYA_ERR_ARG);
     int st = check_shapes(gu_type, d_type, w->k, w->n_embd, w->n_ff);
@@ -642,7 +606,7 @@ int win_experts(int gu_type, int d_type, const maya_moe_win* w, const maya_peer_
     if (ar != nullptr && (w->out_stride != (size_t) w->n_embd || w->n_embd % 4 || !aligned16(w->out) || !aligned16(w->part) ||
                           (w->sh_out && !aligned16(w->sh_out)) || (w->cpu_part && !aligned16(w->cpu_part))))
         return refuse(MAYA_ERR_ARG);
-    st = maya_moe_win_group(w, s);
+    if (!grouped) st = maya_moe_win_group(w, s);
     if (st != MAYA_OK) return st;
     const int cap = w->T * 8;
     const size_t up_off = row_bytes(gu_type, w->n_embd) * (size_t) w->n_ff;
@@ -653,12 +617,12 @@ int win_experts(int gu_type, int d_type, const maya_moe_win* w, const maya_peer_
     A.n_groups = w->n_groups;
     A.ent_slot = w->grp_ent;
     A.tok_from_slot = 1;
-    st = window_gate_up(gu_type, A, cap, w->n_embd, w->n_ff, up_off, w->limit, w->xq, w->xq_stride, w->hq, s);
+    st = window_gate_up(gu_type, A, cap, w->n_embd, w->n_ff, up_off, w->limit, w->xq, w->xq_stride, w->hq, sh, s);
     if (st == kWindowTooWide)
         st = gate_up_groups(gu_type, A, cap, w->n_embd, w->n_ff, up_off, w->limit, w->xq, w->xq_stride, w->hq, nullptr, 0, nullptr, 0,
                             nullptr, s);
     if (st != MAYA_OK) return st;
-    st = window_down(d_type, A, cap, w->n_embd, w->n_ff, w->down_off, w->hq, w->part, s);
+    st = window_down(d_type, A, cap, w->n_embd, w->n_ff, w->down_off, w->hq, w->part, sh, s);
     if (st == kWindowTooWide) st = down_groups(d_type, A, cap, w->n_embd, w->n_ff, w->down_off, w->hq, w->part, s);
     if (st != MAYA_OK) return st;
     if (ar != nullptr)
@@ -702,13 +666,13 @@ extern "C" int maya_moe_down(int d_type, const maya_moe_plan* plan, int k, int n
 extern "C" int maya_moe_win_group(const maya_moe_win* w, void* stream) {
     if (!w || !w->plan_ptr || !w->grp_ptr || !w->grp_start || !w->grp_ent || !w->n_groups) return refuse(MAYA_ERR_ARG);
     if (w->T < 1 || w->T > MAYA_MAX_WIN_TOKENS || w->k < 1 || w->k > MAYA_MAX_K) return refuse(MAYA_ERR_LIMIT);
-    win_group_kernel<<<1, 128, 0, as_stream(stream)>>>(w->plan_ptr, w->T, w->k, w->grp_ptr, w->grp_start, w->grp_ent,
-                                                       w->n_groups);
+    launch_dependent(win_group_kernel, dim3(1), dim3(128), 0, as_stream(stream), w->plan_ptr, w->T, w->k,
+                     GroupOut{w->grp_ptr, w->grp_start, w->grp_ent, w->n_groups});
     return note_launch("moe_win_group");
 }
 
 extern "C" int maya_moe_win_experts(int gu_type, int d_type, const maya_moe_win* w, void* stream) {
-    return win_experts(gu_type, d_type, w, nullptr, 0, 0u, as_stream(stream));
+    return win_experts(gu_type, d_type, w, false, nullptr, nullptr, 0, 0u, as_stream(stream));
 }
 
 extern "C" size_t maya_expert_scratch_bytes(int64_t cap_entries, int64_t n_ff) {

@@ -4,7 +4,9 @@
 // blob addresses of its k routed experts (0 for experts outside [expert_lo, expert_hi): another rank's).
 #include <math.h>
 
+#include "maya_group.cuh"
 #include "maya_internal.cuh"
+#include "maya_router.cuh"
 
 namespace maya {
 namespace {
@@ -16,7 +18,7 @@ struct Scratch {
     int* ids;                    // [T][k]
     float* weights;              // [T][k]
     uint8_t* hq;                 // [T*8][n_ff/32] q8_1
-    float* part;                 // [T*8][n_embd]      (T > 1)
+    float* part;                 // [T*8][n_embd]
     unsigned long long* grp_ptr; // [T*8]
     int* grp_start;              // [T*8 + 1]
     int* grp_ent;                // [T*8]
@@ -25,7 +27,8 @@ struct Scratch {
     uint8_t* sh_hq;              // [T][n_ff_sh/32] q8_1
     float* sh_out;               // [T][n_embd]
     float* h;                    // the fused single-token kernel's h: q8_1 image, shared-unit halves, counters
-    unsigned* sync;              // [16]: the fused kernel's barrier counter, epoch, error word (zero before first use)
+    unsigned* sync;              // [16]: the fused kernel's barrier counter, epoch, error word; [3] prep_kernel's ticket; stamps (zero
+                                 // before first use)
     size_t bytes;
 };
 
@@ -50,7 +53,7 @@ Scratch carve(const maya_moe_layer& L, int T, uint8_t* base) {
     s.ids = (int*) take((size_t) T * L.k * sizeof(int));
     s.weights = (float*) take((size_t) T * L.k * sizeof(float));
     s.hq = take((size_t) T * 8 * (L.n_ff / 32) * kQ81Bytes);
-    s.part = (float*) take(T > 1 ? (size_t) T * 8 * L.n_embd * sizeof(float) : 0);
+    s.part = (float*) take((size_t) T * 8 * L.n_embd * sizeof(float));
     s.grp_ptr = (unsigned long long*) take((size_t) T * 8 * sizeof(unsigned long long));
     s.grp_start = (int*) take(((size_t) T * 8 + 1) * sizeof(int));
     s.grp_ent = (int*) take((size_t) T * 8 * sizeof(int));
@@ -64,21 +67,91 @@ Scratch carve(const maya_moe_layer& L, int T, uint8_t* base) {
     return s;
 }
 
-__global__ void plan_kernel(const int* __restrict__ ids, const float* __restrict__ weights, int T, int k,
-                            const uint8_t* experts, size_t stride, int lo, int hi,
-                            unsigned long long* __restrict__ plan_ptr, float* __restrict__ plan_w) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= T * 8) return;
-    const int t = i >> 3, j = i & 7;
-    unsigned long long p = 0ull;
-    float w = 0.0f;
-    if (j < k) {
-        const int e = ids[t * k + j];
-        w = weights[t * k + j];
-        if (e >= lo && e < hi) p = (unsigned long long) (experts + (size_t) e * stride);
+// Everything in front of the experts in one launch: block (t, 0) routes token t and writes its plan (blob addresses, weights),
+// blocks (t, 1 ..) round its activations to q8_1, and the last routing block to finish groups all the tokens' entries by
+// expert.  As launches of their own - router, quantizer, plan, grouping - these took 12 to 17 us of a window.
+struct PrepArgs {
+    const float* logits;
+    const float* bias;           // sigmoid router
+    float w_scale;
+    int norm_w;
+    int n_expert, k;
+    const void* x;
+    int x_is_bf16, n_embd;
+    uint8_t* xq;                 // [T][n_embd / 32] q8_1
+    const uint8_t* experts;
+    size_t stride;
+    int lo, hi;                  // this rank's experts
+    int* ids;
+    float* weights;
+    unsigned long long* plan_ptr;
+    float* plan_w;
+    GroupOut group;
+    unsigned* ticket;            // zero between launches
+};
+
+template<int RT, int PER>
+__global__ void __launch_bounds__(256) prep_kernel(const PrepArgs P) {
+    extern __shared__ __align__(16) double s_ex[];           // n_expert doubles
+    __shared__ RouterShared route;
+    __shared__ GroupShared grp;
+    __shared__ int s_last;
+    const int t = blockIdx.x, T = gridDim.x, tid = threadIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (blockIdx.y > 0) {
+        const int lane = tid & 31, nblk = P.n_embd / 32, step = 8 * (gridDim.y - 1);
+        for (int b0 = 8 * (blockIdx.y - 1) + (tid >> 5); b0 < nblk; b0 += 4 * step) {        // four blocks in flight a warp
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int b = b0 + i * step;
+                const size_t at = (size_t) t * P.n_embd + (size_t) b * 32 + lane;
+                v[i] = 0.0f;
+                if (b < nblk) v[i] = P.x_is_bf16 ? __uint_as_float((uint32_t) ((const uint16_t*) P.x)[at] << 16) : ((const float*) P.x)[at];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (b0 + i * step < nblk) q8_1_store_warp(v[i], P.xq + ((size_t) t * nblk + b0 + i * step) * kQ81Bytes, lane);
+        }
+        return;
     }
-    plan_ptr[i] = p;
-    plan_w[i] = w;
+    const float* logits = P.logits + (size_t) t * P.n_expert;
+    if constexpr (RT == 1) route_sigmoid<PER, BlockSync>(logits, P.bias, P.n_expert, P.k, P.w_scale, P.norm_w, tid, 256, route);
+    else route_softmax<PER, BlockSync>(logits, P.n_expert, P.k, tid, 256, s_ex, route);
+    if (tid < 8) {
+        unsigned long long p = 0ull;
+        float w = 0.0f;
+        if (tid < P.k) {
+            const int e = route.ids[tid];
+            w = route.val[tid];
+            if (e >= P.lo && e < P.hi) p = (unsigned long long) (P.experts + (size_t) e * P.stride);
+            P.ids[(size_t) t * P.k + tid] = e;
+            P.weights[(size_t) t * P.k + tid] = w;
+        }
+        P.plan_ptr[t * 8 + tid] = p;
+        P.plan_w[t * 8 + tid] = w;
+        __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) {
+        s_last = atomicAdd(P.ticket, 1u) == (unsigned) T - 1u;
+        if (s_last) *P.ticket = 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) group_entries(tid < T * 8 ? __ldcg(P.plan_ptr + tid) : 0ull, T * 8, P.group, grp);
+}
+
+template<int RT> int launch_prep(const PrepArgs& P, int T, cudaStream_t s) {
+    const int per = (P.n_expert + 255) / 256, nblk = P.n_embd / 32;
+    const dim3 grid((unsigned) T, (unsigned) (1 + (nblk >= 256 ? 8 : (nblk + 31) / 32)));
+    const size_t smem = RT == 0 ? (size_t) P.n_expert * sizeof(double) : 0;
+    if (per <= 1) launch_dependent(prep_kernel<RT, 1>, grid, dim3(256), smem, s, P);
+    else if (per <= 2) launch_dependent(prep_kernel<RT, 2>, grid, dim3(256), smem, s, P);
+    else if (per <= 4) launch_dependent(prep_kernel<RT, 4>, grid, dim3(256), smem, s, P);
+    else launch_dependent(prep_kernel<RT, 8>, grid, dim3(256), smem, s, P);
+    return note_launch("moe_prep");
 }
 
 int check_layer(const maya_moe_layer* L) {
@@ -198,23 +271,26 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
     if (L->n_ff_sh > 0 && L->shared_here && (L->sh_lo != 0 || (L->sh_hi != 0 && L->sh_hi != L->n_ff_sh)))
         return refuse(MAYA_ERR_ARG);                 // only the fused kernel slices the shared expert
 
-    st = L->router == 1 ? maya_router_sigmoid(logits, L->router_bias, T, L->n_expert, L->k, L->router_w_scale, L->router_norm_w,
-                                              d_ids, d_w, stream)
-                        : maya_router_top10(logits, T, L->n_expert, L->k, d_ids, d_w, stream);
-    if (st != MAYA_OK) return st;
-    st = x_is_bf16 ? maya_quantize_q8_1_bf16((const uint16_t*) x, S.xq, L->n_embd, T, stream)
-                   : maya_quantize_q8_1((const float*) x, S.xq, L->n_embd, T, stream);
-    if (st != MAYA_OK) return st;
-    plan_kernel<<<(T * 8 + 127) / 128, 128, 0, s>>>(d_ids, d_w, T, L->k, (const uint8_t*) L->experts, L->expert_stride,
-                                                    L->expert_lo, L->expert_hi, S.plan_ptr, S.plan_w);
-    st = note_launch("moe_plan");
+    if (L->k > 64 || L->n_expert > 256 * kRouterMaxPerThread) return refuse(MAYA_ERR_LIMIT);
+    PrepArgs P{};
+    P.logits = logits; P.bias = L->router_bias; P.w_scale = L->router_w_scale; P.norm_w = L->router_norm_w;
+    P.n_expert = L->n_expert; P.k = L->k; P.x = x; P.x_is_bf16 = x_is_bf16; P.n_embd = L->n_embd; P.xq = S.xq;
+    P.experts = (const uint8_t*) L->experts; P.stride = L->expert_stride; P.lo = L->expert_lo; P.hi = L->expert_hi;
+    P.ids = d_ids; P.weights = d_w; P.plan_ptr = S.plan_ptr; P.plan_w = S.plan_w;
+    P.group = GroupOut{S.grp_ptr, S.grp_start, S.grp_ent, S.n_groups};
+    P.ticket = S.sync + 3;
+    st = L->router == 1 ? launch_prep<1>(P, T, s) : launch_prep<0>(P, T, s);
     if (st != MAYA_OK) return st;
 
     const bool shared = L->n_ff_sh > 0 && L->shared_here;
     const uint8_t* sh_blob = (const uint8_t*) L->shared;
-    size_t sh_down_off = 0;
-    if (shared) {
-        sh_down_off = row_bytes(L->sh_gu_type, L->n_embd) * (size_t) L->n_ff_sh * 2;
+    const size_t up_off = row_bytes(L->gu_type, L->n_embd) * (size_t) L->n_ff, down_off = 2 * up_off;
+    // a Q8_0 shared expert rides in the routed experts' launches where the shapes fit them
+    const bool ride = shared && L->sh_gu_type == MAYA_Q8_0 && L->sh_d_type == MAYA_Q8_0 && (((uintptr_t) sh_blob) & 15u) == 0 &&
+                      window_fits(L->n_embd, L->n_ff, L->n_ff_sh);
+    const SharedArgs sh{sh_blob, L->n_ff_sh, T, S.sh_hq, S.sh_out};
+    if (shared && !ride) {
+        const size_t sh_down_off = row_bytes(L->sh_gu_type, L->n_embd) * (size_t) L->n_ff_sh * 2;
         for (int c0 = 0; c0 < T; c0 += MAYA_MAX_COLS) {   // gate and up rows are contiguous: one GEMV of 2 * n_ff_sh rows
             const int nc = T - c0 < MAYA_MAX_COLS ? T - c0 : MAYA_MAX_COLS;
             // column-major output [c][2 * n_ff_sh] per call: offset by the columns already done
@@ -227,20 +303,6 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
                                   L->limit, L->n_ff_sh, S.sh_hq + (size_t) c * (L->n_ff_sh / 32) * kQ81Bytes, stream);
             if (st != MAYA_OK) return st;
         }
-    }
-
-    const size_t up_off = row_bytes(L->gu_type, L->n_embd) * (size_t) L->n_ff;
-    const size_t down_off = 2 * up_off;
-    if (T == 1) {
-        maya_moe_plan P{S.plan_ptr, S.plan_w, L->cpu_flag ? L->cpu_part : nullptr, L->cpu_flag, nullptr};
-        st = maya_moe_gate_up(L->gu_type, &P, L->k, L->n_embd, L->n_ff, L->limit, S.xq, S.hq,
-                              shared ? sh_blob + sh_down_off : nullptr, L->sh_d_type, S.sh_hq, L->n_ff_sh, S.sh_out, stream);
-        if (st != MAYA_OK) return st;
-        st = maya_moe_down(L->d_type, &P, L->k, L->n_embd, L->n_ff, down_off, S.hq, shared ? S.sh_out : nullptr, out, stream);
-        if (st == MAYA_OK && ar != nullptr) st = maya_allreduce_peer(out, L->n_embd, ar, mi, seq, stream);
-        return st == MAYA_OK ? hc_post_tokens(hc, out, 1, L->n_embd, stream) : st;
-    }
-    if (shared) {
         for (int c0 = 0; c0 < T; c0 += MAYA_MAX_COLS) {
             const int nc = T - c0 < MAYA_MAX_COLS ? T - c0 : MAYA_MAX_COLS;
             st = maya_mmvq(L->sh_d_type, sh_blob + sh_down_off, S.sh_hq + (size_t) c0 * (L->n_ff_sh / 32) * kQ81Bytes,
@@ -270,6 +332,8 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
     W.n_ff = L->n_ff;
     W.limit = L->limit;
     W.down_off = down_off;
-    st = win_experts(L->gu_type, L->d_type, &W, ar, mi, seq, s);       // with `ar`: the sum runs in the combine launch
+    // one token: a window of one, its cross-rank sum a launch of its own; more: with `ar` the sum runs in the combine launch
+    st = win_experts(L->gu_type, L->d_type, &W, true, ride ? &sh : nullptr, T > 1 ? ar : nullptr, mi, seq, s);
+    if (st == MAYA_OK && T == 1 && ar != nullptr) st = maya_allreduce_peer(out, L->n_embd, ar, mi, seq, stream);
     return st == MAYA_OK ? hc_post_tokens(hc, out, T, L->n_embd, stream) : st;
 }

@@ -1,0 +1,614 @@
+// moe_window.cuh - the routed experts (and the shared one) of a window (2..16 tokens) or of a short plan: gate/up + SwiGLU + q8_1(h), and the down
+// rows, with the weight rows streamed through shared memory.
+//
+// What bounds this path: on a B200 neither HBM nor the dot products but instruction issue and the shared-memory pipe - a
+// 2-4 bit weight costs 60-90 instructions per 32 to decode and 14-38 per column to dot - so everything around them has to
+// be cheap and no warp may wait for its loads.  One 512-thread block an SM; its warps never meet inside a row:
+//   * the work is a list of jobs - a group (distinct expert) and up to `ncm` of its entries (activation columns) - times
+//     chunks of 64 weight rows (32 gate + the same 32 up rows, or 64 down rows).  Every block takes one contiguous share of
+//     that list, equal in estimated COST (decode + columns x dot), not in count: a chunk with eight columns costs several
+//     times one with a single column.  Contiguous, so that a block stages a job's columns once for all its chunks.
+//   * a warp owns four rows of a chunk and streams their K segments into a private ring with cp.async.bulk, two segments
+//     ahead, across chunk and job boundaries: no block barrier stands between a warp and its next bytes, and decoding reads
+//     shared memory, where a lane's 2-byte aligned fields cost one or two wavefronts a warp instead of the four to five
+//     cache lines they touch in global memory.
+//   * the always-on shared expert, when it is Q8_0, is one more job list in the same launches - its rows against all the tokens -
+//     so that its 40 MB hide behind an instruction-bound phase instead of taking two GEMV launches and a SwiGLU launch a token.
+//   * codebooks lie in several copies side by side in shared memory, lane l reading copy l % n.
+// Read in place by a grid of (chunk, group) blocks (gate/up) and streamed 64 rows a stage (down), an 8-token Q4_K window took
+// 318 us, a 16-token IQ3_S one 570; now 263 and 433.  (32 warps of two rows: 266 and 484, the activation reads then bind.)
+//
+// The arithmetic is rows_dot's (maya_dots.cuh), value for value - the same integers, the same lane order, the same sums - so
+// every token's result is bit-identical to the single-token kernels'.
+//
+// Plain bulk copies (one destination: this block) of this GPU's own memory.  A row need not start on a 16-byte boundary: the
+// aligned window around a segment is copied (expert blobs are 16-byte aligned and a whole number of 16-byte words long, so
+// it stays inside).  Every wait is bounded; one that runs out makes the block skip what is left (its outputs are then
+// missing) after the copies in flight were given the same bounded time to land.  A blob that is not 16-byte aligned is
+// copied with ordinary loads instead.
+#pragma once
+
+#include "maya_dots.cuh"
+#include "maya_internal.cuh"
+#include "maya_stream.cuh"
+#include "moe_window_args.cuh"
+
+#include <atomic>
+#include <type_traits>
+
+namespace maya {
+namespace {
+
+constexpr int kWNC = 8;            // most activation columns of a job
+constexpr int kWStages = 2;        // segments in flight a warp
+constexpr int kWMaxGroups = 128;   // T <= 16 tokens x 8 routes
+constexpr int kWMaxJobs = kWMaxGroups + 16;      // a job has at least one entry; the shared expert's at least one token
+constexpr int kWChunkRows = 64;    // weight rows of a chunk
+constexpr int kChunkCost = 40;     // a chunk's own overhead, in the units of WGeo's costs
+
+// ---- decoders: Dec<T>'s fields and dot, loaded from shared memory - byte `o` of `s` is the block's first - with fewer
+//      instructions.  rep: copies of the codebook, `tab` = this lane's copy.  ONE: for a single column, where it is cheaper to
+//      correct the dot for the signs (see maya_dots_t1.cuh) than to negate the weights.
+__device__ __forceinline__ uint32_t s_u32(const uint8_t* s, uint32_t o) { return *(const uint32_t*) (s + o); }
+// 4 bytes at an even place; sel: 0x3210 where o is a multiple of 4, else 0x5432
+__device__ __forceinline__ uint32_t s_u32_a2(const uint8_t* s, uint32_t o, uint32_t sel) {
+    const uint32_t a = o & ~3u;
+    return prmt_raw(s_u32(s, a), s_u32(s, a + 4), sel);
+}
+// the selector for fields 2 bytes (and a multiple of 4) into a block at o
+__device__ __forceinline__ uint32_t sel_2(uint32_t o) { return (o & 2u) ? 0x3210u : 0x5432u; }
+
+template<int T, bool ONE> struct WDec : Dec<T> {
+    static constexpr int rep = 1;
+    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) { Dec<T>::load(s + o, c, tab); }
+};
+// eight signed weight words (or, with ONE, codebook words XOR mask and the masks) and their dots
+template<bool ONE> struct WSigned {
+    int w[8];
+    uint32_t mk[ONE ? 8 : 1];
+    __device__ __forceinline__ void set(int i, uint32_t g, uint32_t m) {
+        if constexpr (ONE) { w[i] = (int) (g ^ m); mk[i] = m; }
+        else w[i] = apply_sign4(g, m);
+    }
+    __device__ __forceinline__ int dot4(const XQ& v, int i0, int s) const {        // words i0 .. i0 + 3
+#pragma unroll
+        for (int i = i0; i < i0 + 4; ++i) s = __dp4a(w[i], v.u[i], s);
+        if constexpr (ONE) {
+            int m = 0;
+#pragma unroll
+            for (int i = i0; i < i0 + 4; ++i) m = __dp4a((int) mk[i], v.u[i], m);
+            s -= m;
+        }
+        return s;
+    }
+};
+template<bool ONE> struct WDec<MAYA_IQ2_S, ONE> : WSigned<ONE> {
+    static constexpr int rep = 8;
+    int ls0, ls1;
+    float d;
+    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
+        const uint32_t sel = sel_2(o);
+        d = ld_f16(s + o);
+        const uint32_t qs = s_u32_a2(s, o + 2 + 4 * c, sel), sg = s_u32_a2(s, o + 34 + 4 * c, sel);
+        const uint32_t qh = s[o + 66 + c], sc = s[o + 74 + c];
+        ls0 = (int) (sc & 0x0F);
+        ls1 = (int) (sc >> 4);
+        const uint2* grid = (const uint2*) tab;
+        const uint32_t hw = ((qh & 0x33u) * 0x1001u + (qh & 0xCCu) * 0x40040u) & 0x03030303u;      // see Dec1<MAYA_IQ2_S>
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const uint2 g = grid[prmt_raw(qs, hw, 0xCC00u + ((4 + l) << 4) + l) * rep];
+            const uint32_t b = byte_of(sg, l);
+            this->set(2 * l, g.x, sign_mask_lo(b));
+            this->set(2 * l + 1, g.y, sign_mask_hi(b));
+        }
+    }
+    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
+        const int s0 = this->dot4(v, 0, 0), s1 = this->dot4(v, 4, 0);
+        return __fmul_rn(__fmul_rn(d, v.d), (float) ((s0 * ls0 + s1 * ls1 + (s0 + s1) / 2) / 4));
+    }
+};
+// IQ3_S: every codebook value is odd, g = 2 b + 1 with b in 0..7.  Flipping b's bits negates it: 2 ~b + 1 = -g.  So the table
+// holds b, a sign is one XOR, and sum(+-g u) = 2 sum((b ^ m) u) + sum(u), the block's sum being at hand.
+template<bool ONE> struct WDec<MAYA_IQ3_S, ONE> {
+    static constexpr int rep = 16;
+    int w[8];
+    int mul;
+    float d;
+    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
+        const uint32_t sel = sel_2(o), qa = (o + 2 + 8 * c) & ~3u;
+        d = ld_f16(s + o);
+        const uint32_t w1 = s_u32(s, qa + 4), q0 = prmt_raw(s_u32(s, qa), w1, sel), q1 = prmt_raw(w1, s_u32(s, qa + 8), sel);
+        const uint32_t qh = s[o + 66 + c], sg = s_u32_a2(s, o + 74 + 4 * c, sel);
+        mul = 1 + 2 * (int) ((s[o + 106 + (c >> 1)] >> (4 * (c & 1))) & 0x0F);
+        // byte l of h0 / h1: bit l / 4 + l of qh, an entry's ninth index bit
+        const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
+#pragma unroll
+        for (int l = 0; l < 8; ++l) {
+            const uint32_t b = tab[prmt_raw(l < 4 ? q0 : q1, l < 4 ? h0 : h1, 0xCC00u + ((4 + l % 4) << 4) + l % 4) * rep];
+            const uint32_t sb = byte_of(sg, l >> 1);
+            w[l] = (int) (b ^ ((l & 1) ? sign_mask_hi(sb) : sign_mask_lo(sb)));
+        }
+    }
+    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
+        int s = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s = __dp4a(w[i], v.u[i], s);
+        return __fmul_rn(__fmul_rn(d, v.d), (float) ((2 * s + v.isum) * mul));
+    }
+};
+template<bool ONE> struct WDec<MAYA_IQ3_XXS, ONE> : WSigned<ONE> {
+    static constexpr int rep = 32;
+    int ls;
+    float d;
+    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
+        const uint32_t sel = sel_2(o), qa = (o + 2 + 8 * c) & ~3u;
+        d = ld_f16(s + o);
+        const uint32_t w1 = s_u32(s, qa + 4), q0 = prmt_raw(s_u32(s, qa), w1, sel), q1 = prmt_raw(w1, s_u32(s, qa + 8), sel);
+        const uint32_t aux = s_u32_a2(s, o + 66 + 4 * c, sel);
+        ls = (int) (aux >> 28);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const uint32_t s8 = ksign8((aux >> (7 * l)) & 127u), q = l < 2 ? q0 : q1;
+            this->set(2 * l, tab[byte_of(q, 2 * (l & 1)) * rep], sign_mask_lo(s8));
+            this->set(2 * l + 1, tab[byte_of(q, 2 * (l & 1) + 1) * rep], sign_mask_hi(s8));
+        }
+    }
+    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
+        const int t = this->dot4(v, 4, this->dot4(v, 0, 0));
+        return __fmul_rn(__fmul_rn(d, v.d), (float) ((ls * t + t / 2) / 2));
+    }
+};
+template<bool ONE> struct WDec<MAYA_IQ2_XXS, ONE> : WSigned<ONE> {
+    static constexpr int rep = 16;
+    int ls;
+    float d;
+    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
+        const uint32_t sel = sel_2(o), qa = (o + 2 + 8 * c) & ~3u;
+        d = ld_f16(s + o);
+        const uint32_t w1 = s_u32(s, qa + 4), qi = prmt_raw(s_u32(s, qa), w1, sel), aux = prmt_raw(w1, s_u32(s, qa + 8), sel);
+        ls = (int) (aux >> 27) | 1;
+        const uint2* grid = (const uint2*) tab;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const uint2 g = grid[byte_of(qi, l) * rep];
+            const uint32_t s8 = ksign8((aux >> (7 * l)) & 127u);
+            this->set(2 * l, g.x, sign_mask_lo(s8));
+            this->set(2 * l + 1, g.y, sign_mask_hi(s8));
+        }
+    }
+    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
+        const int t = this->dot4(v, 4, this->dot4(v, 0, 0));
+        return __fmul_rn(__fmul_rn(d, v.d), (float) (t * ls / 8));
+    }
+};
+
+// ---- the geometry of a type's stream.  A segment: kSegVals values of a row (a multiple of what 32 lanes take in one step, so
+//      that a lane's calls are the same whatever the segments are).  kPitch: a segment's room in a stage, its bytes and 16 for
+//      the aligned window.
+template<int T, int SPLIT = 1> struct WGeo {
+    static constexpr int split = SPLIT;          // a segment comes in this many stages, rw / SPLIT rows each
+    static constexpr int warps = 16, threads = warps * 32, rw = kWChunkRows / warps;      // a warp's rows: 4
+    // most columns of a job: four where a call spans two q8_1 blocks (six or eight spill 1.3 KB: 617 against 263 us on the window above)
+    static constexpr int nc = Dec<T>::xblk == 2 ? 4 : kWNC;
+    static constexpr int vals = T == MAYA_Q8_0 || T == MAYA_Q6_K ? 1024 : 2048;
+    static constexpr int qk = Fmt<T>::qk, cpb = Dec<T>::cpb;
+    static constexpr int blocks = vals / qk;                                 // weight blocks of a segment
+    static constexpr int bytes = blocks * Fmt<T>::bytes;
+    static constexpr int pitch = (bytes + 15 + 16) & ~15;
+    static constexpr int stage = rw / SPLIT * pitch;                                 // a warp's stage
+    static constexpr int tab = Fmt<T>::tab_words * 4 * WDec<T, false>::rep;
+    // The cost of 32 calls of a row against nc columns, in instructions: decoding, nc dots - or, where that is more, what their
+    // bytes cost at an SM's share of HBM; and a chunk's own overhead.
+    static constexpr int dec_cost = T == MAYA_Q8_0 ? 25 : T == MAYA_Q4_K || T == MAYA_IQ1_S ? 45 : T == MAYA_Q5_K ? 60 : T == MAYA_IQ3_S || T == MAYA_IQ3_XXS ? 90 : 75;
+    static constexpr int col_cost = Dec<T>::xblk == 2 ? 40 : 15;
+    static constexpr int byte_cost = 32 / cpb * Fmt<T>::bytes / 8;
+    __device__ __forceinline__ static int cost(int nc, int n_in) { return max(dec_cost + nc * col_cost, byte_cost) * ((n_in / qk * cpb + 31) / 32) + kChunkCost; }
+};
+using WShGeo = WGeo<MAYA_Q8_0, 2>;           // the shared expert's rows: a stage no larger than the 2-bit types'
+
+// what differs between the routed experts' jobs and the shared one's
+struct WKind { int n_in, n_rows, nchunk, nseg, bytes, pitch, split; size_t rb, up, off; };
+struct WJob { unsigned long long ptr; int e0, nc, shared, per; };     // per: cost of one chunk
+struct WShared {
+    uint64_t full[16][kWStages];
+    WJob job[kWMaxJobs];
+    int cost[kWMaxJobs + 1];         // cost of the jobs before job j
+    int njobs, fail;
+    float s_g[2][kWNC][32], s_u[2][kWNC][32];
+    WKind kind[2];
+};
+
+// ---- the columns in shared memory.  A column has room for CB q8_1 blocks, a compile-time number, so that the loads of every
+//      column, plane and half differ from one another by constants only (computed addresses were a sixth of the kernel's
+//      instructions): the planes of 16-byte pieces of maya_dots.cuh's planar form, then as many planes of scales and of sums.
+template<int CB> constexpr int kColBytes = CB * 40;
+template<int XB, int CB> __device__ __forceinline__ XQ col_load(const uint8_t* cols, int c, int j, int i16, int i4) {
+    constexpr int P = CB / XB;
+    const uint8_t* p = cols + c * kColBytes<CB> + 2 * j * P * 16 + i16;
+    const int4 a = *(const int4*) p, b = *(const int4*) (p + P * 16);
+    XQ v;
+    v.u[0] = a.x; v.u[1] = a.y; v.u[2] = a.z; v.u[3] = a.w;
+    v.u[4] = b.x; v.u[5] = b.y; v.u[6] = b.z; v.u[7] = b.w;
+    v.d = *(const float*) (cols + c * kColBytes<CB> + CB * 32 + j * P * 4 + i4);
+    v.isum = *(const int*) (cols + c * kColBytes<CB> + CB * 36 + j * P * 4 + i4);
+    return v;
+}
+// Block i of a column, a thread's: nine words in flight (word by word the columns of a job took 8 us to stage).
+template<int XB, int CB, bool SUM_F16> __device__ __forceinline__ void col_store(const uint8_t* xq, uint8_t* cols, int c, int i) {
+    constexpr int P = CB / XB;
+    const uint32_t* src = (const uint32_t*) (xq + (size_t) i * kQ81Bytes);
+    uint32_t w[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) w[j] = src[j];
+    uint8_t* col = cols + c * kColBytes<CB>;
+    const int j = i % XB, n = i / XB;
+    *(int4*) (col + (2 * j * P + n) * 16) = make_int4((int) w[1], (int) w[2], (int) w[3], (int) w[4]);
+    *(int4*) (col + ((2 * j + 1) * P + n) * 16) = make_int4((int) w[5], (int) w[6], (int) w[7], (int) w[8]);
+    *(float*) (col + CB * 32 + (j * P + n) * 4) = __half2float(__ushort_as_half((unsigned short) (w[0] & 0xFFFFu)));
+    int s = 0;
+    if constexpr (SUM_F16) s = __float_as_int(__half2float(__ushort_as_half((unsigned short) (w[0] >> 16))));
+    else {
+#pragma unroll
+        for (int k = 1; k < 9; ++k) s = __dp4a((int) w[k], 0x01010101, s);
+    }
+    *(int*) (col + CB * 36 + (j * P + n) * 4) = s;
+}
+
+// One segment of a warp's rows against NC columns: rows_dot's loop (maya_dots.cuh), all four rows decoded before the
+// columns, two where four would not fit the registers.  NC
+// is exact (or one more than the job's columns: a column that is not there is computed from whatever lies in its place and
+// dropped), so that no branch parts one column's loads from the next one's arithmetic.
+template<int T, class G, int NC, int RW, int CB>
+__device__ __forceinline__ void segment_dot(const uint8_t* s, const uint32_t (&row)[RW], const uint8_t* cols, int blk0, int ncalls, int lane,
+                                            const uint32_t* tab, float (&acc)[RW][NC]) {
+    constexpr int XB = Dec<T>::xblk, RP = XB == 2 || NC > 4 || RW < 4 ? 2 : 4;
+    for (int k = lane; k < ncalls; k += 32) {
+        const int kb = k / G::cpb, ci = k - kb * G::cpb;
+        const int n = ((blk0 + kb) * (G::qk / 32) + ci * XB) / XB;
+#pragma unroll
+        for (int r0 = 0; r0 < RW; r0 += RP) {
+            if (r0 > 0) asm volatile("" ::: "memory");       // the second two rows' loads stay behind: their registers are the first two's
+            WDec<T, NC == 1> dec[RP];
+#pragma unroll
+            for (int j = 0; j < RP; ++j) dec[j].load(s, row[r0 + j] + kb * Fmt<T>::bytes, ci, tab);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const XQ a = col_load<XB, CB>(cols, c, 0, n * 16, n * 4);
+                XQ b = a;
+                if constexpr (XB == 2) b = col_load<XB, CB>(cols, c, 1, n * 16, n * 4);
+#pragma unroll
+                for (int j = 0; j < RP; ++j) acc[r0 + j][c] = __fadd_rn(acc[r0 + j][c], dec[j].dot(a, b));
+            }
+        }
+    }
+}
+
+// UP: gate/up (chunk = 32 FFN rows: a warp's rows are 2 gate + 2 up); else down (chunk = 64 rows).  SH: with a Q8_0 shared expert.
+template<int T, bool SH, bool UP, int CB>
+__global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs A) {
+    using G = WGeo<T>;
+    using GS = WShGeo;
+    using D = WDec<T, false>;
+    constexpr int RW = G::rw, kWThreads = G::threads, kStage = SH && GS::stage > G::stage ? GS::stage : G::stage;
+    constexpr int kRing = G::warps * kWStages * kStage;
+    extern __shared__ __align__(128) uint8_t s_raw[];
+    __shared__ WShared sh;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t ring = warp * kWStages * kStage;              // the warp's ring in s_raw
+    uint32_t* const s_tab = (uint32_t*) (s_raw + kRing);
+    uint8_t* const cols = s_raw + kRing + G::tab;
+
+    grid_launch_dependents();
+    if constexpr (G::tab > 0) {                                  // the codebook's copies: constants of the library
+        constexpr int W = (T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1, R = D::rep;
+        const uint32_t* src = tab_source<T>();
+        for (int i = tid; i < G::tab / 4; i += kWThreads) {
+            const uint32_t g = src[i / (W * R) * W + i % W];
+            s_tab[i] = T == MAYA_IQ3_S ? (g >> 1) & 0x07070707u : g;
+        }
+    }
+    if (lane == 0) {
+        for (int s = 0; s < kWStages; ++s) mbar_init(&sh.full[warp][s], RW);
+        if (warp == 0) sh.fail = 0;
+        if (warp < 2) {
+            WKind& k = sh.kind[warp];
+            const int ff = warp ? A.n_ff_sh : A.n_ff;
+            k.n_in = UP ? A.n_embd : ff;
+            k.n_rows = UP ? ff : A.n_embd;
+            k.nchunk = UP ? ff / 32 : (A.n_embd + kWChunkRows - 1) / kWChunkRows;
+            k.nseg = warp ? (k.n_in + GS::vals - 1) / GS::vals : (k.n_in + G::vals - 1) / G::vals;
+            k.bytes = warp ? GS::bytes : G::bytes;
+            k.split = warp ? GS::split : 1;
+            k.pitch = warp ? GS::pitch : G::pitch;
+            k.rb = row_bytes(warp ? (int) MAYA_Q8_0 : T, k.n_in);
+            k.up = warp ? (size_t) A.n_ff_sh * k.rb : A.up_off;
+            k.off = warp ? 0 : A.row_off;
+        }
+    }
+    mbar_fence_init();
+    __syncthreads();
+    grid_dependency_wait();
+    if (A.skip != nullptr && *A.skip) return;
+
+    // ---- the jobs, by one warp
+    if (warp == 0) {
+        int ng = A.n_groups ? *A.n_groups : A.cap;
+        ng = min(min(ng, A.cap), kWMaxGroups);
+        int base = 0, run = 0;
+        const int nsh = SH && A.sh != nullptr ? (A.n_tok + A.ncm - 1) / A.ncm : 0;
+        const WKind &kr = sh.kind[0], &ks = sh.kind[1];
+        for (int g0 = 0; g0 < ng + nsh; g0 += 32) {              // a lane: one group, or one of the shared expert's jobs
+            const int g = g0 + lane;
+            WJob J{0ull, 0, 0, 0, 0};
+            int ne = 0;
+            if (g < ng) {
+                J.ptr = A.ptr[g];
+                J.e0 = A.start ? A.start[g] : g;
+                ne = (A.start ? A.start[g + 1] : g + 1) - J.e0;
+            } else if (g < ng + nsh) {
+                J.ptr = (unsigned long long) A.sh;
+                J.e0 = (g - ng) * A.ncm;
+                ne = min(A.ncm, A.n_tok - J.e0);
+                J.shared = 1;
+            }
+            const int nj = J.ptr != 0ull && ne > 0 ? (ne + A.ncm - 1) / A.ncm : 0;
+            auto job_of = [&](int j) {
+                WJob r = J;
+                r.e0 = J.e0 + j * A.ncm;
+                r.nc = min(A.ncm, ne - j * A.ncm);
+                r.per = J.shared ? GS::cost(r.nc, ks.n_in) : G::cost(r.nc, kr.n_in);
+                return r;
+            };
+            int mine = 0;
+            for (int j = 0; j < nj; ++j) mine += job_of(j).per * (J.shared ? ks.nchunk : kr.nchunk);
+            int incl = nj, cost = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o), w = __shfl_up_sync(0xffffffffu, cost, o);
+                if (lane >= o) { incl += v; cost += w; }
+            }
+            int at = base + incl - nj, before = run + cost - mine;
+            for (int j = 0; j < nj; ++j, ++at) {
+                const WJob r = job_of(j);
+                if (at < kWMaxJobs) { sh.job[at] = r; sh.cost[at] = before; }
+                before += r.per * (J.shared ? ks.nchunk : kr.nchunk);
+            }
+            base += __shfl_sync(0xffffffffu, incl, 31);
+            run += __shfl_sync(0xffffffffu, cost, 31);
+        }
+        if (lane == 0) { sh.njobs = min(base, kWMaxJobs); sh.cost[min(base, kWMaxJobs)] = run; }
+    }
+    __syncthreads();
+    const int njobs = sh.njobs;
+    // chunk c of job j starts at cost[j] + c * per; this block takes those that start in its share [x0, x1) of the whole
+    const long long total = sh.cost[njobs];
+    auto first_at = [&](long long at, int& j, int& c) {
+        j = 0;
+        while (j < njobs && sh.cost[j + 1] <= at) ++j;
+        c = 0;
+        if (j < njobs) {
+            const int per = sh.job[j].per;
+            c = (int) ((at - sh.cost[j] + per - 1) / per);
+            if (c * per >= sh.cost[j + 1] - sh.cost[j]) { ++j; c = 0; }
+        }
+    };
+    int job, chunk, job1, chunk1;
+    first_at((long long) blockIdx.x * total / gridDim.x, job, chunk);
+    first_at((long long) (blockIdx.x + 1) * total / gridDim.x, job1, chunk1);
+    if (job > job1 || (job == job1 && chunk >= chunk1)) return;
+
+    // row r of this warp in a chunk: gate rows, then the same up rows; or down rows (the last chunk's rows past the end are its
+    // last row again: read, and not written)
+    auto row_ptr = [&](unsigned long long blob, const WKind& k, int ch, int r) -> const uint8_t* {
+        constexpr int H = RW / 2;
+        const uint8_t* base = (const uint8_t*) blob + k.off;
+        if constexpr (UP) return base + (r / H) * k.up + (size_t) (ch * 32 + H * warp + r % H) * k.rb;
+        else return base + (size_t) min(ch * kWChunkRows + RW * warp + r, k.n_rows - 1) * k.rb;
+    };
+    // ---- the stream: what the warp asks for next - job, chunk, segment, and which of the segment's stages
+    int pj = job, pc = chunk, ps = 0, pq = 0, pstage = 0;
+    auto ask = [&] {
+        if (pj > job1 || (pj == job1 && pc >= chunk1)) return;
+        const WJob& J = sh.job[pj];
+        const WKind& k = sh.kind[SH ? J.shared : 0];
+        __syncwarp();                                            // every lane has read the stage's last bytes
+        const uint32_t at = (uint32_t) (ps * k.bytes), len = min((uint32_t) k.bytes, (uint32_t) k.rb - at);
+        const uint32_t dst = ring + pstage * kStage;
+        const int rows = SH ? RW / k.split : RW, first = SH ? pq * rows : 0;      // the stage's rows
+        if ((J.ptr & 15ull) == 0 && (!A.plain || (SH && J.shared))) {
+            if (lane < rows) {
+                const uint8_t* src = row_ptr(J.ptr, k, pc, first + lane) + at;
+                const uint32_t off = (uint32_t) (uintptr_t) src & 15u, bytes = (off + len + 15u) & ~15u;
+                fence_proxy_async();
+                mbar_expect_tx(&sh.full[warp][pstage], bytes);
+                bulk_load(s_raw + dst + lane * k.pitch, src - off, bytes, &sh.full[warp][pstage]);
+            } else if (SH && lane < RW) {
+                mbar_arrive_one(&sh.full[warp][pstage]);
+            }
+        } else {                                                 // ordinary loads, two bytes at a time
+            for (int r = 0; r < rows; ++r) {
+                const uint8_t* src = row_ptr(J.ptr, k, pc, first + r) + at;
+                const uint32_t off = (uint32_t) (uintptr_t) src & 15u;
+                for (uint32_t i = 2 * lane; i < len; i += 64) *(uint16_t*) (s_raw + dst + r * k.pitch + off + i) = *(const uint16_t*) (src + i);
+            }
+            __syncwarp();
+            if (lane < RW) mbar_arrive_one(&sh.full[warp][pstage]);
+        }
+        pstage = pstage + 1 == kWStages ? 0 : pstage + 1;
+        if (SH && ++pq < k.split) return;
+        pq = 0;
+        if (++ps == k.nseg) {
+            ps = 0;
+            if (++pc == k.nchunk) { pc = 0; ++pj; }
+        }
+    };
+    for (int s = 0; s < kWStages; ++s) ask();
+
+    const uint32_t* const tab = s_tab + (lane % D::rep) * ((T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1);
+    int cur = -1, stage = 0, buf = 0;
+    uint32_t phase = 0;
+    while (job < job1 || (job == job1 && chunk < chunk1)) {
+        const WJob& J = sh.job[job];
+        const bool shd = SH && J.shared;
+        const WKind& K = sh.kind[shd ? 1 : 0];
+        const int nc = J.nc, n_in = K.n_in;
+        auto slot_of = [&](int c) { return shd ? J.e0 + c : A.ent_slot ? A.ent_slot[J.e0 + c] : J.e0 + c; };     // shared: the token
+        if (job != cur) {                                        // the job's columns
+            __syncthreads();                                     // everyone is done with the old ones
+            for (int c = 0; c < nc; ++c) {
+                const int slot = slot_of(c);
+                const uint8_t* src;
+                if constexpr (UP) src = A.xq + (size_t) (shd ? slot : A.tok_from_slot ? slot >> 3 : 0) * A.xq_stride;
+                else src = shd ? A.sh_hq + (size_t) slot * (A.n_ff_sh / 32) * kQ81Bytes : A.xq + (size_t) slot * A.xq_stride;
+                for (int i = tid; i < n_in / 32; i += kWThreads) {
+                    if (SH && shd) col_store<1, CB, false>(src, cols, c, i);
+                    else col_store<Dec<T>::xblk, CB, T == MAYA_IQ1_S>(src, cols, c, i);
+                }
+            }
+            cur = job;
+            __syncthreads();
+        }
+        // where the warp's first row starts in its 16-byte window, and how far on the next rows do
+        const uint32_t p0 = (uint32_t) (uintptr_t) row_ptr(J.ptr, K, chunk, 0), rb16 = (uint32_t) K.rb & 15u;
+        auto row_at = [&](int r) -> uint32_t {
+            if constexpr (UP) return (p0 + (r / (RW / 2)) * (uint32_t) K.up + (r % (RW / 2)) * rb16) & 15u;
+            else return (p0 + (min(chunk * kWChunkRows + RW * warp + r, K.n_rows - 1) - min(chunk * kWChunkRows + RW * warp, K.n_rows - 1)) * rb16) & 15u;
+        };
+        const uint32_t r0_ = row_at(0), r1_ = row_at(1), r2_ = row_at(2), r3_ = row_at(3);
+        static_assert(RW == 4, "four rows a warp");
+        // a sum's row is its place in the reduction below: bits 4 and 3 of the lane
+        const int my_row = 2 * (lane >> 4) + ((lane >> 3) & 1);
+        auto chunk_dot = [&](auto type_c, auto geo, auto nc_c) {
+            constexpr int TY = decltype(type_c)::value, NC = decltype(nc_c)::value;
+            using GT = decltype(geo);
+            float acc[RW][NC];
+#pragma unroll
+            for (int r = 0; r < RW; ++r)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) acc[r][c] = 0.0f;
+            const uint32_t start[RW] = {r0_, r1_, r2_, r3_};
+            constexpr int RS = RW / GT::split;                   // rows of a stage
+            for (int sg = 0; sg < K.nseg; ++sg) {
+                const uint32_t so = (uint32_t) (sg * GT::bytes);            // (a row's segments can start anywhere, too)
+                const int blk0 = sg * GT::blocks, ncalls = min(GT::blocks, n_in / GT::qk - blk0) * GT::cpb;
+#pragma unroll
+                for (int p = 0; p < GT::split; ++p) {
+                    if (!*(volatile int*) &sh.fail && !mbar_wait(&sh.full[warp][stage], phase)) *(volatile int*) &sh.fail = 1;    // bounded
+                    uint32_t row[RS];
+#pragma unroll
+                    for (int r = 0; r < RS; ++r) row[r] = ring + stage * kStage + r * GT::pitch + ((start[p * RS + r] + so) & 15u);
+                    segment_dot<TY, GT, NC, RS, CB>(s_raw, row, cols, blk0, ncalls, lane, tab, *(float(*)[RS][NC]) &acc[p * RS]);
+                    stage = stage + 1 == kWStages ? 0 : stage + 1;
+                    if (stage == 0) phase ^= 1u;
+                    ask();
+                }
+            }
+            // warp_sum's tree (lanes 16 apart first, then 8, 4, 2, 1) on four rows at once: after the first exchange a lane keeps two
+            // of them, after the second one - six shuffles a column instead of twenty, the same additions
+            const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0, failed = *(volatile int*) &sh.fail != 0;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                float a = up16 ? acc[2][c] : acc[0][c], b = up16 ? acc[3][c] : acc[1][c];
+                a += __shfl_xor_sync(0xffffffffu, up16 ? acc[0][c] : acc[2][c], 16);
+                b += __shfl_xor_sync(0xffffffffu, up16 ? acc[1][c] : acc[3][c], 16);
+                float v = up8 ? b : a;
+                v += __shfl_xor_sync(0xffffffffu, up8 ? a : b, 8);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if ((lane & 7) == 0 && c < nc) {
+                    if constexpr (UP) {
+                        (my_row < 2 ? sh.s_g : sh.s_u)[buf][c][2 * warp + (my_row & 1)] = v;
+                    } else {
+                        const int row = chunk * kWChunkRows + RW * warp + my_row;
+                        if (row < K.n_rows && !failed) (shd ? A.sh_out : A.part)[(size_t) slot_of(c) * A.n_embd + row] = v;
+                    }
+                }
+            }
+        };
+        auto chunk_any = [&](auto type_c, auto geo) {
+            switch (nc) {
+                case 1: chunk_dot(type_c, geo, std::integral_constant<int, 1>{}); break;
+                case 2: chunk_dot(type_c, geo, std::integral_constant<int, 2>{}); break;
+                case 3: chunk_dot(type_c, geo, std::integral_constant<int, 3>{}); break;
+                case 4: chunk_dot(type_c, geo, std::integral_constant<int, 4>{}); break;
+                default:
+                    if constexpr (G::nc > 4) {
+                        if (nc <= 6) chunk_dot(type_c, geo, std::integral_constant<int, 6>{});
+                        else chunk_dot(type_c, geo, std::integral_constant<int, 8>{});
+                    }
+            }
+        };
+        if constexpr (SH) {
+            if (shd) chunk_any(std::integral_constant<int, MAYA_Q8_0>{}, GS{});
+            else chunk_any(std::integral_constant<int, T>{}, G{});
+        } else {
+            chunk_any(std::integral_constant<int, T>{}, G{});
+        }
+        if constexpr (UP) {
+            __syncthreads();                                     // two buffers: one barrier a chunk
+            if (warp < nc && !*(volatile int*) &sh.fail)
+                q8_1_store_warp(swiglu(sh.s_g[buf][warp][lane], sh.s_u[buf][warp][lane], A.limit),
+                                (shd ? A.sh_hq : A.hq) + ((size_t) slot_of(warp) * K.nchunk + chunk) * kQ81Bytes, lane);
+            buf ^= 1;
+        }
+        if (++chunk == K.nchunk) { chunk = 0; ++job; }
+    }
+    if (*(volatile int*) &sh.fail) {
+        // let what may still be in flight land (bounded as well) before the block's shared memory goes away
+        for (int s = 0; s < kWStages; ++s) mbar_wait(&sh.full[warp][s], phase ^ (uint32_t) (s < stage));
+        __syncthreads();
+    }
+}
+
+template<int T, bool SH, bool UP, int CB>
+int launch_window_cb(WArgs A, cudaStream_t s) {
+    using G = WGeo<T>;
+    constexpr int kStage = SH && WShGeo::stage > G::stage ? WShGeo::stage : G::stage, kRing = G::warps * kWStages * kStage;
+    // columns of a job: what fits beside the ring and the codebook, eight at most (a job's rows are decoded once for them all)
+    const long room = 232448l - (long) sizeof(WShared) - 256 - kRing - G::tab;
+    A.ncm = (int) (room / kColBytes<CB>);
+    if (A.ncm > G::nc) A.ncm = G::nc;
+    if (A.ncm == 5 || A.ncm == 7) --A.ncm;            // five columns are dotted as six, seven as eight: the room has to be there
+    if (A.ncm < 1) return kWindowTooWide;
+    A.plain = ((A.row_off | A.up_off | (size_t) (UP ? A.n_ff : A.n_embd) * row_bytes(T, UP ? A.n_embd : A.n_ff)) & 15) != 0;
+    const size_t smem = (size_t) kRing + G::tab + (size_t) A.ncm * kColBytes<CB>;
+    static std::atomic<size_t> set_for{0};            // per instantiation: the size the attribute was last raised to
+    static std::atomic<int> set_dev{-1};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (set_dev.load() != dev || set_for.load() < smem) {
+        if (cudaFuncSetAttribute(window_kernel<T, SH, UP, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
+            return note_launch("window smem attribute");
+        set_for.store(smem);
+        set_dev.store(dev);
+    }
+    const int sms = sm_count();
+    if (sms <= 0) return refuse(MAYA_ERR_DEVICE);
+    launch_dependent(window_kernel<T, SH, UP, CB>, dim3((unsigned) sms), dim3(G::threads), smem, s, A);
+    return note_launch(UP ? "window_gate_up" : "window_down");
+}
+
+// The smallest column capacity that holds the row.
+template<int T, bool SH, bool UP> int launch_window(const WArgs& A, cudaStream_t s) {
+    int n_in = UP ? A.n_embd : A.n_ff;
+    if (!UP && SH && A.n_ff_sh > n_in) n_in = A.n_ff_sh;
+    if (n_in <= 128 * 32) return launch_window_cb<T, SH, UP, 128>(A, s);
+    if (n_in <= 256 * 32) return launch_window_cb<T, SH, UP, 256>(A, s);
+    return kWindowTooWide;
+}
+
+}  // namespace
+
+// Instantiated in moe_window_{up,down}[_sh].cu, one translation unit each: they compile side by side.
+template<bool SH, bool UP> int launch_window_type(int type, const WArgs& A, cudaStream_t s) {
+#define MAYA_WIN(TT) case TT: return launch_window<TT, SH, UP>(A, s);
+    switch (type) {
+        MAYA_WIN(MAYA_Q8_0) MAYA_WIN(MAYA_Q4_K) MAYA_WIN(MAYA_IQ2_S) MAYA_WIN(MAYA_IQ3_S) MAYA_WIN(MAYA_Q5_K)
+        MAYA_WIN(MAYA_Q6_K) MAYA_WIN(MAYA_IQ4_XS) MAYA_WIN(MAYA_IQ3_XXS) MAYA_WIN(MAYA_IQ2_XXS) MAYA_WIN(MAYA_IQ1_S)
+        default: return refuse(MAYA_ERR_TYPE);
+    }
+#undef MAYA_WIN
+}
+
+}  // namespace maya

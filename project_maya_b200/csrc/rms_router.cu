@@ -55,10 +55,10 @@ __global__ void __launch_bounds__(kRmsThreads) rms_router_kernel(const float* __
     const size_t rb = (size_t) n * (BF16 ? 2 : 4);
     const int e0 = blockIdx.x * epb, ne = min(epb, n_expert - e0);
     // Programmatic dependent launch: nothing is read or written before the wait; a prefetch into L2 is neither.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    grid_launch_dependents();
     for (size_t b = (size_t) tid * 128; b < ne * rb; b += kRmsThreads * 128)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(router + (size_t) e0 * rb + b));
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    grid_dependency_wait();
 
     // the block's warps split evenly over its experts (epb divides kRmsWarps): expert e0 + warp / wpe, part warp % wpe
     const int wpe = kRmsWarps / epb, ex = e0 + warp / wpe, first = (warp % wpe) * 32 + lane, step = 32 * wpe;
@@ -165,17 +165,8 @@ int launch(const float* h, const float* add, const float* w, float eps, int n, c
     // chip (beyond 8 x 148 experts blocks share SMs)
     int epb = 1;
     while (epb < kRmsWarps && (n_expert + epb - 1) / epb > 148) epb *= 2;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned) ((n_expert + epb - 1) / epb));
-    cfg.blockDim = dim3(kRmsThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, rms_router_kernel<BF16, VEC>, h, add, w, eps, n, (const uint8_t*) router, n_expert, epb, h_out, x_out, logits);
+    launch_dependent(rms_router_kernel<BF16, VEC>, dim3((unsigned) ((n_expert + epb - 1) / epb)), dim3(kRmsThreads), smem, s, h, add, w, eps,
+                     n, (const uint8_t*) router, n_expert, epb, h_out, x_out, logits);
     return note_launch("rms_router");
 }
 

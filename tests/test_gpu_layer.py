@@ -253,6 +253,30 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
     assert H.rel_err(out.cpu().numpy()[0], want) <= TIGHT
 
 
+@pytest.mark.parametrize("t,n_embd,n_ff,n_ff_sh,n_expert,n_tok,sigmoid", [
+    (H.IQ2_S, 1024, 256, 512, 12, 2, False), (H.Q4_K, 1280, 768, 1312, 12, 9, False),      # the shared expert's jobs: one; three of 4, 4, 1
+    (H.Q8_0, 1056, 288, 4128, 300, 7, True), (H.IQ3_S, 4352, 512, 256, 600, 16, False)])   # rows beyond 4096 values; 2 and 4 experts a thread
+def test_window_with_shared_expert_equals_fused_tokens_bitwise(T, api, t, n_embd, n_ff, n_ff_sh, n_expert, n_tok, sigmoid):
+    """A window whose shared expert rides in the routed experts' launches, behind the one launch that routes, quantizes and
+    groups: every token has the fused single-token kernel's ids, weights and output, bit for bit."""
+    cfg = dict(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, k=5, gu_type=t, d_type=t, n_ff_sh=n_ff_sh, sh_gu_type=H.Q8_0, sh_d_type=H.Q8_0)
+    lc = layer_cfg(api, cfg)
+    lc.limit = 7.0
+    four = dev(T, np.stack([H.constructed_expert(t, t, n_embd, n_ff, H.rng_for("wsh", t, e)) for e in range(4)]))
+    experts = four[T.arange(n_expert, device="cuda") % 4].contiguous()
+    sh = dev(T, H.constructed_expert(H.Q8_0, H.Q8_0, n_embd, n_ff_sh, H.rng_for("wsh-shared", t)))
+    route = (dev(T, (0.1 * H.rng_for("wsh", t).standard_normal(n_expert)).astype(np.float32)), 2.5, True) if sigmoid else None
+    layer = api.MoeLayer(lc, experts, sh, expert_range=(1, n_expert), sigmoid=route)
+    logits = dev(T, H.router_logits("wsh", n_tok, n_expert, 1.1))
+    x = dev(T, H.activations("wsh", n_tok, n_embd, "bf16"), T.bfloat16)
+    for _ in range(2):                                                   # twice: the launches leave their counters as they found them
+        ids, w, out = layer.forward(logits, x)
+        for i in range(n_tok):
+            ids1, w1, out1 = layer.forward(logits[i:i + 1], x[i:i + 1])
+            assert T.equal(ids[i], ids1[0]) and T.equal(w[i], w1[0]) and T.equal(out[i], out1[0]), f"token {i}"
+    assert layer.error() == 0
+
+
 def test_fused_kernel_many_calls_one_scratch(T, api):
     """The grid barrier's counter lives in the scratch: hundreds of calls, single tokens and windows interleaved."""
     cfg = dict(n_embd=512, n_ff=256, n_expert=8, k=4, gu_type=H.Q4_K, d_type=H.Q4_K)
