@@ -5,17 +5,16 @@
 // 2-4 bit weight costs 60-90 instructions per 32 to decode and 14-38 per column to dot - so everything around them has to
 // be cheap and no warp may wait for its loads.  One 512-thread block an SM; its warps never meet inside a row:
 //   * the work is a list of jobs - a group (distinct expert) and up to `ncm` of its entries (activation columns) - times
-//     chunks of 64 weight rows (32 gate + the same 32 up rows, or 64 down rows).  Every block takes one contiguous share of
-//     that list, equal in estimated COST (decode + columns x dot), not in count: a chunk with eight columns costs several
-//     times one with a single column.  Contiguous, so that a block stages a job's columns once for all its chunks.
-//   * a warp owns four rows of a chunk and streams their K segments into a private ring with cp.async.bulk, two segments
-//     ahead, across chunk and job boundaries: no block barrier stands between a warp and its next bytes, and decoding reads
+//     units of weight rows.  Every block takes one contiguous share of that list, equal in measured COST, not in count: rows
+//     with eight columns cost several times those with one.  Contiguous, so that a block stages a job's columns once.
+//   * a warp works on four rows at a time and streams their K segments into a private ring with cp.async.bulk, two segments
+//     ahead, across unit and job boundaries: no block barrier stands between a warp and its next bytes, and decoding reads
 //     shared memory, where a lane's 2-byte aligned fields cost one or two wavefronts a warp instead of the four to five
 //     cache lines they touch in global memory.
 //   * the always-on shared expert, when it is Q8_0, is one more job list in the same launches - its rows against all the tokens -
 //     so that its 40 MB hide behind an instruction-bound phase instead of taking two GEMV launches and a SwiGLU launch a token.
 //   * codebooks lie in several copies side by side in shared memory, lane l reading copy l % n.
-// Read in place by a grid of (chunk, group) blocks (gate/up) and streamed 64 rows a stage (down), an 8-token Q4_K window took
+// Read in place by a grid of (rows, group) blocks (gate/up) and streamed 64 rows a stage (down), an 8-token Q4_K window took
 // 318 us, a 16-token IQ3_S one 570; now 263 and 433.  (32 warps of two rows: 266 and 484, the activation reads then bind.)
 //
 // The arithmetic is rows_dot's (maya_dots.cuh), value for value - the same integers, the same lane order, the same sums - so
@@ -43,8 +42,7 @@ constexpr int kWNC = 8;            // most activation columns of a job
 constexpr int kWStages = 2;        // segments in flight a warp
 constexpr int kWMaxGroups = 128;   // T <= 16 tokens x 8 routes
 constexpr int kWMaxJobs = kWMaxGroups + 16;      // a job has at least one entry; the shared expert's at least one token
-constexpr int kWChunkRows = 64;    // weight rows of a chunk
-constexpr int kChunkCost = 40;     // a chunk's own overhead, in the units of WGeo's costs
+constexpr int kWChunkRows = 64;    // weight rows of a block's step: 16 warps x 4
 
 // ---- decoders: Dec<T>'s fields and dot, loaded from shared memory - byte `o` of `s` is the block's first - with fewer
 //      instructions.  rep: copies of the codebook, `tab` = this lane's copy.  ONE: for a single column, where it is cheaper to
@@ -198,22 +196,30 @@ template<int T, int SPLIT = 1> struct WGeo {
     static constexpr int pitch = (bytes + 15 + 16) & ~15;
     static constexpr int stage = rw / SPLIT * pitch;                                 // a warp's stage
     static constexpr int tab = Fmt<T>::tab_words * 4 * WDec<T, false>::rep;
-    // The cost of 32 calls of a row against nc columns, in instructions: decoding, nc dots - or, where that is more, what their
-    // bytes cost at an SM's share of HBM; and a chunk's own overhead.
-    static constexpr int dec_cost = T == MAYA_Q8_0 ? 25 : T == MAYA_Q4_K || T == MAYA_IQ1_S ? 45 : T == MAYA_Q5_K ? 60 : T == MAYA_IQ3_S || T == MAYA_IQ3_XXS ? 90 : 75;
-    static constexpr int col_cost = Dec<T>::xblk == 2 ? 40 : 15;
-    static constexpr int byte_cost = 32 / cpb * Fmt<T>::bytes / 8;
-    __device__ __forceinline__ static int cost(int nc, int n_in) { return max(dec_cost + nc * col_cost, byte_cost) * ((n_in / qk * cpb + 31) / 32) + kChunkCost; }
+    // What a warp's four rows cost against nc columns, in units of 30 cycles, fitted to clock stamps of 16-token windows: per 32
+    // calls of a row the decoding (for Q8_0: waiting for its bytes) and every column's dot, and every column's sums at the end.
+    // A share that is off by a tenth is a tenth of the launch: with costs counted in instructions instead the slowest of 148
+    // blocks took 27 % longer than the mean.
+    static constexpr int dec_cost = T == MAYA_Q8_0 ? (SPLIT > 1 ? 129 : 72) : T == MAYA_Q4_K ? 92 : T == MAYA_Q5_K ? 125 : T == MAYA_Q6_K ? 115
+                                    : T == MAYA_IQ4_XS ? 92 : T == MAYA_IQ2_XXS ? 70 : T == MAYA_IQ1_S ? 58 : 77;
+    static constexpr int col_cost = Dec<T>::xblk == 2 ? 24 : T == MAYA_IQ2_S || T == MAYA_Q6_K || T == MAYA_IQ3_XXS || T == MAYA_IQ2_XXS ? 11 : 8;
+    static constexpr int sum_cost = 21, glu_cost = 40;       // a column's sums; gate/up: a unit's SwiGLU and barrier
+    static constexpr int job_cost = 350;                     // a block's change of job: its columns, and code it has not run
+    __device__ __forceinline__ static int cost(int nc, int n_in) {
+        if (nc > 4) nc = (nc + 1) & ~1;          // dotted as six, as eight
+        const int spilled = T == MAYA_IQ2_S && nc == 8 ? 60 : 0;
+        return (dec_cost + nc * col_cost + spilled) * ((n_in / qk * cpb + 31) / 32) + nc * sum_cost;
+    }
 };
 using WShGeo = WGeo<MAYA_Q8_0, 2>;           // the shared expert's rows: a stage no larger than the 2-bit types'
 
 // what differs between the routed experts' jobs and the shared one's
-struct WKind { int n_in, n_rows, nchunk, nseg, bytes, pitch, split; size_t rb, up, off; };
-struct WJob { unsigned long long ptr; int e0, nc, shared, per; };     // per: cost of one chunk
+struct WKind { int n_in, nunit, nseg, bytes, pitch, split; size_t rb, up, off; };
+struct WJob { unsigned long long ptr; int e0, nc, shared, per; };     // per: cost of one unit
 struct WShared {
     uint64_t full[16][kWStages];
     WJob job[kWMaxJobs];
-    int cost[kWMaxJobs + 1];         // cost of the jobs before job j
+    long long cost[kWMaxJobs + 1];   // cost of the jobs before job j
     int njobs, fail;
     float s_g[2][kWNC][32], s_u[2][kWNC][32];
     WKind kind[2];
@@ -234,13 +240,16 @@ template<int XB, int CB> __device__ __forceinline__ XQ col_load(const uint8_t* c
     v.isum = *(const int*) (cols + c * kColBytes<CB> + CB * 36 + j * P * 4 + i4);
     return v;
 }
-// Block i of a column, a thread's: nine words in flight (word by word the columns of a job took 8 us to stage).
-template<int XB, int CB, bool SUM_F16> __device__ __forceinline__ void col_store(const uint8_t* xq, uint8_t* cols, int c, int i) {
-    constexpr int P = CB / XB;
+// Block i of a column: its nine words are a thread's loads.
+struct ColBlock { uint32_t w[9]; };
+__device__ __forceinline__ void col_read(const uint8_t* xq, int i, ColBlock& v) {
     const uint32_t* src = (const uint32_t*) (xq + (size_t) i * kQ81Bytes);
-    uint32_t w[9];
 #pragma unroll
-    for (int j = 0; j < 9; ++j) w[j] = src[j];
+    for (int j = 0; j < 9; ++j) v.w[j] = src[j];
+}
+template<int XB, int CB, bool SUM_F16> __device__ __forceinline__ void col_store(const ColBlock& v, uint8_t* cols, int c, int i) {
+    constexpr int P = CB / XB;
+    const uint32_t* w = v.w;
     uint8_t* col = cols + c * kColBytes<CB>;
     const int j = i % XB, n = i / XB;
     *(int4*) (col + (2 * j * P + n) * 16) = make_int4((int) w[1], (int) w[2], (int) w[3], (int) w[4]);
@@ -284,7 +293,9 @@ __device__ __forceinline__ void segment_dot(const uint8_t* s, const uint32_t (&r
     }
 }
 
-// UP: gate/up (chunk = 32 FFN rows: a warp's rows are 2 gate + 2 up); else down (chunk = 64 rows).  SH: with a Q8_0 shared expert.
+// UP: gate/up - a unit of work is a block's: 32 FFN rows (one q8_1 block of h), two of them a warp with their gate and up rows.
+// Else down - a unit is a warp's: four rows.  (Blocks' shares in units of 64 rows ended up to one such step apart.)
+// SH: with a Q8_0 shared expert.
 template<int T, bool SH, bool UP, int CB>
 __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs A) {
     using G = WGeo<T>;
@@ -300,14 +311,6 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     uint8_t* const cols = s_raw + kRing + G::tab;
 
     grid_launch_dependents();
-    if constexpr (G::tab > 0) {                                  // the codebook's copies: constants of the library
-        constexpr int W = (T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1, R = D::rep;
-        const uint32_t* src = tab_source<T>();
-        for (int i = tid; i < G::tab / 4; i += kWThreads) {
-            const uint32_t g = src[i / (W * R) * W + i % W];
-            s_tab[i] = T == MAYA_IQ3_S ? (g >> 1) & 0x07070707u : g;
-        }
-    }
     if (lane == 0) {
         for (int s = 0; s < kWStages; ++s) mbar_init(&sh.full[warp][s], RW);
         if (warp == 0) sh.fail = 0;
@@ -315,8 +318,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             WKind& k = sh.kind[warp];
             const int ff = warp ? A.n_ff_sh : A.n_ff;
             k.n_in = UP ? A.n_embd : ff;
-            k.n_rows = UP ? ff : A.n_embd;
-            k.nchunk = UP ? ff / 32 : (A.n_embd + kWChunkRows - 1) / kWChunkRows;
+            k.nunit = UP ? ff / 32 : A.n_embd / RW;
             k.nseg = warp ? (k.n_in + GS::vals - 1) / GS::vals : (k.n_in + G::vals - 1) / G::vals;
             k.bytes = warp ? GS::bytes : G::bytes;
             k.split = warp ? GS::split : 1;
@@ -331,11 +333,31 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     grid_dependency_wait();
     if (A.skip != nullptr && *A.skip) return;
 
-    // ---- the jobs, by one warp
-    if (warp == 0) {
+    // ---- the jobs, by one warp; the codebook's copies, by the others
+    if (warp > 0) {
+        if constexpr (G::tab > 0) {
+            constexpr int W = (T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1, R = D::rep, NT = kWThreads - 32;
+            const uint32_t* src = tab_source<T>();
+#pragma unroll 4
+            for (int e = tid - 32; e < G::tab / 4 / R; e += NT) {                // a codebook word, and its copies: R / 4 16-byte stores
+                uint32_t g = src[e];
+                if constexpr (T == MAYA_IQ3_S) g = (g >> 1) & 0x07070707u;
+                if constexpr (W == 1) {
+#pragma unroll
+                    for (int r = 0; r < R; r += 4)
+                        if constexpr (R >= 4) ((uint4*) s_tab)[e * (R / 4) + r / 4] = make_uint4(g, g, g, g);
+                        else s_tab[e] = g;
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) s_tab[((e / 2) * R + r) * 2 + (e & 1)] = g;
+                }
+            }
+        }
+    } else {
         int ng = A.n_groups ? *A.n_groups : A.cap;
         ng = min(min(ng, A.cap), kWMaxGroups);
-        int base = 0, run = 0;
+        int base = 0;
+        long long run = 0;
         const int nsh = SH && A.sh != nullptr ? (A.n_tok + A.ncm - 1) / A.ncm : 0;
         const WKind &kr = sh.kind[0], &ks = sh.kind[1];
         for (int g0 = 0; g0 < ng + nsh; g0 += 32) {              // a lane: one group, or one of the shared expert's jobs
@@ -357,22 +379,26 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                 WJob r = J;
                 r.e0 = J.e0 + j * A.ncm;
                 r.nc = min(A.ncm, ne - j * A.ncm);
-                r.per = J.shared ? GS::cost(r.nc, ks.n_in) : G::cost(r.nc, kr.n_in);
+                r.per = (J.shared ? GS::cost(r.nc, ks.n_in) : G::cost(r.nc, kr.n_in)) + (UP ? G::glu_cost : 0);
                 return r;
             };
-            int mine = 0;
-            for (int j = 0; j < nj; ++j) mine += job_of(j).per * (J.shared ? ks.nchunk : kr.nchunk);
-            int incl = nj, cost = mine;
+            constexpr int kStart = G::job_cost * (UP ? 1 : G::warps);        // (down: in units of a warp's work)
+            long long mine = 0;
+            for (int j = 0; j < nj; ++j) mine += kStart + (long long) job_of(j).per * (J.shared ? ks.nunit : kr.nunit);
+            int incl = nj;
+            long long cost = mine;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o), w = __shfl_up_sync(0xffffffffu, cost, o);
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                const long long w = __shfl_up_sync(0xffffffffu, cost, o);
                 if (lane >= o) { incl += v; cost += w; }
             }
-            int at = base + incl - nj, before = run + cost - mine;
+            int at = base + incl - nj;
+            long long before = run + cost - mine;
             for (int j = 0; j < nj; ++j, ++at) {
                 const WJob r = job_of(j);
                 if (at < kWMaxJobs) { sh.job[at] = r; sh.cost[at] = before; }
-                before += r.per * (J.shared ? ks.nchunk : kr.nchunk);
+                before += kStart + (long long) r.per * (J.shared ? ks.nunit : kr.nunit);
             }
             base += __shfl_sync(0xffffffffu, incl, 31);
             run += __shfl_sync(0xffffffffu, cost, 31);
@@ -381,7 +407,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     }
     __syncthreads();
     const int njobs = sh.njobs;
-    // chunk c of job j starts at cost[j] + c * per; this block takes those that start in its share [x0, x1) of the whole
+    // unit c of job j starts at cost[j] + job_cost + c * per; this block takes those that start in its share of the whole
     const long long total = sh.cost[njobs];
     auto first_at = [&](long long at, int& j, int& c) {
         j = 0;
@@ -389,27 +415,31 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         c = 0;
         if (j < njobs) {
             const int per = sh.job[j].per;
-            c = (int) ((at - sh.cost[j] + per - 1) / per);
-            if (c * per >= sh.cost[j + 1] - sh.cost[j]) { ++j; c = 0; }
+            const long long in = at - sh.cost[j] - G::job_cost * (UP ? 1 : G::warps);
+            c = in > 0 ? (int) ((in + per - 1) / per) : 0;
+            if (c >= sh.kind[SH ? sh.job[j].shared : 0].nunit) { ++j; c = 0; }
         }
     };
-    int job, chunk, job1, chunk1;
-    first_at((long long) blockIdx.x * total / gridDim.x, job, chunk);
-    first_at((long long) (blockIdx.x + 1) * total / gridDim.x, job1, chunk1);
-    if (job > job1 || (job == job1 && chunk >= chunk1)) return;
+    int job, unit0, job1, unit1;
+    first_at((long long) blockIdx.x * total / gridDim.x, job, unit0);
+    first_at((long long) (blockIdx.x + 1) * total / gridDim.x, job1, unit1);
+    if (job > job1 || (job == job1 && unit0 >= unit1)) return;
+    constexpr int kStep = UP ? 1 : G::warps;                     // a warp's next unit
+    const int off = UP ? 0 : warp;
+    auto limit_of = [&](int j) { return j == job1 ? unit1 : sh.kind[SH ? sh.job[j].shared : 0].nunit; };     // j <= job1, j < njobs
 
-    // row r of this warp in a chunk: gate rows, then the same up rows; or down rows (the last chunk's rows past the end are its
-    // last row again: read, and not written)
-    auto row_ptr = [&](unsigned long long blob, const WKind& k, int ch, int r) -> const uint8_t* {
+    // row r of this warp in a unit: gate rows, then the same up rows; or down rows
+    auto row_ptr = [&](unsigned long long blob, const WKind& k, int unit, int r) -> const uint8_t* {
         constexpr int H = RW / 2;
         const uint8_t* base = (const uint8_t*) blob + k.off;
-        if constexpr (UP) return base + (r / H) * k.up + (size_t) (ch * 32 + H * warp + r % H) * k.rb;
-        else return base + (size_t) min(ch * kWChunkRows + RW * warp + r, k.n_rows - 1) * k.rb;
+        if constexpr (UP) return base + (r / H) * k.up + (size_t) (unit * 32 + H * warp + r % H) * k.rb;
+        else return base + (size_t) (RW * unit + r) * k.rb;
     };
-    // ---- the stream: what the warp asks for next - job, chunk, segment, and which of the segment's stages
-    int pj = job, pc = chunk, ps = 0, pq = 0, pstage = 0;
+    // ---- the stream: what the warp asks for next - job, unit, segment, and which of the segment's stages
+    int pj = job, pc = unit0 + off, ps = 0, pq = 0, pstage = 0;
     auto ask = [&] {
-        if (pj > job1 || (pj == job1 && pc >= chunk1)) return;
+        while (pj < njobs && pj <= job1 && pc >= limit_of(pj)) { ++pj; pc = off; }
+        if (pj >= njobs || pj > job1) return;
         const WJob& J = sh.job[pj];
         const WKind& k = sh.kind[SH ? J.shared : 0];
         __syncwarp();                                            // every lane has read the stage's last bytes
@@ -440,46 +470,56 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         pq = 0;
         if (++ps == k.nseg) {
             ps = 0;
-            if (++pc == k.nchunk) { pc = 0; ++pj; }
+            pc += kStep;
         }
     };
     for (int s = 0; s < kWStages; ++s) ask();
 
     const uint32_t* const tab = s_tab + (lane % D::rep) * ((T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1);
-    int cur = -1, stage = 0, buf = 0;
+    int stage = 0, buf = 0;
     uint32_t phase = 0;
-    while (job < job1 || (job == job1 && chunk < chunk1)) {
+    for (int first_unit = unit0; job <= job1 && job < njobs; ++job, first_unit = 0) {
+        const int limit = limit_of(job);
+        if (first_unit >= limit) continue;
         const WJob& J = sh.job[job];
         const bool shd = SH && J.shared;
         const WKind& K = sh.kind[shd ? 1 : 0];
         const int nc = J.nc, n_in = K.n_in;
         auto slot_of = [&](int c) { return shd ? J.e0 + c : A.ent_slot ? A.ent_slot[J.e0 + c] : J.e0 + c; };     // shared: the token
-        if (job != cur) {                                        // the job's columns
-            __syncthreads();                                     // everyone is done with the old ones
-            for (int c = 0; c < nc; ++c) {
-                const int slot = slot_of(c);
-                const uint8_t* src;
-                if constexpr (UP) src = A.xq + (size_t) (shd ? slot : A.tok_from_slot ? slot >> 3 : 0) * A.xq_stride;
-                else src = shd ? A.sh_hq + (size_t) slot * (A.n_ff_sh / 32) * kQ81Bytes : A.xq + (size_t) slot * A.xq_stride;
-                for (int i = tid; i < n_in / 32; i += kWThreads) {
-                    if (SH && shd) col_store<1, CB, false>(src, cols, c, i);
-                    else col_store<Dec<T>::xblk, CB, T == MAYA_IQ1_S>(src, cols, c, i);
+        __syncthreads();                                         // everyone is done with the old columns
+        {
+            const int nblk = n_in / 32, items = nc * nblk;
+            for (int i0 = tid; i0 < items; i0 += 2 * kWThreads) {                // two q8_1 blocks a thread in flight
+                ColBlock v[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int i = i0 + u * kWThreads;
+                    if (i >= items) continue;
+                    const int c = i / nblk, slot = slot_of(c);
+                    const uint8_t* src;
+                    if constexpr (UP) src = A.xq + (size_t) (shd ? slot : A.tok_from_slot ? slot >> 3 : 0) * A.xq_stride;
+                    else src = shd ? A.sh_hq + (size_t) slot * nblk * kQ81Bytes : A.xq + (size_t) slot * A.xq_stride;
+                    col_read(src, i - c * nblk, v[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int i = i0 + u * kWThreads;
+                    if (i >= items) continue;
+                    const int c = i / nblk;
+                    if (SH && shd) col_store<1, CB, false>(v[u], cols, c, i - c * nblk);
+                    else col_store<Dec<T>::xblk, CB, T == MAYA_IQ1_S>(v[u], cols, c, i - c * nblk);
                 }
             }
-            cur = job;
-            __syncthreads();
         }
-        // where the warp's first row starts in its 16-byte window, and how far on the next rows do
-        const uint32_t p0 = (uint32_t) (uintptr_t) row_ptr(J.ptr, K, chunk, 0), rb16 = (uint32_t) K.rb & 15u;
-        auto row_at = [&](int r) -> uint32_t {
-            if constexpr (UP) return (p0 + (r / (RW / 2)) * (uint32_t) K.up + (r % (RW / 2)) * rb16) & 15u;
-            else return (p0 + (min(chunk * kWChunkRows + RW * warp + r, K.n_rows - 1) - min(chunk * kWChunkRows + RW * warp, K.n_rows - 1)) * rb16) & 15u;
-        };
-        const uint32_t r0_ = row_at(0), r1_ = row_at(1), r2_ = row_at(2), r3_ = row_at(3);
+        __syncthreads();
+        for (int unit = first_unit + off; unit < limit; unit += kStep) {
+        // where the warp's rows start in their 16-byte windows
+        const uint32_t p0 = (uint32_t) (uintptr_t) row_ptr(J.ptr, K, unit, 0), rb16 = (uint32_t) K.rb & 15u, up16b = (uint32_t) K.up & 15u;
+        const uint32_t start[RW] = {p0, p0 + rb16, UP ? p0 + up16b : p0 + 2 * rb16, UP ? p0 + up16b + rb16 : p0 + 3 * rb16};
         static_assert(RW == 4, "four rows a warp");
         // a sum's row is its place in the reduction below: bits 4 and 3 of the lane
         const int my_row = 2 * (lane >> 4) + ((lane >> 3) & 1);
-        auto chunk_dot = [&](auto type_c, auto geo, auto nc_c) {
+        auto unit_dot = [&](auto type_c, auto geo, auto nc_c) {
             constexpr int TY = decltype(type_c)::value, NC = decltype(nc_c)::value;
             using GT = decltype(geo);
             float acc[RW][NC];
@@ -487,7 +527,6 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             for (int r = 0; r < RW; ++r)
 #pragma unroll
                 for (int c = 0; c < NC; ++c) acc[r][c] = 0.0f;
-            const uint32_t start[RW] = {r0_, r1_, r2_, r3_};
             constexpr int RS = RW / GT::split;                   // rows of a stage
             for (int sg = 0; sg < K.nseg; ++sg) {
                 const uint32_t so = (uint32_t) (sg * GT::bytes);            // (a row's segments can start anywhere, too)
@@ -520,39 +559,38 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                     if constexpr (UP) {
                         (my_row < 2 ? sh.s_g : sh.s_u)[buf][c][2 * warp + (my_row & 1)] = v;
                     } else {
-                        const int row = chunk * kWChunkRows + RW * warp + my_row;
-                        if (row < K.n_rows && !failed) (shd ? A.sh_out : A.part)[(size_t) slot_of(c) * A.n_embd + row] = v;
+                        if (!failed) (shd ? A.sh_out : A.part)[(size_t) slot_of(c) * A.n_embd + RW * unit + my_row] = v;
                     }
                 }
             }
         };
-        auto chunk_any = [&](auto type_c, auto geo) {
+        auto unit_any = [&](auto type_c, auto geo) {
             switch (nc) {
-                case 1: chunk_dot(type_c, geo, std::integral_constant<int, 1>{}); break;
-                case 2: chunk_dot(type_c, geo, std::integral_constant<int, 2>{}); break;
-                case 3: chunk_dot(type_c, geo, std::integral_constant<int, 3>{}); break;
-                case 4: chunk_dot(type_c, geo, std::integral_constant<int, 4>{}); break;
+                case 1: unit_dot(type_c, geo, std::integral_constant<int, 1>{}); break;
+                case 2: unit_dot(type_c, geo, std::integral_constant<int, 2>{}); break;
+                case 3: unit_dot(type_c, geo, std::integral_constant<int, 3>{}); break;
+                case 4: unit_dot(type_c, geo, std::integral_constant<int, 4>{}); break;
                 default:
                     if constexpr (G::nc > 4) {
-                        if (nc <= 6) chunk_dot(type_c, geo, std::integral_constant<int, 6>{});
-                        else chunk_dot(type_c, geo, std::integral_constant<int, 8>{});
+                        if (nc <= 6) unit_dot(type_c, geo, std::integral_constant<int, 6>{});
+                        else unit_dot(type_c, geo, std::integral_constant<int, 8>{});
                     }
             }
         };
         if constexpr (SH) {
-            if (shd) chunk_any(std::integral_constant<int, MAYA_Q8_0>{}, GS{});
-            else chunk_any(std::integral_constant<int, T>{}, G{});
+            if (shd) unit_any(std::integral_constant<int, MAYA_Q8_0>{}, GS{});
+            else unit_any(std::integral_constant<int, T>{}, G{});
         } else {
-            chunk_any(std::integral_constant<int, T>{}, G{});
+            unit_any(std::integral_constant<int, T>{}, G{});
         }
         if constexpr (UP) {
-            __syncthreads();                                     // two buffers: one barrier a chunk
+            __syncthreads();                                     // two buffers: one barrier a unit
             if (warp < nc && !*(volatile int*) &sh.fail)
                 q8_1_store_warp(swiglu(sh.s_g[buf][warp][lane], sh.s_u[buf][warp][lane], A.limit),
-                                (shd ? A.sh_hq : A.hq) + ((size_t) slot_of(warp) * K.nchunk + chunk) * kQ81Bytes, lane);
+                                (shd ? A.sh_hq : A.hq) + ((size_t) slot_of(warp) * K.nunit + unit) * kQ81Bytes, lane);
             buf ^= 1;
         }
-        if (++chunk == K.nchunk) { chunk = 0; ++job; }
+        }
     }
     if (*(volatile int*) &sh.fail) {
         // let what may still be in flight land (bounded as well) before the block's shared memory goes away
