@@ -275,6 +275,16 @@ MAYA_API int maya_mmq_run(const maya_mmq_product* p, void* stream);
  * bit for bit to maya_mmq_run followed by maya_swiglu_rows.  n_ff % 128 == 0. */
 MAYA_API int maya_mmq_run_glu(const maya_mmq_product* p, float limit, void* stream);
 
+/* No counterpart in the reference: n_pairs maya_mmq_run_glu(gate_up[i], limit) and n_pairs maya_mmq_run(down[i]) in one go, the
+ * same bits.  down[i] multiplies the h that gate_up[i] leaves in its xq_out (down[i].xq == gate_up[i].xq_out; the same n, bounds,
+ * expert_map and total_rows), and its blocks start as soon as SMs have no gate/up tile left, each tile waiting only for its own
+ * rows of h (bounded: see `error`), so that the last, partly filled round of tiles of one product runs beside the next.
+ * counters: maya_mmq_chain_bytes(total_rows, matrices of all pairs, n_pairs) bytes, zeroed before the first use (and after an
+ * error); a chain leaves them zero.  One buffer serves one stream at a time. */
+MAYA_API size_t maya_mmq_chain_bytes(int64_t total_rows, int n_matrices, int n_pairs);
+MAYA_API int maya_mmq_run_chain(const maya_mmq_product* gate_up, const maya_mmq_product* down, int n_pairs, float limit,
+                                void* counters, size_t counter_bytes, void* stream);
+
 /* The producer in front of the layer: glmf::rms_q8 (glm_fast.hpp:534: h += add; x = rms(h) * norm_w, eps inside the
  * square root) and the router job of the GEMV batch Glm5Model::fast_moe issues next (glm_fast_path.cu:6925:
  * logits = router_w . x, router_w [n_expert][n_embd] F32 or BF16 bits) in ONE launch, so that a decode layer is this call

@@ -111,6 +111,8 @@ _SIGNATURES = {
     "maya_mmq_quantize_routed_bf16": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int64, c_int64, c_int64, c_void_p]),
     "maya_mmq_run": (c_int, [C.POINTER(MmqProduct), c_void_p]),
     "maya_mmq_run_glu": (c_int, [C.POINTER(MmqProduct), c_float, c_void_p]),
+    "maya_mmq_chain_bytes": (c_size_t, [c_int64, c_int, c_int]),
+    "maya_mmq_run_chain": (c_int, [C.POINTER(MmqProduct), C.POINTER(MmqProduct), c_int, c_float, c_void_p, c_size_t, c_void_p]),
     "maya_moe_combine_rows_local": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int,
                                             c_void_p, c_void_p]),
     "maya_moe_combine_rows_local_ar": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int,

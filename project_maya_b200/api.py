@@ -298,6 +298,17 @@ def mmq_run_glu(p: MmqProduct, limit: float = INF, stream=None) -> None:
     _check("mmq_run_glu", _lib.load().maya_mmq_run_glu(C.byref(p), limit, _stream(stream)))
 
 
+def mmq_run_chain(gate_up, down, limit: float, counters, stream=None) -> None:
+    """No counterpart in the reference: mmq_run_glu of every gate_up product, then mmq_run of every down product (down[i] on
+    gate_up[i].xq_out), overlapped where one product's last tiles leave SMs idle.  counters: uint8, zeroed once,
+    maya_mmq_chain_bytes long."""
+    n = len(gate_up)
+    if n == 0:
+        return
+    _check("mmq_run_chain", _lib.load().maya_mmq_run_chain((MmqProduct * n)(*gate_up), (MmqProduct * n)(*down), n, limit,
+                                                           _ptr(counters), counters.numel(), _stream(stream)))
+
+
 # ---------------------------------------------------------------- whole layer
 @dataclass
 class MoeLayerConfig:
@@ -497,6 +508,8 @@ class MoePrefill:
         self.hq = torch.empty(mmq_q8_bytes(n, FF), **u8)
         self.out, self.ffn = torch.empty((n, H), **f32), torch.empty((T, H), **f32)
         self.err = torch.zeros(1, dtype=torch.int32, device=dev)
+        chain_bytes = _lib.load().maya_mmq_chain_bytes
+        self.chain = torch.zeros(chain_bytes(n, sum(p[5] for p in self.pools) + 1, len(self.pools) + 1), **u8)      # + the shared expert
         if shared is not None:
             FS = cfg.n_ff_sh
             self.sh_bounds, self._sh_T = torch.zeros(2, **i32), -1
@@ -523,27 +536,23 @@ class MoePrefill:
         qtype = self.pools[0][0] if self.pools else cfg.gu_type
         # each token rounded once, its image stored to its k sorted rows (the bytes quant(x, row_tok, ...) would write)
         _check("mmq_quantize_routed", quant_routed(_ptr(x), _ptr(self.pos), k, _ptr(self.xq), qtype, H, x.stride(0), T, s))
-        for gt, dt, blobs, stride, down_off, n_p, emap in self.pools:
-            gu = mmq_product(blobs, gt, 2 * FF, H, stride, n_p, self.xq, self.bounds, None, n, None, FF, expert_map=emap,
-                             error=self.err, xq_out=self.hq)        # h leaves the product already quantized
-            _check("mmq_run_glu", lib.maya_mmq_run_glu(C.byref(gu), cfg.limit, s))
-        for gt, dt, blobs, stride, down_off, n_p, emap in self.pools:
-            dn = mmq_product(blobs.data_ptr() + down_off, dt, H, FF, stride, n_p, self.hq, self.bounds, None, n, self.out, H,
-                             expert_map=emap, error=self.err)
-            _check("mmq_run", lib.maya_mmq_run(C.byref(dn), s))
+        # h leaves the gate/up products already quantized
+        gu = [mmq_product(blobs, gt, 2 * FF, H, stride, n_p, self.xq, self.bounds, None, n, None, FF, expert_map=emap,
+                          error=self.err, xq_out=self.hq) for gt, dt, blobs, stride, down_off, n_p, emap in self.pools]
+        dn = [mmq_product(blobs.data_ptr() + down_off, dt, H, FF, stride, n_p, self.hq, self.bounds, None, n, self.out, H,
+                          expert_map=emap, error=self.err) for gt, dt, blobs, stride, down_off, n_p, emap in self.pools]
         sh_out = None
-        if self.shared is not None:
+        if self.shared is not None:  # one more pair of products, in the same chain
             FS = cfg.n_ff_sh
             if self._sh_T != T:      # the shared expert is one more "expert" that owns every row
                 self.sh_bounds[1], self._sh_T = T, T
             _check("mmq_quantize", quant(_ptr(x), None, _ptr(self.sh_xq), cfg.sh_gu_type, H, x.stride(0), T, s))
-            sgu = mmq_product(self.shared, cfg.sh_gu_type, 2 * FS, H, cfg.shared_bytes, 1, self.sh_xq, self.sh_bounds, None, T,
-                              None, FS, error=self.err, xq_out=self.sh_hq)
-            _check("mmq_run_glu", lib.maya_mmq_run_glu(C.byref(sgu), cfg.limit, s))
-            sdn = mmq_product(self.shared.data_ptr() + self.sh_down_off, cfg.sh_d_type, H, FS, cfg.shared_bytes, 1, self.sh_hq,
-                              self.sh_bounds, None, T, self.sh_out, H, error=self.err)
-            _check("mmq_run", lib.maya_mmq_run(C.byref(sdn), s))
+            gu.append(mmq_product(self.shared, cfg.sh_gu_type, 2 * FS, H, cfg.shared_bytes, 1, self.sh_xq, self.sh_bounds, None, T,
+                                  None, FS, error=self.err, xq_out=self.sh_hq))
+            dn.append(mmq_product(self.shared.data_ptr() + self.sh_down_off, cfg.sh_d_type, H, FS, cfg.shared_bytes, 1, self.sh_hq,
+                                  self.sh_bounds, None, T, self.sh_out, H, error=self.err))
             sh_out = self.sh_out
+        mmq_run_chain(gu, dn, cfg.limit, self.chain, s)
         ffn = self.ffn[:T]
         if self.expert_range is None:
             _check("moe_combine_rows", lib.maya_moe_combine_rows(_ptr(self.out), _ptr(self.pos), _ptr(w), _ptr(sh_out), T, k, H,

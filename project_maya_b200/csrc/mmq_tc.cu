@@ -24,7 +24,7 @@
 //               memory), one commit per two steps -> the steps' buffers are free (the warp cannot issue products as fast as
 //               the tensor core retires them unless their operands stay in uniform registers: see there);
 //   warps 0..15 afterwards: the epilogue - tcgen05.ld (lane = weight row, column = activation row), SwiGLU, optional
-//               q8_1 rounding of h for the next product, then through shared memory: one bulk copy per activation row.
+//               q8_1 rounding of h for the next product; f32 results leave through shared memory, one bulk copy per activation row.
 // Which expert and which 160-row group of it a block handles is found on the device from `bounds`; no count travels
 // to the host.  Every mbarrier wait is bounded: a wait that runs out sets the error word, the roles stop, copies in
 // flight are waited for (bounded), tensor memory is freed and the block returns.
@@ -107,6 +107,12 @@ struct MmqArgs {
     __half* xq_out;              // fused form, optional: q8_1-rounded h as f16, [sorted row][w_rows]
     float limit;
     unsigned* error;             // optional sticky error word
+    // In a chain of products (maya_mmq_run_chain), else NULL.  claim: [0] the next tile to be taken, [1] blocks that found none
+    // left.  ready: per group of rows [0] how often one of its h rows has left a gate/up tile, [1] down tiles that have waited for
+    // it; the down product of the group starts when [0] reaches its rows times ready_slabs.  All zero between chains.
+    unsigned* claim;
+    unsigned* ready;
+    int ready_slabs;             // down: gate/up tiles of a group; gate/up: unused
 };
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *(uint32_t*) &h; }
@@ -303,7 +309,7 @@ template<int J> __device__ __forceinline__ void iq_finish(const IqFields<MAYA_IQ
 }
 
 // A block works on tile after tile (see mmq_kernel): what the roles share of one of them.  e < 0: no tile left.
-struct TileInfo { int e, row0, nrows, m0; };
+struct TileInfo { int e, row0, nrows, m0, lin; };     // lin: its place in the list
 constexpr int kTiles = 8;            // ring of tile entries: the raw-unit loader, which makes them, is at most kMaxUnits / 4 + 1
                                      // tiles ahead of the slowest reader (it waits for every unit to be read)
 
@@ -338,7 +344,7 @@ __device__ __forceinline__ bool wait_or_fail(Pipe& P, uint64_t* bar, uint32_t pa
 
 // A group's activation rows as the write-back leaves them in shared memory: rows rounded up to 8, and the bytes of the whole
 __device__ __forceinline__ int rows_up8(int nrows) { return (nrows + 7) & ~7; }
-template<bool GLU> __device__ __forceinline__ int staging_bytes(int nrows) { return rows_up8(nrows) * (GLU ? 128 * 6 + 8 : TM * 4); }
+template<bool GLU> __device__ __forceinline__ int staging_bytes(int nrows) { return rows_up8(nrows) * (GLU ? 128 * 4 : TM * 4); }
 
 // Persistent: one block an SM takes tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the list (group-major, a group's slabs
 // of weight rows side by side, so that the blocks at work share its activation rows in L2).  How many groups there are is
@@ -346,6 +352,28 @@ template<bool GLU> __device__ __forceinline__ int staging_bytes(int nrows) { ret
 // (64 tokens over 256 experts: 259 group rows launched, 55 in use), and every tile paid the block's set-up - tensor-memory
 // allocation, codebook, barriers - and its first loads' latency behind the previous block's write-back.  Here the barriers'
 // phases run on from tile to tile, and the raw loader starts the next tile's units while the last one is written back.
+// A tile's rows of h are written by threads this one has met at a barrier since: count them for the down product ...
+__device__ __forceinline__ void red_release(unsigned* counter, unsigned n) {
+    fence_proxy_async_all();                         // they are read by tensor copies
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(counter), "r"(n) : "memory");
+}
+// ... whose activation loader waits here (a second at most).  false: the wait ran out or another role has failed.
+__device__ __forceinline__ bool wait_rows(Pipe& P, const unsigned* counter, unsigned want) {
+    unsigned long long t0 = 0, now;
+    for (unsigned i = 0;; ++i) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+        if (v >= want) break;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (i == 0) t0 = now;
+        if (now - t0 > 1000000000ull) { *(volatile int*) &P.fail = 1; return false; }
+        if (failed(P)) return false;
+        __nanosleep(200);
+    }
+    fence_proxy_async_all();                         // the tensor copies that follow read what the counter vouches for
+    return true;
+}
+
 template<int T, bool GLU>
 __global__ void __launch_bounds__(kMmqThreads, 1)
 mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -363,13 +391,13 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
     constexpr int kSlab = GLU ? 128 : TM;
     const int nslab = (A.w_rows + kSlab - 1) / kSlab;
 #ifdef MAYA_MMQ_STAMPS
-    // stamps of tile t of this block: the tile's place in the list is blockIdx.x + t * gridDim.x
-    auto stamps_of = [&](int t) -> long long* {
-        const int lin = (int) blockIdx.x + t * (int) gridDim.x;
+    auto stamps_of = [&](int lin) -> long long* {
         return lin < 4096 ? g_stamps + ((size_t) ((T == MAYA_Q4_K || T == MAYA_IQ3_S ? 2 : 0) + (GLU ? 1 : 0)) * 4096 + lin) * 16 : nullptr;
     };
 #endif
 
+    // In a chain the next product's blocks start where this one's have ended; what they wait for is in `ready`.
+    grid_launch_dependents();
     uint8_t* const raw = smem + kBRing<T>;
     if (tid == 0) {
         for (int s = 0; s < kSt; ++s) mbar_init(&P.a_full[s], 8);
@@ -458,7 +486,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         if (named_bar_or(3, kDqWarps * 32, !ok) || ti.e < 0) break;      // the same for every expanding warp
         const int nrows = ti.nrows, row0 = ti.row0, m0 = ti.m0;
 #ifdef MAYA_MMQ_STAMPS
-        long long* const stamps = tid == 0 && ok ? stamps_of(t) : nullptr;
+        long long* const stamps = tid == 0 && ok ? stamps_of(ti.lin) : nullptr;
         if (stamps) { stamps[0] = stamps[1] = clock64(); stamps[14] = nrows; stamps[15] = npairs; }
 #endif
         for (int kb = 0; kb < nkb && ok; ++kb) {
@@ -567,12 +595,11 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 // Two passes.  First the tile goes from tensor memory to shared memory as h = SwiGLU(gate, up) in f32,
                 // [activation row][128]: 16 warps = 4 lane quadrants x 4 groups, a group takes every 4th chunk of 8
                 // activation rows.  Then, for the f16 image, every thread rounds 8 consecutive values of a row at a time
-                // (4 threads a 32-value group, as maya_mmq_quantize does: the same function, the same bytes) - the
-                // groups' amax and sums cost two shuffles each instead of a warp-wide reduction per value.
-                const int r8 = rows_up8(nrows);
-                __half* b16 = (__half*) stg;                             // [rows][128] f16 image of h
-                float* b32 = (float*) (stg + r8 * 128 * 2);              // [rows][128] h
-                __half* bxa = (__half*) (stg + r8 * 128 * 6);            // [rows][4] sum corrections of the row's four 32-value groups
+                // (4 threads a 32-value group, as maya_mmq_quantize does: the same function, the same bytes) - the groups' amax
+                // and sums cost two shuffles each instead of a warp-wide reduction per value - and stores them from its
+                // registers, 256 bytes a half warp.  (Through shared memory and one bulk copy a row the block waited for
+                // the copies' reads, and in a chain for their completion.)
+                float* b32 = (float*) stg;                               // [rows][128] h
                 const int nchunk = (nrows + 7) >> 3;
                 const int mcol = 32 * q + lane;
                 for (int c = hs; c < nchunk; c += 4) {
@@ -591,6 +618,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 if (A.xq_out) {
                     named_bar_sync(2, kThreadsEpi);
                     const int ch = tid & 15;                             // the row's 8-value chunk; a warp covers two rows
+                    const int64_t ldq = xq_ld(A.w_rows);
                     for (int r0 = 0; r0 < nrows; r0 += kThreadsEpi / 16) {
                         const int r = r0 + (tid >> 4);
                         const bool live = r < nrows;                     // the same for a group's four threads
@@ -600,27 +628,25 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                         uint32_t o[4];
                         const __half xa = q8_1_round8(v, o);
                         if (live) {
-                            *(uint4*) (b16 + r * 128 + 8 * ch) = make_uint4(o[0], o[1], o[2], o[3]);
-                            if ((ch & 3) == 0) bxa[r * 4 + (ch >> 2)] = xa;
+                            __half* const dst = A.xq_out + (int64_t) (row0 + r) * ldq;
+                            *(uint4*) (dst + m0 + 8 * ch) = make_uint4(o[0], o[1], o[2], o[3]);
+                            if ((ch & 3) == 0) dst[A.w_rows + (m0 >> 5) + (ch >> 2)] = xa;
+                            if (m0 == 0)                                 // the zero padding behind the row's corrections
+                                for (int64_t c = A.w_rows + A.w_rows / 32 + ch; c < ldq; c += 16) dst[c] = __float2half_rn(0.0f);
                         }
                     }
                 }
 #ifdef MAYA_MMQ_STAMPS
                 if (stamps) stamps[6] = clock64();       // tile rounded
 #endif
-                fence_proxy_async();
-                named_bar_sync(1, kThreadsEpi);
-                if (tid < nrows) {                                       // one activation row each
-                    const int64_t row_g = row0 + tid;
-                    if (A.xq_out) {
-                        const int64_t ldq = xq_ld(A.w_rows);
-                        bulk_store(A.xq_out + row_g * ldq + m0, b16 + tid * 128, 128 * 2);
-                        *(uint2*) (A.xq_out + row_g * ldq + A.w_rows + (m0 >> 5)) = *(const uint2*) (bxa + tid * 4);
-                        if (m0 == 0)                                     // the zero padding behind the row's corrections
-                            for (int64_t c = A.w_rows + A.w_rows / 32; c < ldq; ++c) A.xq_out[row_g * ldq + c] = __float2half_rn(0.0f);
+                if (A.dst) {                                             // h itself, a bulk copy a row
+                    fence_proxy_async();
+                    named_bar_sync(1, kThreadsEpi);
+                    if (tid < nrows) {
+                        const int64_t row_g = row0 + tid;
+                        bulk_store(A.dst + (int64_t) (A.ids ? A.ids[row_g] : row_g) * A.ld_dst + m0, b32 + tid * 128, 128 * 4);
+                        bulk_commit();
                     }
-                    if (A.dst) bulk_store(A.dst + (int64_t) (A.ids ? A.ids[row_g] : row_g) * A.ld_dst + m0, b32 + tid * 128, 128 * 4);
-                    bulk_commit();
                 }
             } else {
                 // 16 warps = 4 lane quadrants x 2 accumulators x 2 groups that take alternate chunks of 16 activation rows
@@ -650,6 +676,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 }
             }
             if (tid < nrows) bulk_wait_read<0>();                        // the copies have read shared memory ...
+            fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&P.stg_free[t & 1]);              // ... which the next tile's loads may overwrite
         }
@@ -660,11 +687,15 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
     } else if (warp == kDqWarps) {
         // ------------------------------------------------------------ the tile list, and raw weight units (one lane)
         int u0 = 0, prev_rows = 0;           // raw units of the tiles before this one; rows of the tile before this one
+        // In a chain the tiles are taken as blocks get to them (blocks of the next product start where this one's have run out of
+        // tiles), a tile ahead of its use; else block b's are b, b + grid, ...
+        int claimed = (int) blockIdx.x;
+        if (A.claim != nullptr && lane == 0) claimed = (int) atomicAdd(A.claim, 1u);
         for (int t = 0;; ++t, u0 += 4 * nkb) {
             // Which (matrix, 160-row group) is this tile's: the warp scans the per-matrix group counts - each lane the counts
             // of a run of consecutive matrices, an exclusive warp scan of the runs' sums, then the lane whose run holds the
             // wanted group walks it - 1024 matrices a round.
-            const int lin = (int) blockIdx.x + t * (int) gridDim.x, want_all = lin / nslab;
+            const int lin = __shfl_sync(0xFFFFFFFFu, claimed, 0), want_all = lin / nslab;
             int found_e = -1, row0 = 0, nrows = 0, base = 0;
             for (int e0 = 0; e0 < A.n; e0 += 1024) {
                 const int per = (min(A.n - e0, 1024) + 31) >> 5;          // matrices a lane (<= 32)
@@ -705,11 +736,13 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             const int m0 = (lin % nslab) * kSlab;
             bool ok = true;
             if (lane == 0) {
+                claimed = lin + (int) gridDim.x;
+                if (A.claim != nullptr && found_e >= 0) claimed = (int) atomicAdd(A.claim, 1u);
                 // Entry t % kTiles was read by every role before tile t - kTiles ended.  The write-back of the tile two before
                 // this one has to be over in any case (so that a barrier's phase is never two behind), that of the tile before
                 // only where it stretches into the raw ring.
                 if (t >= 2) ok = wait_or_fail(P, &P.stg_free[t & 1], ((t - 2) >> 1) & 1);
-                P.tile[t % kTiles] = TileInfo{found_e, row0, nrows, m0};
+                P.tile[t % kTiles] = TileInfo{found_e, row0, nrows, m0, lin};
                 mbar_arrive(&P.tile_full[t % kTiles]);
                 if (found_e >= 0) {
                     if (ok && t >= 1 && staging_bytes<GLU>(prev_rows) > kBRing<T>)
@@ -735,6 +768,10 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
             if (!ok || found_e < 0) break;
             prev_rows = nrows;
+        }
+        if (A.claim != nullptr && lane == 0 && atomicAdd(A.claim + 1, 1u) == gridDim.x - 1u) {       // no block will claim again
+            A.claim[0] = 0u;
+            A.claim[1] = 0u;
         }
     } else if (warp == kDqWarps + 1 || warp == kDqWarps + 3) {
         // ------------------------------------------------------------ tensor-core issue (two warps, one accumulator each, on
@@ -774,7 +811,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 }
                 tc_fence_after();
 #ifdef MAYA_MMQ_STAMPS
-                if (my == 0 && kp == 0 && lane == 0 && stamps_of(t)) stamps_of(t)[2] = clock64();       // the first product
+                if (my == 0 && kp == 0 && lane == 0 && stamps_of(ti.lin)) stamps_of(ti.lin)[2] = clock64();       // the first product
 #endif
                 mma_f16_ts_x4_commit(d0, at, b_lo, b_hi, idesc, first, done0 + done_at);
                 first = 1;
@@ -785,7 +822,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 if (b_lo == b_lo_end) { b_lo = b_lo0; bfull = bfull0; ph_b ^= 1; }
             }
 #ifdef MAYA_MMQ_STAMPS
-            if (my == 0 && lane == 0 && stamps_of(t)) stamps_of(t)[3] = clock64();                      // the last product issued
+            if (my == 0 && lane == 0 && stamps_of(ti.lin)) stamps_of(ti.lin)[3] = clock64();                      // the last product issued
 #endif
             if (!ok) break;
             mma_commit_elect(smem_u32(&P.final));
@@ -796,12 +833,27 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             const int nmain = nkt / 2;
             int p0 = 0, issued = 0;                  // pairs of the tiles before this one; tiles of activations asked for
             bool ok = true;
+            unsigned* counter = nullptr;             // gate/up in a chain: the counter of the tile before's rows, not counted yet
+            unsigned written = 0;
+            auto count_rows = [&] {
+                if (counter != nullptr) red_release(counter, written);
+                counter = nullptr;
+            };
             for (int t = 0;; ++t, p0 += npairs) {
                 TileInfo ti;
                 ok = tile_of(t, ti);
-                if (!ok || ti.e < 0) break;
                 // the write-back of the tile before uses the activation ring
-                if (t > 0) ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
+                if (ok && t > 0) ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
+                if (!ok || ti.e < 0) {
+                    if (ok) count_rows();
+                    break;
+                }
+                if (!GLU && A.ready != nullptr) {
+                    unsigned* const r = A.ready + 2 * (ti.lin / nslab);
+                    ok = wait_rows(P, r, (unsigned) (ti.nrows * A.ready_slabs));
+                    if (!ok) break;
+                    if (atomicAdd(r + 1, 1u) == (unsigned) nslab - 1u) { r[0] = 0u; r[1] = 0u; }     // the group's last tile to wait
+                }
                 const bool big = ti.nrows > 128;     // the activation tile is a 128-row box and a 32-row box
                 const uint32_t tx_bytes = big ? kBStage : kBBox;
                 for (int kb2 = 0; kb2 < npairs && ok; ++kb2) {
@@ -824,8 +876,10 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     tma_load_2d(bt, &tm_x, &P.b_full[sb], xcol, ti.row0);
                     if (big) tma_load_2d(bt + kBBox, &tm_x32, &P.b_full[sb], xcol, ti.row0 + 128);
                     issued = pg + 1;
+                    if (kb2 == min(NB, npairs) - 1) count_rows();        // behind the loads the expansion waits for
                 }
                 if (!ok) break;
+                if (GLU && A.ready != nullptr) { counter = A.ready + 2 * (ti.lin / nslab); written = (unsigned) ti.nrows; }
             }
             if (!ok)                                         // let the copies in flight land before the block ends
                 for (int pg = max(0, issued - NB); pg < issued; ++pg) wait_or_fail(P, &P.b_full[pg % NB], (pg / NB) & 1);
@@ -834,6 +888,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, 512);
+    grid_dependency_wait();                          // a block ends after the products in front of its own
     if (tid == 0 && failed(P) && A.error != nullptr) atomicExch(A.error, 1u);
 }
 
@@ -925,7 +980,7 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, const void* base
 }
 
 template<int T, bool GLU>
-int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
+int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, bool dependent, cudaStream_t s) {
     const int64_t mat_rows = p->w_rows, K = p->w_cols;
     const size_t rbw = row_bytes(T, K);
     CUtensorMap tw, tx, tx32;
@@ -960,11 +1015,15 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
     const int slab = GLU ? 128 : TM, sms = sm_count();
     if (sms <= 0) return refuse(MAYA_ERR_DEVICE);
     const int64_t most = (int64_t) ((A.w_rows + slab - 1) / slab) * groups;      // tiles there can be
-    mmq_kernel<T, GLU><<<(unsigned) (most < sms ? most : sms), kMmqThreads, smem, s>>>(tw, tx, tx32, A);
+    const dim3 grid((unsigned) (most < sms ? most : sms));
+    if (dependent) launch_dependent(mmq_kernel<T, GLU>, grid, dim3(kMmqThreads), smem, s, tw, tx, tx32, A);
+    else mmq_kernel<T, GLU><<<grid, kMmqThreads, smem, s>>>(tw, tx, tx32, A);
     return note_launch("mmq");
 }
 
-int run_product(const maya_mmq_product* p, bool glu, float limit, cudaStream_t s) {
+struct Chain { unsigned *claim, *ready; int ready_slabs; bool dependent; };
+
+int run_product(const maya_mmq_product* p, bool glu, float limit, const Chain* chain, cudaStream_t s) {
     if (!p || !p->w || !p->xq || !p->bounds) return refuse(MAYA_ERR_ARG);
     if (!p->dst && !(glu && p->xq_out)) return refuse(MAYA_ERR_ARG);
     if (!maya_mmq_supported(p->type)) return refuse(MAYA_ERR_TYPE);
@@ -984,11 +1043,13 @@ int run_product(const maya_mmq_product* p, bool glu, float limit, cudaStream_t s
     A.w_rows = (int) out_rows; A.w_cols = (int) p->w_cols; A.n = p->n; A.expert_map = p->expert_map; A.bounds = p->bounds;
     A.ids = p->ids; A.dst = p->dst; A.ld_dst = p->ld_dst; A.xq_out = glu ? (__half*) p->xq_out : nullptr; A.limit = limit;
     A.error = p->error;
+    const bool dep = chain != nullptr && chain->dependent;
+    if (chain != nullptr) { A.claim = chain->claim; A.ready = chain->ready; A.ready_slabs = chain->ready_slabs; }
     switch (p->type) {
-        case MAYA_Q4_K: return glu ? launch_mmq<MAYA_Q4_K, true>(p, A, s) : launch_mmq<MAYA_Q4_K, false>(p, A, s);
-        case MAYA_Q8_0: return glu ? launch_mmq<MAYA_Q8_0, true>(p, A, s) : launch_mmq<MAYA_Q8_0, false>(p, A, s);
-        case MAYA_IQ2_S: return glu ? launch_mmq<MAYA_IQ2_S, true>(p, A, s) : launch_mmq<MAYA_IQ2_S, false>(p, A, s);
-        default: return glu ? launch_mmq<MAYA_IQ3_S, true>(p, A, s) : launch_mmq<MAYA_IQ3_S, false>(p, A, s);
+        case MAYA_Q4_K: return glu ? launch_mmq<MAYA_Q4_K, true>(p, A, dep, s) : launch_mmq<MAYA_Q4_K, false>(p, A, dep, s);
+        case MAYA_Q8_0: return glu ? launch_mmq<MAYA_Q8_0, true>(p, A, dep, s) : launch_mmq<MAYA_Q8_0, false>(p, A, dep, s);
+        case MAYA_IQ2_S: return glu ? launch_mmq<MAYA_IQ2_S, true>(p, A, dep, s) : launch_mmq<MAYA_IQ2_S, false>(p, A, dep, s);
+        default: return glu ? launch_mmq<MAYA_IQ3_S, true>(p, A, dep, s) : launch_mmq<MAYA_IQ3_S, false>(p, A, dep, s);
     }
 }
 
@@ -1028,7 +1089,41 @@ extern "C" int maya_mmq_quantize_routed_bf16(const uint16_t* x, const int32_t* p
     if (k <= 0) return refuse(MAYA_ERR_ARG);
     return launch_quantize<uint16_t>(x, pos, xq, type, cols, ld, tokens, k, stream);
 }
-extern "C" int maya_mmq_run(const maya_mmq_product* p, void* stream) { return run_product(p, false, 0.0f, as_stream(stream)); }
+extern "C" int maya_mmq_run(const maya_mmq_product* p, void* stream) { return run_product(p, false, 0.0f, nullptr, as_stream(stream)); }
 extern "C" int maya_mmq_run_glu(const maya_mmq_product* p, float limit, void* stream) {
-    return run_product(p, true, limit, as_stream(stream));
+    return run_product(p, true, limit, nullptr, as_stream(stream));
+}
+// Words of a chain's counters: two claim words a product, two ready words a group of a pair (an upper bound of the groups).
+static size_t chain_groups(int64_t total_rows, int n) { return (size_t) (total_rows / TN + n); }
+extern "C" size_t maya_mmq_chain_bytes(int64_t total_rows, int n_matrices, int n_pairs) {
+    if (total_rows <= 0 || n_matrices <= 0 || n_pairs <= 0) return 0;
+    return sizeof(unsigned) * (4 * (size_t) n_pairs + 2 * ((size_t) n_pairs * (size_t) (total_rows / TN) + (size_t) n_matrices));
+}
+extern "C" int maya_mmq_run_chain(const maya_mmq_product* gate_up, const maya_mmq_product* down, int n_pairs, float limit, void* counters,
+                                  size_t counter_bytes, void* stream) {
+    if (n_pairs <= 0) return MAYA_OK;
+    if (!gate_up || !down || !counters || ((uintptr_t) counters & 3u)) return refuse(MAYA_ERR_ARG);
+    size_t need = 4 * (size_t) n_pairs;
+    for (int i = 0; i < n_pairs; ++i) {
+        if (gate_up[i].n != down[i].n || gate_up[i].bounds != down[i].bounds || gate_up[i].expert_map != down[i].expert_map ||
+            gate_up[i].total_rows != down[i].total_rows || gate_up[i].xq_out != down[i].xq || !gate_up[i].xq_out || gate_up[i].n < 0)
+            return refuse(MAYA_ERR_ARG);
+        need += 2 * chain_groups(gate_up[i].total_rows, gate_up[i].n);
+    }
+    if (need * sizeof(unsigned) > counter_bytes) return refuse(MAYA_ERR_LIMIT);
+    unsigned* const words = (unsigned*) counters;
+    bool first = true;
+    for (int pass = 0; pass < 2; ++pass) {
+        unsigned* ready = words + 4 * n_pairs;
+        for (int i = 0; i < n_pairs; ++i) {
+            const maya_mmq_product& p = pass ? down[i] : gate_up[i];
+            const Chain c{words + 4 * i + 2 * pass, ready, (int) (gate_up[i].w_rows / 256), !first};
+            ready += 2 * chain_groups(p.total_rows, p.n);
+            if (p.n == 0 || p.total_rows <= 0) continue;
+            const int st = run_product(&p, pass == 0, limit, &c, as_stream(stream));
+            if (st != MAYA_OK) return st;
+            first = false;
+        }
+    }
+    return MAYA_OK;
 }

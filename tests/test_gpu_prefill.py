@@ -233,6 +233,47 @@ def test_fused_glu_equals_product_then_swiglu_bitwise(T, api, t, limit):
     assert T.equal(hq, want_hq)
 
 
+@pytest.mark.parametrize("ta,tb,counts,n_ff", [
+    (H.Q8_0, H.Q4_K, [1, 0, 161, 7, 320, 33], 256),                                       # fewer tiles than blocks, remainders of 160 rows
+    (H.IQ2_S, H.IQ3_S, [5] * 24 + [0] * 3 + [170] * 3, 2048),                             # several rounds of tiles
+    (H.Q4_K, H.Q8_0, [0] * 6, 256)])                                                      # no rows at all in one pair
+def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
+    """Two pairs of gate/up and down products in one chain, each down tile starting when its own rows of h are there: the bits
+    of the four products run one after another - twice, on the same counters, which end at zero."""
+    cols = 2048
+    pairs = []
+    for t, c in ((ta, counts), (tb, counts[::-1] if sum(counts) else [3, 200, 0, 9, 1, 64])):
+        w, total = synth_matrices(T, api, t, len(c), 2 * n_ff, cols, 31), sum(c)
+        wd = synth_matrices(T, api, t, len(c), 512, n_ff, 37)
+        x = (H.rng_for("chain", t).standard_normal((max(total, 1), cols)) * 2.0).astype(np.float32)
+        pairs.append(dict(t=t, n=len(c), w=w, wd=wd, total=total, xq=api.mmq_quantize(dev(T, x), None, t),
+                          bounds=dev(T, np.concatenate([[0], np.cumsum(c)]).astype(np.int32))))
+    err = T.zeros(1, dtype=T.int32, device="cuda")
+
+    def products(p):
+        hq = T.zeros(max(api.mmq_q8_bytes(p["total"], n_ff), 16), dtype=T.uint8, device="cuda")
+        out = T.zeros((max(p["total"], 1), 512), dtype=T.float32, device="cuda")
+        return (api.mmq_product(p["w"], p["t"], 2 * n_ff, cols, p["w"].shape[1], p["n"], p["xq"], p["bounds"], None, p["total"], None, n_ff,
+                                error=err, xq_out=hq),
+                api.mmq_product(p["wd"], p["t"], 512, n_ff, p["wd"].shape[1], p["n"], hq, p["bounds"], None, p["total"], out, 512, error=err), hq, out)
+
+    want = [products(p) for p in pairs]
+    for gu, dn, _, _ in want:
+        api.mmq_run_glu(gu, 7.0)
+        api.mmq_run(dn)
+    counters = T.zeros(4096, dtype=T.uint8, device="cuda")
+    for _ in range(2):
+        got = [products(p) for p in pairs]
+        api.mmq_run_chain([g[0] for g in got], [g[1] for g in got], 7.0, counters)
+        T.cuda.synchronize()
+        assert int(err.item()) == 0 and not counters.any()
+        for a, b in zip(got, want):
+            assert T.equal(a[2], b[2]) and T.equal(a[3], b[3])
+    assert want[1][3].abs().max() > 0.01
+    with pytest.raises(api.MayaError):                                                    # the down product reads another h
+        api.mmq_run_chain([want[0][0]], [got[0][1]], 7.0, counters)
+
+
 def test_expert_map_selects_bounds_entries(T, api):
     """A staged group: matrix i of the product owns the rows of expert expert_map[i]."""
     t, rows, cols = H.Q4_K, 128, 256
