@@ -84,13 +84,14 @@ __device__ __forceinline__ void select_topk(float (&sel)[PER], const float (&val
     }
 }
 
-// Selection by rank for one expert per thread (nt >= n_expert).  `keys`: n_expert 64-bit words of shared memory.  p >= 0
-// (or NaN): its bit pattern orders like the value; the low word makes equal values rank by ascending index, the stable
-// descending order.  The keys are distinct whatever p holds, so exactly one thread has each rank.
+// Selection by rank for one expert per thread (nt >= n_expert).  `keys`: n_expert 64-bit words of shared memory.  `order`: a
+// number that orders like the value selected on (the bits of a value >= 0 do); the low word makes equal values rank by
+// ascending index, the stable descending order.  The keys are distinct, so exactly one thread has each rank.  The chosen ids
+// and their p land in sh.ids / sh.val.
 template<class Sync>
-__device__ __forceinline__ void select_rank(float p, int n_expert, int k, int tid, unsigned long long* keys,
+__device__ __forceinline__ void select_rank(uint32_t order, float p, int n_expert, int k, int tid, unsigned long long* keys,
                                             RouterShared& sh) {
-    const unsigned long long mine = ((unsigned long long) __float_as_uint(p) << 32) | (unsigned) (0xffffffffu - (unsigned) tid);
+    const unsigned long long mine = ((unsigned long long) order << 32) | (unsigned) (0xffffffffu - (unsigned) tid);
     if (tid < n_expert) keys[tid] = mine;
     if (k <= 8) {
         // Two levels: a key's rank among its own warp's 32 keys first; the k best of every warp are the only candidates
@@ -205,7 +206,7 @@ __device__ __forceinline__ void route_softmax(const float* __restrict__ l, int n
         p[j] = (j * nt + tid) < n_expert ? (float) (ex[j] * inv) : -INFINITY;
         sel[j] = p[j];
     }
-    if constexpr (PER == 1) select_rank<Sync>(p[0], n_expert, k, tid, (unsigned long long*) s_ex, sh);
+    if constexpr (PER == 1) select_rank<Sync>(__float_as_uint(p[0]), p[0], n_expert, k, tid, (unsigned long long*) s_ex, sh);
     else select_topk<PER, Sync>(sel, p, n_expert, k, tid, nt, sh);
     // weights renormalised in double by max(their sum in selection order, 2^-14): every thread adds, k threads divide
     double s = 0.0;
@@ -220,9 +221,11 @@ __device__ __forceinline__ void route_softmax(const float* __restrict__ l, int n
 // One token's sigmoid routing (router_sigmoid.cu:29-74, glm_batch.cu:2063-2100): p = sigmoid(logit) in FP32, selection on
 // p + bias (bias NULL: none), the stable descending top-k, weights from the unbiased p - divided in double by
 // max(their sum, 2^-14) when norm_w - times w_scale.  On return sh.ids[0..k) / sh.val[0..k) hold ids and final weights.
+// s_keys: n_expert 64-bit words of shared memory, 16-byte aligned (one expert per thread: selection by rank, one pass instead of
+// k rounds of arg-max with two barriers each).
 template<int PER, class Sync>
 __device__ __forceinline__ void route_sigmoid(const float* __restrict__ l, const float* __restrict__ bias, int n_expert, int k,
-                                              float w_scale, int norm_w, int tid, int nt, RouterShared& sh) {
+                                              float w_scale, int norm_w, int tid, int nt, double* s_keys, RouterShared& sh) {
     float p[PER], sel[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
@@ -235,17 +238,21 @@ __device__ __forceinline__ void route_sigmoid(const float* __restrict__ l, const
             sel[j] = -INFINITY;
         }
     }
-    select_topk<PER, Sync>(sel, p, n_expert, k, tid, nt, sh);
-    if (tid == 0) {
-        double s = 0.0;
-        for (int i = 0; i < k; ++i) s += (double) sh.val[i];
-        const double sc = fmax(s, 6.103515625e-05);
-        for (int i = 0; i < k; ++i) {
-            float w = sh.val[i];
-            if (norm_w) w = (float) ((double) w / sc);
-            sh.val[i] = w * w_scale;
-        }
+    if constexpr (PER == 1) {
+        uint32_t u = __float_as_uint(sel[0] + 0.0f);             // (-0 counts as 0)
+        u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;              // orders like the value, negative ones included
+        if (sel[0] != sel[0]) u = 0u;                            // no number: last
+        select_rank<Sync>(u, p[0], n_expert, k, tid, (unsigned long long*) s_keys, sh);
+    } else {
+        select_topk<PER, Sync>(sel, p, n_expert, k, tid, nt, sh);
     }
+    double s = 0.0;                                              // every thread adds, k threads divide
+    for (int i = 0; i < k; ++i) s += (double) sh.val[i];
+    const double sc = fmax(s, 6.103515625e-05);
+    float mine = tid < k ? sh.val[tid] : 0.0f;
+    if (norm_w) mine = (float) ((double) mine / sc);
+    Sync::sync();
+    if (tid < k) sh.val[tid] = mine * w_scale;
     Sync::sync();
 }
 

@@ -120,10 +120,10 @@ __device__ __noinline__ void route_token(const float* logits, const float* bias,
     using RS = NamedSync<1, kRouteThreads>;
     const int per = (n_expert + kRouteThreads - 1) / kRouteThreads;
     if constexpr (RT == 1) {
-        if (per <= 1) route_sigmoid<1, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, *route);
-        else if (per <= 2) route_sigmoid<2, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, *route);
-        else if (per <= 4) route_sigmoid<4, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, *route);
-        else route_sigmoid<8, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, *route);
+        if (per <= 1) route_sigmoid<1, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        else if (per <= 2) route_sigmoid<2, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        else if (per <= 4) route_sigmoid<4, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        else route_sigmoid<8, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
     } else {
         if (per <= 1) route_softmax<1, RS>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
         else if (per <= 2) route_softmax<2, RS>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepArgs P) {
         return;
     }
     const float* logits = P.logits + (size_t) t * P.n_expert;
-    if constexpr (RT == 1) route_sigmoid<PER, BlockSync>(logits, P.bias, P.n_expert, P.k, P.w_scale, P.norm_w, tid, 256, route);
+    if constexpr (RT == 1) route_sigmoid<PER, BlockSync>(logits, P.bias, P.n_expert, P.k, P.w_scale, P.norm_w, tid, 256, s_ex, route);
     else route_softmax<PER, BlockSync>(logits, P.n_expert, P.k, tid, 256, s_ex, route);
     if (tid < 8) {
         unsigned long long p = 0ull;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const PrepArgs P) {
 template<int RT> int launch_prep(const PrepArgs& P, int T, cudaStream_t s) {
     const int per = (P.n_expert + 255) / 256, nblk = P.n_embd / 32;
     const dim3 grid((unsigned) T, (unsigned) (1 + (nblk >= 256 ? 8 : (nblk + 31) / 32)));
-    const size_t smem = RT == 0 ? (size_t) P.n_expert * sizeof(double) : 0;
+    const size_t smem = (size_t) P.n_expert * sizeof(double);
     if (per <= 1) launch_dependent(prep_kernel<RT, 1>, grid, dim3(256), smem, s, P);
     else if (per <= 2) launch_dependent(prep_kernel<RT, 2>, grid, dim3(256), smem, s, P);
     else if (per <= 4) launch_dependent(prep_kernel<RT, 4>, grid, dim3(256), smem, s, P);

@@ -28,9 +28,10 @@ __global__ void __launch_bounds__(kRouterThreads) router_sigmoid_kernel(const fl
                                                                         int k, float w_scale, int norm_w,
                                                                         int* __restrict__ ids,
                                                                         float* __restrict__ weights) {
+    extern __shared__ double s_keys[];        // n_expert 64-bit words
     __shared__ RouterShared sh;
     const int t = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
-    route_sigmoid<PER, BlockSync>(logits + (size_t) t * n_expert, bias, n_expert, k, w_scale, norm_w, tid, nt, sh);
+    route_sigmoid<PER, BlockSync>(logits + (size_t) t * n_expert, bias, n_expert, k, w_scale, norm_w, tid, nt, s_keys, sh);
     if (tid < k) {
         ids[(size_t) t * k + tid] = sh.ids[tid];
         weights[(size_t) t * k + tid] = sh.val[tid];
@@ -70,10 +71,11 @@ extern "C" int maya_router_sigmoid(const float* logits, const float* bias, int n
     if (k > 64 || k > n_expert || n_expert > kRouterThreads * kRouterMaxPerThread) return refuse(MAYA_ERR_LIMIT);
     const int nt = router_threads(n_expert);
     const int per = (n_expert + nt - 1) / nt;
+    const size_t smem = (size_t) n_expert * sizeof(double);
     cudaStream_t s = as_stream(stream);
-    if (per <= 1) router_sigmoid_kernel<1><<<n_tokens, nt, 0, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
-    else if (per <= 2) router_sigmoid_kernel<2><<<n_tokens, nt, 0, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
-    else if (per <= 4) router_sigmoid_kernel<4><<<n_tokens, nt, 0, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
-    else router_sigmoid_kernel<8><<<n_tokens, nt, 0, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    if (per <= 1) router_sigmoid_kernel<1><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    else if (per <= 2) router_sigmoid_kernel<2><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    else if (per <= 4) router_sigmoid_kernel<4><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    else router_sigmoid_kernel<8><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
     return note_launch("router_sigmoid");
 }

@@ -96,6 +96,23 @@ def test_router_sigmoid_golden(T, api):
         assert (np.abs(w.cpu().numpy() - g["weights"][i]) / g["weights"][i]).max() <= 1e-6
 
 
+@pytest.mark.parametrize("E,k", [(64, 8), (160, 6), (256, 10), (33, 33), (300, 8)])       # one and two experts a thread; k beyond 8
+def test_router_sigmoid_ties_and_signs(T, api, oracle, E, k):
+    """Scores of both signs, exact ties (lower index first), -0 beside +0, a masked expert: the oracle's ids and weights."""
+    rng = H.rng_for("sigmoid-ties", E, k)
+    logits = rng.standard_normal((6, E)).astype(np.float32)
+    logits[1] = 0.25                                                                       # all equal
+    logits[2, ::3] = logits[2, 0]
+    bias = (rng.standard_normal(E) - 1.0).astype(np.float32)                               # most p + bias below zero
+    bias[5], bias[7] = -0.5, -0.5
+    logits[3, 5], logits[3, 7] = 0.0, -0.0                                                 # p + bias = 0 twice
+    for b, norm in ((bias, True), (np.zeros(E, np.float32), False)):
+        ids, w = api.router_sigmoid(dev(T, logits), dev(T, b), k, 2.5, norm)
+        ids_o, w_o = oracle.router_sigmoid(logits, b, k, 2.5, norm)
+        assert np.array_equal(ids.cpu().numpy(), ids_o)
+        assert (np.abs(w.cpu().numpy() - w_o) / np.abs(w_o)).max() <= 1e-6
+
+
 # ------------------------------------------------------------------------------------------------ q8_1
 @pytest.mark.parametrize("act", ["f32", "bf16"])
 def test_quantize_q8_1_bytes(T, api, oracle, act):
