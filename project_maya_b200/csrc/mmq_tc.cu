@@ -113,6 +113,7 @@ struct MmqArgs {
     unsigned* claim;
     unsigned* ready;
     int ready_slabs;             // down: gate/up tiles of a group; gate/up: unused
+    int alone;                   // not behind another product of its chain: everything in front has to be done first
 };
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *(uint32_t*) &h; }
@@ -396,8 +397,6 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
     };
 #endif
 
-    // In a chain the next product's blocks start where this one's have ended; what they wait for is in `ready`.
-    grid_launch_dependents();
     uint8_t* const raw = smem + kBRing<T>;
     if (tid == 0) {
         for (int s = 0; s < kSt; ++s) mbar_init(&P.a_full[s], 8);
@@ -419,6 +418,10 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = P.tmem;
+    if (A.alone) grid_dependency_wait();             // (its set-up overlaps the launch in front)
+    // In a chain the next product's blocks may start from here on, where this one's have ended: after the wait, since they do not
+    // wait for what is in front of this one.  What they do wait for is in `ready`.
+    grid_launch_dependents();
     // the block's t-th tile, for a role that waits for its entry; false: the wait ran out or another role has failed
     auto tile_of = [&](int t, TileInfo& ti) -> bool {
         if (!wait_or_fail(P, &P.tile_full[t % kTiles], (t / kTiles) & 1)) return false;
@@ -901,6 +904,8 @@ template<typename X, bool ROUTED>
 __global__ void __launch_bounds__(256) mmq_quantize_kernel(const X* __restrict__ x, const int* __restrict__ ids,
                                                            __half* __restrict__ xq, int cols, int64_t ld, int k) {
     const int64_t row = blockIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int cpr = cols >> 3, c = (int) blockIdx.y * 256 + (int) threadIdx.x;
     const bool live = c < cpr;                       // cpr is a multiple of 4: a block's 4 threads live together
     const int64_t src = (!ROUTED && ids) ? ids[row] : row;
@@ -954,8 +959,8 @@ int launch_quantize(const X* x, const int32_t* ids, void* xq, int type, int64_t 
     const int64_t by = (cols / 8 + 255) / 256;
     if (rows > 0x7FFFFFFFll || by > 65535) return refuse(MAYA_ERR_LIMIT);
     const dim3 grid((unsigned) rows, (unsigned) by);
-    if (k > 0) mmq_quantize_kernel<X, true><<<grid, 256, 0, as_stream(stream)>>>(x, ids, (__half*) xq, (int) cols, ld, k);
-    else mmq_quantize_kernel<X, false><<<grid, 256, 0, as_stream(stream)>>>(x, ids, (__half*) xq, (int) cols, ld, 0);
+    launch_dependent(k > 0 ? mmq_quantize_kernel<X, true> : mmq_quantize_kernel<X, false>, grid, dim3(256), 0, as_stream(stream), x, ids,
+                     (__half*) xq, (int) cols, ld, k > 0 ? k : 0);
     return note_launch(k > 0 ? "mmq_quantize_routed" : "mmq_quantize");
 }
 
@@ -980,7 +985,7 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, const void* base
 }
 
 template<int T, bool GLU>
-int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, bool dependent, cudaStream_t s) {
+int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
     const int64_t mat_rows = p->w_rows, K = p->w_cols;
     const size_t rbw = row_bytes(T, K);
     CUtensorMap tw, tx, tx32;
@@ -1016,12 +1021,11 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, bool dependent, cuda
     if (sms <= 0) return refuse(MAYA_ERR_DEVICE);
     const int64_t most = (int64_t) ((A.w_rows + slab - 1) / slab) * groups;      // tiles there can be
     const dim3 grid((unsigned) (most < sms ? most : sms));
-    if (dependent) launch_dependent(mmq_kernel<T, GLU>, grid, dim3(kMmqThreads), smem, s, tw, tx, tx32, A);
-    else mmq_kernel<T, GLU><<<grid, kMmqThreads, smem, s>>>(tw, tx, tx32, A);
+    launch_dependent(mmq_kernel<T, GLU>, grid, dim3(kMmqThreads), smem, s, tw, tx, tx32, A);
     return note_launch("mmq");
 }
 
-struct Chain { unsigned *claim, *ready; int ready_slabs; bool dependent; };
+struct Chain { unsigned *claim, *ready; int ready_slabs; bool first; };
 
 int run_product(const maya_mmq_product* p, bool glu, float limit, const Chain* chain, cudaStream_t s) {
     if (!p || !p->w || !p->xq || !p->bounds) return refuse(MAYA_ERR_ARG);
@@ -1043,13 +1047,13 @@ int run_product(const maya_mmq_product* p, bool glu, float limit, const Chain* c
     A.w_rows = (int) out_rows; A.w_cols = (int) p->w_cols; A.n = p->n; A.expert_map = p->expert_map; A.bounds = p->bounds;
     A.ids = p->ids; A.dst = p->dst; A.ld_dst = p->ld_dst; A.xq_out = glu ? (__half*) p->xq_out : nullptr; A.limit = limit;
     A.error = p->error;
-    const bool dep = chain != nullptr && chain->dependent;
+    A.alone = chain == nullptr || chain->first;
     if (chain != nullptr) { A.claim = chain->claim; A.ready = chain->ready; A.ready_slabs = chain->ready_slabs; }
     switch (p->type) {
-        case MAYA_Q4_K: return glu ? launch_mmq<MAYA_Q4_K, true>(p, A, dep, s) : launch_mmq<MAYA_Q4_K, false>(p, A, dep, s);
-        case MAYA_Q8_0: return glu ? launch_mmq<MAYA_Q8_0, true>(p, A, dep, s) : launch_mmq<MAYA_Q8_0, false>(p, A, dep, s);
-        case MAYA_IQ2_S: return glu ? launch_mmq<MAYA_IQ2_S, true>(p, A, dep, s) : launch_mmq<MAYA_IQ2_S, false>(p, A, dep, s);
-        default: return glu ? launch_mmq<MAYA_IQ3_S, true>(p, A, dep, s) : launch_mmq<MAYA_IQ3_S, false>(p, A, dep, s);
+        case MAYA_Q4_K: return glu ? launch_mmq<MAYA_Q4_K, true>(p, A, s) : launch_mmq<MAYA_Q4_K, false>(p, A, s);
+        case MAYA_Q8_0: return glu ? launch_mmq<MAYA_Q8_0, true>(p, A, s) : launch_mmq<MAYA_Q8_0, false>(p, A, s);
+        case MAYA_IQ2_S: return glu ? launch_mmq<MAYA_IQ2_S, true>(p, A, s) : launch_mmq<MAYA_IQ2_S, false>(p, A, s);
+        default: return glu ? launch_mmq<MAYA_IQ3_S, true>(p, A, s) : launch_mmq<MAYA_IQ3_S, false>(p, A, s);
     }
 }
 
@@ -1117,7 +1121,7 @@ extern "C" int maya_mmq_run_chain(const maya_mmq_product* gate_up, const maya_mm
         unsigned* ready = words + 4 * n_pairs;
         for (int i = 0; i < n_pairs; ++i) {
             const maya_mmq_product& p = pass ? down[i] : gate_up[i];
-            const Chain c{words + 4 * i + 2 * pass, ready, (int) (gate_up[i].w_rows / 256), !first};
+            const Chain c{words + 4 * i + 2 * pass, ready, (int) (gate_up[i].w_rows / 256), first};
             ready += 2 * chain_groups(p.total_rows, p.n);
             if (p.n == 0 || p.total_rows <= 0) continue;
             const int st = run_product(&p, pass == 0, limit, &c, as_stream(stream));

@@ -12,6 +12,12 @@ WArgs common(const GroupArgs& A, int cap_groups, int n_embd, int n_ff, const Sha
     if (sh != nullptr) { W.n_ff_sh = sh->n_ff; W.n_tok = sh->n_tok; W.sh_hq = (uint8_t*) sh->hq; W.sh_out = sh->out; }
     return W;
 }
+template<bool SH, bool UP> int launch_window_type(int type, const WArgs& W, cudaStream_t s) {
+    switch (type) {
+        case MAYA_Q8_0: case MAYA_Q4_K: case MAYA_Q5_K: case MAYA_Q6_K: case MAYA_IQ4_XS: return launch_window_group<SH, UP, 0>(type, W, s);
+        default: return launch_window_group<SH, UP, 1>(type, W, s);
+    }
+}
 }  // namespace
 
 int window_gate_up(int gu_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t up_off, float limit, const void* xq,

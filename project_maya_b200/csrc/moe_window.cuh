@@ -638,15 +638,21 @@ template<int T, bool SH, bool UP> int launch_window(const WArgs& A, cudaStream_t
 
 }  // namespace
 
-// Instantiated in moe_window_{up,down}[_sh].cu, one translation unit each: they compile side by side.
-template<bool SH, bool UP> int launch_window_type(int type, const WArgs& A, cudaStream_t s) {
+// Instantiated in moe_window_{up,down}[_sh]_{k,i}.cu - GROUP 0: Q8_0, the K-quants and IQ4_XS, 1: the codebook types - a
+// translation unit each, so that they compile side by side.
+template<bool SH, bool UP, int GROUP> int launch_window_group(int type, const WArgs& A, cudaStream_t s) {
 #define MAYA_WIN(TT) case TT: return launch_window<TT, SH, UP>(A, s);
-    switch (type) {
-        MAYA_WIN(MAYA_Q8_0) MAYA_WIN(MAYA_Q4_K) MAYA_WIN(MAYA_IQ2_S) MAYA_WIN(MAYA_IQ3_S) MAYA_WIN(MAYA_Q5_K)
-        MAYA_WIN(MAYA_Q6_K) MAYA_WIN(MAYA_IQ4_XS) MAYA_WIN(MAYA_IQ3_XXS) MAYA_WIN(MAYA_IQ2_XXS) MAYA_WIN(MAYA_IQ1_S)
-        default: return refuse(MAYA_ERR_TYPE);
+    if constexpr (GROUP == 0) {
+        switch (type) {
+            MAYA_WIN(MAYA_Q8_0) MAYA_WIN(MAYA_Q4_K) MAYA_WIN(MAYA_Q5_K) MAYA_WIN(MAYA_Q6_K) MAYA_WIN(MAYA_IQ4_XS)
+        }
+    } else {
+        switch (type) {
+            MAYA_WIN(MAYA_IQ2_S) MAYA_WIN(MAYA_IQ3_S) MAYA_WIN(MAYA_IQ3_XXS) MAYA_WIN(MAYA_IQ2_XXS) MAYA_WIN(MAYA_IQ1_S)
+        }
     }
 #undef MAYA_WIN
+    return refuse(MAYA_ERR_TYPE);
 }
 
 }  // namespace maya

@@ -30,7 +30,8 @@ struct WArgs {
     float* sh_out;                   // down out: [n_tok][n_embd]
 };
 
-// By type; SH: with A.sh.  kWindowTooWide: the shapes leave no room for a column, nothing launched.
-template<bool SH, bool UP> int launch_window_type(int type, const WArgs& A, cudaStream_t s);
+// By type (GROUP 0: Q8_0, the K-quants and IQ4_XS, 1: the codebook types); SH: with A.sh.  kWindowTooWide: the shapes leave no
+// room for a column, nothing launched.
+template<bool SH, bool UP, int GROUP> int launch_window_group(int type, const WArgs& A, cudaStream_t s);
 
 }  // namespace maya

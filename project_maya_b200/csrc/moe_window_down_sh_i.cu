@@ -1,0 +1,6 @@
+// moe_window_down_sh_i.cu - the window kernel, down with a Q8_0 shared expert, the codebook types (see moe_window.cuh).
+#include "moe_window.cuh"
+
+namespace maya {
+template int launch_window_group<true, false, 1>(int, const WArgs&, cudaStream_t);
+}

@@ -20,6 +20,8 @@ __global__ void __launch_bounds__(1024) expert_count_kernel(const int* __restric
                                                             int* __restrict__ rank) {
     const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __shared__ int s_wc[32];
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int per = ((n + 1023) / 1024) * 32;
     const int i0 = warp * per, i1 = min(n, i0 + per);
     int cnt = 0;
@@ -50,6 +52,8 @@ __global__ void __launch_bounds__(1024) expert_count_kernel(const int* __restric
 __global__ void __launch_bounds__(1024) expert_bounds_kernel(const int* __restrict__ counts, int n_expert,
                                                              int* __restrict__ bounds) {
     __shared__ int s_part[1024];
+    grid_launch_dependents();
+    grid_dependency_wait();
     const int tid = threadIdx.x, per = (n_expert + 1023) / 1024;
     int local = 0;
     for (int j = 0; j < per; ++j) {
@@ -76,6 +80,8 @@ __global__ void __launch_bounds__(256) expert_scatter_kernel(const int* __restri
                                                              const int* __restrict__ base, int n, int k,
                                                              int* __restrict__ row_tok, int* __restrict__ pos) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
     if (i >= n) return;
     const int row = base[ids[i]] + rank[i];
     row_tok[row] = i / k;
@@ -109,6 +115,8 @@ __global__ void __launch_bounds__(256) combine_rows4_kernel(const float* __restr
                                                             const float* __restrict__ w, const float* __restrict__ sh,
                                                             int k, int n_embd, float* __restrict__ ffn) {
     const int t = blockIdx.y, e = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    grid_launch_dependents();
+    grid_dependency_wait();
     if (e >= n_embd) return;
     const int kk = K > 0 ? K : k;
     float4 m = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -210,19 +218,19 @@ using namespace maya;
 extern "C" int maya_expert_count(const int* ids, int n, int n_expert, int* counts, int* rank, void* stream) {
     if (n_expert <= 0) return MAYA_OK;
     if (!counts || n < 0 || (n > 0 && (!ids || !rank))) return refuse(MAYA_ERR_ARG);
-    expert_count_kernel<<<n_expert, 1024, 0, as_stream(stream)>>>(ids, n, counts, rank);
+    launch_dependent(expert_count_kernel, dim3((unsigned) n_expert), dim3(1024), 0, as_stream(stream), ids, n, counts, rank);
     return note_launch("expert_count");
 }
 extern "C" int maya_expert_bounds(const int* counts, int n_expert, int* bounds, void* stream) {
     if (!counts || !bounds || n_expert <= 0) return refuse(MAYA_ERR_ARG);
-    expert_bounds_kernel<<<1, 1024, 0, as_stream(stream)>>>(counts, n_expert, bounds);
+    launch_dependent(expert_bounds_kernel, dim3(1), dim3(1024), 0, as_stream(stream), counts, n_expert, bounds);
     return note_launch("expert_bounds");
 }
 extern "C" int maya_expert_scatter(const int* ids, const int* rank, const int* base, int n, int k, int* row_tok, int* pos,
                                    void* stream) {
     if (n <= 0) return MAYA_OK;
     if (!ids || !rank || !base || !row_tok || !pos || k <= 0) return refuse(MAYA_ERR_ARG);
-    expert_scatter_kernel<<<(n + 255) / 256, 256, 0, as_stream(stream)>>>(ids, rank, base, n, k, row_tok, pos);
+    launch_dependent(expert_scatter_kernel, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, as_stream(stream), ids, rank, base, n, k, row_tok, pos);
     return note_launch("expert_scatter");
 }
 extern "C" int maya_swiglu_rows(const float* gu, float* h, int rows, int n_ff, float limit, int ld_h, void* stream) {
@@ -239,8 +247,8 @@ extern "C" int maya_moe_combine_rows(const float* out, const int* pos, const flo
     if (!out || !pos || !w || !ffn || k <= 0 || n_embd <= 0) return refuse(MAYA_ERR_ARG);
     if (n_embd % 4 == 0 && aligned16(out) && aligned16(ffn) && (!sh || aligned16(sh))) {
         const dim3 grid4((unsigned) ((n_embd / 4 + 255) / 256), (unsigned) T);
-        if (k == 8) combine_rows4_kernel<8><<<grid4, 256, 0, as_stream(stream)>>>(out, pos, w, sh, k, n_embd, ffn);
-        else combine_rows4_kernel<0><<<grid4, 256, 0, as_stream(stream)>>>(out, pos, w, sh, k, n_embd, ffn);
+        launch_dependent(k == 8 ? combine_rows4_kernel<8> : combine_rows4_kernel<0>, grid4, dim3(256), 0, as_stream(stream), out, pos, w, sh, k,
+                         n_embd, ffn);
         return note_launch("moe_combine_rows");
     }
     const dim3 grid((unsigned) ((n_embd + 255) / 256), (unsigned) T);

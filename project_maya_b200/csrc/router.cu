@@ -15,6 +15,8 @@ __global__ void __launch_bounds__(kRouterThreads) router_softmax_kernel(const fl
     extern __shared__ double s_ex[];          // n_expert doubles
     __shared__ RouterShared sh;
     const int t = blockIdx.x, tid = threadIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
     route_softmax<PER, BlockSync>(logits + (size_t) t * n_expert, n_expert, k, tid, blockDim.x, s_ex, sh);
     if (tid < k) {
         ids[(size_t) t * k + tid] = sh.ids[tid];
@@ -31,6 +33,8 @@ __global__ void __launch_bounds__(kRouterThreads) router_sigmoid_kernel(const fl
     extern __shared__ double s_keys[];        // n_expert 64-bit words
     __shared__ RouterShared sh;
     const int t = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
     route_sigmoid<PER, BlockSync>(logits + (size_t) t * n_expert, bias, n_expert, k, w_scale, norm_w, tid, nt, s_keys, sh);
     if (tid < k) {
         ids[(size_t) t * k + tid] = sh.ids[tid];
@@ -57,10 +61,10 @@ extern "C" int maya_router_top10(const float* logits, int n_tokens, int n_expert
     const int per = (n_expert + nt - 1) / nt;
     const size_t smem = (size_t) n_expert * sizeof(double);
     cudaStream_t s = as_stream(stream);
-    if (per <= 1) router_softmax_kernel<1><<<n_tokens, nt, smem, s>>>(logits, n_expert, k, ids, weights);
-    else if (per <= 2) router_softmax_kernel<2><<<n_tokens, nt, smem, s>>>(logits, n_expert, k, ids, weights);
-    else if (per <= 4) router_softmax_kernel<4><<<n_tokens, nt, smem, s>>>(logits, n_expert, k, ids, weights);
-    else router_softmax_kernel<8><<<n_tokens, nt, smem, s>>>(logits, n_expert, k, ids, weights);
+    if (per <= 1) launch_dependent(router_softmax_kernel<1>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, n_expert, k, ids, weights);
+    else if (per <= 2) launch_dependent(router_softmax_kernel<2>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, n_expert, k, ids, weights);
+    else if (per <= 4) launch_dependent(router_softmax_kernel<4>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, n_expert, k, ids, weights);
+    else launch_dependent(router_softmax_kernel<8>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, n_expert, k, ids, weights);
     return note_launch("router_top10");
 }
 
@@ -73,9 +77,9 @@ extern "C" int maya_router_sigmoid(const float* logits, const float* bias, int n
     const int per = (n_expert + nt - 1) / nt;
     const size_t smem = (size_t) n_expert * sizeof(double);
     cudaStream_t s = as_stream(stream);
-    if (per <= 1) router_sigmoid_kernel<1><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
-    else if (per <= 2) router_sigmoid_kernel<2><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
-    else if (per <= 4) router_sigmoid_kernel<4><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
-    else router_sigmoid_kernel<8><<<n_tokens, nt, smem, s>>>(logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    if (per <= 1) launch_dependent(router_sigmoid_kernel<1>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    else if (per <= 2) launch_dependent(router_sigmoid_kernel<2>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    else if (per <= 4) launch_dependent(router_sigmoid_kernel<4>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
+    else launch_dependent(router_sigmoid_kernel<8>, dim3((unsigned) n_tokens), dim3((unsigned) nt), smem, s, logits, bias, n_expert, k, w_scale, norm_w, ids, weights);
     return note_launch("router_sigmoid");
 }
