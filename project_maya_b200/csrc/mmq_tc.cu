@@ -75,7 +75,8 @@ template<int T> constexpr int kBRing = kBStages<T> * kBStage;
 // is bound by those instructions: 64 tokens of IQ3_S 553 -> 475 us, 777 of IQ2_S 1436 -> 1316.)
 template<int T> constexpr int kCopies = T == MAYA_IQ2_S ? 4 : T == MAYA_IQ3_S ? 16 : 0;
 template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 16 * kCopies<T> : T == MAYA_IQ3_S ? 512 * 8 * kCopies<T> : 0;
-template<int T> constexpr int kTabOff = kBRing<T> + kUnits<T> * kUnitBytes<T>;
+// the codebook lies behind the rings - and behind a finished tile, which takes their place: 160 rows of 256 f32 values
+template<int T> constexpr int kTabOff = kBRing<T> + kUnits<T> * kUnitBytes<T> > TN * TM * 4 ? kBRing<T> + kUnits<T> * kUnitBytes<T> : TN * TM * 4;
 template<int T> constexpr size_t kSmemBytes = (size_t) kTabOff<T> + kTabBytes<T>;
 static_assert(kUnits<MAYA_Q4_K> <= kMaxUnits && kUnits<MAYA_Q8_0> <= kMaxUnits && kUnits<MAYA_IQ2_S> <= kMaxUnits &&
               kUnits<MAYA_IQ3_S> <= kMaxUnits, "one mbarrier pair per raw unit");

@@ -233,6 +233,30 @@ def test_fused_glu_equals_product_then_swiglu_bitwise(T, api, t, limit):
     assert T.equal(hq, want_hq)
 
 
+@pytest.mark.parametrize("t", [H.Q4_K, H.Q8_0, H.IQ2_S, H.IQ3_S])
+@pytest.mark.parametrize("rows", [160, 157, 129])
+def test_tall_groups_equal_short_groups_bitwise(T, api, t, rows):
+    """Groups of up to 160 rows, whose finished tiles fill the rings' shared memory, on blocks that take several tiles one after
+    another: the bits of the same rows in groups of half the height."""
+    n, cols, w_rows, half = 40, 2048, 2048, rows // 2
+    w = synth_matrices(T, api, t, n, w_rows, cols, 41)
+    xq = api.mmq_quantize(dev(T, H.rng_for("tall", t, rows).standard_normal((n * rows, cols)).astype(np.float32)), None, t)
+    image = xq.view(n, rows, -1)
+
+    def run(x, c):
+        out = T.zeros((n * c, w_rows), dtype=T.float32, device="cuda")
+        err = T.zeros(1, dtype=T.int32, device="cuda")
+        api.mmq_run(api.mmq_product(w, t, w_rows, cols, w.shape[1], n, x, dev(T, np.arange(n + 1, dtype=np.int32) * c), None, n * c, out, w_rows, error=err))
+        T.cuda.synchronize()
+        assert int(err.item()) == 0
+        return out.view(n, c, w_rows)
+
+    got = run(xq, rows)
+    assert T.isfinite(got).all()
+    assert T.equal(got[:, :half], run(image[:, :half].contiguous(), half))
+    assert T.equal(got[:, half:], run(image[:, half:].contiguous(), rows - half))
+
+
 @pytest.mark.parametrize("ta,tb,counts,n_ff", [
     (H.Q8_0, H.Q4_K, [1, 0, 161, 7, 320, 33], 256),                                       # fewer tiles than blocks, remainders of 160 rows
     (H.IQ2_S, H.IQ3_S, [5] * 24 + [0] * 3 + [170] * 3, 2048),                             # several rounds of tiles
