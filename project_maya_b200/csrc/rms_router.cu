@@ -24,7 +24,7 @@ namespace {
 
 constexpr int kRmsThreads = 256;
 constexpr int kRmsWarps = kRmsThreads / 32;
-constexpr int kAhead = 4;              // 16-byte pieces of a router row a lane holds before the norm is known
+constexpr int kAhead = 8;              // 16-byte pieces of a router row a lane holds before the norm is known
 
 // Dot of 16 bytes of a router row with the values of x they meet.
 template<bool BF16> __device__ __forceinline__ float dot16(const uint4 r, const float* xv, float acc) {
