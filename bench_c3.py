@@ -85,7 +85,7 @@ def run(torch, api) -> dict:
            "us_per_step": us, "tok_s_layer": T * 1e6 / us, "launch": f"CUDA graph of {N_WIN} windows",
            "roofline": {"bound": "hbm", "algorithmic_bytes_per_step": bytes_step, "achieved": bytes_step / us / 1e3, "peak": peak,
                         "peak_kind": kind, "unit": "GB/s", "frac": bytes_step / us / 1e3 / peak,
-                        "kernels": "win_group + gate_up_kernel + down_groups_kernel + win_combine_kernel per window"},
+                        "kernels": "prep_kernel + window_kernel (gate/up) + window_kernel (down) + win_combine_kernel per window"},
            "error": layer.error()}
 
     # ---- the same windows through the prompt path (tensor-core grouped product over f16 operands: within 1e-2 of the

@@ -15,9 +15,9 @@ import sys
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
-PHASES = [(1, "set-up (tile scan, barriers, tensor-memory allocation)"), (2, "to the first product"), (3, "K loop"),
+PHASES = [(2, "to the first product"), (3, "K loop"),
           (4, "drain, expanding warps meet"), (5, "tensor memory -> SwiGLU -> shared memory"),
-          (6, "q8_1 rounding of the tile"), (7, "bulk stores (down: + tensor memory -> shared memory)")]
+          (6, "q8_1 rounding of the tile"), (7, "stores done (down: + tensor memory -> shared memory)")]
 KINDS = ["Q8_0 / IQ2_S down", "Q8_0 / IQ2_S gate/up", "Q4_K / IQ3_S down", "Q4_K / IQ3_S gate/up"]
 
 
