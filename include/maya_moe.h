@@ -279,8 +279,10 @@ MAYA_API int maya_mmq_run_glu(const maya_mmq_product* p, float limit, void* stre
  * same bits.  down[i] multiplies the h that gate_up[i] leaves in its xq_out (down[i].xq == gate_up[i].xq_out; the same n, bounds,
  * expert_map and total_rows), and its blocks start as soon as SMs have no gate/up tile left, each tile waiting only for its own
  * rows of h (bounded: see `error`), so that the last, partly filled round of tiles of one product runs beside the next.
- * counters: maya_mmq_chain_bytes(total_rows, matrices of all pairs, n_pairs) bytes, zeroed before the first use (and after an
- * error); a chain leaves them zero.  One buffer serves one stream at a time. */
+ * down[i].w_cols == gate_up[i].w_rows / 2.  Every product is checked before the first is launched: a refused chain has launched
+ * nothing and not touched the counters.
+ * counters: maya_mmq_chain_bytes(total_rows, matrices of all pairs, n_pairs) bytes, zeroed before the first use and after a chain
+ * whose `error` word was set; every other chain leaves them zero.  One buffer serves one stream at a time. */
 MAYA_API size_t maya_mmq_chain_bytes(int64_t total_rows, int n_matrices, int n_pairs);
 MAYA_API int maya_mmq_run_chain(const maya_mmq_product* gate_up, const maya_mmq_product* down, int n_pairs, float limit,
                                 void* counters, size_t counter_bytes, void* stream);

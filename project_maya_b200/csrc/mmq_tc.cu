@@ -985,6 +985,9 @@ bool make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, const void* base
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// An upper bound of sum(ceil(rows_e / 160)), known without the counts.
+int64_t most_groups(const maya_mmq_product* p) { return (p->total_rows > 0 ? p->total_rows / TN : 0) + p->n; }
+
 template<int T, bool GLU>
 int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
     const int64_t mat_rows = p->w_rows, K = p->w_cols;
@@ -1016,8 +1019,7 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
     constexpr size_t smem = kSmemBytes<T>;
     if (cudaFuncSetAttribute(mmq_kernel<T, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
         return note_launch("mmq smem attribute");
-    const int64_t groups = p->total_rows / TN + p->n;   // an upper bound of sum(ceil(rows_e / 160)), known without the counts
-    if (groups > 65535) return refuse(MAYA_ERR_LIMIT);
+    const int64_t groups = most_groups(p);
     const int slab = GLU ? 128 : TM, sms = sm_count();
     if (sms <= 0) return refuse(MAYA_ERR_DEVICE);
     const int64_t most = (int64_t) ((A.w_rows + slab - 1) / slab) * groups;      // tiles there can be
@@ -1026,23 +1028,33 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
     return note_launch("mmq");
 }
 
-struct Chain { unsigned *claim, *ready; int ready_slabs; bool first; };
-
-int run_product(const maya_mmq_product* p, bool glu, float limit, const Chain* chain, cudaStream_t s) {
-    if (!p || !p->w || !p->xq || !p->bounds) return refuse(MAYA_ERR_ARG);
-    if (!p->dst && !(glu && p->xq_out)) return refuse(MAYA_ERR_ARG);
-    if (!maya_mmq_supported(p->type)) return refuse(MAYA_ERR_TYPE);
-    if ((p->type == MAYA_IQ2_S || p->type == MAYA_IQ3_S) && p->w_cols % 2048) return refuse(MAYA_ERR_ARG);   // 16-byte aligned rows
+// Everything about a product that can be refused, before anything is launched.
+int check_product(const maya_mmq_product* p, bool glu) {
+    if (!p || !p->w || !p->xq || !p->bounds) return MAYA_ERR_ARG;
+    if (!p->dst && !(glu && p->xq_out)) return MAYA_ERR_ARG;
+    if (!maya_mmq_supported(p->type)) return MAYA_ERR_TYPE;
+    if ((p->type == MAYA_IQ2_S || p->type == MAYA_IQ3_S) && p->w_cols % 2048) return MAYA_ERR_ARG;   // 16-byte aligned rows
     if (p->n <= 0 || p->total_rows <= 0) return MAYA_OK;
     const int64_t out_rows = glu ? p->w_rows / 2 : p->w_rows;
-    if (p->w_cols <= 0 || p->w_cols % 256 || out_rows <= 0 || out_rows % 128 || (glu && p->w_rows % 2)) return refuse(MAYA_ERR_ARG);
+    if (p->w_cols <= 0 || p->w_cols % 256 || out_rows <= 0 || out_rows % 128 || (glu && p->w_rows % 2)) return MAYA_ERR_ARG;
     if (p->expert_bytes % (size_t) type_bytes(p->type) || p->expert_bytes % 16 || (p->dst && p->ld_dst < out_rows)) {
         std::fprintf(stderr, "maya_mmq_run: expert_bytes %zu is not a whole number of blocks and of 16 bytes, or ld_dst too small\n",
                      p->expert_bytes);
-        return refuse(MAYA_ERR_ARG);
+        return MAYA_ERR_ARG;
     }
-    if (!aligned16(p->w) || !aligned16(p->xq) || (p->xq_out && !aligned16(p->xq_out))) return refuse(MAYA_ERR_ARG);
-    if (p->dst && (!aligned16(p->dst) || p->ld_dst % 4)) return refuse(MAYA_ERR_ARG);      // rows leave as 16-byte aligned bulk copies
+    if (!aligned16(p->w) || !aligned16(p->xq) || (p->xq_out && !aligned16(p->xq_out))) return MAYA_ERR_ARG;
+    if (p->dst && (!aligned16(p->dst) || p->ld_dst % 4)) return MAYA_ERR_ARG;      // rows leave as 16-byte aligned bulk copies
+    if (most_groups(p) > 65535) return MAYA_ERR_LIMIT;
+    return MAYA_OK;
+}
+
+struct Chain { unsigned *claim, *ready; int ready_slabs; bool first; };
+
+int run_product(const maya_mmq_product* p, bool glu, float limit, const Chain* chain, cudaStream_t s) {
+    const int st = check_product(p, glu);
+    if (st != MAYA_OK) return refuse(st);
+    if (p->n <= 0 || p->total_rows <= 0) return MAYA_OK;
+    const int64_t out_rows = glu ? p->w_rows / 2 : p->w_rows;
     MmqArgs A{};
     A.w = (const uint8_t*) p->w; A.expert_bytes = p->expert_bytes; A.mat_rows = (int) p->w_rows;
     A.w_rows = (int) out_rows; A.w_cols = (int) p->w_cols; A.n = p->n; A.expert_map = p->expert_map; A.bounds = p->bounds;
@@ -1099,7 +1111,6 @@ extern "C" int maya_mmq_run_glu(const maya_mmq_product* p, float limit, void* st
     return run_product(p, true, limit, nullptr, as_stream(stream));
 }
 // Words of a chain's counters: two claim words a product, two ready words a group of a pair (an upper bound of the groups).
-static size_t chain_groups(int64_t total_rows, int n) { return (size_t) (total_rows / TN + n); }
 extern "C" size_t maya_mmq_chain_bytes(int64_t total_rows, int n_matrices, int n_pairs) {
     if (total_rows <= 0 || n_matrices <= 0 || n_pairs <= 0) return 0;
     return sizeof(unsigned) * (4 * (size_t) n_pairs + 2 * ((size_t) n_pairs * (size_t) (total_rows / TN) + (size_t) n_matrices));
@@ -1108,12 +1119,21 @@ extern "C" int maya_mmq_run_chain(const maya_mmq_product* gate_up, const maya_mm
                                   size_t counter_bytes, void* stream) {
     if (n_pairs <= 0) return MAYA_OK;
     if (!gate_up || !down || !counters || ((uintptr_t) counters & 3u)) return refuse(MAYA_ERR_ARG);
+    // Nothing is launched before every product has been looked at: a gate/up product without its down product would leave its
+    // rows counted, and the next chain on these counters would take them for its own.
     size_t need = 4 * (size_t) n_pairs;
+    auto empty = [&](int i) { return gate_up[i].n == 0 || gate_up[i].total_rows <= 0; };
     for (int i = 0; i < n_pairs; ++i) {
-        if (gate_up[i].n != down[i].n || gate_up[i].bounds != down[i].bounds || gate_up[i].expert_map != down[i].expert_map ||
-            gate_up[i].total_rows != down[i].total_rows || gate_up[i].xq_out != down[i].xq || !gate_up[i].xq_out || gate_up[i].n < 0)
+        const maya_mmq_product &g = gate_up[i], &d = down[i];
+        if (g.n != d.n || g.bounds != d.bounds || g.expert_map != d.expert_map || g.total_rows != d.total_rows || g.xq_out != d.xq ||
+            !g.xq_out || g.n < 0)
             return refuse(MAYA_ERR_ARG);
-        need += 2 * chain_groups(gate_up[i].total_rows, gate_up[i].n);
+        need += 2 * (size_t) most_groups(&g);
+        if (empty(i)) continue;
+        int st = check_product(&g, true);
+        if (st == MAYA_OK) st = check_product(&d, false);
+        if (st == MAYA_OK && d.w_cols != g.w_rows / 2) st = MAYA_ERR_ARG;          // the rows of h it reads are n_ff values long
+        if (st != MAYA_OK) return refuse(st);
     }
     if (need * sizeof(unsigned) > counter_bytes) return refuse(MAYA_ERR_LIMIT);
     unsigned* const words = (unsigned*) counters;
@@ -1123,10 +1143,13 @@ extern "C" int maya_mmq_run_chain(const maya_mmq_product* gate_up, const maya_mm
         for (int i = 0; i < n_pairs; ++i) {
             const maya_mmq_product& p = pass ? down[i] : gate_up[i];
             const Chain c{words + 4 * i + 2 * pass, ready, (int) (gate_up[i].w_rows / 256), first};
-            ready += 2 * chain_groups(p.total_rows, p.n);
-            if (p.n == 0 || p.total_rows <= 0) continue;
+            ready += 2 * most_groups(&p);
+            if (empty(i)) continue;
             const int st = run_product(&p, pass == 0, limit, &c, as_stream(stream));
-            if (st != MAYA_OK) return st;
+            if (st != MAYA_OK) {                     // the launch itself failed: the products before it leave counts behind
+                cudaMemsetAsync(counters, 0, need * sizeof(unsigned), as_stream(stream));
+                return st;
+            }
             first = false;
         }
     }

@@ -298,6 +298,41 @@ def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
         api.mmq_run_chain([want[0][0]], [got[0][1]], 7.0, counters)
 
 
+def test_refused_chain_launches_nothing_and_leaves_its_counters_alone(T, api, lib):
+    """A chain with one product that cannot run is refused before its first launch, whichever product it is; the next chain on the
+    same counters gives the bits of its products run one after another."""
+    t, n_ff, cols, counts = H.Q8_0, 256, 256, [70, 5, 0, 200]
+    n, total = len(counts), sum(counts)
+    w, wd = synth_matrices(T, api, t, n, 2 * n_ff, cols, 41), synth_matrices(T, api, t, n, 256, n_ff, 43)
+    bounds = dev(T, np.concatenate([[0], np.cumsum(counts)]).astype(np.int32))
+    xq = api.mmq_quantize(dev(T, H.rng_for("refused-chain").standard_normal((total, cols)).astype(np.float32)), None, t)
+    hq = T.zeros(api.mmq_q8_bytes(total, 2 * n_ff), dtype=T.uint8, device="cuda")         # (room for the wider h asked for below)
+    out = T.zeros((total, 256), dtype=T.float32, device="cuda")
+    gu = lambda **kw: api.mmq_product(**{**dict(w=w, ggml_type=t, w_rows=2 * n_ff, w_cols=cols, expert_bytes=w.shape[1], n=n, xq=xq,  # noqa: E731
+                                                 bounds=bounds, ids=None, total_rows=total, dst=None, ld_dst=n_ff, xq_out=hq), **kw})
+    dn = lambda **kw: api.mmq_product(**{**dict(w=wd, ggml_type=t, w_rows=256, w_cols=n_ff, expert_bytes=wd.shape[1], n=n, xq=hq,     # noqa: E731
+                                                 bounds=bounds, ids=None, total_rows=total, dst=out, ld_dst=256), **kw})
+    api.mmq_run_glu(gu(), H.INF)
+    api.mmq_run(dn())
+    want = out.clone()
+    counters = T.zeros(api._lib.load().maya_mmq_chain_bytes(total, 2 * n, 2), dtype=T.uint8, device="cuda")
+    T.cuda.synchronize()
+    launches = lib.maya_launch_count()
+    for bad in (dn(ld_dst=128), dn(dst=None), dn(ggml_type=H.Q5_K), dn(ggml_type=H.IQ3_S), dn(w_rows=200), dn(w_cols=2 * n_ff)):
+        for pairs in ([(gu(), bad)], [(gu(), dn()), (gu(), bad)]):
+            with pytest.raises(api.MayaError):
+                api.mmq_run_chain([p[0] for p in pairs], [p[1] for p in pairs], H.INF, counters)
+            T.cuda.synchronize()
+            assert lib.maya_launch_count() == launches and not counters.any()
+    with pytest.raises(api.MayaError):
+        api.mmq_run_chain([gu(w_rows=100)], [dn()], H.INF, counters)
+    assert lib.maya_launch_count() == launches
+    out.zero_(), hq.zero_()
+    api.mmq_run_chain([gu()], [dn()], H.INF, counters)
+    T.cuda.synchronize()
+    assert T.equal(out, want) and not counters.any()
+
+
 def test_expert_map_selects_bounds_entries(T, api):
     """A staged group: matrix i of the product owns the rows of expert expert_map[i]."""
     t, rows, cols = H.Q4_K, 128, 256
