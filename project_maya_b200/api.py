@@ -569,5 +569,10 @@ class MoePrefill:
         return ids, w, ffn
 
     def error(self) -> int:
-        """1 when a bounded wait inside a grouped-GEMM launch ran out (synchronises)."""
-        return int(self.err.item())
+        """1 when a bounded wait inside a grouped-GEMM launch ran out (synchronises; sticky).  A chain that ended that way leaves its
+        counters somewhere in between, and the next one would start from there: they are zeroed here, so that the passes after
+        this call are sound again."""
+        code = int(self.err.item())
+        if code:
+            self.chain.zero_()
+        return code

@@ -413,6 +413,23 @@ def test_prefill_layer_small(T, api, oracle, t, n_tok, E):
         assert H.rel_err(got[tok], want) <= 2.5e-2 and H.rel_l2(got[tok], want) <= 2.5e-2
 
 
+def test_prefill_layer_recovers_after_a_chain_that_gave_up(T, api):
+    """A chain whose bounded wait ran out leaves its counters part-way and sets the error word - the state is made here on the host;
+    error() reports it and the passes after it give the right bits again."""
+    cfg = api.MoeLayerConfig(512, 256, 8, 2, H.Q4_K, H.Q4_K)
+    experts = T.empty((8, cfg.blob_bytes), dtype=T.uint8, device="cuda")
+    api.synth_weights(H.Q4_K, 5, 0.02, experts.numel() // H.row_bytes(H.Q4_K, 256), 256, experts)
+    layer = api.MoePrefill(cfg, experts, max_tokens=40)
+    passes = [(dev(T, H.router_logits("recover", 40, 8, None)) * s, dev(T, H.activations("recover", 40, 512, "f32")) * s) for s in (1.0, -0.5)]
+    want = [layer.forward(*p)[2].clone() for p in passes]
+    assert layer.error() == 0 and not T.equal(want[0], want[1])
+    layer.chain.fill_(1)
+    layer.err.fill_(1)
+    assert layer.error() == 1
+    for p, w in zip(passes, want):
+        assert T.equal(layer.forward(*p)[2], w)
+
+
 def build_pools(T, api, cfg, types, seed, sigma=0.02):
     """One pool of synthetic [gate | up | down] blobs per storage type; returns (pools for MoePrefill, blob of expert e)."""
     H_, FF = cfg["n_embd"], cfg["n_ff"]
