@@ -149,12 +149,17 @@ typedef struct maya_moe_win {
     unsigned long long* grp_ptr;         /* scratch: [T * 8] */
     int* grp_start;                      /* scratch: [T * 8 + 1] */
     int* grp_ent;                        /* scratch: [T * 8] */
-    int* n_groups;                       /* scratch: [1] */
+    int* n_groups;                       /* scratch: [1]; -1 after a call whose bounded wait ran out: its outputs are not valid */
     int T, k, n_embd, n_ff;
     float limit;
     size_t down_off;
 } maya_moe_win;
 MAYA_API int maya_moe_win_experts(int gu_type, int d_type, const maya_moe_win* w, void* stream);
+/* No counterpart in the reference: the same with the caller's bound on the kernels' waits for weight rows (`polls` looks at a
+ * copy before a warp gives up; maya_moe_win_experts takes 2^22, some seconds) and, when one ran out, *error (NULL: not wanted)
+ * set to 1 beside n_groups. */
+MAYA_API int maya_moe_win_experts_checked(int gu_type, int d_type, const maya_moe_win* w, unsigned polls, unsigned* error,
+                                          void* stream);
 /* glmf::moe_win_group (glm_fast.hpp:468): the grouping alone. */
 MAYA_API int maya_moe_win_group(const maya_moe_win* w, void* stream);
 
@@ -329,10 +334,11 @@ typedef struct maya_moe_layer {
 } maya_moe_layer;
 /* Bytes of scratch maya_moe_layer_decode needs for n_tokens tokens.  The scratch must be 256-byte aligned and ZEROED
  * once before its first use (it holds the fused kernel's grid-barrier counter); one scratch serves one stream at a
- * time.  After a device-side barrier time-out (a block never arrived) the word returned by maya_moe_layer_error is
- * non-zero and the outputs of that and later calls on the scratch are undefined. */
+ * time.  After a device-side wait that ran out (a block never arrived at the fused kernel's barrier, weight rows of a window
+ * or a staged token never landed) the word returned by maya_moe_layer_error is non-zero and the outputs of that and later
+ * calls on the scratch are undefined. */
 MAYA_API size_t maya_moe_layer_scratch_bytes(const maya_moe_layer* L, int n_tokens);
-/* Reads the sticky barrier-error word of a layer scratch (synchronises the stream first). 0 = no error. */
+/* Reads the sticky error word of a layer scratch (synchronises the stream first). 0 = no error. */
 MAYA_API int maya_moe_layer_error(const maya_moe_layer* L, int n_tokens, const void* scratch, void* stream);
 /* Diagnostic: block 0's wall-clock stamps (ns, %globaltimer) of the last fused single-token launch on this scratch:
  * start, end of routing/quantizing, end of its gate/up work, past the grid barrier, end of down + combine, end of the

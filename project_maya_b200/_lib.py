@@ -88,6 +88,7 @@ _SIGNATURES = {
     "maya_moe_down": (c_int, [c_int, C.POINTER(MoePlan), c_int, c_int, c_int, c_size_t, c_void_p, c_void_p, c_void_p,
                               c_void_p]),
     "maya_moe_win_experts": (c_int, [c_int, c_int, C.POINTER(MoeWin), c_void_p]),
+    "maya_moe_win_experts_checked": (c_int, [c_int, c_int, C.POINTER(MoeWin), C.c_uint, c_void_p, c_void_p]),
     "maya_moe_win_group": (c_int, [C.POINTER(MoeWin), c_void_p]),
     "maya_expert_scratch_bytes": (c_size_t, [c_int64, c_int64]),
     "maya_expert_grouped": (c_int, [C.POINTER(ExpertLayout), c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,

@@ -161,6 +161,12 @@ def moe_win_experts(gu_type: int, d_type: int, win: MoeWin, stream=None) -> None
     _check("moe_win_experts", _lib.load().maya_moe_win_experts(gu_type, d_type, C.byref(win), _stream(stream)))
 
 
+def moe_win_experts_checked(gu_type: int, d_type: int, win: MoeWin, polls: int, error=None, stream=None) -> None:
+    """moe_win_experts with the caller's bound on the waits for weight rows; error: int32 [1], set to 1 when one ran out."""
+    _check("moe_win_experts_checked",
+           _lib.load().maya_moe_win_experts_checked(gu_type, d_type, C.byref(win), polls, _ptr(error), _stream(stream)))
+
+
 def native_expert_scratch_bytes(cap_entries: int, n_ff: int) -> int:
     return int(_lib.load().maya_expert_scratch_bytes(cap_entries, n_ff))
 

@@ -32,6 +32,7 @@ inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+constexpr unsigned kMbarPolls = 1u << 22;   // how often a warp looks at an mbarrier before it gives up (seconds)
 inline bool aligned16(const void* p) { return (((uintptr_t) p) & 15u) == 0; }
 
 // ---------------------------------------------------------------- GGUF block geometry

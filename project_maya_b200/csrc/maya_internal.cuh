@@ -37,17 +37,24 @@ struct SharedArgs {
     void* hq;
     float* out;
 };
+// How often a warp looks at its rows' copies before it gives up, and who is told: `error` (optional, a sticky word) is set to 1 and
+// *n_groups, the launch's group count, to -1.
+struct WaitArgs {
+    int* n_groups;
+    unsigned* error;
+    unsigned polls;
+};
 inline bool window_fits(int n_embd, int n_ff, int n_ff_sh) { return n_embd <= 8192 && n_ff <= 8192 && n_ff_sh <= 8192; }
 int window_gate_up(int gu_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t up_off, float limit, const void* xq,
-                   size_t xq_stride, void* hq, const SharedArgs* sh, cudaStream_t s);
+                   size_t xq_stride, void* hq, const SharedArgs* sh, const WaitArgs& wait, cudaStream_t s);
 int window_down(int d_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t down_off, const void* hq, float* part,
-                const SharedArgs* sh, cudaStream_t s);
+                const SharedArgs* sh, const WaitArgs& wait, cudaStream_t s);
 int win_combine(const unsigned long long* plan_ptr, const float* plan_w, int T, int k, int n_embd, const float* part,
                 const float* cpu_part, const int* cpu_flag, const float* sh_out, float* out, size_t out_stride,
                 cudaStream_t s);
 
-int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, const maya_peer_ar* ar, int mi,
-                unsigned seq, cudaStream_t s);
+int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, unsigned polls, unsigned* error,
+                const maya_peer_ar* ar, int mi, unsigned seq, cudaStream_t s);
 
 // The fused single-token layer kernel (moe_fused.cu).
 bool fused_t1_supported(const maya_moe_layer& L);

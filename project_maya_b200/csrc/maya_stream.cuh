@@ -1,5 +1,5 @@
 // maya_stream.cuh - mbarrier and bulk-copy (TMA) helpers: rows streamed into shared memory with completion counted on an
-// mbarrier.  Used by the prompt-path GEMM (mmq_tc.cu).
+// mbarrier.  Used by the window kernel (moe_window.cuh) and the prompt-path GEMM (mmq_tc.cu).
 //
 // The copies are plain (non-multicast) bulk copies from this GPU's own memory.  Every wait on an mbarrier is bounded;
 // a wait that runs out returns false and the caller carries on to its end without touching the data.
@@ -57,9 +57,9 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait (every lane polls).  false: gave up.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    for (unsigned i = 0; i < (1u << 22); ++i) {
+// Bounded wait (every lane polls, at most `polls` times).  false: gave up.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned polls = kMbarPolls) {
+    for (unsigned i = 0; i < polls; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (i > 64) __nanosleep(32);
     }

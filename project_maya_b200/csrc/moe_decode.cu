@@ -596,9 +596,9 @@ int win_combine_ar(const unsigned long long* plan_ptr, const float* plan_w, int 
 
 // moe_win_experts; with `ar` the cross-rank sum of out[T][n_embd] (contiguous) runs inside the combine launch.  grouped: the
 // group arrays are filled already.  sh: the shared expert in the same launches (w->sh_out == sh->out); the caller has asked
-// window_fits.
-int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, const maya_peer_ar* ar, int mi,
-                unsigned seq, cudaStream_t s) {
+// window_fits.  polls, error: see WaitArgs.
+int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, unsigned polls, unsigned* error,
+                const maya_peer_ar* ar, int mi, unsigned seq, cudaStream_t s) {
     if (!w || !w->plan_w || !w->xq || !w->hq || !w->part || !w->out) return refuse(MAYA_ERR_ARG);
     if (w->cpu_flag != nullptr && w->cpu_part == nullptr) return refuse(MAYA_ERR_ARG);
     int st = check_shapes(gu_type, d_type, w->k, w->n_embd, w->n_ff);
@@ -617,12 +617,13 @@ int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, co
     A.n_groups = w->n_groups;
     A.ent_slot = w->grp_ent;
     A.tok_from_slot = 1;
-    st = window_gate_up(gu_type, A, cap, w->n_embd, w->n_ff, up_off, w->limit, w->xq, w->xq_stride, w->hq, sh, s);
+    const WaitArgs wait{w->n_groups, error, polls};
+    st = window_gate_up(gu_type, A, cap, w->n_embd, w->n_ff, up_off, w->limit, w->xq, w->xq_stride, w->hq, sh, wait, s);
     if (st == kWindowTooWide)
         st = gate_up_groups(gu_type, A, cap, w->n_embd, w->n_ff, up_off, w->limit, w->xq, w->xq_stride, w->hq, nullptr, 0, nullptr, 0,
                             nullptr, s);
     if (st != MAYA_OK) return st;
-    st = window_down(d_type, A, cap, w->n_embd, w->n_ff, w->down_off, w->hq, w->part, sh, s);
+    st = window_down(d_type, A, cap, w->n_embd, w->n_ff, w->down_off, w->hq, w->part, sh, wait, s);
     if (st == kWindowTooWide) st = down_groups(d_type, A, cap, w->n_embd, w->n_ff, w->down_off, w->hq, w->part, s);
     if (st != MAYA_OK) return st;
     if (ar != nullptr)
@@ -672,7 +673,10 @@ extern "C" int maya_moe_win_group(const maya_moe_win* w, void* stream) {
 }
 
 extern "C" int maya_moe_win_experts(int gu_type, int d_type, const maya_moe_win* w, void* stream) {
-    return win_experts(gu_type, d_type, w, false, nullptr, nullptr, 0, 0u, as_stream(stream));
+    return win_experts(gu_type, d_type, w, false, nullptr, kMbarPolls, nullptr, nullptr, 0, 0u, as_stream(stream));
+}
+extern "C" int maya_moe_win_experts_checked(int gu_type, int d_type, const maya_moe_win* w, unsigned polls, unsigned* error, void* stream) {
+    return win_experts(gu_type, d_type, w, false, nullptr, polls, error, nullptr, 0, 0u, as_stream(stream));
 }
 
 extern "C" size_t maya_expert_scratch_bytes(int64_t cap_entries, int64_t n_ff) {

@@ -27,7 +27,7 @@ struct Scratch {
     uint8_t* sh_hq;              // [T][n_ff_sh/32] q8_1
     float* sh_out;               // [T][n_embd]
     float* h;                    // the fused single-token kernel's h: q8_1 image, shared-unit halves, counters
-    unsigned* sync;              // [16]: the fused kernel's barrier counter, epoch, error word; [3] prep_kernel's ticket; stamps (zero
+    unsigned* sync;              // [16]: the fused kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket; stamps (zero
                                  // before first use)
     size_t bytes;
 };
@@ -333,7 +333,7 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
     W.limit = L->limit;
     W.down_off = down_off;
     // one token: a window of one, its cross-rank sum a launch of its own; more: with `ar` the sum runs in the combine launch
-    st = win_experts(L->gu_type, L->d_type, &W, true, ride ? &sh : nullptr, T > 1 ? ar : nullptr, mi, seq, s);
+    st = win_experts(L->gu_type, L->d_type, &W, true, ride ? &sh : nullptr, kMbarPolls, S.sync + 2, T > 1 ? ar : nullptr, mi, seq, s);
     if (st == MAYA_OK && T == 1 && ar != nullptr) st = maya_allreduce_peer(out, L->n_embd, ar, mi, seq, stream);
     return st == MAYA_OK ? hc_post_tokens(hc, out, T, L->n_embd, stream) : st;
 }

@@ -22,9 +22,9 @@
 //
 // Plain bulk copies (one destination: this block) of this GPU's own memory.  A row need not start on a 16-byte boundary: the
 // aligned window around a segment is copied (expert blobs are 16-byte aligned and a whole number of 16-byte words long, so
-// it stays inside).  Every wait is bounded; one that runs out makes the block skip what is left (its outputs are then
-// missing) after the copies in flight were given the same bounded time to land.  A blob that is not 16-byte aligned is
-// copied with ordinary loads instead.
+// it stays inside).  A blob that is not 16-byte aligned is copied with ordinary loads instead.  Every wait is bounded.  A warp whose
+// wait ran out asks for nothing more, and its block leaves - together, at the next barrier - after the copies in flight have had
+// the same bounded time to land; the outputs of what was left are missing, and the error word and the group count say so.
 #pragma once
 
 #include "maya_dots.cuh"
@@ -220,7 +220,8 @@ struct WShared {
     uint64_t full[16][kWStages];
     WJob job[kWMaxJobs];
     long long cost[kWMaxJobs + 1];   // cost of the jobs before job j
-    int njobs, fail;
+    int njobs;
+    int gave_up[16];                 // a wait of this warp ran out
     float s_g[2][kWNC][32], s_u[2][kWNC][32];
     WKind kind[2];
 };
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     grid_launch_dependents();
     if (lane == 0) {
         for (int s = 0; s < kWStages; ++s) mbar_init(&sh.full[warp][s], RW);
-        if (warp == 0) sh.fail = 0;
+        sh.gave_up[warp] = 0;
         if (warp < 2) {
             WKind& k = sh.kind[warp];
             const int ff = warp ? A.n_ff_sh : A.n_ff;
@@ -354,11 +355,12 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             }
         }
     } else {
-        int ng = A.n_groups ? *A.n_groups : A.cap;
-        ng = min(min(ng, A.cap), kWMaxGroups);
+        int ng = *A.n_groups;
+        const bool lost = ng < 0;                                // a wait of the launch in front ran out: no work
+        ng = max(0, min(min(ng, A.cap), kWMaxGroups));
         int base = 0;
         long long run = 0;
-        const int nsh = SH && A.sh != nullptr ? (A.n_tok + A.ncm - 1) / A.ncm : 0;
+        const int nsh = SH && A.sh != nullptr && !lost ? (A.n_tok + A.ncm - 1) / A.ncm : 0;
         const WKind &kr = sh.kind[0], &ks = sh.kind[1];
         for (int g0 = 0; g0 < ng + nsh; g0 += 32) {              // a lane: one group, or one of the shared expert's jobs
             const int g = g0 + lane;
@@ -436,7 +438,9 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         else return base + (size_t) (RW * unit + r) * k.rb;
     };
     // ---- the stream: what the warp asks for next - job, unit, segment, and which of the segment's stages
-    int pj = job, pc = unit0 + off, ps = 0, pq = 0, pstage = 0;
+    int pj = job, pc = unit0 + off, ps = 0, pq = 0;
+    uint32_t asked = 0;                                          // stages asked for, modulo 2 kWStages: the next one's place is asked % kWStages
+    static_assert(kWStages == 2, "a stage is a bit of `asked`");
     auto ask = [&] {
         while (pj < njobs && pj <= job1 && pc >= limit_of(pj)) { ++pj; pc = off; }
         if (pj >= njobs || pj > job1) return;
@@ -444,7 +448,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         const WKind& k = sh.kind[SH ? J.shared : 0];
         __syncwarp();                                            // every lane has read the stage's last bytes
         const uint32_t at = (uint32_t) (ps * k.bytes), len = min((uint32_t) k.bytes, (uint32_t) k.rb - at);
-        const uint32_t dst = ring + pstage * kStage;
+        const uint32_t pstage = asked & 1u, dst = ring + pstage * kStage;
         const int rows = SH ? RW / k.split : RW, first = SH ? pq * rows : 0;      // the stage's rows
         if ((J.ptr & 15ull) == 0 && (!A.plain || (SH && J.shared))) {
             if (lane < rows) {
@@ -465,7 +469,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             __syncwarp();
             if (lane < RW) mbar_arrive_one(&sh.full[warp][pstage]);
         }
-        pstage = pstage + 1 == kWStages ? 0 : pstage + 1;
+        asked = (asked + 1) & 3u;
         if (SH && ++pq < k.split) return;
         pq = 0;
         if (++ps == k.nseg) {
@@ -478,6 +482,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     const uint32_t* const tab = s_tab + (lane % D::rep) * ((T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1);
     int stage = 0, buf = 0;
     uint32_t phase = 0;
+    auto gave_up = [&](int w) { return *(volatile int*) &sh.gave_up[w]; };
     for (int first_unit = unit0; job <= job1 && job < njobs; ++job, first_unit = 0) {
         const int limit = limit_of(job);
         if (first_unit >= limit) continue;
@@ -486,7 +491,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         const WKind& K = sh.kind[shd ? 1 : 0];
         const int nc = J.nc, n_in = K.n_in;
         auto slot_of = [&](int c) { return shd ? J.e0 + c : A.ent_slot ? A.ent_slot[J.e0 + c] : J.e0 + c; };     // shared: the token
-        __syncthreads();                                         // everyone is done with the old columns
+        if (__syncthreads_or(gave_up(warp))) goto leave;         // everyone is done with the old columns; or has to leave
         {
             const int nblk = n_in / 32, items = nc * nblk;
             for (int i0 = tid; i0 < items; i0 += 2 * kWThreads) {                // two q8_1 blocks a thread in flight
@@ -533,7 +538,10 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                 const int blk0 = sg * GT::blocks, ncalls = min(GT::blocks, n_in / GT::qk - blk0) * GT::cpb;
 #pragma unroll
                 for (int p = 0; p < GT::split; ++p) {
-                    if (!*(volatile int*) &sh.fail && !mbar_wait(&sh.full[warp][stage], phase)) *(volatile int*) &sh.fail = 1;    // bounded
+                    if (!__all_sync(0xffffffffu, mbar_wait(&sh.full[warp][stage], phase, A.polls))) {
+                        *(volatile int*) &sh.gave_up[warp] = 1;
+                        return;
+                    }
                     uint32_t row[RS];
 #pragma unroll
                     for (int r = 0; r < RS; ++r) row[r] = ring + stage * kStage + r * GT::pitch + ((start[p * RS + r] + so) & 15u);
@@ -545,7 +553,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             }
             // warp_sum's tree (lanes 16 apart first, then 8, 4, 2, 1) on four rows at once: after the first exchange a lane keeps two
             // of them, after the second one - six shuffles a column instead of twenty, the same additions
-            const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0, failed = *(volatile int*) &sh.fail != 0;
+            const bool up16 = (lane & 16) != 0, up8 = (lane & 8) != 0;
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 float a = up16 ? acc[2][c] : acc[0][c], b = up16 ? acc[3][c] : acc[1][c];
@@ -559,7 +567,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                     if constexpr (UP) {
                         (my_row < 2 ? sh.s_g : sh.s_u)[buf][c][2 * warp + (my_row & 1)] = v;
                     } else {
-                        if (!failed) (shd ? A.sh_out : A.part)[(size_t) slot_of(c) * A.n_embd + RW * unit + my_row] = v;
+                        (shd ? A.sh_out : A.part)[(size_t) slot_of(c) * A.n_embd + RW * unit + my_row] = v;
                     }
                 }
             }
@@ -584,18 +592,23 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             unit_any(std::integral_constant<int, T>{}, G{});
         }
         if constexpr (UP) {
-            __syncthreads();                                     // two buffers: one barrier a unit
-            if (warp < nc && !*(volatile int*) &sh.fail)
+            if (__syncthreads_or(gave_up(warp))) goto leave;     // two buffers: one barrier a unit
+            if (warp < nc)
                 q8_1_store_warp(swiglu(sh.s_g[buf][warp][lane], sh.s_u[buf][warp][lane], A.limit),
                                 (shd ? A.sh_hq : A.hq) + ((size_t) slot_of(warp) * K.nunit + unit) * kQ81Bytes, lane);
             buf ^= 1;
+        } else if (gave_up(warp)) {
+            break;                                               // (the warps meet again at the change of job)
         }
         }
     }
-    if (*(volatile int*) &sh.fail) {
-        // let what may still be in flight land (bounded as well) before the block's shared memory goes away
-        for (int s = 0; s < kWStages; ++s) mbar_wait(&sh.full[warp][s], phase ^ (uint32_t) (s < stage));
-        __syncthreads();
+    if (!gave_up(warp)) return;
+leave:
+    // let what this warp has in flight land - the stages asked for and not yet read - before the block's shared memory goes away
+    for (uint32_t i = 2 * phase + stage; i != asked; i = (i + 1) & 3u) mbar_wait(&sh.full[warp][i & 1u], i >> 1);     // modulo 4, as `asked`
+    if (gave_up(warp) && lane == 0) {
+        if (A.error != nullptr) atomicExch(A.error, 1u);
+        atomicExch(A.n_groups, -1);
     }
 }
 

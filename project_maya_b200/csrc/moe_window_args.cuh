@@ -9,10 +9,12 @@ namespace maya {
 struct WArgs {
     const unsigned long long* ptr;   // [groups] blob addresses (0: skipped)
     const int* start;                // [groups + 1] entry ranges, or NULL: group g has the single entry g
-    const int* n_groups;             // device count, or NULL: `cap`
+    int* n_groups;                   // device count; set to -1 when a wait ran out
     const int* ent_slot;             // [entries] an entry's h / partial slot, or NULL: the entry number
     const int* skip;                 // optional "do nothing" flag
-    int cap;                         // most groups (<= kWMaxJobs)
+    unsigned* error;                 // optional: set to 1 when a wait ran out
+    unsigned polls;                  // looks at a row's copy before a warp gives up
+    int cap;                         // most groups (<= kWMaxGroups)
     int tok_from_slot;               // gate/up: an entry's column is slot >> 3 (a window), else column 0 (one token)
     int ncm;                         // columns of a job, <= kWNC
     int plain;                       // the rows do not start and end on 16-byte boundaries inside a blob: no bulk copies

@@ -302,7 +302,7 @@ def test_plan_refusals(T, api):
 
 
 # ------------------------------------------------------------------------------------------------ window form
-def run_window(T, api, t, n_embd, n_ff, store, ids, w, x, limit):
+def run_window(T, api, t, n_embd, n_ff, store, ids, w, x, limit, call=None):
     from project_maya_b200._lib import MoeWin
     n_tok, k = ids.shape
     ptr = np.zeros((n_tok, 8), np.int64)
@@ -321,7 +321,7 @@ def run_window(T, api, t, n_embd, n_ff, store, ids, w, x, limit):
                  keep["part"].data_ptr(), None, keep["out"].data_ptr(), n_embd, keep["gp"].data_ptr(),
                  keep["gs"].data_ptr(), keep["ge"].data_ptr(), keep["ng"].data_ptr(), n_tok, k, n_embd, n_ff, limit,
                  2 * n_ff * H.row_bytes(t, n_embd))
-    api.moe_win_experts(t, t, win)
+    (call or api.moe_win_experts)(t, t, win)
     T.cuda.synchronize()
     return keep["out"].reshape(n_tok, n_embd), plan_ptr, plan_w, xq, keep
 
@@ -350,6 +350,35 @@ def test_window_equals_token_by_token_bitwise(T, api, oracle, t, n_tok):
     blobs = [store[int(e)].cpu().numpy() for e in ids[0]]
     want = oracle_plan(oracle, t, n_embd, n_ff, blobs, w[0], x[0], 7.0)
     assert H.rel_err(out[0].cpu().numpy(), want) <= TIGHT
+
+
+@pytest.mark.parametrize("t,n_tok", [(H.Q4_K, 8), (H.IQ2_S, 1), (H.Q8_0, 16)])
+def test_window_reports_a_wait_that_ran_out(T, api, t, n_tok):
+    """The kernels' waits for weight rows are bounded: with no look at the copies at all every warp gives up with its copies in
+    flight, the launch ends, and the group count and the error word say so; with one look either all of them were there or it
+    says so too.  The same buffers then serve a call with the usual bound, which gives the usual bits."""
+    n_embd, n_ff, E, k = 512, 256, 6, 4
+    store = dev(T, np.stack([expert_blob(t, n_embd, n_ff, e, False) for e in range(E)]))
+    rng = H.rng_for("win-wait", t)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(n_tok)]).astype(np.int64)
+    w, x = rng.random((n_tok, k)).astype(np.float32), rng.standard_normal((n_tok, n_embd)).astype(np.float32)
+    want, groups = run_window(T, api, t, n_embd, n_ff, store, ids, w, x, 7.0)[0], len(set(ids.reshape(-1).tolist()))
+    seen = []
+
+    def calls(gu, d, win):
+        out = T.zeros((n_tok, n_embd), dtype=T.float32, device="cuda")
+        n_groups, err = T.zeros(1, dtype=T.int32, device="cuda"), T.zeros(1, dtype=T.int32, device="cuda")
+        win.out, win.n_groups = out.data_ptr(), n_groups.data_ptr()
+        for polls in (0, 1, 1 << 22):
+            err.zero_()
+            api.moe_win_experts_checked(gu, d, win, polls, err)
+            T.cuda.synchronize()
+            seen.append((polls, int(err.item()), int(n_groups.item()), T.equal(out, want)))
+
+    run_window(T, api, t, n_embd, n_ff, store, ids, w, x, 7.0, calls)
+    assert seen[0][:3] == (0, 1, -1)
+    assert seen[1] == (1, 0, groups, True) or seen[1][:3] == (1, 1, -1)
+    assert seen[2] == (1 << 22, 0, groups, True)
 
 
 @pytest.mark.parametrize("t,n_embd,n_ff,n_tok", [
