@@ -32,6 +32,9 @@ inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Dynamic shared memory up to which a launch leaves its kernel's limit alone.  The 48 KB that need no raised limit are for static
+// and dynamic shared memory together; no kernel here whose limit depends on the call has more than 16 KB of static.
+constexpr size_t kSmemNoLimit = 32 * 1024;
 constexpr unsigned kMbarPolls = 1u << 22;   // how often a warp looks at an mbarrier before it gives up (seconds)
 inline bool aligned16(const void* p) { return (((uintptr_t) p) & 15u) == 0; }
 

@@ -46,7 +46,7 @@ template<int T, int NC>
 int launch_mmvq(const void* w, const void* xq, float* y, int n_in, int n_out, int ncols, cudaStream_t s) {
     const size_t smem = (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_in / 32, ncols);
     if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > 48 * 1024) {
+    if (smem > kSmemNoLimit) {
         if (cudaFuncSetAttribute(mmvq_kernel<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
             return note_launch("mmvq smem attribute");
     }

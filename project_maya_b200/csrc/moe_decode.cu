@@ -453,7 +453,7 @@ int launch_gate_up(const Groups& G, int n_groups_grid, int n_embd, int n_ff, siz
         if (sh > smem) smem = sh;
     }
     if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > 48 * 1024 &&
+    if (smem > kSmemNoLimit &&
         cudaFuncSetAttribute(gate_up_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
         return note_launch("gate_up smem attribute");
     const dim3 grid((unsigned) (n_ff / kGuRows), (unsigned) (n_groups_grid + (sh_down != nullptr ? 1 : 0)));
@@ -468,7 +468,7 @@ int launch_down_plan(const maya_moe_plan& P, int k, int n_embd, int n_ff, size_t
                      const float* sh_out, float* out, cudaStream_t s) {
     const size_t smem = (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_ff / 32, k);
     if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > 48 * 1024 &&
+    if (smem > kSmemNoLimit &&
         cudaFuncSetAttribute(down_plan_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
         return note_launch("down smem attribute");
     down_plan_kernel<T><<<(n_embd + kDownRows - 1) / kDownRows, kDownWarps * 32, smem, s>>>(
@@ -481,7 +481,7 @@ int launch_down_groups(const Groups& G, int n_groups_grid, int n_embd, int n_ff,
                        float* part, cudaStream_t s) {
     const size_t smem = (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_ff / 32, kNC);
     if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > 48 * 1024 &&
+    if (smem > kSmemNoLimit &&
         cudaFuncSetAttribute(down_groups_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
         return note_launch("down_groups smem attribute");
     const dim3 grid((unsigned) ((n_embd + kDownRows - 1) / kDownRows), (unsigned) n_groups_grid);
@@ -494,7 +494,7 @@ int launch_gate_up_mixed(const Groups& G, int n_groups_grid, int n_embd, int n_f
                          size_t xq_stride, void* hq, cudaStream_t s) {
     const size_t smem = (size_t) (Fmt<TG>::tab_words + Fmt<TU>::tab_words) * 4 + xcols_bytes(n_embd / 32, kNC);
     if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > 48 * 1024 &&
+    if (smem > kSmemNoLimit &&
         cudaFuncSetAttribute(gate_up_mixed_kernel<TG, TU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
         return note_launch("gate_up_mixed smem attribute");
     const dim3 grid((unsigned) (n_ff / kGuRows), (unsigned) n_groups_grid);

@@ -151,11 +151,11 @@ template<bool BF16, bool VEC>
 int launch(const float* h, const float* add, const float* w, float eps, int n, const void* router, int n_expert, float* h_out,
            float* x_out, float* logits, cudaStream_t s) {
     const size_t smem = (size_t) n * sizeof(float);
-    static std::atomic<size_t> set_for{48 * 1024};        // dynamic shared memory the attribute was last raised to ...
+    static std::atomic<size_t> set_for{kSmemNoLimit};        // dynamic shared memory the attribute was last raised to ...
     static std::atomic<int> set_dev{-1};                  // ... on this device
     int dev = 0;
     cudaGetDevice(&dev);
-    if (smem > 48 * 1024 && (set_dev.load() != dev || set_for.load() < smem)) {
+    if (smem > kSmemNoLimit && (set_dev.load() != dev || set_for.load() < smem)) {
         if (cudaFuncSetAttribute(rms_router_kernel<BF16, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
             return note_launch("rms_router smem attribute");
         set_dev.store(dev);

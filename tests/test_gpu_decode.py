@@ -272,6 +272,16 @@ def test_plan_edge_cases(T, api, oracle):
     assert not got0.any()
 
 
+@pytest.mark.parametrize("t,n_embd,n_ff", [(H.IQ2_S, 8192, 256), (H.Q4_K, 9728, 256), (H.Q8_0, 9632, 32), (H.Q8_0, 9792, 32)])
+def test_plan_widths_around_the_shared_memory_limit(T, api, oracle, t, n_embd, n_ff):
+    """Columns that leave less than the kernel's static shared memory of the 48 KB it has without a raised limit."""
+    blob = expert_blob(t, n_embd, n_ff, "edge", False)
+    x = H.rng_for("plan-edge", t).standard_normal(n_embd).astype(np.float32)
+    w = np.ones(1, np.float32)
+    got, _ = run_plan(T, api, t, n_embd, n_ff, [blob], w, x, 7.0)
+    assert H.rel_err(got, oracle_plan(oracle, t, n_embd, n_ff, [blob], w, x, 7.0)) <= TIGHT
+
+
 def test_plan_skip_flag_leaves_output_alone(T, api):
     t, n_embd, n_ff, k = H.Q4_K, 512, 256, 2
     store = dev(T, np.stack([expert_blob(t, n_embd, n_ff, i, False) for i in range(k)]))

@@ -434,6 +434,20 @@ def test_rms_router_and_two_launch_layer(T, api, oracle, router_dtype):
     assert H.rel_err(out.cpu().numpy()[0], want) <= TIGHT
 
 
+@pytest.mark.parametrize("n", [8184, 8193, 12272, 12273, 12280, 12288, 12289])
+@pytest.mark.parametrize("router_dtype", ["f32", "bf16"])
+def test_rms_router_row_widths_around_the_shared_memory_limit(T, api, n, router_dtype):
+    """Rows whose f32 image fills the 48 KB a kernel has without a raised limit - up to the last bytes, and beyond: x against
+    float64, the logits against the float64 product with that x (f32 sums of n terms, added in up to 256 partial sums)."""
+    rng = H.rng_for("rms-width", n, router_dtype)
+    h, nw = (dev(T, rng.standard_normal(n).astype(np.float32)) for _ in range(2))
+    rw = dev(T, (rng.standard_normal((5, n)) / np.sqrt(n)).astype(np.float32), T.bfloat16 if router_dtype == "bf16" else None)
+    x, logits = api.rms_router(h, None, nw, 1e-6, rw)
+    want = h.double() * T.rsqrt(h.double().pow(2).mean() + 1e-6) * nw.double()
+    assert float((x.double() - want).abs().max()) <= 4e-6 * float(want.abs().max())
+    assert float((logits.double() - rw.double() @ x.double()).abs().max()) <= 1e-5
+
+
 def _word_area(T, r):
     """The {seq, value} words of rank r's receive buffer: they follow its 2 x nm x stride floats of rows."""
     return r.keep[0][r.mi][2 * r.nm * r.stride * 4:].view(T.int64).view(2, r.nm, r.stride)
