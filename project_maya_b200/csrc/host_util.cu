@@ -22,17 +22,26 @@ int refuse(int status) {
     return status;
 }
 
+constexpr int kDevices = 64;                 // devices something is remembered for; beyond them it is asked again each time
+
 int sm_count() {
-    static std::atomic<int> cached_dev{-1}, cached_n{0};
+    static std::atomic<int> count[kDevices];
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (dev < kDevices && (n = count[dev].load()) > 0) return n;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (dev < kDevices) count[dev].store(n);
+    return n;
+}
+
+bool SmemLimit::raise(const void* kernel, size_t bytes) {
     int dev = 0;
     cudaGetDevice(&dev);
-    if (cached_dev.load() != dev) {
-        int n = 0;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        cached_n.store(n);
-        cached_dev.store(dev);
-    }
-    return cached_n.load();
+    const unsigned long long bit = dev < kDevices ? 1ull << dev : 0ull;
+    if (raised.load() & bit) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes) != cudaSuccess) return false;
+    raised.fetch_or(bit);
+    return true;
 }
 
 }  // namespace maya

@@ -1,6 +1,7 @@
 // maya_common.cuh - shared device helpers: GGUF block geometry, packed loads, warp reductions, launch checks.
 #pragma once
 
+#include <atomic>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -13,6 +14,14 @@ namespace maya {
 int note_launch(const char* what);          // cudaGetLastError -> status; counts failures
 int refuse(int status);                     // counts a refused call, returns status
 int sm_count();                             // multiprocessors of the current device
+// A kernel's limit of dynamic shared memory, raised once per device - always to the same `bytes`, so that what is remembered (one
+// bit a device, set behind the call it stands for) holds whichever threads and devices get here in whatever order.
+class SmemLimit {
+public:
+    bool raise(const void* kernel, size_t bytes);
+private:
+    std::atomic<unsigned long long> raised{0ull};
+};
 inline cudaStream_t as_stream(void* s) { return (cudaStream_t) s; }
 // A launch whose set-up may overlap the tail of the launch in front of it (programmatic dependent launch): the kernel must call
 // grid_dependency_wait() before it reads or writes anything that launch could touch.
@@ -35,6 +44,7 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 // Dynamic shared memory up to which a launch leaves its kernel's limit alone.  The 48 KB that need no raised limit are for static
 // and dynamic shared memory together; no kernel here whose limit depends on the call has more than 16 KB of static.
 constexpr size_t kSmemNoLimit = 32 * 1024;
+constexpr size_t kSmemMost = 200 * 1024;    // dynamic shared memory of a launch whose need depends on the call, at most
 constexpr unsigned kMbarPolls = 1u << 22;   // how often a warp looks at an mbarrier before it gives up (seconds)
 inline bool aligned16(const void* p) { return (((uintptr_t) p) & 15u) == 0; }
 

@@ -45,11 +45,9 @@ __global__ void __launch_bounds__(kMvWarps * 32) mmvq_kernel(const uint8_t* __re
 template<int T, int NC>
 int launch_mmvq(const void* w, const void* xq, float* y, int n_in, int n_out, int ncols, cudaStream_t s) {
     const size_t smem = (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_in / 32, ncols);
-    if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > kSmemNoLimit) {
-        if (cudaFuncSetAttribute(mmvq_kernel<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-            return note_launch("mmvq smem attribute");
-    }
+    if (smem > kSmemMost) return refuse(MAYA_ERR_LIMIT);
+    static SmemLimit smem_limit;
+    if (smem > kSmemNoLimit && !smem_limit.raise((const void*) mmvq_kernel<T, NC>, kSmemMost)) return note_launch("mmvq smem attribute");
     const int rows_per_block = kMvWarps * kRowsPerWarp;
     mmvq_kernel<T, NC><<<(n_out + rows_per_block - 1) / rows_per_block, kMvWarps * 32, smem, s>>>(
         (const uint8_t*) w, (const uint8_t*) xq, y, n_in, n_out, ncols);

@@ -452,10 +452,9 @@ int launch_gate_up(const Groups& G, int n_groups_grid, int n_embd, int n_ff, siz
         const size_t sh = 8192 + xcols_bytes(n_ff_sh / 32, 1);
         if (sh > smem) smem = sh;
     }
-    if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > kSmemNoLimit &&
-        cudaFuncSetAttribute(gate_up_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-        return note_launch("gate_up smem attribute");
+    if (smem > kSmemMost) return refuse(MAYA_ERR_LIMIT);
+    static SmemLimit smem_limit;
+    if (smem > kSmemNoLimit && !smem_limit.raise((const void*) gate_up_kernel<T>, kSmemMost)) return note_launch("gate_up smem attribute");
     const dim3 grid((unsigned) (n_ff / kGuRows), (unsigned) (n_groups_grid + (sh_down != nullptr ? 1 : 0)));
     gate_up_kernel<T><<<grid, kGuWarps * 32, smem, s>>>(G, n_groups_grid, n_embd, n_ff, up_off, limit, (const uint8_t*) xq,
                                                         xq_stride, (uint8_t*) hq, (const uint8_t*) sh_down, sh_type,
@@ -467,10 +466,9 @@ template<int T>
 int launch_down_plan(const maya_moe_plan& P, int k, int n_embd, int n_ff, size_t down_off, const void* hq,
                      const float* sh_out, float* out, cudaStream_t s) {
     const size_t smem = (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_ff / 32, k);
-    if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > kSmemNoLimit &&
-        cudaFuncSetAttribute(down_plan_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-        return note_launch("down smem attribute");
+    if (smem > kSmemMost) return refuse(MAYA_ERR_LIMIT);
+    static SmemLimit smem_limit;
+    if (smem > kSmemNoLimit && !smem_limit.raise((const void*) down_plan_kernel<T>, kSmemMost)) return note_launch("down smem attribute");
     down_plan_kernel<T><<<(n_embd + kDownRows - 1) / kDownRows, kDownWarps * 32, smem, s>>>(
         P, k, n_embd, n_ff, down_off, (const uint8_t*) hq, sh_out, out);
     return note_launch("moe_down");
@@ -480,10 +478,9 @@ template<int T>
 int launch_down_groups(const Groups& G, int n_groups_grid, int n_embd, int n_ff, size_t down_off, const void* hq,
                        float* part, cudaStream_t s) {
     const size_t smem = (size_t) Fmt<T>::tab_words * 4 + xcols_bytes(n_ff / 32, kNC);
-    if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > kSmemNoLimit &&
-        cudaFuncSetAttribute(down_groups_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-        return note_launch("down_groups smem attribute");
+    if (smem > kSmemMost) return refuse(MAYA_ERR_LIMIT);
+    static SmemLimit smem_limit;
+    if (smem > kSmemNoLimit && !smem_limit.raise((const void*) down_groups_kernel<T>, kSmemMost)) return note_launch("down_groups smem attribute");
     const dim3 grid((unsigned) ((n_embd + kDownRows - 1) / kDownRows), (unsigned) n_groups_grid);
     down_groups_kernel<T><<<grid, kDownWarps * 32, smem, s>>>(G, n_embd, n_ff, down_off, (const uint8_t*) hq, part);
     return note_launch("down_groups");
@@ -493,10 +490,9 @@ template<int TG, int TU>
 int launch_gate_up_mixed(const Groups& G, int n_groups_grid, int n_embd, int n_ff, size_t up_off, float limit, const void* xq,
                          size_t xq_stride, void* hq, cudaStream_t s) {
     const size_t smem = (size_t) (Fmt<TG>::tab_words + Fmt<TU>::tab_words) * 4 + xcols_bytes(n_embd / 32, kNC);
-    if (smem > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (smem > kSmemNoLimit &&
-        cudaFuncSetAttribute(gate_up_mixed_kernel<TG, TU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-        return note_launch("gate_up_mixed smem attribute");
+    if (smem > kSmemMost) return refuse(MAYA_ERR_LIMIT);
+    static SmemLimit smem_limit;
+    if (smem > kSmemNoLimit && !smem_limit.raise((const void*) gate_up_mixed_kernel<TG, TU>, kSmemMost)) return note_launch("gate_up_mixed smem attribute");
     const dim3 grid((unsigned) (n_ff / kGuRows), (unsigned) n_groups_grid);
     gate_up_mixed_kernel<TG, TU><<<grid, kGuWarps * 32, smem, s>>>(G, n_embd, n_ff, up_off, limit, (const uint8_t*) xq, xq_stride,
                                                                   (uint8_t*) hq);

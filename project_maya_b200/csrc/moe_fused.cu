@@ -490,30 +490,18 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
 
 template<int T, int TS, int RT, bool HV>
 int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
-    // per instantiation: the device and dynamic shared-memory size the attribute was last set for, and whether the
-    // programmatic-serialization attribute is in use (1), was refused by the driver (0) or has not been tried (-1)
-    static std::atomic<int> attr_dev{-1}, pdl{-1};
-    static std::atomic<size_t> attr_smem{0};
-    static thread_local int cached_dev = -1, cached_grid = 0;
-    int dev = 0;
-    cudaGetDevice(&dev);
+    // per instantiation: whether the programmatic-serialization attribute is in use (1), was refused by the driver (0) or has not
+    // been tried (-1)
+    static std::atomic<int> pdl{-1};
+    static SmemLimit smem_limit;
+    constexpr size_t kMost = 220 * 1024;
     const int nblk_x = A.n_embd / 32, nblk_h = (A.n_ff > A.n_ff_sh ? A.n_ff : A.n_ff_sh) / 32;
     const int cols_blocks = ((nblk_x > (MAYA_MAX_K + 1) * nblk_h ? nblk_x : (MAYA_MAX_K + 1) * nblk_h) + 1) & ~1;
     const size_t smem = (size_t) kRepTabBytes<T> + (size_t) cols_blocks * 40 + (size_t) A.n_expert * sizeof(double);
-    if (smem > 220 * 1024) return refuse(MAYA_ERR_LIMIT);
-    if (cached_dev != dev) {
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cached_grid = sms;
-        cached_dev = dev;
-    }
-    if (attr_dev.load() != dev || attr_smem.load() != smem) {
-        if (cudaFuncSetAttribute(moe_layer_t1_kernel<T, TS, RT, HV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-            return note_launch("fused smem attribute");
-        attr_dev.store(dev);
-        attr_smem.store(smem);
-    }
-    int grid = cached_grid;
+    if (smem > kMost) return refuse(MAYA_ERR_LIMIT);
+    if (!smem_limit.raise((const void*) moe_layer_t1_kernel<T, TS, RT, HV>, kMost)) return note_launch("fused smem attribute");
+    const int grid = sm_count();
+    if (grid <= 0) return refuse(MAYA_ERR_DEVICE);
     if (4 * ((A.n_embd / 4 + grid - 1) / grid) > kMaxSliceRows || A.n_embd % 4) return refuse(MAYA_ERR_LIMIT);
     if (A.ar.nm >= 2 && grid > MAYA_PEER_AR_BLOCKS) return refuse(MAYA_ERR_LIMIT);
     FusedArgs args = A;

@@ -32,7 +32,6 @@
 #include "maya_stream.cuh"
 #include "moe_window_args.cuh"
 
-#include <atomic>
 #include <type_traits>
 
 namespace maya {
@@ -624,16 +623,8 @@ int launch_window_cb(WArgs A, cudaStream_t s) {
     if (A.ncm < 1) return kWindowTooWide;
     A.plain = ((A.row_off | A.up_off | (size_t) (UP ? A.n_ff : A.n_embd) * row_bytes(T, UP ? A.n_embd : A.n_ff)) & 15) != 0;
     const size_t smem = (size_t) kRing + G::tab + (size_t) A.ncm * kColBytes<CB>;
-    static std::atomic<size_t> set_for{0};            // per instantiation: the size the attribute was last raised to
-    static std::atomic<int> set_dev{-1};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (set_dev.load() != dev || set_for.load() < smem) {
-        if (cudaFuncSetAttribute(window_kernel<T, SH, UP, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-            return note_launch("window smem attribute");
-        set_for.store(smem);
-        set_dev.store(dev);
-    }
+    static SmemLimit smem_limit;                           // (smem is the same in every call of an instantiation)
+    if (!smem_limit.raise((const void*) window_kernel<T, SH, UP, CB>, smem)) return note_launch("window smem attribute");
     const int sms = sm_count();
     if (sms <= 0) return refuse(MAYA_ERR_DEVICE);
     launch_dependent(window_kernel<T, SH, UP, CB>, dim3((unsigned) sms), dim3(G::threads), smem, s, A);

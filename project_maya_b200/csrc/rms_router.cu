@@ -17,8 +17,6 @@
 // of dependent 2-byte loads: 19.7 us a call at that size, about 7 us now.
 #include "maya_common.cuh"
 
-#include <atomic>
-
 namespace maya {
 namespace {
 
@@ -151,16 +149,8 @@ template<bool BF16, bool VEC>
 int launch(const float* h, const float* add, const float* w, float eps, int n, const void* router, int n_expert, float* h_out,
            float* x_out, float* logits, cudaStream_t s) {
     const size_t smem = (size_t) n * sizeof(float);
-    static std::atomic<size_t> set_for{kSmemNoLimit};        // dynamic shared memory the attribute was last raised to ...
-    static std::atomic<int> set_dev{-1};                  // ... on this device
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (smem > kSmemNoLimit && (set_dev.load() != dev || set_for.load() < smem)) {
-        if (cudaFuncSetAttribute(rms_router_kernel<BF16, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)
-            return note_launch("rms_router smem attribute");
-        set_dev.store(dev);
-        set_for.store(smem);
-    }
+    static SmemLimit smem_limit;
+    if (smem > kSmemNoLimit && !smem_limit.raise((const void*) rms_router_kernel<BF16, VEC>, kSmemMost)) return note_launch("rms_router smem attribute");
     // experts a block: the fewest (1, 2, 4 or 8) that leave at most one block an SM, so that a small router spreads over the
     // chip (beyond 8 x 148 experts blocks share SMs)
     int epb = 1;
@@ -180,7 +170,7 @@ extern "C" int maya_rms_router(const float* h, const float* add, const float* no
                                float* logits, void* stream) {
     if (!h || !norm_w || !router_w || !x_out || !logits || n_embd <= 0 || n_expert <= 0) return refuse(MAYA_ERR_ARG);
     if (add != nullptr && h_out == h) return refuse(MAYA_ERR_ARG);       // other blocks still read h
-    if ((size_t) n_embd * sizeof(float) > 200 * 1024) return refuse(MAYA_ERR_LIMIT);
+    if ((size_t) n_embd * sizeof(float) > kSmemMost) return refuse(MAYA_ERR_LIMIT);
     const bool vec = n_embd % 8 == 0 && aligned16(h) && (!add || aligned16(add)) && aligned16(norm_w) && aligned16(router_w) &&
                      (!h_out || aligned16(h_out)) && aligned16(x_out);
     cudaStream_t s = as_stream(stream);

@@ -448,6 +448,50 @@ def test_rms_router_row_widths_around_the_shared_memory_limit(T, api, n, router_
     assert float((logits.double() - rw.double() @ x.double()).abs().max()) <= 1e-5
 
 
+def test_two_threads_with_calls_of_different_sizes(T, api):
+    """The kernels' shared-memory limits are process-wide state: two host threads whose calls need different amounts are both
+    served - on one stream, so that the GPU sees one call after another - and get the bits they get alone."""
+    import threading
+    rng = H.rng_for("two-threads")
+
+    def mmvq(n_in):
+        w = dev(T, H.constructed_blocks(H.Q8_0, 64, n_in, rng))
+        xq = api.native_quantize_q8_1(dev(T, rng.standard_normal((8, n_in)).astype(np.float32)))
+        return lambda: (api.native_mmvq(H.Q8_0, w, xq, n_in, 64, ncols=8),)
+
+    def rms(n):
+        h, nw, rw = (T.randn(s, device="cuda") for s in (n, n, (5, n)))
+        return lambda: api.rms_router(h, None, nw, 1e-6, rw)
+
+    def layer(n_embd, n_ff):
+        lc, experts, _ = synth_layer(T, api, dict(n_embd=n_embd, n_ff=n_ff, n_expert=4, k=2, gu_type=H.Q4_K, d_type=H.Q4_K), 4, seed=9)
+        m = api.MoeLayer(lc, experts)
+        logits, x = T.randn(1, 4, device="cuda"), T.randn(1, n_embd, device="cuda")
+        return lambda: m.forward(logits, x)
+
+    for make, small, large in ((rms, (13000,), (50000,)), (mmvq, (5120,), (16384,)), (layer, (512, 256), (1024, 4096))):
+        calls, failed = [make(*small), make(*large)], []
+        gate, outs = threading.Barrier(2), [None, None]
+
+        def work(i):
+            try:
+                gate.wait()
+                for _ in range(500):
+                    outs[i] = calls[i]()
+            except Exception as e:
+                failed.append(e)
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        T.cuda.synchronize()
+        assert not failed, f"{make.__name__}: {failed[0]}"
+        for call, out in zip(calls, outs):
+            assert all(T.equal(a, b) for a, b in zip(call(), out))
+
+
 def _word_area(T, r):
     """The {seq, value} words of rank r's receive buffer: they follow its 2 x nm x stride floats of rows."""
     return r.keep[0][r.mi][2 * r.nm * r.stride * 4:].view(T.int64).view(2, r.nm, r.stride)
