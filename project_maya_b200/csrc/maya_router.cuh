@@ -37,6 +37,7 @@ template<int ID, int N> struct NamedSync {
 
 struct RouterShared {
     float rv[kRouterMaxWarps], rw[kRouterMaxWarps];
+    uint32_t ro[kRouterMaxWarps];
     int ri[kRouterMaxWarps];
     int ids[64];
     float val[64];
@@ -45,41 +46,46 @@ struct RouterShared {
     alignas(16) unsigned long long cand[kRouterMaxWarps * 8];   // select_rank: every warp's k best keys (k <= 8)
 };
 
-// k rounds of arg-max over `sel` (expert e = j * nt + tid), "greater value, or equal value and lower index" - the
-// stable descending order.  The chosen ids and their companions `val` land in sh.ids / sh.val.
+// A number that orders like the value: -inf before every other, no number (NaN) before -inf.  Never 0.
+__device__ __forceinline__ uint32_t order_of(float v) {
+    const uint32_t u = __float_as_uint(v);
+    return v != v ? 1u : u ^ ((u >> 31) ? 0xffffffffu : 0x80000000u);
+}
+// k rounds of arg-max over `order` (order_of the value selected on; expert e = j * nt + tid; 0: no expert), "greater, or equal and
+// lower index" - the stable descending order.  The chosen ids and their companions `val` land in sh.ids / sh.val.  k <= n_expert:
+// every round finds one, whatever the values are (masked to -inf, NaN).
 template<int PER, class Sync>
-__device__ __forceinline__ void select_topk(float (&sel)[PER], const float (&val)[PER], int n_expert, int k, int tid,
+__device__ __forceinline__ void select_topk(uint32_t (&order)[PER], const float (&val)[PER], int n_expert, int k, int tid,
                                             int nt, RouterShared& sh) {
     const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     for (int i = 0; i < k; ++i) {
-        float bv = -INFINITY, bw = 0.0f;
+        uint32_t bv = 0u;
+        float bw = 0.0f;
         int bi = n_expert;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int e = j * nt + tid;
-            if (e < n_expert && sel[j] > bv) { bv = sel[j]; bi = e; bw = val[j]; }   // ascending e: lowest index on ties
-        }
+        for (int j = 0; j < PER; ++j)
+            if (order[j] > bv) { bv = order[j]; bi = j * nt + tid; bw = val[j]; }    // ascending e: lowest index on ties
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const uint32_t ov = __shfl_xor_sync(0xffffffffu, bv, o);
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             const float ow = __shfl_xor_sync(0xffffffffu, bw, o);
             if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; bw = ow; }
         }
-        if (lane == 0) { sh.rv[warp] = bv; sh.ri[warp] = bi; sh.rw[warp] = bw; }
+        if (lane == 0) { sh.ro[warp] = bv; sh.ri[warp] = bi; sh.rw[warp] = bw; }
         Sync::sync();
-        float v = sh.rv[0], w = sh.rw[0];
+        uint32_t v = sh.ro[0];
+        float w = sh.rw[0];
         int ix = sh.ri[0];
         for (int q = 1; q < nw; ++q) {
-            const float ov = sh.rv[q];
+            const uint32_t ov = sh.ro[q];
             const int oi = sh.ri[q];
             if (ov > v || (ov == v && oi < ix)) { v = ov; ix = oi; w = sh.rw[q]; }
         }
-        if (tid == 0 && ix < n_expert) { sh.ids[i] = ix; sh.val[i] = w; }
-        // retire the winner: -inf never beats the -inf start, so it cannot be picked again
+        if (tid == 0) { sh.ids[i] = ix; sh.val[i] = w; }
 #pragma unroll
         for (int j = 0; j < PER; ++j)
-            if (j * nt + tid == ix) sel[j] = -INFINITY;
+            if (j * nt + tid == ix) order[j] = 0u;               // taken
         Sync::sync();
     }
 }
@@ -200,14 +206,15 @@ __device__ __forceinline__ void route_softmax(const float* __restrict__ l, int n
         inv = sh.inv;
         Sync::sync();                                            // s_ex is reused below
     }
-    float p[PER], sel[PER];
+    float p[PER];
+    uint32_t order[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
-        p[j] = (j * nt + tid) < n_expert ? (float) (ex[j] * inv) : -INFINITY;
-        sel[j] = p[j];
+        p[j] = (float) (ex[j] * inv);
+        order[j] = j * nt + tid < n_expert ? order_of(p[j]) : 0u;
     }
-    if constexpr (PER == 1) select_rank<Sync>(__float_as_uint(p[0]), p[0], n_expert, k, tid, (unsigned long long*) s_ex, sh);
-    else select_topk<PER, Sync>(sel, p, n_expert, k, tid, nt, sh);
+    if constexpr (PER == 1) select_rank<Sync>(order[0], p[0], n_expert, k, tid, (unsigned long long*) s_ex, sh);
+    else select_topk<PER, Sync>(order, p, n_expert, k, tid, nt, sh);
     // weights renormalised in double by max(their sum in selection order, 2^-14): every thread adds, k threads divide
     double s = 0.0;
     for (int i = 0; i < k; ++i) s += (double) sh.val[i];
@@ -226,26 +233,20 @@ __device__ __forceinline__ void route_softmax(const float* __restrict__ l, int n
 template<int PER, class Sync>
 __device__ __forceinline__ void route_sigmoid(const float* __restrict__ l, const float* __restrict__ bias, int n_expert, int k,
                                               float w_scale, int norm_w, int tid, int nt, double* s_keys, RouterShared& sh) {
-    float p[PER], sel[PER];
+    float p[PER];
+    uint32_t order[PER];
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
         const int e = j * nt + tid;
+        p[j] = 0.0f;
+        order[j] = 0u;
         if (e < n_expert) {
             p[j] = __fdiv_rn(1.0f, 1.0f + expf(-l[e]));
-            sel[j] = bias ? p[j] + bias[e] : p[j];
-        } else {
-            p[j] = 0.0f;
-            sel[j] = -INFINITY;
+            order[j] = order_of(bias ? p[j] + bias[e] : p[j]);   // (p >= +0: a sum of zero is +0)
         }
     }
-    if constexpr (PER == 1) {
-        uint32_t u = __float_as_uint(sel[0] + 0.0f);             // (-0 counts as 0)
-        u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;              // orders like the value, negative ones included
-        if (sel[0] != sel[0]) u = 0u;                            // no number: last
-        select_rank<Sync>(u, p[0], n_expert, k, tid, (unsigned long long*) s_keys, sh);
-    } else {
-        select_topk<PER, Sync>(sel, p, n_expert, k, tid, nt, sh);
-    }
+    if constexpr (PER == 1) select_rank<Sync>(order[0], p[0], n_expert, k, tid, (unsigned long long*) s_keys, sh);
+    else select_topk<PER, Sync>(order, p, n_expert, k, tid, nt, sh);
     double s = 0.0;                                              // every thread adds, k threads divide
     for (int i = 0; i < k; ++i) s += (double) sh.val[i];
     const double sc = fmax(s, 6.103515625e-05);

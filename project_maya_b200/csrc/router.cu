@@ -12,7 +12,7 @@ template<int PER>
 __global__ void __launch_bounds__(kRouterThreads) router_softmax_kernel(const float* __restrict__ logits, int n_expert,
                                                                         int k, int* __restrict__ ids,
                                                                         float* __restrict__ weights) {
-    extern __shared__ double s_ex[];          // n_expert doubles
+    extern __shared__ __align__(16) double s_ex[];          // n_expert doubles
     __shared__ RouterShared sh;
     const int t = blockIdx.x, tid = threadIdx.x;
     grid_launch_dependents();
@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(kRouterThreads) router_sigmoid_kernel(const fl
                                                                         int k, float w_scale, int norm_w,
                                                                         int* __restrict__ ids,
                                                                         float* __restrict__ weights) {
-    extern __shared__ double s_keys[];        // n_expert 64-bit words
+    extern __shared__ __align__(16) double s_keys[];        // n_expert 64-bit words
     __shared__ RouterShared sh;
     const int t = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
     grid_launch_dependents();

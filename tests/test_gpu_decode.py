@@ -96,21 +96,53 @@ def test_router_sigmoid_golden(T, api):
         assert (np.abs(w.cpu().numpy() - g["weights"][i]) / g["weights"][i]).max() <= 1e-6
 
 
-@pytest.mark.parametrize("E,k", [(64, 8), (160, 6), (256, 10), (33, 33), (300, 8)])       # one and two experts a thread; k beyond 8
+ROUTER_SIZES = [(64, 8), (160, 6), (256, 10), (33, 33), (300, 8)]                          # one and two experts a thread; k beyond 8
+
+
+@pytest.mark.parametrize("E,k", ROUTER_SIZES)
 def test_router_sigmoid_ties_and_signs(T, api, oracle, E, k):
-    """Scores of both signs, exact ties (lower index first), -0 beside +0, a masked expert: the oracle's ids and weights."""
+    """Scores of both signs and exact ties (lower index first), with the tied scores - two zeros and one just below - the best of
+    all in one bias, and more experts masked to -inf than leaves k in another: the oracle's ids and weights."""
     rng = H.rng_for("sigmoid-ties", E, k)
     logits = rng.standard_normal((6, E)).astype(np.float32)
     logits[1] = 0.25                                                                       # all equal
     logits[2, ::3] = logits[2, 0]
+    logits[3, 5], logits[3, 7] = 0.0, -0.0
     bias = (rng.standard_normal(E) - 1.0).astype(np.float32)                               # most p + bias below zero
-    bias[5], bias[7] = -0.5, -0.5
-    logits[3, 5], logits[3, 7] = 0.0, -0.0                                                 # p + bias = 0 twice
-    for b, norm in ((bias, True), (np.zeros(E, np.float32), False)):
+    bias[5], bias[7] = -0.5, -0.5                                                          # p + bias = 0 twice in row 3
+    zeros = np.full(E, -3.0, np.float32)
+    zeros[5], zeros[7], zeros[9] = -0.5, -0.5, -1.0
+    masked = np.full(E, -np.inf, np.float32)
+    masked[[3, 11, E - 2]] = 0.25, -2.0, 0.25
+    for b, norm in ((bias, True), (np.zeros(E, np.float32), False), (zeros, True), (masked, True)):
         ids, w = api.router_sigmoid(dev(T, logits), dev(T, b), k, 2.5, norm)
         ids_o, w_o = oracle.router_sigmoid(logits, b, k, 2.5, norm)
         assert np.array_equal(ids.cpu().numpy(), ids_o)
         assert (np.abs(w.cpu().numpy() - w_o) / np.abs(w_o)).max() <= 1e-6
+        if b is zeros:
+            assert ids_o[3, :2].tolist() == [5, 7] and ids_o[3, 2] == 9
+
+
+@pytest.mark.parametrize("E,k", ROUTER_SIZES)
+def test_router_without_numbers(T, api, oracle, E, k):
+    """Logits that are no number: such an expert comes after every other one, masked ones included; where nothing is a number the ids
+    are still k different experts, the lowest first."""
+    rng = H.rng_for("router-nan", E, k)
+    logits = rng.standard_normal((4, E)).astype(np.float32)
+    bias = (0.1 * rng.standard_normal(E)).astype(np.float32)
+    bias[2] = -np.inf
+    lost = logits.copy()
+    lost[:, 6] = np.nan
+    ids, _ = api.router_sigmoid(dev(T, lost), dev(T, bias), k, 1.0, True)
+    # the oracle without expert 6, the others numbered on
+    rest = [e for e in range(E) if e != 6]
+    want = np.array(rest, np.int32)[oracle.router_sigmoid(np.ascontiguousarray(logits[:, rest]), bias[rest], min(k, E - 1), 1.0, True)[0]]
+    if k == E:
+        want = np.concatenate([want, np.full((4, 1), 6, np.int32)], 1)
+    assert np.array_equal(ids.cpu().numpy(), want)
+    lost[:] = np.nan
+    for ids, _ in (api.router_sigmoid(dev(T, lost), None, k, 1.0, True), api.router_top10(dev(T, lost), k)):
+        assert np.array_equal(ids.cpu().numpy(), np.tile(np.arange(k, dtype=np.int32), (4, 1)))
 
 
 # ------------------------------------------------------------------------------------------------ q8_1
