@@ -976,6 +976,11 @@ PFN_cuTensorMapEncodeTiled encode_fn() {
     }();
     return fn;
 }
+// The driver refused a tensor map (a stride or an extent beyond what a map can hold): nothing is launched.
+int no_map(const char* what) {
+    std::fprintf(stderr, "maya_moe: %s tensor map refused\n", what);
+    return refuse(MAYA_ERR_LAUNCH);
+}
 bool make_map(CUtensorMap* m, CUtensorMapDataType dt, int rank, const void* base, const cuuint64_t* dim, const cuuint64_t* stride,
               const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
     PFN_cuTensorMapEncodeTiled fn = encode_fn();
@@ -999,14 +1004,14 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
         const cuuint64_t st[2] = {(cuuint64_t) rbw, (cuuint64_t) p->expert_bytes};
         const cuuint32_t box[3] = {(cuuint32_t) (kRawRow<T> / 4), kUnitRows, 1};
         if (!make_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, p->w, dim, st, box, CU_TENSOR_MAP_SWIZZLE_NONE))
-            return note_launch("mmq weight tensor map");
+            return no_map("mmq weight");
     } else {                   // i-quants as bytes: a box = the 112 / 144 bytes of 64 rows that hold the block's window;
                                // a row is a multiple of 16 bytes (K a multiple of 2048) and so is every window's start
         const cuuint64_t dim[3] = {(cuuint64_t) rbw, (cuuint64_t) mat_rows, (cuuint64_t) p->n};
         const cuuint64_t st[2] = {(cuuint64_t) rbw, (cuuint64_t) p->expert_bytes};
         const cuuint32_t box[3] = {(cuuint32_t) kRawRow<T>, kUnitRows, 1};
         if (!make_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, p->w, dim, st, box, CU_TENSOR_MAP_SWIZZLE_NONE))
-            return note_launch("mmq weight tensor map");
+            return no_map("mmq weight");
     }
     {   // activations: f16 [row][K + tail] (xq_ld); a box = 64 K-values (128 bytes) of 128 or 32 rows, written with the 128-byte swizzle
         const cuuint64_t dim[2] = {(cuuint64_t) xq_ld(K), (cuuint64_t) p->total_rows};
@@ -1014,7 +1019,7 @@ int launch_mmq(const maya_mmq_product* p, const MmqArgs& A, cudaStream_t s) {
         const cuuint32_t box[2] = {64, 128}, box32[2] = {64, 32};
         if (!make_map(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p->xq, dim, st, box, CU_TENSOR_MAP_SWIZZLE_128B) ||
             !make_map(&tx32, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p->xq, dim, st, box32, CU_TENSOR_MAP_SWIZZLE_128B))
-            return note_launch("mmq activation tensor map");
+            return no_map("mmq activation");
     }
     constexpr size_t smem = kSmemBytes<T>;
     if (cudaFuncSetAttribute(mmq_kernel<T, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess)

@@ -367,6 +367,9 @@ def test_refusals(T, api):
     for bad in (dict(ggml_type=H.IQ2_S), dict(w_rows=100), dict(w_cols=96), dict(ld_dst=64), dict(expert_bytes=w.numel() + 8)):
         with pytest.raises(api.MayaError):
             api.mmq_run(ok(**bad))
+    far = H.row_bytes(t, 256) * 128
+    with pytest.raises(api.MayaError):                    # matrices further apart than a tensor map's 40-bit stride: not launched, not 0
+        api.mmq_run(ok(expert_bytes=far * ((1 << 40) // far + 1)))
     with pytest.raises(api.MayaError):
         api.mmq_run_glu(ok(w_rows=128), H.INF)            # n_ff = 64 is not a multiple of 128
     assert api.mmq_q8_bytes(3, 100) == 0 and api.mmq_q8_bytes(3, 256) == 3 * xq_ld(256) * 2
