@@ -45,18 +45,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// The non-suspending form: one look at the barrier.
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // Bounded wait (every lane polls, at most `polls` times).  false: gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned polls = kMbarPolls) {
     for (unsigned i = 0; i < polls; ++i) {

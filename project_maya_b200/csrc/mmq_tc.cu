@@ -491,7 +491,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         const int nrows = ti.nrows, row0 = ti.row0, m0 = ti.m0;
 #ifdef MAYA_MMQ_STAMPS
         long long* const stamps = tid == 0 && ok ? stamps_of(ti.lin) : nullptr;
-        if (stamps) { stamps[0] = stamps[1] = clock64(); stamps[14] = nrows; stamps[15] = npairs; }
+        if (stamps) { stamps[0] = clock64(); stamps[14] = nrows; stamps[15] = npairs; }
 #endif
         for (int kb = 0; kb < nkb && ok; ++kb) {
             const int u = u0 + kb * 4 + slab, slot = u % NU;

@@ -3,12 +3,10 @@
 
 namespace maya {
 namespace {
-constexpr int kWMaxGroupsHost = 128;         // as moe_window.cuh's
-
 WArgs common(const GroupArgs& A, int cap_groups, int n_embd, int n_ff, const SharedArgs* sh, const WaitArgs& wait) {
     WArgs W{};
-    W.ptr = A.ptr; W.start = A.start; W.n_groups = wait.n_groups; W.error = wait.error; W.polls = wait.polls; W.ent_slot = A.ent_slot; W.skip = A.skip; W.cap = cap_groups;
-    W.tok_from_slot = A.tok_from_slot; W.n_embd = n_embd; W.n_ff = n_ff;
+    W.ptr = A.ptr; W.start = A.start; W.n_groups = wait.n_groups; W.error = wait.error; W.polls = wait.polls; W.ent_slot = A.ent_slot;
+    W.cap = cap_groups; W.n_embd = n_embd; W.n_ff = n_ff;
     if (sh != nullptr) { W.n_ff_sh = sh->n_ff; W.n_tok = sh->n_tok; W.sh_hq = (uint8_t*) sh->hq; W.sh_out = sh->out; }
     return W;
 }
@@ -22,7 +20,7 @@ template<bool SH, bool UP> int launch_window_type(int type, const WArgs& W, cuda
 
 int window_gate_up(int gu_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t up_off, float limit, const void* xq,
                    size_t xq_stride, void* hq, const SharedArgs* sh, const WaitArgs& wait, cudaStream_t s) {
-    if (cap_groups > kWMaxGroupsHost) return kWindowTooWide;
+    if (cap_groups > kWMaxGroups) return kWindowTooWide;
     WArgs W = common(A, cap_groups, n_embd, n_ff, sh, wait);
     W.up_off = up_off; W.limit = limit;
     W.xq = (const uint8_t*) xq; W.xq_stride = xq_stride; W.hq = (uint8_t*) hq;
@@ -32,7 +30,7 @@ int window_gate_up(int gu_type, const GroupArgs& A, int cap_groups, int n_embd, 
 }
 int window_down(int d_type, const GroupArgs& A, int cap_groups, int n_embd, int n_ff, size_t down_off, const void* hq, float* part,
                 const SharedArgs* sh, const WaitArgs& wait, cudaStream_t s) {
-    if (cap_groups > kWMaxGroupsHost) return kWindowTooWide;
+    if (cap_groups > kWMaxGroups) return kWindowTooWide;
     WArgs W = common(A, cap_groups, n_embd, n_ff, sh, wait);
     W.row_off = down_off;
     W.xq = (const uint8_t*) hq; W.xq_stride = (size_t) (n_ff / 32) * kQ81Bytes; W.part = part;

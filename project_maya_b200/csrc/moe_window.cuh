@@ -1,5 +1,5 @@
-// moe_window.cuh - the routed experts (and the shared one) of a window (2..16 tokens) or of a short plan: gate/up + SwiGLU + q8_1(h), and the down
-// rows, with the weight rows streamed through shared memory.
+// moe_window.cuh - the routed experts (and the shared one) of a window (1..16 tokens): gate/up + SwiGLU + q8_1(h),
+// and the down rows, with the weight rows streamed through shared memory.
 //
 // What bounds this path: on a B200 neither HBM nor the dot products but instruction issue and the shared-memory pipe - a
 // 2-4 bit weight costs 60-90 instructions per 32 to decode and 14-38 per column to dot - so everything around them has to
@@ -39,7 +39,6 @@ namespace {
 
 constexpr int kWNC = 8;            // most activation columns of a job
 constexpr int kWStages = 2;        // segments in flight a warp
-constexpr int kWMaxGroups = 128;   // T <= 16 tokens x 8 routes
 constexpr int kWMaxJobs = kWMaxGroups + 16;      // a job has at least one entry; the shared expert's at least one token
 constexpr int kWChunkRows = 64;    // weight rows of a block's step: 16 warps x 4
 
@@ -331,7 +330,6 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     mbar_fence_init();
     __syncthreads();
     grid_dependency_wait();
-    if (A.skip != nullptr && *A.skip) return;
 
     // ---- the jobs, by one warp; the codebook's copies, by the others
     if (warp > 0) {
@@ -367,8 +365,8 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             int ne = 0;
             if (g < ng) {
                 J.ptr = A.ptr[g];
-                J.e0 = A.start ? A.start[g] : g;
-                ne = (A.start ? A.start[g + 1] : g + 1) - J.e0;
+                J.e0 = A.start[g];
+                ne = A.start[g + 1] - J.e0;
             } else if (g < ng + nsh) {
                 J.ptr = (unsigned long long) A.sh;
                 J.e0 = (g - ng) * A.ncm;
@@ -489,7 +487,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         const bool shd = SH && J.shared;
         const WKind& K = sh.kind[shd ? 1 : 0];
         const int nc = J.nc, n_in = K.n_in;
-        auto slot_of = [&](int c) { return shd ? J.e0 + c : A.ent_slot ? A.ent_slot[J.e0 + c] : J.e0 + c; };     // shared: the token
+        auto slot_of = [&](int c) { return shd ? J.e0 + c : A.ent_slot[J.e0 + c]; };     // shared: the token
         if (__syncthreads_or(gave_up(warp))) goto leave;         // everyone is done with the old columns; or has to leave
         {
             const int nblk = n_in / 32, items = nc * nblk;
@@ -501,7 +499,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                     if (i >= items) continue;
                     const int c = i / nblk, slot = slot_of(c);
                     const uint8_t* src;
-                    if constexpr (UP) src = A.xq + (size_t) (shd ? slot : A.tok_from_slot ? slot >> 3 : 0) * A.xq_stride;
+                    if constexpr (UP) src = A.xq + (size_t) (shd ? slot : slot >> 3) * A.xq_stride;
                     else src = shd ? A.sh_hq + (size_t) slot * nblk * kQ81Bytes : A.xq + (size_t) slot * A.xq_stride;
                     col_read(src, i - c * nblk, v[u]);
                 }
@@ -616,11 +614,11 @@ int launch_window_cb(WArgs A, cudaStream_t s) {
     using G = WGeo<T>;
     constexpr int kStage = SH && WShGeo::stage > G::stage ? WShGeo::stage : G::stage, kRing = G::warps * kWStages * kStage;
     // columns of a job: what fits beside the ring and the codebook, eight at most (a job's rows are decoded once for them all)
-    const long room = 232448l - (long) sizeof(WShared) - 256 - kRing - G::tab;
+    constexpr long room = 232448l - (long) sizeof(WShared) - 256 - kRing - G::tab;
+    static_assert(room >= kColBytes<CB>, "a column has to fit");
     A.ncm = (int) (room / kColBytes<CB>);
     if (A.ncm > G::nc) A.ncm = G::nc;
     if (A.ncm == 5 || A.ncm == 7) --A.ncm;            // five columns are dotted as six, seven as eight: the room has to be there
-    if (A.ncm < 1) return kWindowTooWide;
     A.plain = ((A.row_off | A.up_off | (size_t) (UP ? A.n_ff : A.n_embd) * row_bytes(T, UP ? A.n_embd : A.n_ff)) & 15) != 0;
     const size_t smem = (size_t) kRing + G::tab + (size_t) A.ncm * kColBytes<CB>;
     static SmemLimit smem_limit;                           // (smem is the same in every call of an instantiation)

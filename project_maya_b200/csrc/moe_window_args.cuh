@@ -5,17 +5,17 @@
 
 namespace maya {
 
+constexpr int kWMaxGroups = 128;     // T <= 16 tokens x 8 routes
+
 // What a launch works on.
 struct WArgs {
     const unsigned long long* ptr;   // [groups] blob addresses (0: skipped)
-    const int* start;                // [groups + 1] entry ranges, or NULL: group g has the single entry g
+    const int* start;                // [groups + 1] entry ranges
     int* n_groups;                   // device count; set to -1 when a wait ran out
-    const int* ent_slot;             // [entries] an entry's h / partial slot, or NULL: the entry number
-    const int* skip;                 // optional "do nothing" flag
+    const int* ent_slot;             // [entries] an entry's h / partial slot: 8 token + route
     unsigned* error;                 // optional: set to 1 when a wait ran out
     unsigned polls;                  // looks at a row's copy before a warp gives up
     int cap;                         // most groups (<= kWMaxGroups)
-    int tok_from_slot;               // gate/up: an entry's column is slot >> 3 (a window), else column 0 (one token)
     int ncm;                         // columns of a job, <= kWNC
     int plain;                       // the rows do not start and end on 16-byte boundaries inside a blob: no bulk copies
     int n_embd, n_ff;
@@ -32,8 +32,8 @@ struct WArgs {
     float* sh_out;                   // down out: [n_tok][n_embd]
 };
 
-// By type (GROUP 0: Q8_0, the K-quants and IQ4_XS, 1: the codebook types); SH: with A.sh.  kWindowTooWide: the shapes leave no
-// room for a column, nothing launched.
+// By type (GROUP 0: Q8_0, the K-quants and IQ4_XS, 1: the codebook types); SH: with A.sh.  kWindowTooWide: the rows are
+// longer than a column has room for, nothing launched.
 template<bool SH, bool UP, int GROUP> int launch_window_group(int type, const WArgs& A, cudaStream_t s);
 
 }  // namespace maya
