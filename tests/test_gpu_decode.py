@@ -426,8 +426,9 @@ def test_window_reports_a_wait_that_ran_out(T, api, t, n_tok):
 @pytest.mark.parametrize("t,n_embd,n_ff,n_tok", [
     (H.IQ2_S, 4096, 256, 5), (H.IQ2_S, 4352, 768, 7), (H.IQ2_S, 8448, 256, 3),     # column capacities 128, 256 and none; 5 and 7 columns
     (H.IQ3_S, 6144, 256, 16), (H.IQ3_S, 2304, 1280, 7), (H.IQ3_XXS, 4352, 768, 5),  # two jobs of one expert; rows off a 16-byte boundary
-    (H.Q4_K, 7168, 256, 9), (H.Q5_K, 6400, 512, 4), (H.Q8_0, 2880, 1056, 6), (H.Q6_K, 3328, 768, 8), (H.IQ2_XXS, 2048, 256, 2)])
-def test_window_edges_bitwise(T, api, t, n_embd, n_ff, n_tok):
+    (H.Q4_K, 7168, 256, 9), (H.Q5_K, 6400, 512, 4), (H.Q8_0, 2880, 1056, 6), (H.Q6_K, 3328, 768, 8), (H.IQ2_XXS, 2048, 256, 2),
+    (H.Q4_K, 512, 8448, 3), (H.Q8_0, 8224, 8224, 2)])                               # down rows alone, and both, beyond the streamed form
+def test_window_edges_bitwise(T, api, oracle, t, n_embd, n_ff, n_tok):
     """Every token shares its experts with every other one, so the jobs are as wide as the shared memory lets them be: each
     token's output equals its single-token window's, in which every job has one column, bit for bit."""
     E, k = 3, 2
@@ -440,6 +441,35 @@ def test_window_edges_bitwise(T, api, t, n_embd, n_ff, n_tok):
     for i in range(n_tok):
         one = run_window(T, api, t, n_embd, n_ff, store, ids[i:i + 1], w[i:i + 1], x[i:i + 1], H.INF)[0]
         assert T.isfinite(one).all() and T.equal(out[i], one[0]), f"token {i}"
+    if n_ff > 8192:
+        want = oracle_plan(oracle, t, n_embd, n_ff, [store[int(e)].cpu().numpy() for e in ids[0]], w[0], x[0], H.INF)
+        assert H.rel_err(out[0].cpu().numpy(), want) <= TIGHT
+
+
+@pytest.mark.parametrize("t", [H.Q8_0, H.IQ2_S, H.IQ3_S, H.Q6_K])              # blocks made of 2-byte fields
+@pytest.mark.parametrize("shift,gap", [(2, 0), (8, 0), (0, 6)])
+def test_window_rows_that_bulk_copies_cannot_take(T, api, t, shift, gap):
+    """Blobs that start off a 16-byte boundary, and down rows that do (a gap in front of them): read with ordinary loads, with the
+    bits of the same rows where bulk copies take them."""
+    n_embd, n_ff, E, k, n_tok = 2304, 512, 3, 2, 5
+    blobs = [H.constructed_expert(t, t, n_embd, n_ff, H.rng_for("win-off", t, e)) for e in range(E)]
+    rng = H.rng_for("win-off", t)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(n_tok)]).astype(np.int64)
+    w, x = rng.random((n_tok, k)).astype(np.float32), rng.standard_normal((n_tok, n_embd)).astype(np.float32)
+    want = run_window(T, api, t, n_embd, n_ff, dev(T, np.stack(blobs)), ids, w, x, 7.0)[0]
+    down = 2 * n_ff * H.row_bytes(t, n_embd)
+    room = (len(blobs[0]) + gap + shift + 31) // 16 * 16
+    store = T.zeros((E, room), dtype=T.uint8, device="cuda")
+    for e, b in enumerate(blobs):
+        store[e, shift:shift + down] = dev(T, b[:down])
+        store[e, shift + down + gap:shift + gap + len(b)] = dev(T, b[down:])
+
+    def call(gu, d, win):
+        win.down_off = down + gap
+        api.moe_win_experts(gu, d, win)
+
+    got = run_window(T, api, t, n_embd, n_ff, store[:, shift:], ids, w, x, 7.0, call)[0]
+    assert T.isfinite(want).all() and want.abs().max() > 0 and T.equal(got, want)
 
 
 # ------------------------------------------------------------------------------------------------ grouped (native) form

@@ -255,7 +255,8 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
 
 @pytest.mark.parametrize("t,n_embd,n_ff,n_ff_sh,n_expert,n_tok,sigmoid", [
     (H.IQ2_S, 1024, 256, 512, 12, 2, False), (H.Q4_K, 1280, 768, 1312, 12, 9, False),      # the shared expert's jobs: one; three of 4, 4, 1
-    (H.Q8_0, 1056, 288, 4128, 300, 7, True), (H.IQ3_S, 4352, 512, 256, 600, 16, False)])   # rows beyond 4096 values; 2 and 4 experts a thread
+    (H.Q8_0, 1056, 288, 4128, 300, 7, True), (H.IQ3_S, 4352, 512, 256, 600, 16, False),    # rows beyond 4096 values; 2 and 4 experts a thread
+    (H.Q4_K, 512, 256, 8448, 8, 3, False)])                                                # too wide to ride: launches of its own
 def test_window_with_shared_expert_equals_fused_tokens_bitwise(T, api, t, n_embd, n_ff, n_ff_sh, n_expert, n_tok, sigmoid):
     """A window whose shared expert rides in the routed experts' launches, behind the one launch that routes, quantizes and
     groups: every token has the fused single-token kernel's ids, weights and output, bit for bit."""
