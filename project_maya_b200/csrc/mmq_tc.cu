@@ -348,12 +348,6 @@ __device__ __forceinline__ bool wait_or_fail(Pipe& P, uint64_t* bar, uint32_t pa
 __device__ __forceinline__ int rows_up8(int nrows) { return (nrows + 7) & ~7; }
 template<bool GLU> __device__ __forceinline__ int staging_bytes(int nrows) { return rows_up8(nrows) * (GLU ? 128 * 4 : TM * 4); }
 
-// Persistent: one block an SM takes tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the list (group-major, a group's slabs
-// of weight rows side by side, so that the blocks at work share its activation rows in L2).  How many groups there are is
-// known only on the device; a grid sized for the most there can be cost 20 to 30 us a launch in blocks that found no tile
-// (64 tokens over 256 experts: 259 group rows launched, 55 in use), and every tile paid the block's set-up - tensor-memory
-// allocation, codebook, barriers - and its first loads' latency behind the previous block's write-back.  Here the barriers'
-// phases run on from tile to tile, and the raw loader starts the next tile's units while the last one is written back.
 // A tile's rows of h are written by threads this one has met at a barrier since: count them for the down product ...
 __device__ __forceinline__ void red_release(unsigned* counter, unsigned n) {
     fence_proxy_async_all();                         // they are read by tensor copies
@@ -376,6 +370,12 @@ __device__ __forceinline__ bool wait_rows(Pipe& P, const unsigned* counter, unsi
     return true;
 }
 
+// Persistent: one block an SM takes tiles blockIdx.x, blockIdx.x + gridDim.x, ... of the list (group-major, a group's slabs
+// of weight rows side by side, so that the blocks at work share its activation rows in L2).  How many groups there are is
+// known only on the device; a grid sized for the most there can be cost 20 to 30 us a launch in blocks that found no tile
+// (64 tokens over 256 experts: 259 group rows launched, 55 in use), and every tile paid the block's set-up - tensor-memory
+// allocation, codebook, barriers - and its first loads' latency behind the previous block's write-back.  Here the barriers'
+// phases run on from tile to tile, and the raw loader starts the next tile's units while the last one is written back.
 template<int T, bool GLU>
 __global__ void __launch_bounds__(kMmqThreads, 1)
 mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -783,8 +783,8 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         // One product of N = rows rounded up to 16 per accumulator and K = 16: an M = 128 product occupies the tensor core
         // for N / 2 cycles, but only if this warp can issue one that often.  The whole warp walks the loop, converged, and
         // one elected lane issues: everything the products take is warp-uniform and stays in uniform registers.  (With a
-        // single lane inside a divergent branch every operand of every product crossed from a vector register - 31 such
-        // moves and 430-550 cycles a pair of K steps, the longest stage of the whole pipeline.)
+        // single lane inside a divergent branch every operand of every product crossed from a vector register first, and
+        // issuing was the longest stage of the pipeline.)
         const int my = warp == kDqWarps + 1 ? 0 : 1;
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
         const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem));

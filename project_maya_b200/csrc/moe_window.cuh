@@ -15,14 +15,16 @@
 //     so that its 40 MB hide behind an instruction-bound phase instead of taking two GEMV launches and a SwiGLU launch a token.
 //   * codebooks lie in several copies side by side in shared memory, lane l reading copy l % n.
 // Read in place by a grid of (rows, group) blocks (gate/up) and streamed 64 rows a stage (down), an 8-token Q4_K window took
-// 318 us, a 16-token IQ3_S one 570; now 263 and 433.  (32 warps of two rows: 266 and 484, the activation reads then bind.)
+// 318 us, a 16-token IQ3_S one 570; now 224 and 368.  (32 warps of two rows, measured when this form took 263 and 433: 266 and
+// 484, the activation reads then bind.)
 //
 // The arithmetic is rows_dot's (maya_dots.cuh), value for value - the same integers, the same lane order, the same sums - so
 // every token's result is bit-identical to the single-token kernels'.
 //
 // Plain bulk copies (one destination: this block) of this GPU's own memory.  A row need not start on a 16-byte boundary: the
 // aligned window around a segment is copied (expert blobs are 16-byte aligned and a whole number of 16-byte words long, so
-// it stays inside).  A blob that is not 16-byte aligned is copied with ordinary loads instead.  Every wait is bounded.  A warp whose
+// it stays inside).  A blob that is not 16-byte aligned is copied with ordinary loads instead (types made of 2-byte fields; blocks
+// of Q4_K, Q5_K and IQ4_XS are read in wider pieces and need the alignment).  Every wait is bounded.  A warp whose
 // wait ran out asks for nothing more, and its block leaves - together, at the next barrier - after the copies in flight have had
 // the same bounded time to land; the outputs of what was left are missing, and the error word and the group count say so.
 #pragma once
@@ -194,7 +196,8 @@ template<int T, int SPLIT = 1> struct WGeo {
     static constexpr int pitch = (bytes + 15 + 16) & ~15;
     static constexpr int stage = rw / SPLIT * pitch;                                 // a warp's stage
     static constexpr int tab = Fmt<T>::tab_words * 4 * WDec<T, false>::rep;
-    // What a warp's four rows cost against nc columns, in units of 30 cycles, fitted to clock stamps of 16-token windows: per 32
+    // What a warp's four rows cost against nc columns, in units of 30 cycles, fitted to clock stamps of 16-token windows
+    // (Q8_0, Q4_K, IQ2_S, IQ3_S, IQ3_XXS, IQ4_XS; the other four types' are estimates without stamps): per 32
     // calls of a row the decoding (for Q8_0: waiting for its bytes) and every column's dot, and every column's sums at the end.
     // A share that is off by a tenth is a tenth of the launch: with costs counted in instructions instead the slowest of 148
     // blocks took 27 % longer than the mean.
@@ -225,8 +228,7 @@ struct WShared {
 };
 
 // ---- the columns in shared memory.  A column has room for CB q8_1 blocks, a compile-time number, so that the loads of every
-//      column, plane and half differ from one another by constants only (computed addresses were a sixth of the kernel's
-//      instructions): the planes of 16-byte pieces of maya_dots.cuh's planar form, then as many planes of scales and of sums.
+//      column, plane and half differ from one another by constants only: the planes of 16-byte pieces of maya_dots.cuh's planar form, then as many planes of scales and of sums.
 template<int CB> constexpr int kColBytes = CB * 40;
 template<int XB, int CB> __device__ __forceinline__ XQ col_load(const uint8_t* cols, int c, int j, int i16, int i4) {
     constexpr int P = CB / XB;

@@ -15,6 +15,10 @@
 // front and into registers before the norm's reduction, 16 bytes a lane; and a block takes only as many experts as leave
 // one block an SM (its eight warps split between them), where one warp per expert kept 32 of 148 SMs busy with a chain
 // of dependent 2-byte loads: 19.7 us a call at that size, about 7 us now.
+//
+// A logit is an f32 sum whose order - and with it its last bits - depends on how many warps share a row (8, 4, 2 or 1, by the
+// number of experts and SMs) and on whether the 16-byte form runs (alignment): equal to rounding, not bit for bit, between calls
+// that differ in these.  The same call gives the same bits.
 #include "maya_common.cuh"
 
 namespace maya {
@@ -152,9 +156,10 @@ int launch(const float* h, const float* add, const float* w, float eps, int n, c
     static SmemLimit smem_limit;
     if (smem > kSmemNoLimit && !smem_limit.raise((const void*) rms_router_kernel<BF16, VEC>, kSmemMost)) return note_launch("rms_router smem attribute");
     // experts a block: the fewest (1, 2, 4 or 8) that leave at most one block an SM, so that a small router spreads over the
-    // chip (beyond 8 x 148 experts blocks share SMs)
+    // chip (beyond 8 experts an SM blocks share SMs)
+    const int sms = sm_count();
     int epb = 1;
-    while (epb < kRmsWarps && (n_expert + epb - 1) / epb > 148) epb *= 2;
+    while (epb < kRmsWarps && (n_expert + epb - 1) / epb > sms) epb *= 2;
     launch_dependent(rms_router_kernel<BF16, VEC>, dim3((unsigned) ((n_expert + epb - 1) / epb)), dim3(kRmsThreads), smem, s, h, add, w, eps,
                      n, (const uint8_t*) router, n_expert, epb, h_out, x_out, logits);
     return note_launch("rms_router");
