@@ -457,8 +457,9 @@ class MoeLayer:
 
 class MoePrefill:
     """The prompt path of one resident layer for a chunk of up to `max_tokens` tokens, with no host round trip:
-    route -> group rows by expert -> q8_1 of the gathered rows -> gate/up grouped GEMM with SwiGLU in its write-back ->
-    q8_1 of h -> down grouped GEMM -> weighted combine (+ the shared expert as one more product over all rows).
+    route -> group rows by expert -> each token rounded to q8_1 once and stored to its k sorted rows -> one chain of grouped
+    GEMMs (gate/up with SwiGLU and the q8_1 rounding of h in its write-back, then down; every pool's products and, over all
+    rows, the shared expert's) -> weighted combine.
 
     Follows the reference's prefill_run expert sequence (src/core/glm_prefill.cu:3230-3420: expert_count, bases,
     expert_scatter, mmq::quantize, Context::run_glu, mmq::quantize, Context::run, moe_combine), except that the bases
