@@ -29,9 +29,8 @@
 // the same bounded time to land; the outputs of what was left are missing, and the error word and the group count say so.
 #pragma once
 
-#include "maya_dots.cuh"
 #include "maya_internal.cuh"
-#include "maya_stream.cuh"
+#include "maya_rows.cuh"
 #include "moe_window_args.cuh"
 
 #include <type_traits>
@@ -44,158 +43,16 @@ constexpr int kWStages = 2;        // segments in flight a warp
 constexpr int kWMaxJobs = kWMaxGroups + 16;      // a job has at least one entry; the shared expert's at least one token
 constexpr int kWChunkRows = 64;    // weight rows of a block's step: 16 warps x 4
 
-// ---- decoders: Dec<T>'s fields and dot, loaded from shared memory - byte `o` of `s` is the block's first - with fewer
-//      instructions.  rep: copies of the codebook, `tab` = this lane's copy.  ONE: for a single column, where it is cheaper to
-//      correct the dot for the signs (see maya_dots_t1.cuh) than to negate the weights.
-__device__ __forceinline__ uint32_t s_u32(const uint8_t* s, uint32_t o) { return *(const uint32_t*) (s + o); }
-// 4 bytes at an even place; sel: 0x3210 where o is a multiple of 4, else 0x5432
-__device__ __forceinline__ uint32_t s_u32_a2(const uint8_t* s, uint32_t o, uint32_t sel) {
-    const uint32_t a = o & ~3u;
-    return prmt_raw(s_u32(s, a), s_u32(s, a + 4), sel);
-}
-// the selector for fields 2 bytes (and a multiple of 4) into a block at o
-__device__ __forceinline__ uint32_t sel_2(uint32_t o) { return (o & 2u) ? 0x3210u : 0x5432u; }
-
-template<int T, bool ONE> struct WDec : Dec<T> {
-    static constexpr int rep = 1;
-    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) { Dec<T>::load(s + o, c, tab); }
-};
-// eight signed weight words (or, with ONE, codebook words XOR mask and the masks) and their dots
-template<bool ONE> struct WSigned {
-    int w[8];
-    uint32_t mk[ONE ? 8 : 1];
-    __device__ __forceinline__ void set(int i, uint32_t g, uint32_t m) {
-        if constexpr (ONE) { w[i] = (int) (g ^ m); mk[i] = m; }
-        else w[i] = apply_sign4(g, m);
-    }
-    __device__ __forceinline__ int dot4(const XQ& v, int i0, int s) const {        // words i0 .. i0 + 3
-#pragma unroll
-        for (int i = i0; i < i0 + 4; ++i) s = __dp4a(w[i], v.u[i], s);
-        if constexpr (ONE) {
-            int m = 0;
-#pragma unroll
-            for (int i = i0; i < i0 + 4; ++i) m = __dp4a((int) mk[i], v.u[i], m);
-            s -= m;
-        }
-        return s;
-    }
-};
-template<bool ONE> struct WDec<MAYA_IQ2_S, ONE> : WSigned<ONE> {
-    static constexpr int rep = 8;
-    int ls0, ls1;
-    float d;
-    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
-        const uint32_t sel = sel_2(o);
-        d = ld_f16(s + o);
-        const uint32_t qs = s_u32_a2(s, o + 2 + 4 * c, sel), sg = s_u32_a2(s, o + 34 + 4 * c, sel);
-        const uint32_t qh = s[o + 66 + c], sc = s[o + 74 + c];
-        ls0 = (int) (sc & 0x0F);
-        ls1 = (int) (sc >> 4);
-        const uint2* grid = (const uint2*) tab;
-        const uint32_t hw = ((qh & 0x33u) * 0x1001u + (qh & 0xCCu) * 0x40040u) & 0x03030303u;      // see Dec1<MAYA_IQ2_S>
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const uint2 g = grid[prmt_raw(qs, hw, 0xCC00u + ((4 + l) << 4) + l) * rep];
-            const uint32_t b = byte_of(sg, l);
-            this->set(2 * l, g.x, sign_mask_lo(b));
-            this->set(2 * l + 1, g.y, sign_mask_hi(b));
-        }
-    }
-    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
-        const int s0 = this->dot4(v, 0, 0), s1 = this->dot4(v, 4, 0);
-        return __fmul_rn(__fmul_rn(d, v.d), (float) ((s0 * ls0 + s1 * ls1 + (s0 + s1) / 2) / 4));
-    }
-};
-// IQ3_S: every codebook value is odd, g = 2 b + 1 with b in 0..7.  Flipping b's bits negates it: 2 ~b + 1 = -g.  So the table
-// holds b, a sign is one XOR, and sum(+-g u) = 2 sum((b ^ m) u) + sum(u), the block's sum being at hand.
-template<bool ONE> struct WDec<MAYA_IQ3_S, ONE> {
-    static constexpr int rep = 16;
-    int w[8];
-    int mul;
-    float d;
-    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
-        const uint32_t sel = sel_2(o), qa = (o + 2 + 8 * c) & ~3u;
-        d = ld_f16(s + o);
-        const uint32_t w1 = s_u32(s, qa + 4), q0 = prmt_raw(s_u32(s, qa), w1, sel), q1 = prmt_raw(w1, s_u32(s, qa + 8), sel);
-        const uint32_t qh = s[o + 66 + c], sg = s_u32_a2(s, o + 74 + 4 * c, sel);
-        mul = 1 + 2 * (int) ((s[o + 106 + (c >> 1)] >> (4 * (c & 1))) & 0x0F);
-        // byte l of h0 / h1: bit l / 4 + l of qh, an entry's ninth index bit
-        const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-            const uint32_t b = tab[prmt_raw(l < 4 ? q0 : q1, l < 4 ? h0 : h1, 0xCC00u + ((4 + l % 4) << 4) + l % 4) * rep];
-            const uint32_t sb = byte_of(sg, l >> 1);
-            w[l] = (int) (b ^ ((l & 1) ? sign_mask_hi(sb) : sign_mask_lo(sb)));
-        }
-    }
-    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
-        int s = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) s = __dp4a(w[i], v.u[i], s);
-        return __fmul_rn(__fmul_rn(d, v.d), (float) ((2 * s + v.isum) * mul));
-    }
-};
-template<bool ONE> struct WDec<MAYA_IQ3_XXS, ONE> : WSigned<ONE> {
-    static constexpr int rep = 32;
-    int ls;
-    float d;
-    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
-        const uint32_t sel = sel_2(o), qa = (o + 2 + 8 * c) & ~3u;
-        d = ld_f16(s + o);
-        const uint32_t w1 = s_u32(s, qa + 4), q0 = prmt_raw(s_u32(s, qa), w1, sel), q1 = prmt_raw(w1, s_u32(s, qa + 8), sel);
-        const uint32_t aux = s_u32_a2(s, o + 66 + 4 * c, sel);
-        ls = (int) (aux >> 28);
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const uint32_t s8 = ksign8((aux >> (7 * l)) & 127u), q = l < 2 ? q0 : q1;
-            this->set(2 * l, tab[byte_of(q, 2 * (l & 1)) * rep], sign_mask_lo(s8));
-            this->set(2 * l + 1, tab[byte_of(q, 2 * (l & 1) + 1) * rep], sign_mask_hi(s8));
-        }
-    }
-    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
-        const int t = this->dot4(v, 4, this->dot4(v, 0, 0));
-        return __fmul_rn(__fmul_rn(d, v.d), (float) ((ls * t + t / 2) / 2));
-    }
-};
-template<bool ONE> struct WDec<MAYA_IQ2_XXS, ONE> : WSigned<ONE> {
-    static constexpr int rep = 16;
-    int ls;
-    float d;
-    __device__ __forceinline__ void load(const uint8_t* s, uint32_t o, int c, const uint32_t* tab) {
-        const uint32_t sel = sel_2(o), qa = (o + 2 + 8 * c) & ~3u;
-        d = ld_f16(s + o);
-        const uint32_t w1 = s_u32(s, qa + 4), qi = prmt_raw(s_u32(s, qa), w1, sel), aux = prmt_raw(w1, s_u32(s, qa + 8), sel);
-        ls = (int) (aux >> 27) | 1;
-        const uint2* grid = (const uint2*) tab;
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const uint2 g = grid[byte_of(qi, l) * rep];
-            const uint32_t s8 = ksign8((aux >> (7 * l)) & 127u);
-            this->set(2 * l, g.x, sign_mask_lo(s8));
-            this->set(2 * l + 1, g.y, sign_mask_hi(s8));
-        }
-    }
-    __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {
-        const int t = this->dot4(v, 4, this->dot4(v, 0, 0));
-        return __fmul_rn(__fmul_rn(d, v.d), (float) (t * ls / 8));
-    }
-};
-
-// ---- the geometry of a type's stream.  A segment: kSegVals values of a row (a multiple of what 32 lanes take in one step, so
-//      that a lane's calls are the same whatever the segments are).  kPitch: a segment's room in a stage, its bytes and 16 for
-//      the aligned window.
-template<int T, int SPLIT = 1> struct WGeo {
+// ---- the geometry of a type's stream here
+template<int T, int SPLIT = 1> struct WGeo : RowGeo<T> {
     static constexpr int split = SPLIT;          // a segment comes in this many stages, rw / SPLIT rows each
     static constexpr int warps = 16, threads = warps * 32, rw = kWChunkRows / warps;      // a warp's rows: 4
     // most columns of a job: four where a call spans two q8_1 blocks (six or eight spill 1.3 KB: 617 against 263 us on the window above)
     static constexpr int nc = Dec<T>::xblk == 2 ? 4 : kWNC;
-    static constexpr int vals = T == MAYA_Q8_0 || T == MAYA_Q6_K ? 1024 : 2048;
-    static constexpr int qk = Fmt<T>::qk, cpb = Dec<T>::cpb;
-    static constexpr int blocks = vals / qk;                                 // weight blocks of a segment
-    static constexpr int bytes = blocks * Fmt<T>::bytes;
-    static constexpr int pitch = (bytes + 15 + 16) & ~15;
-    static constexpr int stage = rw / SPLIT * pitch;                                 // a warp's stage
-    static constexpr int tab = Fmt<T>::tab_words * 4 * WDec<T, false>::rep;
+    using RowGeo<T>::qk;
+    using RowGeo<T>::cpb;
+    static constexpr int stage = rw / SPLIT * RowGeo<T>::pitch;                                 // a warp's stage
+    static constexpr int tab = RowTab<T, false>::bytes;
     // What a warp's four rows cost against nc columns, in units of 30 cycles, fitted to clock stamps of 16-token windows
     // (Q8_0, Q4_K, IQ2_S, IQ3_S, IQ3_XXS, IQ4_XS; the other four types' are estimates without stamps): per 32
     // calls of a row the decoding (for Q8_0: waiting for its bytes) and every column's dot, and every column's sums at the end.
@@ -271,24 +128,26 @@ template<int XB, int CB, bool SUM_F16> __device__ __forceinline__ void col_store
 // dropped), so that no branch parts one column's loads from the next one's arithmetic.
 template<int T, class G, int NC, int RW, int CB>
 __device__ __forceinline__ void segment_dot(const uint8_t* s, const uint32_t (&row)[RW], const uint8_t* cols, int blk0, int ncalls, int lane,
-                                            const uint32_t* tab, float (&acc)[RW][NC]) {
+                                            const RowLut<T, false>& lut, float (&acc)[RW][NC]) {
     constexpr int XB = Dec<T>::xblk, RP = XB == 2 || NC > 4 || RW < 4 ? 2 : 4;
+    using D = SDec<T, NC == 1, false>;
     for (int k = lane; k < ncalls; k += 32) {
         const int kb = k / G::cpb, ci = k - kb * G::cpb;
-        const int n = ((blk0 + kb) * (G::qk / 32) + ci * XB) / XB;
+        // the call's place in the row, and its blocks' in a plane (the same number; written so that it costs fewest registers)
+        const int n = Fmt<T>::tab_words > 0 ? blk0 * G::cpb + k : ((blk0 + kb) * (G::qk / 32) + ci * XB) / XB;
 #pragma unroll
         for (int r0 = 0; r0 < RW; r0 += RP) {
             if (r0 > 0) asm volatile("" ::: "memory");       // the second two rows' loads stay behind: their registers are the first two's
-            WDec<T, NC == 1> dec[RP];
+            D dec[RP];
 #pragma unroll
-            for (int j = 0; j < RP; ++j) dec[j].load(s, row[r0 + j] + kb * Fmt<T>::bytes, ci, tab);
+            for (int i = 0; i < RP; ++i) dec[i].load(s, D::at(row[r0 + i] + kb * Fmt<T>::bytes, ci), 0, ci, lut);
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
                 const XQ a = col_load<XB, CB>(cols, c, 0, n * 16, n * 4);
                 XQ b = a;
                 if constexpr (XB == 2) b = col_load<XB, CB>(cols, c, 1, n * 16, n * 4);
 #pragma unroll
-                for (int j = 0; j < RP; ++j) acc[r0 + j][c] = __fadd_rn(acc[r0 + j][c], dec[j].dot(a, b));
+                for (int i = 0; i < RP; ++i) acc[r0 + i][c] = __fadd_rn(acc[r0 + i][c], dec[i].dot(a, b));
             }
         }
     }
@@ -301,7 +160,6 @@ template<int T, bool SH, bool UP, int CB>
 __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs A) {
     using G = WGeo<T>;
     using GS = WShGeo;
-    using D = WDec<T, false>;
     constexpr int RW = G::rw, kWThreads = G::threads, kStage = SH && GS::stage > G::stage ? GS::stage : G::stage;
     constexpr int kRing = G::warps * kWStages * kStage;
     extern __shared__ __align__(128) uint8_t s_raw[];
@@ -335,24 +193,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
 
     // ---- the jobs, by one warp; the codebook's copies, by the others
     if (warp > 0) {
-        if constexpr (G::tab > 0) {
-            constexpr int W = (T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1, R = D::rep, NT = kWThreads - 32;
-            const uint32_t* src = tab_source<T>();
-#pragma unroll 4
-            for (int e = tid - 32; e < G::tab / 4 / R; e += NT) {                // a codebook word, and its copies: R / 4 16-byte stores
-                uint32_t g = src[e];
-                if constexpr (T == MAYA_IQ3_S) g = (g >> 1) & 0x07070707u;
-                if constexpr (W == 1) {
-#pragma unroll
-                    for (int r = 0; r < R; r += 4)
-                        if constexpr (R >= 4) ((uint4*) s_tab)[e * (R / 4) + r / 4] = make_uint4(g, g, g, g);
-                        else s_tab[e] = g;
-                } else {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) s_tab[((e / 2) * R + r) * 2 + (e & 1)] = g;
-                }
-            }
-        }
+        RowTab<T, false>::fill(s_tab, tid - 32, kWThreads - 32);
     } else {
         int ng = *A.n_groups;
         const bool lost = ng < 0;                                // a wait of the launch in front ran out: no work
@@ -478,7 +319,8 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
     };
     for (int s = 0; s < kWStages; ++s) ask();
 
-    const uint32_t* const tab = s_tab + (lane % D::rep) * ((T == MAYA_IQ2_S || T == MAYA_IQ2_XXS) ? 2 : 1);
+    const RowLut<T, false> lut(s_tab, lane);
+    const RowLut<MAYA_Q8_0, false> lut_sh(s_tab, lane);          // (no codebook)
     int stage = 0, buf = 0;
     uint32_t phase = 0;
     auto gave_up = [&](int w) { return *(volatile int*) &sh.gave_up[w]; };
@@ -544,7 +386,8 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                     uint32_t row[RS];
 #pragma unroll
                     for (int r = 0; r < RS; ++r) row[r] = ring + stage * kStage + r * GT::pitch + ((start[p * RS + r] + so) & 15u);
-                    segment_dot<TY, GT, NC, RS, CB>(s_raw, row, cols, blk0, ncalls, lane, tab, *(float(*)[RS][NC]) &acc[p * RS]);
+                    if constexpr (TY == T) segment_dot<TY, GT, NC, RS, CB>(s_raw, row, cols, blk0, ncalls, lane, lut, *(float(*)[RS][NC]) &acc[p * RS]);
+                    else segment_dot<TY, GT, NC, RS, CB>(s_raw, row, cols, blk0, ncalls, lane, lut_sh, *(float(*)[RS][NC]) &acc[p * RS]);
                     stage = stage + 1 == kWStages ? 0 : stage + 1;
                     if (stage == 0) phase ^= 1u;
                     ask();
