@@ -77,7 +77,7 @@ def run(torch, api) -> dict:
            "us_per_token": us, "tok_s_layer": 1e6 / us, "launch": f"CUDA graph of {N_STEPS} steps",
            "roofline": {"bound": "hbm", "algorithmic_bytes_per_step": nbytes, "achieved": nbytes / us / 1e3, "peak": peak,
                         "peak_kind": kind, "unit": "GB/s", "frac": nbytes / us / 1e3 / peak,
-                        "kernel": "moe_layer_t1_kernel<Q4_K, none> (one launch a step)"},
+                        "kernel": "token_kernel<Q4_K, none> (one launch a step)"},
            "error": max(l.error() for l in layers)}
 
     from oracle import ref_gpu

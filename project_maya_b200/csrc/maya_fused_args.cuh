@@ -1,4 +1,4 @@
-// maya_fused_args.cuh - the argument block of the single-token layer kernels (moe_fused.cu, moe_stream.cu).
+// maya_fused_args.cuh - the argument blocks of the single-token layer kernels (moe_fused.cu, moe_token.cuh).
 #pragma once
 
 #include "maya_common.cuh"
@@ -33,6 +33,16 @@ struct FusedArgs {
     unsigned ar_seq;
     maya_hc_post_args hc;      // hc.R_new != NULL: the hyper-connection write of `out` into the residual stack, last
     unsigned* sync;            // scratch: [0] arrivals, [1] epoch, [2] error, [4..13] block 0's phase time stamps (ns)
+};
+
+// moe_token.cuh: the rows' places in a blob, and the launch's carve-up of shared memory.
+struct TokArgs : FusedArgs {
+    int d_type;
+    size_t up_off, down_off;   // byte offsets of the up and of the down rows in a routed blob
+    unsigned* unit_count;      // scratch [(MAYA_MAX_K + 1) * blocks of h]: items done of units that two blocks share, modulo 16
+    unsigned polls;            // looks at a row's copy before a warp gives up
+    int stage, tab, cols;      // bytes of a ring stage, of the codebook, of the activation columns
+    int units;                 // units of h a block may work on
 };
 
 }  // namespace maya

@@ -56,10 +56,14 @@ int win_combine(const unsigned long long* plan_ptr, const float* plan_w, int T, 
 int win_experts(int gu_type, int d_type, const maya_moe_win* w, bool grouped, const SharedArgs* sh, unsigned polls, unsigned* error,
                 const maya_peer_ar* ar, int mi, unsigned seq, cudaStream_t s);
 
-// The fused single-token layer kernel (moe_fused.cu).
+// One token through a layer in one launch: the token kernel (moe_token.cuh) or the fused kernel (moe_fused.cu).  kNotHere: neither
+// takes the layer, nothing launched.
+constexpr int kNotHere = 1;
+struct FusedArgs;
 bool fused_t1_supported(const maya_moe_layer& L);
 int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_is_bf16, int* ids, float* weights,
-             float* out, float* h_scratch, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
+             float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
              const maya_hc_post_args* hc, cudaStream_t s);
+int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_count, cudaStream_t s);
 
 }  // namespace maya

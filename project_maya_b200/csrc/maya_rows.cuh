@@ -27,10 +27,15 @@ __device__ __forceinline__ uint32_t s_u32_a2(const uint8_t* s, uint32_t o, uint3
 }
 // the selector for fields 2 bytes (and a multiple of 4) into a block at o
 __device__ __forceinline__ uint32_t sel_2(uint32_t o) { return (o & 2u) ? 0x3210u : 0x5432u; }
-// c + a's low (b = f) or high (b = f << 8) 16 bits times f, f < 256
-__device__ __forceinline__ uint32_t dp2a_lo(uint32_t a, uint32_t b, uint32_t c) {
+// c + a's low or high 16 bits times f, b = f | f << 24, f < 256
+__device__ __forceinline__ uint32_t dp2a_low(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
     asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t dp2a_high(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("dp2a.hi.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
 // c + byte l of a times f (b = f << 8 l), f < 256
@@ -83,45 +88,50 @@ template<int T, bool MANY> struct RowTab {
     static constexpr int words = T == MAYA_IQ2_S ? 1024 : Fmt<T>::tab_words;   // of one copy
     static constexpr int sign_off = words * 4 * copies, bytes = sign_off + 256 * 4 * signs;
 
-    // by threads tid of nt; 16 bytes a store where there are four copies of a word
+    // by threads tid of nt, 16 bytes a store: consecutive threads to consecutive places
     __device__ __forceinline__ static void fill(uint32_t* tab, int tid, int nt) {
         if constexpr (bytes > 0) {
             const uint32_t* src = tab_source<T>();
+            if constexpr (W == 2) {                                              // two words an entry: two copies a store
+                constexpr int P = copies / 2;
 #pragma unroll 4
-            for (int e = tid; e < words; e += nt) {
-                uint32_t g;
-                if constexpr (T == MAYA_IQ2_S) {                                 // eight nibbles: 0, 1, 2 for 8, 25, 43
-                    const uint2 v = ((const uint2*) src)[e];
-                    auto code = [](uint32_t b) { return (b >> 4) & 0x03030303u; };      // 0x08, 0x19, 0x2b
-                    auto pack = [](uint32_t c) { c = (c | c >> 4) & 0x00FF00FFu; return (c | c >> 8) & 0xFFFFu; };
-                    g = pack(code(v.x)) | pack(code(v.y)) << 16;
-                } else {
-                    g = src[e];
-                    if constexpr (T == MAYA_IQ3_S) g = (g >> 1) & 0x07070707u;   // see SDec<MAYA_IQ3_S>
+                for (int i = tid; i < words / 2 * P; i += nt) {
+                    const uint2 g = ((const uint2*) src)[i / P];
+                    ((uint4*) tab)[i] = make_uint4(g.x, g.y, g.x, g.y);
                 }
-                put<copies>(tab, e, g);
+            } else if constexpr (copies == 1) {
+                for (int i = tid; i < words; i += nt) tab[i] = src[i];
+            } else {
+                constexpr int P = copies / 4;
+#pragma unroll 4
+                for (int i = tid; i < words * P; i += nt) {
+                    uint32_t g;
+                    if constexpr (T == MAYA_IQ2_S) {                             // eight nibbles: 0, 1, 2 for 8, 25, 43
+                        const uint2 v = ((const uint2*) src)[i / P];
+                        auto pack = [](uint32_t c) {                             // 0x08, 0x19, 0x2b
+                            c = (c >> 4) & 0x03030303u;
+                            c = (c | c >> 4) & 0x00FF00FFu;
+                            return (c | c >> 8) & 0xFFFFu;
+                        };
+                        g = pack(v.x) | pack(v.y) << 16;
+                    } else {
+                        g = src[i / P];
+                        if constexpr (T == MAYA_IQ3_S) g = (g >> 1) & 0x07070707u;       // see SDec<MAYA_IQ3_S>
+                    }
+                    ((uint4*) tab)[i] = make_uint4(g, g, g, g);
+                }
             }
             if constexpr (signs > 0) {
+                constexpr int P = signs / 4;
 #pragma unroll 2
-                for (int e = tid; e < 256; e += nt) {                            // bit i of the byte at bit 4 i + 2
-                    uint32_t g = 0u;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) g |= (((uint32_t) e >> i) & 1u) << (4 * i + 2);
-                    put<signs>(tab + sign_off / 4, e, g);
+                for (int i = tid; i < 256 * P; i += nt) {                        // bit j of the byte at bit 4 j + 2
+                    const uint32_t e = (uint32_t) (i / P);
+                    uint32_t g = (e & 0x0Fu) | (e & 0xF0u) << 12;                // bits 0..3 and 16..19
+                    g = (g & 0x00030003u) | (g & 0x000C000Cu) << 6;              // two to a byte
+                    g = ((g & 0x01010101u) | (g & 0x02020202u) << 3) << 2;
+                    ((uint4*) (tab + sign_off / 4))[i] = make_uint4(g, g, g, g);
                 }
             }
-        }
-    }
-private:
-    template<int N> __device__ __forceinline__ static void put(uint32_t* t, int e, uint32_t g) {
-        if constexpr (W == 2) {
-#pragma unroll
-            for (int r = 0; r < N; ++r) t[((e / 2) * N + r) * 2 + (e & 1)] = g;
-        } else if constexpr (N >= 4) {
-#pragma unroll
-            for (int r = 0; r < N; r += 4) ((uint4*) t)[e * (N / 4) + r / 4] = make_uint4(g, g, g, g);
-        } else {
-            t[e] = g;
         }
     }
 };
@@ -129,10 +139,14 @@ private:
 template<int T, bool MANY> struct RowLut {
     const uint32_t* p;
     uint32_t a, s;               // shared-memory addresses of the codebook and of the sign words
+    uint32_t fa, fs;             // the entries' distances, as dp2a takes them
     __device__ __forceinline__ RowLut(const uint32_t* tab, int lane) {
         using R = RowTab<T, MANY>;
         p = tab + (lane % R::copies) * R::W;
         a = smem_u32(p);
+        constexpr uint32_t ca = R::copies * R::W * 4, cs = R::signs * 4;
+        asm volatile("mov.u32 %0, %1;" : "=r"(fa) : "n"(ca | ca << 24));      // (opaque: kept in registers)
+        asm volatile("mov.u32 %0, %1;" : "=r"(fs) : "n"(cs | cs << 24));
         s = smem_u32(tab) + R::sign_off + (R::signs > 0 ? lane % (R::signs > 0 ? R::signs : 1) * 4 : 0);
     }
 };
@@ -169,27 +183,28 @@ private:
 };
 // IQ2_S: the weights as nibble selectors (see the head of the file).
 template<bool ONE, bool MANY> struct SDec<MAYA_IQ2_S, ONE, MANY> {
-    struct At { uint32_t q, o, sel; };           // the index bytes' aligned word, the block
+    struct At { uint32_t q, o, c, sel; };        // the index bytes' aligned word, the block, its byte `call`
     int w[8];
     int ls0, ls1;
     float d;
     __device__ __forceinline__ static At at(uint32_t row, int l) {
         const uint32_t o = row + (l >> 3) * 82;
-        return {(o + 2 + 4 * (l & 7)) & ~3u, o, sel_2(o)};
+        return {(o + 2 + 4 * (l & 7)) & ~3u, o, o + (l & 7), sel_2(o)};
     }
-    __device__ __forceinline__ void load(const uint8_t* s, const At& A, int j, int l, const RowLut<MAYA_IQ2_S, MANY>& L) {
-        constexpr int R = RowTab<MAYA_IQ2_S, MANY>::copies * 4, S = RowTab<MAYA_IQ2_S, MANY>::signs * 4;
-        const uint8_t *q = s + A.q + j * 328, *b = s + A.o + j * 328;
+    __device__ __forceinline__ void load(const uint8_t* s, const At& A, int j, int, const RowLut<MAYA_IQ2_S, MANY>& L) {
+        const uint8_t *q = s + A.q + j * 328, *c = s + A.c + j * 328;
         const uint32_t qs = prmt_raw(s_u32(q, 0), s_u32(q, 4), A.sel), sg = prmt_raw(s_u32(q, 32), s_u32(q, 36), A.sel);
-        const uint32_t qh = b[66 + (l & 7)], sc = b[74 + (l & 7)];
-        d = ld_f16(b);
+        const uint32_t qh = c[66], sc = c[74];
+        d = ld_f16(s + A.o + j * 328);
         ls0 = (int) (sc & 0x0F);
         ls1 = (int) (sc >> 4);
         const uint32_t hw = ((qh & 0x33u) * 0x1001u + (qh & 0xCCu) * 0x40040u) & 0x03030303u;      // see Dec1<MAYA_IQ2_S>
         const uint32_t p0 = prmt_raw(qs, hw, 0x5140u), p1 = prmt_raw(qs, hw, 0x7362u);             // the indices, two to a word
+        const uint32_t g0 = __byte_perm(sg, 0, 0x4140), g1 = __byte_perm(sg, 0, 0x4342);           // and the sign bytes
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t n = lds_u32(dp2a_lo(i < 2 ? p0 : p1, (i & 1) ? R << 8 : R, L.a)) | lds_u32(dp4a_u(sg, (uint32_t) S << (8 * i), L.s));
+            const uint32_t p = i < 2 ? p0 : p1, q = i < 2 ? g0 : g1;
+            const uint32_t n = lds_u32((i & 1) ? dp2a_high(p, L.fa, L.a) : dp2a_low(p, L.fa, L.a)) | lds_u32((i & 1) ? dp2a_high(q, L.fs, L.s) : dp2a_low(q, L.fs, L.s));
             w[2 * i] = (int) prmt_raw(0x002B1908u, 0x00D5E7F8u, n);
             w[2 * i + 1] = (int) prmt_raw(0x002B1908u, 0x00D5E7F8u, n >> 16);
         }
@@ -204,30 +219,28 @@ template<bool ONE, bool MANY> struct SDec<MAYA_IQ2_S, ONE, MANY> {
 // IQ3_S: every codebook value is odd, g = 2 b + 1 with b in 0..7.  Flipping b's bits negates it: 2 ~b + 1 = -g.  So the table
 // holds b, a sign is one XOR, and sum(+-g u) = 2 sum((b ^ m) u) + sum(u), the block's sum being at hand.
 template<bool ONE, bool MANY> struct SDec<MAYA_IQ3_S, ONE, MANY> {
-    struct At { uint32_t q, g, o, sel; };        // the aligned words of the index and of the sign bytes, the block
+    struct At { uint32_t q, g, o, c, n, sel; };  // the aligned words of the index and of the sign bytes, the block, its bytes `call` and `call` / 2
     int w[8];
     int mul;
     float d;
     __device__ __forceinline__ static At at(uint32_t row, int l) {
         const uint32_t o = row + (l >> 3) * 110;
-        return {(o + 2 + 8 * (l & 7)) & ~3u, (o + 74 + 4 * (l & 7)) & ~3u, o, sel_2(o)};
+        return {(o + 2 + 8 * (l & 7)) & ~3u, (o + 74 + 4 * (l & 7)) & ~3u, o, o + (l & 7), o + ((l & 7) >> 1), sel_2(o)};
     }
     __device__ __forceinline__ void load(const uint8_t* s, const At& A, int j, int l, const RowLut<MAYA_IQ3_S, MANY>& L) {
-        constexpr int R = RowTab<MAYA_IQ3_S, MANY>::copies * 4;
-        const int c = l & 7;
-        const uint8_t *q = s + A.q + j * 440, *b = s + A.o + j * 440, *g = s + A.g + j * 440;
+        const uint8_t *q = s + A.q + j * 440, *g = s + A.g + j * 440;
         const uint32_t w1 = s_u32(q, 4), q0 = prmt_raw(s_u32(q, 0), w1, A.sel), q1 = prmt_raw(w1, s_u32(q, 8), A.sel);
-        const uint32_t sg = prmt_raw(s_u32(g, 0), s_u32(g, 4), A.sel), qh = b[66 + c];
-        d = ld_f16(b);
-        mul = 1 + 2 * (int) ((b[106 + (c >> 1)] >> (4 * (c & 1))) & 0x0F);
+        const uint32_t sg = prmt_raw(s_u32(g, 0), s_u32(g, 4), A.sel), qh = s[A.c + j * 440 + 66];
+        d = ld_f16(s + A.o + j * 440);
+        mul = 1 + 2 * (int) ((s[A.n + j * 440 + 106] >> (4 * (l & 1))) & 0x0F);
         // byte i of h0 / h1: bit i / 4 + i of qh, an entry's ninth index bit
         const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
         const uint32_t p[4] = {prmt_raw(q0, h0, 0x5140u), prmt_raw(q0, h0, 0x7362u), prmt_raw(q1, h1, 0x5140u), prmt_raw(q1, h1, 0x7362u)};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t sb = byte_of(sg, i);
-            w[2 * i] = (int) (lds_u32(dp2a_lo(p[i], R, L.a)) ^ sign_mask_lo(sb));
-            w[2 * i + 1] = (int) (lds_u32(dp2a_lo(p[i], R << 8, L.a)) ^ sign_mask_hi(sb));
+            w[2 * i] = (int) (lds_u32(dp2a_low(p[i], L.fa, L.a)) ^ sign_mask_lo(sb));
+            w[2 * i + 1] = (int) (lds_u32(dp2a_high(p[i], L.fa, L.a)) ^ sign_mask_hi(sb));
         }
     }
     __device__ __forceinline__ float dot(const XQ& v, const XQ&) const {

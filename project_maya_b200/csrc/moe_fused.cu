@@ -31,16 +31,12 @@
 #include "maya_hc_post.cuh"
 #include "maya_router.cuh"
 #include "maya_fused_args.cuh"
+#include "maya_token_phase.cuh"
 
 namespace maya {
 namespace {
 
 constexpr int kFusedThreads = 1024;
-constexpr int kRouteThreads = 256;
-constexpr int kMaxSliceRows = 96;          // output rows a block may own (n_embd / grid rounded up)
-constexpr unsigned long long kBarrierTimeoutNs = 1000000000ull;   // the grid barrier gives up after a second
-
-
 constexpr int kUnitBatch = 4;   // units of 32 FFN rows a block works on at a time (64 four-row items: two per warp)
 
 struct FusedShared {
@@ -55,13 +51,6 @@ struct FusedShared {
     float hbuf[kUnitBatch][32];   // the h values of the (expert, 32-row group) units this block is working on
     int bar_ok;                   // the grid barrier's outcome, for every thread of the block
 };
-
-// balanced contiguous split of n rows over nb blocks
-__device__ __forceinline__ void slice(int n, int nb, int b, int& r0, int& r1) {
-    const int base = n / nb, rem = n % nb;
-    r0 = b * base + min(b, rem);
-    r1 = r0 + base + (b < rem ? 1 : 0);
-}
 
 // q8_1 of 32 values (one per lane) straight into the shared structure-of-arrays form the dots read.
 __device__ __forceinline__ void q8_1_to_smem(float v, int4* q, float* d, int* isum, int blk, int lane) {
@@ -78,60 +67,9 @@ __device__ __forceinline__ void q8_1_to_smem(float v, int4* q, float* d, int* is
     }
 }
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-// block 0's wall-clock stamp of a phase boundary (a 64-bit ns count in two scratch words)
-__device__ __forceinline__ void stamp(unsigned* sync, int i) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile unsigned long long*) &sync[4 + 2 * i] = global_ns();
-}
-
-// All blocks of the (cooperative) grid meet here.  false in EVERY thread of the block when the wait ran out: thread 0
-// leaves the outcome in shared memory before the closing barrier.
-__device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned epoch, int* s_ok) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        __threadfence();
-        atomicAdd(&sync[0], 1u);
-        const unsigned target = (epoch + 1u) * gridDim.x;
-        const unsigned long long t0 = global_ns();
-        while ((int) (*(volatile unsigned*) &sync[0] - target) < 0) {
-            if (global_ns() - t0 > kBarrierTimeoutNs) { ok = 0; atomicExch(&sync[2], 1u); break; }
-            __nanosleep(20);
-        }
-        __threadfence();
-        *s_ok = ok;
-    }
-    __syncthreads();
-    return *s_ok != 0;
-}
-
 // RT: the router - 0 softmax, 1 sigmoid.  A template parameter, not a branch on A.router: with both routers compiled into
 // one kernel the softmax layer's routing phase ran 2 us longer (the 64-register cap of a 1024-thread block is shared by
 // everything the phase may call).
-// The token's routing by the block's first kRouteThreads threads, as a function of its own: run once a launch, it is
-// kept out of the kernel's register allocation and instruction scheduling (which proved sensitive to what phase 0 holds).
-template<int RT>
-__device__ __noinline__ void route_token(const float* logits, const float* bias, int n_expert, int k, float w_scale, int norm_w,
-                                         int tid, double* s_ex, RouterShared* route) {
-    using RS = NamedSync<1, kRouteThreads>;
-    const int per = (n_expert + kRouteThreads - 1) / kRouteThreads;
-    if constexpr (RT == 1) {
-        if (per <= 1) route_sigmoid<1, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 2) route_sigmoid<2, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 4) route_sigmoid<4, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-        else route_sigmoid<8, RS>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-    } else {
-        if (per <= 1) route_softmax<1, RS>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 2) route_softmax<2, RS>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 4) route_softmax<4, RS>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-        else route_softmax<8, RS>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-    }
-}
-
 // HV: the kernel may cut phase-1 units in halves (decided per launch on the device; the code for it is compiled in only
 // where a rank's units can be that few - in the one-GPU kernel it cost 1 us by its mere presence).
 template<int T, int TS, int RT, bool HV>
@@ -490,9 +428,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
 
 template<int T, int TS, int RT, bool HV>
 int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
-    // per instantiation: whether the programmatic-serialization attribute is in use (1), was refused by the driver (0) or has not
-    // been tried (-1)
-    static std::atomic<int> pdl{-1};
     static SmemLimit smem_limit;
     constexpr size_t kMost = 220 * 1024;
     const int nblk_x = A.n_embd / 32, nblk_h = (A.n_ff > A.n_ff_sh ? A.n_ff : A.n_ff_sh) / 32;
@@ -506,48 +441,40 @@ int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
     if (A.ar.nm >= 2 && grid > MAYA_PEER_AR_BLOCKS) return refuse(MAYA_ERR_LIMIT);
     FusedArgs args = A;
     void* params[] = {&args};
-    // Cooperative (the grid barrier needs every block resident) and, where the driver accepts the attribute,
-    // programmatically serialized after the launch in front of it: its set-up then overlaps that launch's tail.
-    if (pdl.load() != 0) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kFusedThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 2;
-        const cudaError_t e = cudaLaunchKernelExC(&cfg, (const void*) moe_layer_t1_kernel<T, TS, RT, HV>, params);
-        if (e == cudaSuccess) { pdl.store(1); return note_launch("moe_layer_t1"); }
-        // only "this attribute / combination is not supported" turns the attribute off; any other failure is the launch's
-        if (e != cudaErrorNotSupported && e != cudaErrorInvalidValue) return note_launch("moe_layer_t1");
-        cudaGetLastError();
-        pdl.store(0);
-    }
-    cudaLaunchCooperativeKernel((const void*) moe_layer_t1_kernel<T, TS, RT, HV>, dim3(grid), dim3(kFusedThreads), params, smem, s);
-    return note_launch("moe_layer_t1");
+    return launch_cooperative((const void*) moe_layer_t1_kernel<T, TS, RT, HV>, dim3(grid), dim3(kFusedThreads), params, smem, s, "moe_layer_t1");
+}
+
+// Units of one routed expert + the shared expert's: when even twice that many fit the grid, a rank with few local experts (or a
+// narrow width slice) may have fewer units than half the blocks.
+bool few_units(const FusedArgs& A) {
+    const int units_min = A.n_ff / 32 + (A.shared != nullptr ? (A.sh_hi - A.sh_lo) / 32 : 0);
+    return 2 * units_min <= sm_count();
+}
+
+// Layers of one core type on which the fused kernel is the faster one (us fused / token kernel, 148 SMs):
+bool fused_better(int type, const FusedArgs& A) {
+    const int units = A.k * A.n_ff / 32 + (A.shared != nullptr ? (A.sh_hi - A.sh_lo) / 32 : 0);
+    // so few units that it cuts every one in two for two blocks
+    if (A.router == 0 && 2 * units <= sm_count()) return true;
+    // 2-bit rows beside a shared expert's 8-bit ones: two of the token kernel's 16 warps wait for those where two of 32 do here
+    // (6144 x 2048: 63.2 / 64.4; without the shared expert 69.6 / 58.0, 3-bit rows with it 71.8 / 65.4)
+    if (type == MAYA_IQ2_S && A.shared != nullptr) return true;
+    // less than an item a warp: the token kernel's codebook is not worth filling (2048 x 512, top 8: IQ2_S 16.9 / 18.5, IQ3_S 18.5 / 18.5)
+    if ((type == MAYA_IQ2_S || type == MAYA_IQ3_S) && units < sm_count()) return true;
+    // short rows, where a stage's handling outweighs its dots (1120 x 2272 Q8_0 30.1 / 31.0, 1280 x 1280 IQ2_S 28.8 / 29.4, 1024 x 1280
+    // IQ3_S 26.7 / 27.1; 1024 x 2560 Q4_K 39.0 / 37.2)
+    return type != MAYA_Q4_K && A.n_embd <= 1280;
 }
 
 template<int T, int TS>
 int launch_fused(const FusedArgs& A, cudaStream_t s) {
     if (A.router == 1) return launch_fused_rt<T, TS, 1, false>(A, s);
-    // units of one routed expert + the shared expert's: when even twice that many fit the grid, a rank with few local
-    // experts (or a narrow width slice) may have fewer units than half the blocks
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    static thread_local int c_dev = -1, c_sms = 0;
-    if (c_dev != dev) { cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); c_dev = dev; c_sms = sms; }
-    const int units_min = A.n_ff / 32 + (A.shared != nullptr ? (A.sh_hi - A.sh_lo) / 32 : 0);
-    return 2 * units_min <= c_sms ? launch_fused_rt<T, TS, 0, true>(A, s) : launch_fused_rt<T, TS, 0, false>(A, s);
+    return few_units(A) ? launch_fused_rt<T, TS, 0, true>(A, s) : launch_fused_rt<T, TS, 0, false>(A, s);
 }
 
 }  // namespace
 
-// Whether the fused single-token kernel covers this layer (else the staged kernels run).
+// Whether the fused single-token kernel covers this layer (else the token kernel or the staged kernels run).
 bool fused_t1_supported(const maya_moe_layer& L) {
     if (L.gu_type != L.d_type || !type_is_core(L.gu_type)) return false;
     if (L.n_ff_sh > 0 && (L.sh_gu_type != MAYA_Q8_0 || L.sh_d_type != MAYA_Q8_0)) return false;
@@ -556,7 +483,7 @@ bool fused_t1_supported(const maya_moe_layer& L) {
 }
 
 int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_is_bf16, int* ids, float* weights,
-             float* out, float* h_scratch, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
+             float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
              const maya_hc_post_args* hc, cudaStream_t s) {
     FusedArgs A{};
     if (hc != nullptr) A.hc = *hc;
@@ -574,6 +501,14 @@ int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_
     A.sh_hi = sh ? (L.sh_hi > 0 ? L.sh_hi : L.n_ff_sh) : 0;
     A.limit = L.limit;
     A.ids = ids; A.weights = weights; A.out = out; A.h = h_scratch; A.sync = sync;
+    const bool here = fused_t1_supported(L);
+    // (a slice of the shared expert beside routed rows of two types, or of a type outside the core, stays refused)
+    const bool sliced = sh && (L.sh_lo != 0 || (L.sh_hi != 0 && L.sh_hi != L.n_ff_sh));
+    if (L.n_expert <= kRouteThreads * kRouterMaxPerThread && (here ? !fused_better(L.gu_type, A) : !sliced)) {
+        const int st = token_layer(L, A, unit_count, s);
+        if (st != kNotHere) return st;
+    }
+    if (!here) return kNotHere;
 #define FUSED_CASE(TT)                                                      \
     case TT: return sh ? launch_fused<TT, MAYA_Q8_0>(A, s) : launch_fused<TT, 0>(A, s);
     switch (L.gu_type) {

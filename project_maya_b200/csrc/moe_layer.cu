@@ -27,6 +27,7 @@ struct Scratch {
     uint8_t* sh_hq;              // [T][n_ff_sh/32] q8_1
     float* sh_out;               // [T][n_embd]
     float* h;                    // the fused single-token kernel's h: q8_1 image, shared-unit halves, counters
+    unsigned* unit_count;        // the token kernel's counters of units that two blocks share (zero before first use)
     unsigned* sync;              // [16]: the fused kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket; stamps (zero
                                  // before first use)
     size_t bytes;
@@ -46,6 +47,7 @@ Scratch carve(const maya_moe_layer& L, int T, uint8_t* base) {
         // per expert and 32-value group of h: the q8_1 image (40 bytes), the f32 halves two blocks leave when a unit is
         // shared between them (128 bytes) and that unit's arrival counter
         s.h = (float*) take((size_t) (MAYA_MAX_K + 1) * (ld / 32) * (40 + 128 + 4));
+        s.unit_count = (unsigned*) take((size_t) (MAYA_MAX_K + 1) * (ld / 32) * 4);
     }
     s.xq = take((size_t) T * (L.n_embd / 32) * kQ81Bytes);
     s.plan_ptr = (unsigned long long*) take((size_t) T * 8 * sizeof(unsigned long long));
@@ -266,8 +268,10 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
     cudaStream_t s = as_stream(stream);
     int* d_ids = ids ? ids : S.ids;
     float* d_w = weights ? weights : S.weights;
-    if (T == 1 && !L->staged && fused_t1_supported(*L))
-        return fused_t1(*L, logits, x, x_is_bf16, d_ids, d_w, out, S.h, S.sync, ar, mi, seq, hc, s);
+    if (T == 1 && !L->staged) {
+        st = fused_t1(*L, logits, x, x_is_bf16, d_ids, d_w, out, S.h, S.unit_count, S.sync, ar, mi, seq, hc, s);
+        if (st != kNotHere) return st;
+    }
     if (L->n_ff_sh > 0 && L->shared_here && (L->sh_lo != 0 || (L->sh_hi != 0 && L->sh_hi != L->n_ff_sh)))
         return refuse(MAYA_ERR_ARG);                 // only the fused kernel slices the shared expert
 

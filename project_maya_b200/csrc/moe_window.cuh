@@ -15,7 +15,7 @@
 //     so that its 40 MB hide behind an instruction-bound phase instead of taking two GEMV launches and a SwiGLU launch a token.
 //   * codebooks lie in several copies side by side in shared memory, lane l reading copy l % n.
 // Read in place by a grid of (rows, group) blocks (gate/up) and streamed 64 rows a stage (down), an 8-token Q4_K window took
-// 318 us, a 16-token IQ3_S one 570; now 224 and 368.  (32 warps of two rows, measured when this form took 263 and 433: 266 and
+// 318 us, a 16-token IQ3_S one 570; now 225 and 351.  (32 warps of two rows, measured when this form took 263 and 433: 266 and
 // 484, the activation reads then bind.)
 //
 // The arithmetic is rows_dot's (maya_dots.cuh), value for value - the same integers, the same lane order, the same sums - so

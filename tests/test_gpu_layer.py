@@ -253,6 +253,43 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
     assert H.rel_err(out.cpu().numpy()[0], want) <= TIGHT
 
 
+@pytest.mark.parametrize("gu,d,n_embd,n_ff,n_ff_sh,k,cut", [
+    (H.Q8_0, H.Q8_0, 1344, 288, 0, 8, None),             # an odd number of blocks a row; 9 calls of a down row
+    (H.Q8_0, H.Q8_0, 2080, 1056, 96, 6, None),           # three segments, the last of one block; two of a down row
+    (H.Q4_K, H.Q4_K, 512, 512, 0, 8, None),              # down rows of 8 calls, four side by side
+    (H.Q4_K, H.Q6_K, 2304, 1536, 4128, 8, None),         # down in segments of 840 bytes
+    (H.Q4_K, H.Q4_K, 2304, 1536, 4128, 6, 64),           # slices of the shared expert
+    (H.Q5_K, H.Q8_0, 1536, 2304, 352, 5, None), (H.Q6_K, H.Q5_K, 1280, 768, 0, 7, None), (H.IQ4_XS, H.IQ3_XXS, 2560, 256, 0, 8, None),
+    (H.IQ2_S, H.IQ3_S, 2304, 2304, 512, 3, None), (H.IQ2_S, H.IQ2_S, 2048, 1280, 0, 8, None), (H.IQ3_S, H.IQ3_S, 4352, 1024, 288, 6, None),
+    (H.IQ3_XXS, H.IQ4_XS, 4096, 1536, 0, 8, None), (H.IQ2_XXS, H.IQ3_XXS, 1792, 512, 64, 8, None), (H.IQ1_S, H.IQ2_XXS, 2304, 768, 0, 8, None),
+    (H.IQ3_S, H.IQ1_S, 2048, 2560, 1024, 8, None), (H.IQ1_S, H.IQ1_S, 1024, 512, 256, 1, None)])
+def test_token_kernel_equals_staged_kernels_bitwise(T, api, gu, d, n_embd, n_ff, n_ff_sh, k, cut):
+    """One token through the streamed single-token kernel and through the separate launches: the same bits, where segments,
+    stages, units shared by two blocks and short down rows end unevenly; twice, so that the counters are seen again."""
+    n_expert = 12
+    cfg = dict(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, k=k, gu_type=gu, d_type=d)
+    if n_ff_sh:
+        cfg.update(n_ff_sh=n_ff_sh, sh_gu_type=H.Q8_0, sh_d_type=H.Q8_0)
+    lc = layer_cfg(api, cfg)
+    lc.limit = 7.0
+    three = dev(T, np.stack([H.constructed_expert(gu, d, n_embd, n_ff, H.rng_for("tok", gu, d, e)) for e in range(3)]))
+    experts = three[T.arange(n_expert, device="cuda") % 3].contiguous()
+    sh = dev(T, H.constructed_expert(H.Q8_0, H.Q8_0, n_embd, n_ff_sh, H.rng_for("tok-shared", gu))) if n_ff_sh else None
+    token = api.MoeLayer(lc, experts, sh, expert_range=(1, n_expert))
+    staged = api.MoeLayer(lc, experts, sh, expert_range=(1, n_expert), staged=True)
+    logits = dev(T, H.router_logits("tok", 4, n_expert, 1.1))
+    x = dev(T, H.activations("tok", 4, n_embd, "f32"))
+    for i in (0, 1, 2, 3, 0):
+        got, want = token.forward(logits[i:i + 1], x[i:i + 1]), staged.forward(logits[i:i + 1], x[i:i + 1])
+        assert all(T.equal(a, b) for a, b in zip(got, want)), f"token {i}"
+        assert T.isfinite(want[2]).all() and want[2].abs().max() > 0
+    assert token.error() == 0
+    if cut:                                                              # two slices of the shared expert add up to it
+        out = [api.MoeLayer(lc, experts, sh, expert_range=(1, n_expert), **kw).forward(logits[:1], x[:1])[2].double()
+               for kw in ({}, dict(shared_here=False), dict(shared_range=(0, cut)), dict(shared_range=(cut, n_ff_sh)))]
+        assert ((out[2] + out[3] - out[1]) - out[0]).abs().max() <= 1e-5 * out[0].abs().max()
+
+
 @pytest.mark.parametrize("t,n_embd,n_ff,n_ff_sh,n_expert,n_tok,sigmoid", [
     (H.IQ2_S, 1024, 256, 512, 12, 2, False), (H.Q4_K, 1280, 768, 1312, 12, 9, False),      # the shared expert's jobs: one; three of 4, 4, 1
     (H.Q8_0, 1056, 288, 4128, 300, 7, True), (H.IQ3_S, 4352, 512, 256, 600, 16, False),    # rows beyond 4096 values; 2 and 4 experts a thread
