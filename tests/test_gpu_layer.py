@@ -254,7 +254,7 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
 
 
 @pytest.mark.parametrize("gu,d,n_embd,n_ff,n_ff_sh,k,cut", [
-    (H.Q8_0, H.Q8_0, 1344, 288, 0, 8, None),             # an odd number of blocks a row; 9 calls of a down row
+    (H.Q8_0, H.Q8_0, 1344, 352, 0, 8, None),             # an odd number of blocks a row; 11 calls of a down row
     (H.Q8_0, H.Q8_0, 2080, 1056, 96, 6, None),           # three segments, the last of one block; two of a down row
     (H.Q4_K, H.Q4_K, 512, 512, 0, 8, None),              # down rows of 8 calls, four side by side
     (H.Q4_K, H.Q6_K, 2304, 1536, 4128, 8, None),         # down in segments of 840 bytes
