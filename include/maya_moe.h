@@ -333,10 +333,11 @@ typedef struct maya_moe_layer {
                                     NULL: no host contribution.  With several ranks give it to one rank only. */
 } maya_moe_layer;
 /* Bytes of scratch maya_moe_layer_decode needs for n_tokens tokens.  The scratch must be 256-byte aligned and ZEROED
- * once before its first use (it holds the fused kernel's grid-barrier counter); one scratch serves one stream at a
- * time.  After a device-side wait that ran out (a block never arrived at the fused kernel's barrier, weight rows of a window
- * or a staged token never landed) the word returned by maya_moe_layer_error is non-zero and the outputs of that and later
- * calls on the scratch are undefined. */
+ * once before its first use (it holds the single-token kernels' grid-barrier counter and the token kernel's counters of units
+ * that blocks share); one scratch serves one stream at a time.  After a device-side wait that ran out (a block never arrived at a
+ * single-token kernel's barrier, weight rows of the token kernel, of a window or of a staged token never landed) the word returned by
+ * maya_moe_layer_error is non-zero and the outputs of that call are incomplete; the scratch has to be zeroed again before its next
+ * use. */
 MAYA_API size_t maya_moe_layer_scratch_bytes(const maya_moe_layer* L, int n_tokens);
 /* Reads the sticky error word of a layer scratch (synchronises the stream first). 0 = no error. */
 MAYA_API int maya_moe_layer_error(const maya_moe_layer* L, int n_tokens, const void* scratch, void* stream);
@@ -349,6 +350,20 @@ MAYA_API int maya_moe_layer_phase_ns(const maya_moe_layer* L, const void* scratc
 MAYA_API int maya_moe_layer_decode(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16,
                                    int n_tokens, int* ids, float* weights, float* out, void* scratch,
                                    size_t scratch_bytes, void* stream);
+
+/* No counterpart in the reference: one token with the caller's choice of kernel and bound on the waits for weight rows (`polls` looks at
+ * a copy before a warp gives up; maya_moe_layer_decode takes 2^22, some seconds).  MAYA_ERR_LIMIT: that kernel does not take the
+ * layer.  hc (optional) as in maya_moe_layer_decode_hc. */
+enum maya_layer_kernel {
+    MAYA_LAYER_CHOICE = 0,      /* maya_moe_layer_decode's */
+    MAYA_LAYER_FUSED = 1,       /* one launch, rows read in place: core types, and with a cross-rank sum the only one-launch form */
+    MAYA_LAYER_TOKEN = 2,       /* one launch, rows streamed through shared memory */
+    MAYA_LAYER_STAGED = 3       /* routing with q8_1, gate/up, down, combine as launches of their own */
+};
+struct maya_hc_post_args;
+MAYA_API int maya_moe_layer_decode_checked(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16, int* ids,
+                                           float* weights, float* out, void* scratch, size_t scratch_bytes, int kernel,
+                                           unsigned polls, const struct maya_hc_post_args* hc, void* stream);
 
 /* Cross-GPU sum of expert partials -------------------------------------------------------------- */
 #define MAYA_PEER_AR_MAX_RANKS 8

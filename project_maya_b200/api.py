@@ -24,6 +24,7 @@ TYPE_NAMES = {Q8_0: "Q8_0", Q4_K: "Q4_K", IQ3_S: "IQ3_S", IQ2_S: "IQ2_S", Q5_K: 
               IQ3_XXS: "IQ3_XXS", IQ4_XS: "IQ4_XS", IQ1_S: "IQ1_S"}
 STATUS = {0: "ok", -1: "bad argument", -2: "unsupported ggml type", -3: "CUDA launch failed", -4: "beyond a limit",
           -5: "no sm_100 device"}
+LAYER_CHOICE, LAYER_FUSED, LAYER_TOKEN, LAYER_STAGED = 0, 1, 2, 3        # maya_layer_kernel
 INF = float("inf")
 
 
@@ -444,8 +445,23 @@ class MoeLayer:
                                                  self.scratch.numel(), _stream(stream)))
         return ids, weights, out
 
+    def forward_checked(self, logits, x, kernel: int, polls: int = 1 << 22, out=None, hc=None, stream=None):
+        """forward of one token with the caller's choice of kernel (LAYER_CHOICE, LAYER_FUSED, LAYER_TOKEN, LAYER_STAGED; a kernel that
+        does not take the layer raises) and bound on its waits for weight rows."""
+        dev = logits.device
+        ids = torch.empty((1, self.cfg.k), dtype=torch.int32, device=dev)
+        weights = torch.empty((1, self.cfg.k), dtype=torch.float32, device=dev)
+        out = out if out is not None else torch.empty((1, self.cfg.n_embd), dtype=torch.float32, device=dev)
+        assert logits.shape[0] == 1 and x.dtype in (torch.float32, torch.bfloat16)
+        args = C.byref(HcPostArgs(*[_ptr(t) for t in hc])) if hc is not None else None
+        _check("moe_layer_decode_checked",
+               _lib.load().maya_moe_layer_decode_checked(C.byref(self.desc), _ptr(logits), _ptr(x), int(x.dtype == torch.bfloat16),
+                                                         _ptr(ids), _ptr(weights), _ptr(out), _ptr(self.scratch), self.scratch.numel(),
+                                                         kernel, polls, args, _stream(stream)))
+        return ids, weights, out
+
     def phase_ns(self, stream=None):
-        """Block 0's phase stamps of the last fused single-token launch, as offsets in ns from its start."""
+        """Block 0's phase stamps of the last single-token launch (fused or token kernel), as offsets in ns from its start."""
         buf = (C.c_ulonglong * 6)()
         _check("moe_layer_phase_ns", _lib.load().maya_moe_layer_phase_ns(C.byref(self.desc), _ptr(self.scratch), _stream(stream), buf))
         return [int(buf[i]) - int(buf[0]) for i in range(6)]

@@ -63,7 +63,7 @@ struct FusedArgs;
 bool fused_t1_supported(const maya_moe_layer& L);
 int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_is_bf16, int* ids, float* weights,
              float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
-             const maya_hc_post_args* hc, cudaStream_t s);
-int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_count, cudaStream_t s);
+             const maya_hc_post_args* hc, int kernel, unsigned polls, cudaStream_t s);
+int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_count, unsigned polls, cudaStream_t s);
 
 }  // namespace maya

@@ -484,7 +484,7 @@ bool fused_t1_supported(const maya_moe_layer& L) {
 
 int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_is_bf16, int* ids, float* weights,
              float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
-             const maya_hc_post_args* hc, cudaStream_t s) {
+             const maya_hc_post_args* hc, int kernel, unsigned polls, cudaStream_t s) {
     FusedArgs A{};
     if (hc != nullptr) A.hc = *hc;
     if (ar != nullptr) { A.ar = *ar; A.ar_rank = ar_rank; A.ar_seq = ar_seq; }
@@ -504,11 +504,12 @@ int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_
     const bool here = fused_t1_supported(L);
     // (a slice of the shared expert beside routed rows of two types, or of a type outside the core, stays refused)
     const bool sliced = sh && (L.sh_lo != 0 || (L.sh_hi != 0 && L.sh_hi != L.n_ff_sh));
-    if (L.n_expert <= kRouteThreads * kRouterMaxPerThread && (here ? !fused_better(L.gu_type, A) : !sliced)) {
-        const int st = token_layer(L, A, unit_count, s);
+    const bool rule = kernel == MAYA_LAYER_CHOICE;
+    if (kernel != MAYA_LAYER_FUSED && L.n_expert <= kRouteThreads * kRouterMaxPerThread && (here ? !rule || !fused_better(L.gu_type, A) : !sliced)) {
+        const int st = token_layer(L, A, unit_count, polls, s);
         if (st != kNotHere) return st;
     }
-    if (!here) return kNotHere;
+    if (!here || kernel == MAYA_LAYER_TOKEN) return kNotHere;
 #define FUSED_CASE(TT)                                                      \
     case TT: return sh ? launch_fused<TT, MAYA_Q8_0>(A, s) : launch_fused<TT, 0>(A, s);
     switch (L.gu_type) {

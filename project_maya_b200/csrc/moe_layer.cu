@@ -28,8 +28,8 @@ struct Scratch {
     float* sh_out;               // [T][n_embd]
     float* h;                    // the fused single-token kernel's h: q8_1 image, shared-unit halves, counters
     unsigned* unit_count;        // the token kernel's counters of units that two blocks share (zero before first use)
-    unsigned* sync;              // [16]: the fused kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket; stamps (zero
-                                 // before first use)
+    unsigned* sync;              // [17]: the fused and the token kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket;
+                                 // stamps; [16] the token kernel's mark of a launch that gave up (zero before first use)
     size_t bytes;
 };
 
@@ -41,7 +41,7 @@ Scratch carve(const maya_moe_layer& L, int T, uint8_t* base) {
     auto take = [&](size_t n) { uint8_t* p = base ? base + off : nullptr; off += align_up(n); return p; };
     // the fused kernel's words first: their place must not depend on T (a scratch sized for a window also serves
     // single tokens, and the barrier counter has to survive the calls in between)
-    s.sync = (unsigned*) take(16 * sizeof(unsigned));
+    s.sync = (unsigned*) take(17 * sizeof(unsigned));
     {
         const int ld = L.n_ff > L.n_ff_sh ? L.n_ff : L.n_ff_sh;
         // per expert and 32-value group of h: the q8_1 image (40 bytes), the f32 halves two blocks leave when a unit is
@@ -207,7 +207,8 @@ extern "C" int maya_moe_layer_phase_ns(const maya_moe_layer* L, const void* scra
 
 static int layer_decode(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16, int n_tokens, int* ids,
                         float* weights, float* out, void* scratch, size_t scratch_bytes, const maya_peer_ar* ar, int mi,
-                        unsigned seq, void* stream, const maya_hc_post_args* hc = nullptr);
+                        unsigned seq, void* stream, const maya_hc_post_args* hc = nullptr, int kernel = MAYA_LAYER_CHOICE,
+                        unsigned polls = kMbarPolls);
 static int ar_args_ok(const maya_moe_layer* L, int n_tokens, float* out, const maya_peer_ar* a, int mi, unsigned seq);
 
 extern "C" int maya_moe_layer_decode(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16,
@@ -244,6 +245,14 @@ extern "C" int maya_moe_layer_decode_hc(const maya_moe_layer* L, const float* lo
     return layer_decode(L, logits, x, x_is_bf16, n_tokens, ids, weights, out, scratch, scratch_bytes, a, mi, seq, stream, hc);
 }
 
+extern "C" int maya_moe_layer_decode_checked(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16, int* ids,
+                                             float* weights, float* out, void* scratch, size_t scratch_bytes, int kernel,
+                                             unsigned polls, const maya_hc_post_args* hc, void* stream) {
+    if (hc && (!hc->R_old || !hc->post || !hc->comb || !hc->R_new || hc->R_new == hc->R_old)) return refuse(MAYA_ERR_ARG);
+    if (kernel < MAYA_LAYER_CHOICE || kernel > MAYA_LAYER_STAGED) return refuse(MAYA_ERR_ARG);
+    return layer_decode(L, logits, x, x_is_bf16, 1, ids, weights, out, scratch, scratch_bytes, nullptr, 0, 0, stream, hc, kernel, polls);
+}
+
 // The staged paths' consumer: one hc_post launch per token, after `out` is complete.
 static int hc_post_tokens(const maya_hc_post_args* hc, const float* out, int T, int n_embd, void* stream) {
     if (hc == nullptr) return MAYA_OK;
@@ -257,7 +266,7 @@ static int hc_post_tokens(const maya_hc_post_args* hc, const float* out, int T, 
 
 static int layer_decode(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16, int n_tokens, int* ids,
                         float* weights, float* out, void* scratch, size_t scratch_bytes, const maya_peer_ar* ar, int mi,
-                        unsigned seq, void* stream, const maya_hc_post_args* hc) {
+                        unsigned seq, void* stream, const maya_hc_post_args* hc, int kernel, unsigned polls) {
     int st = check_layer(L);
     if (st != MAYA_OK) return refuse(st);
     if (n_tokens < 1 || n_tokens > MAYA_MAX_WIN_TOKENS) return refuse(MAYA_ERR_LIMIT);
@@ -268,9 +277,10 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
     cudaStream_t s = as_stream(stream);
     int* d_ids = ids ? ids : S.ids;
     float* d_w = weights ? weights : S.weights;
-    if (T == 1 && !L->staged) {
-        st = fused_t1(*L, logits, x, x_is_bf16, d_ids, d_w, out, S.h, S.unit_count, S.sync, ar, mi, seq, hc, s);
+    if (T == 1 && (kernel == MAYA_LAYER_CHOICE ? !L->staged : kernel != MAYA_LAYER_STAGED)) {
+        st = fused_t1(*L, logits, x, x_is_bf16, d_ids, d_w, out, S.h, S.unit_count, S.sync, ar, mi, seq, hc, kernel, polls, s);
         if (st != kNotHere) return st;
+        if (kernel != MAYA_LAYER_CHOICE) return refuse(MAYA_ERR_LIMIT);
     }
     if (L->n_ff_sh > 0 && L->shared_here && (L->sh_lo != 0 || (L->sh_hi != 0 && L->sh_hi != L->n_ff_sh)))
         return refuse(MAYA_ERR_ARG);                 // only the fused kernel slices the shared expert
@@ -337,7 +347,7 @@ static int layer_decode(const maya_moe_layer* L, const float* logits, const void
     W.limit = L->limit;
     W.down_off = down_off;
     // one token: a window of one, its cross-rank sum a launch of its own; more: with `ar` the sum runs in the combine launch
-    st = win_experts(L->gu_type, L->d_type, &W, true, ride ? &sh : nullptr, kMbarPolls, S.sync + 2, T > 1 ? ar : nullptr, mi, seq, s);
+    st = win_experts(L->gu_type, L->d_type, &W, true, ride ? &sh : nullptr, polls, S.sync + 2, T > 1 ? ar : nullptr, mi, seq, s);
     if (st == MAYA_OK && T == 1 && ar != nullptr) st = maya_allreduce_peer(out, L->n_embd, ar, mi, seq, stream);
     return st == MAYA_OK ? hc_post_tokens(hc, out, T, L->n_embd, stream) : st;
 }

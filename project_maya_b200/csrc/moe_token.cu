@@ -7,7 +7,7 @@ namespace maya {
 template<int T> int token_by_type(const TokArgs& A, cudaStream_t s);
 
 // kNotHere: not this kernel's, nothing launched.
-int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_count, cudaStream_t s) {
+int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_count, unsigned polls, cudaStream_t s) {
     if (F.ar.nm >= 2) return kNotHere;                 // the cross-rank sum is moe_fused.cu's
     // bulk copies take aligned 16-byte windows around the rows: blobs have to start and end on 16-byte boundaries
     if ((((uintptr_t) F.experts) | F.expert_stride | (uintptr_t) F.shared) & 15u) return kNotHere;
@@ -18,7 +18,7 @@ int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_coun
     A.up_off = row_bytes(L.gu_type, L.n_embd) * (size_t) L.n_ff;
     A.down_off = 2 * A.up_off;
     A.unit_count = unit_count;
-    A.polls = kMbarPolls;
+    A.polls = polls;
     switch (L.gu_type) {
         case MAYA_Q8_0: return token_by_type<MAYA_Q8_0>(A, s);
         case MAYA_Q4_K: return token_by_type<MAYA_Q4_K>(A, s);

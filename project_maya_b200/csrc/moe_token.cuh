@@ -23,8 +23,10 @@
 // The (row, expert) dots, q8_1 of h and the combine chain are rows_dot1's and the staged kernels', value for value: results are
 // bit-identical to every other path's.
 //
-// Every wait is bounded.  A warp whose copies never land asks for nothing more; its block says so in the error word, still
-// meets the others at the grid barrier, and leaves after the copies in flight have had the same bounded time.
+// Every wait is bounded.  A warp whose copies never land asks for nothing more; its block says so in the error word and, with the
+// launch's mark, in sync[16], still meets the others at the grid barrier, and leaves after the copies in flight have had a bounded
+// time.  The other blocks find the mark behind the barrier, where the h that they read is incomplete: none writes `out` or the
+// residual stack, and the counters of split units, some of which stay short of a launch's 16, are set to zero for the next launch.
 #pragma once
 
 #include "maya_fused_args.cuh"
@@ -200,6 +202,20 @@ struct Spread {
     __device__ __forceinline__ int before(int p) const { return (int) (((uint32_t) p * q) >> 16); }
     __device__ __forceinline__ bool at(int p) const { return before(p + 1) > before(p); }
 };
+
+// What only a launch in which a wait ran out comes to: as functions of their own, out of the kernel's register allocation.
+__device__ __noinline__ void tok_gave_up(unsigned* sync, unsigned mark) {
+    atomicExch(&sync[2], 1u);
+    atomicExch(&sync[16], mark);
+}
+// (every block of the launch is past its counters)
+__device__ __noinline__ void tok_reset(unsigned* count, int n) {
+    for (int i = threadIdx.x; i < n; i += kTokThreads) count[i] = 0u;
+}
+// what a warp has in flight lands before the block's shared memory goes away
+__device__ __noinline__ void tok_drain(uint64_t* full, int got, int asked) {
+    for (; got < asked; ++got) mbar_wait(&full[got & 1], (got >> 1) & 1);
+}
 
 // T: gate/up type; SH: with a Q8_0 shared expert.
 template<int T, bool SH>
@@ -503,7 +519,8 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
         if (ok) { open2(); ask2(); ask2(); }             // the first down rows, under the barrier
     }
     ok = __syncthreads_or(ok ? 0 : 1) == 0;              // the block agrees
-    if (!ok && tid == 0) atomicExch(&A.sync[2], 1u);
+    const unsigned mark = (sh.epoch + 1u) | 0x80000000u;             // this launch's, never zero
+    if (!ok && tid == 0) tok_gave_up(A.sync, mark);
     if (A.d_type != T) tok_fill(A.d_type, s_tab, tid);
     stamp(A.sync, 2);
     const bool met = grid_barrier(A.sync, sh.epoch, &sh.bar_ok);
@@ -512,6 +529,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
 
     // ---------------------------------------------------------------- phase 2: q8_1(h), down, combine
     if (done) {
+        const unsigned lost = tid == 0 ? __ldcg(A.sync + 16) : 0u;   // (asked for ahead of h: both arrive together)
         const int nb_r = n_ff / 32, total_r = nv * nb_r, b_s = has_sh ? A.sh_lo / 32 : 0, nb_s = has_sh ? (A.sh_hi - A.sh_lo) / 32 : 0;
         const int xb2 = A.d_type == MAYA_Q4_K || A.d_type == MAYA_Q5_K ? 2 : 1;
         for (int i = tid; i < 2 * (total_r + nb_s); i += kTokThreads) {          // half a block each, its scale or its sum
@@ -527,7 +545,10 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             *(uint4*) (col + (two ? tok_piece<2>(n, blk, hf) : tok_piece<1>(n, blk, hf))) = v;
             *(uint32_t*) (col + (two ? tok_scale<2>(n, blk) : tok_scale<1>(n, blk)) + hf * n * 4) = ds;
         }
-        __syncthreads();
+        done = __syncthreads_or(lost == mark ? 1 : 0) == 0;         // no block gave up
+    }
+    if (done) {
+        const int nb_r = n_ff / 32, nb_s = has_sh ? (A.sh_hi - A.sh_lo) / 32 : 0;
         if (SH) {                                        // the shared expert's rows, by the warps that have an item less (in the loop
                                                          // below, spread among the others, this phase took 21.1 us instead of 18.6)
             const TokCol H{cols + nv * tok_col_bytes(nb_r), nb_s};
@@ -588,8 +609,9 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             A.out[o0 + tid] = __fadd_rn(m, has_sh ? sh.part[tid][k] : 0.0f);
         }
     }
-    // what a warp has in flight lands before the block's shared memory goes away (nothing, unless a wait ran out)
-    for (; got < asked; ++got) mbar_wait(&sh.full[warp][got & 1], (got >> 1) & 1, A.polls);
+    if (met && !done)                                    // every block is past its counters: whole again for the next launch
+        tok_reset(A.unit_count, (MAYA_MAX_K + 1) * nblk_h);
+    if (got < asked) tok_drain(sh.full[warp], got, asked);       // (nothing in flight, unless a wait ran out)
     stamp(A.sync, 4);
     __syncthreads();
     if (A.hc.R_new != nullptr && done) hc_post_rows(A.out, A.hc, n_embd, o0, o1, tid, kTokThreads);

@@ -290,6 +290,59 @@ def test_token_kernel_equals_staged_kernels_bitwise(T, api, gu, d, n_embd, n_ff,
         assert ((out[2] + out[3] - out[1]) - out[0]).abs().max() <= 1e-5 * out[0].abs().max()
 
 
+@pytest.mark.parametrize("gu,d,n_embd,n_ff,n_ff_sh,k", [
+    (H.Q4_K, H.Q4_K, 2304, 1536, 0, 8), (H.IQ3_S, H.IQ1_S, 2048, 1280, 1024, 6), (H.Q8_0, H.Q8_0, 1344, 352, 2080, 1)])
+def test_token_kernel_reports_a_wait_that_ran_out(T, api, gu, d, n_embd, n_ff, n_ff_sh, k):
+    """The token kernel's waits for weight rows given no or one look: where one runs out the error word says so, no block writes an
+    output or a residual row made of another block's missing h, and - with the word cleared - the next call is whole again: the
+    counters of split units did not keep what the lost call left."""
+    n_expert = 8
+    cfg = dict(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, k=k, gu_type=gu, d_type=d)
+    if n_ff_sh:
+        cfg.update(n_ff_sh=n_ff_sh, sh_gu_type=H.Q8_0, sh_d_type=H.Q8_0)
+    three = dev(T, np.stack([H.constructed_expert(gu, d, n_embd, n_ff, H.rng_for("lost", gu, d, e)) for e in range(3)]))
+    experts = three[T.arange(n_expert, device="cuda") % 3].contiguous()
+    sh = dev(T, H.constructed_expert(H.Q8_0, H.Q8_0, n_embd, n_ff_sh, H.rng_for("lost-shared", gu))) if n_ff_sh else None
+    layer = api.MoeLayer(layer_cfg(api, cfg), experts, sh, max_tokens=1)
+    rng = H.rng_for("lost", n_embd)
+    logits, x = dev(T, H.router_logits("lost", 2, n_expert, None)), dev(T, H.activations("lost", 2, n_embd, "f32"))
+    R_old, post, comb = (dev(T, rng.standard_normal(s).astype(np.float32)) for s in ((4, n_embd), 4, (4, 4)))
+    lost = 0
+
+    def call(i, kernel, polls=1 << 22):
+        out, R_new = T.full((1, n_embd), -7.5, device="cuda"), T.full((4, n_embd), -7.5, device="cuda")
+        layer.forward_checked(logits[i:i + 1], x[i:i + 1], kernel, polls, out=out, hc=(R_old, post, comb, R_new))
+        return out, R_new
+
+    want = [call(i, api.LAYER_STAGED) for i in range(2)]
+    for polls in (0, 1, 0, 1, 1 << 22):
+        out, R_new = call(1, api.LAYER_TOKEN, polls)
+        err = layer.error()
+        lost += err
+        assert err == (1 if polls == 0 else 0 if polls > 1 else err)
+        for got, full in ((out, want[1][0]), (R_new, want[1][1])):
+            assert bool((got == -7.5).all()) if polls == 0 else bool(((got == full) | (got == -7.5)).all()) if err else T.equal(got, full)
+        layer.scratch[8:12].zero_()                                      # the sticky word alone
+        for i in (0, 1):
+            out, R_new = call(i, api.LAYER_TOKEN)
+            assert layer.error() == 0 and T.equal(out, want[i][0]) and T.equal(R_new, want[i][1])
+    assert lost >= 2
+
+
+def test_token_kernel_barrier_times_out_and_reports(T, api):
+    """The token kernel's grid barrier, as the fused kernel's below: the call returns, the sticky word says so, nothing is written."""
+    cfg = dict(n_embd=2304, n_ff=768, n_expert=8, k=4, gu_type=H.Q4_K, d_type=H.Q4_K)
+    lc, experts, _ = synth_layer(T, api, cfg, 8, seed=3)
+    layer = api.MoeLayer(lc, experts)
+    logits, x = dev(T, H.router_logits("timeout", 1, 8, None)), dev(T, H.activations("timeout", 1, 2304, "f32"))
+    layer.forward_checked(logits, x, api.LAYER_TOKEN)
+    assert layer.error() == 0
+    layer.scratch[:16].view(T.int32)[1] += 7
+    out = T.full((1, 2304), -7.5, device="cuda")
+    layer.forward_checked(logits, x, api.LAYER_TOKEN, out=out)
+    assert layer.error() != 0 and bool((out == -7.5).all())
+
+
 @pytest.mark.parametrize("t,n_embd,n_ff,n_ff_sh,n_expert,n_tok,sigmoid", [
     (H.IQ2_S, 1024, 256, 512, 12, 2, False), (H.Q4_K, 1280, 768, 1312, 12, 9, False),      # the shared expert's jobs: one; three of 4, 4, 1
     (H.Q8_0, 1056, 288, 4128, 300, 7, True), (H.IQ3_S, 4352, 512, 256, 600, 16, False),    # rows beyond 4096 values; 2 and 4 experts a thread
