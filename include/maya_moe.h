@@ -360,6 +360,9 @@ enum maya_layer_kernel {
     MAYA_LAYER_TOKEN = 2,       /* one launch, rows streamed through shared memory */
     MAYA_LAYER_STAGED = 3       /* routing with q8_1, gate/up, down, combine as launches of their own */
 };
+/* Which of them maya_moe_layer_decode[_ar, _hc] takes for one token of L on a GPU of n_sms SMs, with a sum over n_ranks ranks where that is
+ * 2 or more; a negative maya_status for a layer that is refused.  Needs no GPU. */
+MAYA_API int maya_moe_layer_kernel(const maya_moe_layer* L, int n_ranks, int n_sms);
 struct maya_hc_post_args;
 MAYA_API int maya_moe_layer_decode_checked(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16, int* ids,
                                            float* weights, float* out, void* scratch, size_t scratch_bytes, int kernel,

@@ -124,6 +124,7 @@ _SIGNATURES = {
     "maya_moe_layer_phase_ns": (c_int, [C.POINTER(MoeLayerDesc), c_void_p, c_void_p, C.POINTER(C.c_ulonglong)]),
     "maya_moe_layer_decode": (c_int, [C.POINTER(MoeLayerDesc), c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_size_t, c_void_p]),
+    "maya_moe_layer_kernel": (c_int, [C.POINTER(MoeLayerDesc), c_int, c_int]),
     "maya_moe_layer_decode_checked": (c_int, [C.POINTER(MoeLayerDesc), c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                               c_size_t, c_int, C.c_uint, C.POINTER(HcPostArgs), c_void_p]),
     "maya_peer_ar_recv_bytes": (c_size_t, [c_int, c_size_t]),

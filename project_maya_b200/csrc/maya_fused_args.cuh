@@ -45,5 +45,11 @@ struct TokArgs : FusedArgs {
     int stage, tab, cols;      // bytes of a ring stage, of the codebook, of the activation columns
     int units;                 // units of h a block may work on
 };
+constexpr int kTokWarps = 16;
+constexpr size_t kTokMostSmem = 232448 - 8192;                  // dynamic shared memory, beside the static part
+#define MAYA_TOK_TYPES(X) X(MAYA_IQ2_S) X(MAYA_IQ3_S) X(MAYA_IQ3_XXS) X(MAYA_IQ2_XXS) X(MAYA_IQ1_S)      // types with a codebook
+__host__ __device__ inline int tok_col_bytes(int nblk) { return (nblk * 40 + 15) & ~15; }       // of an activation column
+// The launch's carve-up, into A; what it takes of shared memory beside the static part, 0: more than there is.
+size_t token_smem(int gu_type, TokArgs& A, int grid);
 
 }  // namespace maya

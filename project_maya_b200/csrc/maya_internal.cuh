@@ -65,5 +65,9 @@ int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_
              float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
              const maya_hc_post_args* hc, int kernel, unsigned polls, cudaStream_t s);
 int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_count, unsigned polls, cudaStream_t s);
+bool token_takes(const maya_moe_layer& L, const FusedArgs& F, int sms);           // the token kernel's limits
+bool token_better(int type, const FusedArgs& A, int sms);
+// The kernel maya_moe_layer_decode runs one token with (enum maya_layer_kernel), with a sum over n_ranks ranks where that is 2 or more.
+int layer_kernel(const maya_moe_layer& L, int n_ranks, int sms);
 
 }  // namespace maya

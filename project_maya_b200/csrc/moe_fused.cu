@@ -451,21 +451,6 @@ bool few_units(const FusedArgs& A) {
     return 2 * units_min <= sm_count();
 }
 
-// Layers of one core type on which the fused kernel is the faster one (us fused / token kernel, 148 SMs):
-bool fused_better(int type, const FusedArgs& A) {
-    const int units = A.k * A.n_ff / 32 + (A.shared != nullptr ? (A.sh_hi - A.sh_lo) / 32 : 0);
-    // so few units that it cuts every one in two for two blocks
-    if (A.router == 0 && 2 * units <= sm_count()) return true;
-    // 2-bit rows beside a shared expert's 8-bit ones: two of the token kernel's 16 warps wait for those where two of 32 do here
-    // (6144 x 2048: 63.2 / 64.4; without the shared expert 69.6 / 58.0, 3-bit rows with it 71.8 / 65.4)
-    if (type == MAYA_IQ2_S && A.shared != nullptr) return true;
-    // less than an item a warp: the token kernel's codebook is not worth filling (2048 x 512, top 8: IQ2_S 16.9 / 18.5, IQ3_S 18.5 / 18.5)
-    if ((type == MAYA_IQ2_S || type == MAYA_IQ3_S) && units < sm_count()) return true;
-    // short rows, where a stage's handling outweighs its dots (1120 x 2272 Q8_0 30.1 / 31.0, 1280 x 1280 IQ2_S 28.8 / 29.4, 1024 x 1280
-    // IQ3_S 26.7 / 27.1; 1024 x 2560 Q4_K 39.0 / 37.2)
-    return type != MAYA_Q4_K && A.n_embd <= 1280;
-}
-
 template<int T, int TS>
 int launch_fused(const FusedArgs& A, cudaStream_t s) {
     if (A.router == 1) return launch_fused_rt<T, TS, 1, false>(A, s);
@@ -482,13 +467,9 @@ bool fused_t1_supported(const maya_moe_layer& L) {
     return true;
 }
 
-int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_is_bf16, int* ids, float* weights,
-             float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
-             const maya_hc_post_args* hc, int kernel, unsigned polls, cudaStream_t s) {
+// What a launch takes from the layer alone.
+static FusedArgs fused_args(const maya_moe_layer& L) {
     FusedArgs A{};
-    if (hc != nullptr) A.hc = *hc;
-    if (ar != nullptr) { A.ar = *ar; A.ar_rank = ar_rank; A.ar_seq = ar_seq; }
-    A.logits = logits; A.x = x; A.x_is_bf16 = x_is_bf16;
     A.router = L.router; A.router_bias = L.router_bias; A.router_w_scale = L.router_w_scale; A.router_norm_w = L.router_norm_w;
     A.cpu_part = L.cpu_flag != nullptr ? L.cpu_part : nullptr; A.cpu_flag = L.cpu_flag;
     A.n_embd = L.n_embd; A.n_ff = L.n_ff; A.n_expert = L.n_expert; A.k = L.k;
@@ -500,16 +481,37 @@ int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_
     A.sh_lo = sh ? L.sh_lo : 0;
     A.sh_hi = sh ? (L.sh_hi > 0 ? L.sh_hi : L.n_ff_sh) : 0;
     A.limit = L.limit;
-    A.ids = ids; A.weights = weights; A.out = out; A.h = h_scratch; A.sync = sync;
-    const bool here = fused_t1_supported(L);
+    return A;
+}
+
+// The kernel for one token (see maya_internal.cuh).
+static int choose(const maya_moe_layer& L, const FusedArgs& A, int sms) {
+    const bool takes = token_takes(L, A, sms);
+    if (fused_t1_supported(L)) return takes && token_better(L.gu_type, A, sms) ? MAYA_LAYER_TOKEN : MAYA_LAYER_FUSED;
     // (a slice of the shared expert beside routed rows of two types, or of a type outside the core, stays refused)
-    const bool sliced = sh && (L.sh_lo != 0 || (L.sh_hi != 0 && L.sh_hi != L.n_ff_sh));
-    const bool rule = kernel == MAYA_LAYER_CHOICE;
-    if (kernel != MAYA_LAYER_FUSED && L.n_expert <= kRouteThreads * kRouterMaxPerThread && (here ? !rule || !fused_better(L.gu_type, A) : !sliced)) {
-        const int st = token_layer(L, A, unit_count, polls, s);
-        if (st != kNotHere) return st;
-    }
-    if (!here || kernel == MAYA_LAYER_TOKEN) return kNotHere;
+    const bool sliced = A.shared != nullptr && (L.sh_lo != 0 || (L.sh_hi != 0 && L.sh_hi != L.n_ff_sh));
+    return takes && !sliced ? MAYA_LAYER_TOKEN : MAYA_LAYER_STAGED;
+}
+int layer_kernel(const maya_moe_layer& L, int n_ranks, int sms) {
+    FusedArgs A = fused_args(L);
+    A.ar.nm = n_ranks;
+    return L.staged ? MAYA_LAYER_STAGED : choose(L, A, sms);
+}
+
+int fused_t1(const maya_moe_layer& L, const float* logits, const void* x, int x_is_bf16, int* ids, float* weights,
+             float* out, float* h_scratch, unsigned* unit_count, unsigned* sync, const maya_peer_ar* ar, int ar_rank, unsigned ar_seq,
+             const maya_hc_post_args* hc, int kernel, unsigned polls, cudaStream_t s) {
+    FusedArgs A = fused_args(L);
+    if (hc != nullptr) A.hc = *hc;
+    if (ar != nullptr) { A.ar = *ar; A.ar_rank = ar_rank; A.ar_seq = ar_seq; }
+    A.logits = logits; A.x = x; A.x_is_bf16 = x_is_bf16;
+    A.ids = ids; A.weights = weights; A.out = out; A.h = h_scratch; A.sync = sync;
+    const int sms = sm_count();
+    if (kernel == MAYA_LAYER_CHOICE) kernel = choose(L, A, sms);
+    else if (kernel == MAYA_LAYER_TOKEN && !token_takes(L, A, sms)) return kNotHere;
+    if (kernel == MAYA_LAYER_TOKEN) return token_layer(L, A, unit_count, polls, s);
+    if (kernel != MAYA_LAYER_FUSED || !fused_t1_supported(L)) return kNotHere;
+    const bool sh = A.shared != nullptr;
 #define FUSED_CASE(TT)                                                      \
     case TT: return sh ? launch_fused<TT, MAYA_Q8_0>(A, s) : launch_fused<TT, 0>(A, s);
     switch (L.gu_type) {

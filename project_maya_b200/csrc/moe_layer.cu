@@ -245,6 +245,11 @@ extern "C" int maya_moe_layer_decode_hc(const maya_moe_layer* L, const float* lo
     return layer_decode(L, logits, x, x_is_bf16, n_tokens, ids, weights, out, scratch, scratch_bytes, a, mi, seq, stream, hc);
 }
 
+extern "C" int maya_moe_layer_kernel(const maya_moe_layer* L, int n_ranks, int n_sms) {
+    const int st = check_layer(L);
+    return st != MAYA_OK ? st : layer_kernel(*L, n_ranks, n_sms);
+}
+
 extern "C" int maya_moe_layer_decode_checked(const maya_moe_layer* L, const float* logits, const void* x, int x_is_bf16, int* ids,
                                              float* weights, float* out, void* scratch, size_t scratch_bytes, int kernel,
                                              unsigned polls, const maya_hc_post_args* hc, void* stream) {

@@ -41,8 +41,7 @@
 namespace maya {
 namespace {
 
-constexpr int kTokWarps = 16, kTokThreads = kTokWarps * 32;
-constexpr size_t kTokMostSmem = 232448 - 8192;                  // dynamic shared memory, beside the static part
+constexpr int kTokThreads = kTokWarps * 32;
 
 // the streamed rows: gate/up [0] and down [1] of the routed experts
 struct TokKind {
@@ -66,7 +65,7 @@ struct TokShared {
     int bar_ok;
 };
 
-static_assert(sizeof(TokShared) <= 8192 - 1024, "with the driver's 1 KB");
+static_assert(sizeof(TokShared) <= 232448 - kTokMostSmem - 1024, "with the driver's 1 KB");
 
 // One q8_1 block of 32 values, one a lane: its lane's quant, the scale as the f16 field holds it, and the sum a dot takes - of the
 // quants, or for IQ1_S the stored f16 sum of the values (float bits).
@@ -113,22 +112,13 @@ template<bool SUM_F16> __device__ __forceinline__ TokBlock4 tok_round4(const flo
     return t;
 }
 // The codebook of a type only known at run time.
-#define MAYA_TOK_TYPES(X) X(MAYA_IQ2_S) X(MAYA_IQ3_S) X(MAYA_IQ3_XXS) X(MAYA_IQ2_XXS) X(MAYA_IQ1_S)
 __device__ __noinline__ void tok_fill(int type, uint32_t* tab, int tid) {
 #define MAYA_TOK_FILL(TT) case TT: RowTab<TT, true>::fill(tab, tid, kTokThreads); break;
     switch (type) { MAYA_TOK_TYPES(MAYA_TOK_FILL) }
 #undef MAYA_TOK_FILL
 }
-inline int tok_tab_bytes(int type) {
-#define MAYA_TOK_BYTES(TT) case TT: return RowTab<TT, true>::bytes;
-    switch (type) { MAYA_TOK_TYPES(MAYA_TOK_BYTES) }
-#undef MAYA_TOK_BYTES
-    return 0;
-}
-
 // One activation column in shared memory, planar (maya_dots.cuh): nblk q8_1 blocks, calls of XB blocks.
 struct TokCol { const uint8_t* p; int nblk; };
-__host__ __device__ inline int tok_col_bytes(int nblk) { return (nblk * 40 + 15) & ~15; }
 template<int XB> __device__ __forceinline__ XQ tok_col(const TokCol& c, int j, int n) {
     const int P = c.nblk / XB;
     const int4 a = *(const int4*) (c.p + (2 * j * P + n) * 16), b = *(const int4*) (c.p + ((2 * j + 1) * P + n) * 16);
@@ -619,27 +609,11 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     if (blockIdx.x == 0 && tid == 0) *(volatile unsigned*) &A.sync[1] = sh.epoch + 1u;       // the next launch's epoch
 }
 
-// What the kernel takes of shared memory beside its static part; 0: more than there is.
-template<int T, bool SH> size_t token_smem(TokArgs& A, int grid) {
-    const RowGeoRt gd = row_geo(A.d_type);
-    int stage = 4 * RowGeo<T>::pitch;
-    if (4 * gd.pitch > stage) stage = 4 * gd.pitch;
-    A.stage = (stage + 15) & ~15;
-    const int td = tok_tab_bytes(A.d_type);
-    A.tab = RowTab<T, true>::bytes > td ? RowTab<T, true>::bytes : td;
-    const int x = tok_col_bytes(A.n_embd / 32) * (SH && Dec<T>::xblk == 2 ? 2 : 1), h = A.k * tok_col_bytes(A.n_ff / 32) + tok_col_bytes(A.n_ff_sh / 32);
-    A.cols = ((x > h ? x : h) + 15) & ~15;
-    A.units = A.k * A.n_ff / 32 / grid + A.n_ff_sh / 32 / grid + 4;          // of a block, parts at both ends of both classes
-    const size_t smem = (size_t) kTokWarps * 2 * A.stage + A.tab + A.cols + ((A.units * 132 + 15) & ~15) + (size_t) A.n_expert * sizeof(double);
-    return smem <= kTokMostSmem ? smem : 0;
-}
-
 template<int T, bool SH> int launch_token(TokArgs A, cudaStream_t s) {
     static SmemLimit smem_limit;
     const int grid = sm_count();
-    if (grid <= 0) return refuse(MAYA_ERR_DEVICE);
-    const size_t smem = token_smem<T, SH>(A, grid);
-    if (smem == 0 || 4 * ((A.n_embd / 4 + grid - 1) / grid) > kMaxSliceRows) return kNotHere;
+    const size_t smem = token_smem(T, A, grid);
+    if (smem == 0) return kNotHere;
     if (!smem_limit.raise((const void*) token_kernel<T, SH>, kTokMostSmem)) return note_launch("token smem attribute");
     void* params[] = {&A};
     return launch_cooperative((const void*) token_kernel<T, SH>, dim3(grid), dim3(kTokThreads), params, smem, s, "moe_token");

@@ -231,7 +231,7 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
     ids_o, w_o = oracle.router_top10(logits, k)
     for i in range(6):
         ld, xd = dev(T, logits[i:i + 1]), dev(T, x[i:i + 1], T.bfloat16)
-        ids_f, w_f, out_f = fused.forward(ld, xd)
+        ids_f, w_f, out_f = fused.forward_checked(ld, xd, api.LAYER_FUSED)
         ids_s, w_s, out_s = staged.forward(ld, xd)
         assert T.equal(ids_f, ids_s) and T.equal(w_f, w_s)
         assert np.array_equal(ids_f.cpu().numpy()[0], ids_o[i])
@@ -239,7 +239,7 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
     assert fused.error() == 0
     # f32 activations and the oracle, experts 17..19 left to "another rank"
     xf = H.activations("fused32", 1, n_embd, "f32")
-    _, _, out = fused.forward(dev(T, logits[:1]), dev(T, xf))
+    _, _, out = fused.forward_checked(dev(T, logits[:1]), dev(T, xf), api.LAYER_FUSED)
     xq = oracle.quantize_q8_1(xf[0])
     parts = np.zeros((k, n_embd), np.float32)
     skip = np.zeros(k, np.uint8)
@@ -280,12 +280,12 @@ def test_token_kernel_equals_staged_kernels_bitwise(T, api, gu, d, n_embd, n_ff,
     logits = dev(T, H.router_logits("tok", 4, n_expert, 1.1))
     x = dev(T, H.activations("tok", 4, n_embd, "f32"))
     for i in (0, 1, 2, 3, 0):
-        got, want = token.forward(logits[i:i + 1], x[i:i + 1]), staged.forward(logits[i:i + 1], x[i:i + 1])
+        got, want = token.forward_checked(logits[i:i + 1], x[i:i + 1], api.LAYER_TOKEN), staged.forward(logits[i:i + 1], x[i:i + 1])
         assert all(T.equal(a, b) for a, b in zip(got, want)), f"token {i}"
         assert T.isfinite(want[2]).all() and want[2].abs().max() > 0
     assert token.error() == 0
     if cut:                                                              # two slices of the shared expert add up to it
-        out = [api.MoeLayer(lc, experts, sh, expert_range=(1, n_expert), **kw).forward(logits[:1], x[:1])[2].double()
+        out = [api.MoeLayer(lc, experts, sh, expert_range=(1, n_expert), **kw).forward_checked(logits[:1], x[:1], api.LAYER_TOKEN)[2].double()
                for kw in ({}, dict(shared_here=False), dict(shared_range=(0, cut)), dict(shared_range=(cut, n_ff_sh)))]
         assert ((out[2] + out[3] - out[1]) - out[0]).abs().max() <= 1e-5 * out[0].abs().max()
 
