@@ -426,15 +426,22 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     }
 }
 
+// What the kernel takes of dynamic shared memory; 0: more than there is.
+constexpr size_t kMostSmem = 220 * 1024;
+size_t fused_smem(int type, const FusedArgs& A) {
+    const size_t tab = type == MAYA_IQ2_S ? kRepTabBytes<MAYA_IQ2_S> : type == MAYA_IQ3_S ? kRepTabBytes<MAYA_IQ3_S> : 0;
+    const int nblk_x = A.n_embd / 32, nblk_h = (A.n_ff > A.n_ff_sh ? A.n_ff : A.n_ff_sh) / 32;
+    const int cols_blocks = ((nblk_x > (MAYA_MAX_K + 1) * nblk_h ? nblk_x : (MAYA_MAX_K + 1) * nblk_h) + 1) & ~1;
+    const size_t smem = tab + (size_t) cols_blocks * 40 + (size_t) A.n_expert * sizeof(double);
+    return smem <= kMostSmem ? smem : 0;
+}
+
 template<int T, int TS, int RT, bool HV>
 int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
     static SmemLimit smem_limit;
-    constexpr size_t kMost = 220 * 1024;
-    const int nblk_x = A.n_embd / 32, nblk_h = (A.n_ff > A.n_ff_sh ? A.n_ff : A.n_ff_sh) / 32;
-    const int cols_blocks = ((nblk_x > (MAYA_MAX_K + 1) * nblk_h ? nblk_x : (MAYA_MAX_K + 1) * nblk_h) + 1) & ~1;
-    const size_t smem = (size_t) kRepTabBytes<T> + (size_t) cols_blocks * 40 + (size_t) A.n_expert * sizeof(double);
-    if (smem > kMost) return refuse(MAYA_ERR_LIMIT);
-    if (!smem_limit.raise((const void*) moe_layer_t1_kernel<T, TS, RT, HV>, kMost)) return note_launch("fused smem attribute");
+    const size_t smem = fused_smem(T, A);
+    if (smem == 0) return refuse(MAYA_ERR_LIMIT);
+    if (!smem_limit.raise((const void*) moe_layer_t1_kernel<T, TS, RT, HV>, kMostSmem)) return note_launch("fused smem attribute");
     const int grid = sm_count();
     if (grid <= 0) return refuse(MAYA_ERR_DEVICE);
     if (4 * ((A.n_embd / 4 + grid - 1) / grid) > kMaxSliceRows || A.n_embd % 4) return refuse(MAYA_ERR_LIMIT);
@@ -487,7 +494,8 @@ static FusedArgs fused_args(const maya_moe_layer& L) {
 // The kernel for one token (see maya_internal.cuh).
 static int choose(const maya_moe_layer& L, const FusedArgs& A, int sms) {
     const bool takes = token_takes(L, A, sms);
-    if (fused_t1_supported(L)) return takes && token_better(L.gu_type, A, sms) ? MAYA_LAYER_TOKEN : MAYA_LAYER_FUSED;
+    if (fused_t1_supported(L))           // (experts too wide for the fused kernel's columns, of which there is one a plan entry that could be)
+        return takes && (fused_smem(L.gu_type, A) == 0 || token_better(L.gu_type, A, sms)) ? MAYA_LAYER_TOKEN : MAYA_LAYER_FUSED;
     // (a slice of the shared expert beside routed rows of two types, or of a type outside the core, stays refused)
     const bool sliced = A.shared != nullptr && (L.sh_lo != 0 || (L.sh_hi != 0 && L.sh_hi != L.n_ff_sh));
     return takes && !sliced ? MAYA_LAYER_TOKEN : MAYA_LAYER_STAGED;

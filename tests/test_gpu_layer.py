@@ -257,6 +257,7 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
     (H.Q8_0, H.Q8_0, 1344, 352, 0, 8, None),             # an odd number of blocks a row; 11 calls of a down row
     (H.Q8_0, H.Q8_0, 2080, 1056, 96, 6, None),           # three segments, the last of one block; two of a down row
     (H.Q4_K, H.Q4_K, 512, 512, 0, 8, None),              # down rows of 8 calls, four side by side
+    (H.Q4_K, H.Q4_K, 512, 20480, 0, 1, None),            # experts wider than the fused kernel takes
     (H.Q4_K, H.Q6_K, 2304, 1536, 4128, 8, None),         # down in segments of 840 bytes
     (H.Q4_K, H.Q4_K, 2304, 1536, 4128, 6, 64),           # slices of the shared expert
     (H.Q5_K, H.Q8_0, 1536, 2304, 352, 5, None), (H.Q6_K, H.Q5_K, 1280, 768, 0, 7, None), (H.IQ4_XS, H.IQ3_XXS, 2560, 256, 0, 8, None),

@@ -51,6 +51,12 @@ def test_pairs_of_types_that_fit_shared_memory(lib):
     assert kernel(lib, desc(H.IQ2_S, H.IQ3_S, 2304, 2304, 3, n_ff_sh=512, n_expert=12)) == TOKEN
 
 
+@pytest.mark.parametrize("t,n_embd,n_ff", [(H.Q8_0, 1024, 20480), (H.Q4_K, 512, 20480), (H.IQ3_S, 2048, 16384), (H.IQ2_S, 2048, 16384)])
+def test_experts_too_wide_for_the_fused_kernel_take_the_other(lib, t, n_embd, n_ff):
+    """The fused kernel holds nine columns of h whatever k is, the token kernel k of them."""
+    assert kernel(lib, desc(t, t, n_embd, n_ff, 1, n_expert=8)) == TOKEN
+
+
 def test_what_the_token_kernel_leaves_to_others(lib):
     core, mixed = (H.IQ3_S, H.IQ3_S, 6144, 2048, 8), (H.Q4_K, H.Q6_K, 4096, 1536, 8)
     for a, other in ((core, FUSED), (mixed, STAGED)):
