@@ -72,8 +72,10 @@ __device__ __noinline__ void route_token(const float* logits, const float* bias,
 
 // A cooperative launch (the grid barrier needs every block resident) and, where the driver accepts the attribute,
 // programmatically serialized after the launch in front of it: its set-up then overlaps that launch's tail.
-inline int launch_cooperative(const void* kernel, dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what) {
-    static std::atomic<int> pdl{-1};           // the attribute is in use (1), was refused by the driver (0), has not been tried (-1)
+template<auto Kernel>
+int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what) {
+    static std::atomic<int> pdl{-1};           // for this kernel: the attribute is in use (1), was refused by the driver (0), has not been tried (-1)
+    const void* const kernel = (const void*) Kernel;
     if (pdl.load() != 0) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = grid;
