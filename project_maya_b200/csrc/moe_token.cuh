@@ -1,7 +1,9 @@
 // moe_token.cuh - one token through one MoE layer in one cooperative launch, every weight row streamed through shared memory.
 //
-// The form for one GPU of what moe_fused.cu does (which keeps the cross-rank sum and layers of very few units), for any pair
-// of the ten block types.  Phases as there: route and round x / gate and up rows, SwiGLU and q8_1 of h / grid barrier / down rows and combine.
+// The form for one GPU of what moe_fused.cu does (which keeps the cross-rank sum and the layers on which it is the faster kernel: see
+// token_better in moe_token.cu), for pairs of the ten block types whose ring and codebook fit shared memory together: at 6144 x 2048,
+// top 8, 68 of the 100 (not IQ2_S / IQ3_S, nor either of these with Q4_K; token_smem).  Phases as there: route and round x / gate and
+// up rows, SwiGLU and q8_1 of h / grid barrier / down rows and combine.
 //
 // What bounds it: HBM for the 4- to 8-bit types, instruction issue and the shared-memory pipe for the codebook types.  Read in
 // place by 32 warps of 64 registers, a codebook type's fields cost three to four L1 lines a load (the load/store pipe was the limit,
@@ -16,7 +18,7 @@
 //     warps wait for them while the rest decode: as stages they would be many (a ring sized for 2-bit rows) and their handling
 //     more than their dots.
 // Measured beside the fused kernel on 6144 x 2048, top 8 (us, 148 SMs, rows in HBM): IQ2_S 69.6 -> 58.0, IQ3_S 71.0 -> 57.5, Q4_K
-// 60.1 -> 48.0, Q8_0 73.3 -> 68.0, with a 2048-wide shared expert IQ3_S 71.8 -> 65.4, Q4_K 66.3 -> 58.0 (and IQ2_S 63.6 -> 64.8: it stays
+// 60.1 -> 48.0, Q8_0 73.3 -> 68.0, with a 2048-wide shared expert IQ3_S 71.8 -> 65.4, Q4_K 66.3 -> 58.0 (and IQ2_S 63.2 -> 64.4: it stays
 // there); two layers of Q4_K / Q6_K, which took four launches a layer, 122.2 -> 97.8.
 // The loops are kept short: with steps, rows and both row classes unrolled side by side a third of all issue slots went to
 // waiting for instructions (81 us on the 6144 x 2048 IQ2_S layer with shared expert).
@@ -53,11 +55,10 @@ struct TokKind {
 
 struct TokShared {
     RouterShared route;
-    unsigned long long ptr[MAYA_MAX_K + 1];
+    unsigned long long ptr[MAYA_MAX_K];
     float w[MAYA_MAX_K];
     float part[kMaxSliceRows][MAYA_MAX_K + 1];
     uint64_t full[kTokWarps][2];
-    int gave_up[kTokWarps];
     TokKind kind[2];
     unsigned epoch;
     int ve[MAYA_MAX_K];
@@ -66,6 +67,12 @@ struct TokShared {
 };
 
 static_assert(sizeof(TokShared) <= 232448 - kTokMostSmem - 1024, "with the driver's 1 KB");
+
+// Whether ring and codebook of a pair (T: gate/up, TD: down) fit shared memory beside nothing else: a stage is the wider type's, the table
+// the larger codebook's.  token_smem turns away the pairs that do not, and those that fit only narrower layers.
+template<int T, int TD> constexpr bool kTokPair =
+    (size_t) kTokWarps * 8 * (RowGeo<T>::pitch > RowGeo<TD>::pitch ? RowGeo<T>::pitch : RowGeo<TD>::pitch) +
+        (RowTab<T, true>::bytes > RowTab<TD, true>::bytes ? RowTab<T, true>::bytes : RowTab<TD, true>::bytes) <= kTokMostSmem;
 
 // One q8_1 block of 32 values, one a lane: its lane's quant, the scale as the f16 field holds it, and the sum a dot takes - of the
 // quants, or for IQ1_S the stored f16 sum of the values (float bits).
@@ -234,7 +241,6 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             for (int w = warp; w < kTokWarps; w += kRouteThreads / 32) {
                 mbar_init(&sh.full[w][0], 4);
                 mbar_init(&sh.full[w][1], 4);
-                sh.gave_up[w] = 0;
             }
             mbar_fence_init();
         }
@@ -342,11 +348,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
 
     const int half = n_ff / 2, nv = sh.nv;
     int asked = 0, got = 0;                              // stages asked for and read: stage i lies in ring place i % 2
-    auto wait = [&]() -> bool {
-        if (__all_sync(0xffffffffu, mbar_wait(&sh.full[warp][got & 1], (got >> 1) & 1, A.polls))) return true;
-        *(volatile int*) &sh.gave_up[warp] = 1;
-        return false;
-    };
+    auto wait = [&]() -> bool { return __all_sync(0xffffffffu, mbar_wait(&sh.full[warp][got & 1], (got >> 1) & 1, A.polls)); };
     // The stream.  A lane r < 4 keeps row r's next byte and how many are left of it.
     const uint8_t* a_row = nullptr;
     uint32_t a_left = 0;
@@ -584,7 +586,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
                 }
             }
         };
-#define MAYA_TOK_DOWN(TT) case TT: down(std::integral_constant<int, TT>{}); break;
+#define MAYA_TOK_DOWN(TT) case TT: if constexpr (kTokPair<T, TT>) down(std::integral_constant<int, TT>{}); break;
         switch (A.d_type) {
             MAYA_TOK_DOWN(MAYA_Q8_0) MAYA_TOK_DOWN(MAYA_Q4_K) MAYA_TOK_DOWN(MAYA_Q5_K) MAYA_TOK_DOWN(MAYA_Q6_K) MAYA_TOK_DOWN(MAYA_IQ4_XS)
             MAYA_TOK_DOWN(MAYA_IQ2_S) MAYA_TOK_DOWN(MAYA_IQ3_S) MAYA_TOK_DOWN(MAYA_IQ3_XXS) MAYA_TOK_DOWN(MAYA_IQ2_XXS) MAYA_TOK_DOWN(MAYA_IQ1_S)
