@@ -253,6 +253,26 @@ def test_fused_token_kernel_equals_staged_kernels_bitwise(T, api, oracle, t, sha
     assert H.rel_err(out.cpu().numpy()[0], want) <= TIGHT
 
 
+@pytest.mark.parametrize("t,n_embd,n_ff,n_ff_sh,k", [
+    (H.Q4_K, 2048, 1024, 0, 8), (H.Q4_K, 7168, 512, 1024, 8), (H.Q8_0, 2080, 1056, 96, 6), (H.Q8_0, 6144, 256, 2048, 8),
+    (H.IQ3_S, 6144, 2048, 0, 4), (H.IQ3_S, 4352, 1024, 288, 6), (H.IQ2_S, 6144, 1024, 2048, 8)])
+def test_fused_kernel_at_the_widths_that_ranks_use(T, api, t, n_embd, n_ff, n_ff_sh, k):
+    """What several ranks run a token with, whichever kernel is the faster one on a single GPU: the staged kernels' bits."""
+    n_expert = 10
+    cfg = dict(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, k=k, gu_type=t, d_type=t, limit=7.0)
+    if n_ff_sh:
+        cfg.update(n_ff_sh=n_ff_sh, sh_gu_type=H.Q8_0, sh_d_type=H.Q8_0)
+    two = dev(T, np.stack([H.constructed_expert(t, t, n_embd, n_ff, H.rng_for("wide", t, e)) for e in range(2)]))
+    experts = two[T.arange(n_expert, device="cuda") % 2].contiguous()
+    sh = dev(T, H.constructed_expert(H.Q8_0, H.Q8_0, n_embd, n_ff_sh, H.rng_for("wide-shared", t))) if n_ff_sh else None
+    layer = api.MoeLayer(layer_cfg(api, cfg), experts, sh, expert_range=(0, 8))
+    logits, x = dev(T, H.router_logits("wide", 3, n_expert, 1.1)), dev(T, H.activations("wide", 3, n_embd, "bf16"), T.bfloat16)
+    for i in (0, 1, 2, 0):
+        got, want = (layer.forward_checked(logits[i:i + 1], x[i:i + 1], kernel) for kernel in (api.LAYER_FUSED, api.LAYER_STAGED))
+        assert all(T.equal(a, b) for a, b in zip(got, want)), f"token {i}"
+    assert layer.error() == 0 and want[2].abs().max() > 0
+
+
 @pytest.mark.parametrize("gu,d,n_embd,n_ff,n_ff_sh,k,cut", [
     (H.Q8_0, H.Q8_0, 1344, 352, 0, 8, None),             # an odd number of blocks a row; 11 calls of a down row
     (H.Q8_0, H.Q8_0, 2080, 1056, 96, 6, None),           # three segments, the last of one block; two of a down row
@@ -370,7 +390,7 @@ def test_window_with_shared_expert_equals_fused_tokens_bitwise(T, api, t, n_embd
 
 
 def test_fused_kernel_many_calls_one_scratch(T, api):
-    """The grid barrier's counter lives in the scratch: hundreds of calls, single tokens and windows interleaved."""
+    """The grid barrier's counter lives in the scratch: hundreds of calls, single tokens (fused) and windows interleaved."""
     cfg = dict(n_embd=512, n_ff=256, n_expert=8, k=4, gu_type=H.Q4_K, d_type=H.Q4_K)
     lc, experts, _ = synth_layer(T, api, cfg, 8, seed=3)
     layer = api.MoeLayer(lc, experts)
@@ -383,6 +403,38 @@ def test_fused_kernel_many_calls_one_scratch(T, api):
         out = layer.forward(logits[:1], x[:1])[2]
     T.cuda.synchronize()
     assert T.equal(out, first)
+    assert layer.error() == 0
+
+
+@pytest.mark.parametrize("gu,d,n_ff_sh", [(H.Q4_K, H.Q6_K, 0), (H.IQ3_S, H.IQ3_S, 1056)])
+def test_token_kernel_many_calls_one_scratch(T, api, gu, d, n_ff_sh):
+    """The counters of units that two blocks share live in the scratch too: hundreds of tokens, whose experts change from call to call
+    and some of which are another rank's, windows, fused tokens and replays of a captured token between them."""
+    n_embd, n_ff, n_expert, k = 768, 1280, 12, 5
+    cfg = dict(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, k=k, gu_type=gu, d_type=d)
+    if n_ff_sh:
+        cfg.update(n_ff_sh=n_ff_sh, sh_gu_type=H.Q8_0, sh_d_type=H.Q8_0)
+    three = dev(T, np.stack([H.constructed_expert(gu, d, n_embd, n_ff, H.rng_for("manytok", gu, e)) for e in range(3)]))
+    experts = three[T.arange(n_expert, device="cuda") % 3].contiguous()
+    sh = dev(T, H.constructed_expert(H.Q8_0, H.Q8_0, n_embd, n_ff_sh, H.rng_for("manytok-shared", gu))) if n_ff_sh else None
+    layer = api.MoeLayer(layer_cfg(api, cfg), experts, sh, expert_range=(2, n_expert))
+    logits, x = dev(T, H.router_logits("manytok", 16, n_expert, None)), dev(T, H.activations("manytok", 16, n_embd, "f32"))
+    want = [layer.forward_checked(logits[i:i + 1], x[i:i + 1], api.LAYER_STAGED) for i in range(16)]
+    stream, graph = T.cuda.Stream(), T.cuda.CUDAGraph()
+    T.cuda.synchronize()
+    with T.cuda.graph(graph, stream=stream):
+        replayed = layer.forward_checked(logits[3:4], x[3:4], api.LAYER_TOKEN)
+    T.cuda.synchronize()
+    for i in range(300):
+        if i % 50 == 7:
+            layer.forward(logits, x)
+        if i % 50 == 23:
+            graph.replay()
+            assert all(T.equal(a, b) for a, b in zip(replayed, want[3]))
+        if gu == d and i % 3 == 1:
+            layer.forward_checked(logits[:1], x[:1], api.LAYER_FUSED)
+        got = layer.forward_checked(logits[i % 16:i % 16 + 1], x[i % 16:i % 16 + 1], api.LAYER_TOKEN)
+        assert all(T.equal(a, b) for a, b in zip(got, want[i % 16])), f"call {i}"
     assert layer.error() == 0
 
 
@@ -685,8 +737,8 @@ def test_fused_layer_exchange_times_out_and_poisons(T, api):
 @pytest.mark.parametrize("t", list(H.MORE_TYPES))
 def test_layer_with_further_block_types(T, api, oracle, t):
     """maya_moe_layer_decode on routed experts stored as Q5_K, Q6_K, IQ4_XS, IQ3_XXS or IQ2_XXS (the rest of
-    glmf::moe_supported's table): the staged kernels run, with a Q8_0 shared expert beside them; single tokens against the
-    oracle, and a 5-token window equal to its tokens bit for bit."""
+    glmf::moe_supported's table) with a Q8_0 shared expert beside them: single tokens (the token kernel) against the oracle, and
+    a 5-token window equal to its tokens bit for bit."""
     n_embd, n_ff, E, k, n_sh = 1024, 512, 12, 4, 256
     cfg = dict(n_embd=n_embd, n_ff=n_ff, n_expert=E, k=k, gu_type=t, d_type=t, n_ff_sh=n_sh, sh_gu_type=H.Q8_0, sh_d_type=H.Q8_0)
     rng = H.rng_for("layer-more", t)
