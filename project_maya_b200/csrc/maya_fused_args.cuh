@@ -32,8 +32,8 @@ struct FusedArgs {
     int ar_rank;
     unsigned ar_seq;
     maya_hc_post_args hc;      // hc.R_new != NULL: the hyper-connection write of `out` into the residual stack, last
-    unsigned* sync;            // scratch: [0] arrivals, [1] epoch, [2] error, [4..15] block 0's phase time stamps (ns), [16] the mark of the
-                               // last launch in which a block of the token kernel gave up
+    unsigned* sync;            // scratch: [0] arrivals, [1] epoch, [2] error, [4..15] block 0's phase time stamps (ns), [kTokMark] the mark
+                               // of the last launch in which a block of the token kernel gave up
 };
 
 // moe_token.cuh: the rows' places in a blob, and the launch's carve-up of shared memory.
@@ -46,6 +46,7 @@ struct TokArgs : FusedArgs {
     int units;                 // units of h a block may work on
 };
 constexpr int kTokWarps = 16;
+constexpr int kTokMark = 32;    // a 128-byte line away from the arrivals, which every block is polling when the mark is read
 constexpr size_t kTokMostSmem = 232448 - 8192;                  // dynamic shared memory, beside the static part
 #define MAYA_TOK_TYPES(X) X(MAYA_IQ2_S) X(MAYA_IQ3_S) X(MAYA_IQ3_XXS) X(MAYA_IQ2_XXS) X(MAYA_IQ1_S)      // types with a codebook
 __host__ __device__ inline int tok_col_bytes(int nblk) { return (nblk * 40 + 15) & ~15; }       // of an activation column

@@ -4,6 +4,7 @@
 // blob addresses of its k routed experts (0 for experts outside [expert_lo, expert_hi): another rank's).
 #include <math.h>
 
+#include "maya_fused_args.cuh"
 #include "maya_group.cuh"
 #include "maya_internal.cuh"
 #include "maya_router.cuh"
@@ -28,8 +29,8 @@ struct Scratch {
     float* sh_out;               // [T][n_embd]
     float* h;                    // the fused single-token kernel's h: q8_1 image, shared-unit halves, counters
     unsigned* unit_count;        // the token kernel's counters of units that two blocks share (zero before first use)
-    unsigned* sync;              // [17]: the fused and the token kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket;
-                                 // stamps; [16] the token kernel's mark of a launch that gave up (zero before first use)
+    unsigned* sync;              // [33]: the fused and the token kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket;
+                                 // stamps; [32] the token kernel's mark of a launch that gave up (zero before first use)
     size_t bytes;
 };
 
@@ -41,7 +42,7 @@ Scratch carve(const maya_moe_layer& L, int T, uint8_t* base) {
     auto take = [&](size_t n) { uint8_t* p = base ? base + off : nullptr; off += align_up(n); return p; };
     // the fused kernel's words first: their place must not depend on T (a scratch sized for a window also serves
     // single tokens, and the barrier counter has to survive the calls in between)
-    s.sync = (unsigned*) take(17 * sizeof(unsigned));
+    s.sync = (unsigned*) take((kTokMark + 1) * sizeof(unsigned));
     {
         const int ld = L.n_ff > L.n_ff_sh ? L.n_ff : L.n_ff_sh;
         // per expert and 32-value group of h: the q8_1 image (40 bytes), the f32 halves two blocks leave when a unit is

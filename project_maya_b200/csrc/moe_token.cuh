@@ -26,9 +26,9 @@
 // bit-identical to every other path's.
 //
 // Every wait is bounded.  A warp whose copies never land asks for nothing more; its block says so in the error word and, with the
-// launch's mark, in sync[16], still meets the others at the grid barrier, and leaves after the copies in flight have had a bounded
-// time.  The other blocks find the mark behind the barrier, where the h that they read is incomplete: none writes `out` or the
-// residual stack, and the counters of split units, some of which stay short of a launch's 16, are set to zero for the next launch.
+// launch's mark, in sync[kTokMark], still meets the others at the grid barrier, and leaves after the copies in flight have had a bounded
+// time.  The other blocks ask for the mark behind the barrier, where the h that they read may be incomplete, and look at it where they
+// vote on their own rows (a vote of its own cost 1 %): none writes `out` or the residual stack, and the counters of split units, some of which stay short of a launch's 16, are set to zero for the next launch.
 #pragma once
 
 #include "maya_fused_args.cuh"
@@ -63,7 +63,7 @@ struct TokShared {
     unsigned epoch;
     int ve[MAYA_MAX_K];
     int nv;
-    int bar_ok;
+    int bar_ok, lost;
 };
 
 static_assert(sizeof(TokShared) <= 232448 - kTokMostSmem - 1024, "with the driver's 1 KB");
@@ -203,14 +203,12 @@ struct Spread {
 // What only a launch in which a wait ran out comes to: as functions of their own, out of the kernel's register allocation.
 __device__ __noinline__ void tok_gave_up(unsigned* sync, unsigned mark) {
     atomicExch(&sync[2], 1u);
-    atomicExch(&sync[16], mark);
+    atomicExch(&sync[kTokMark], mark);
 }
-// (every block of the launch is past its counters)
-__device__ __noinline__ void tok_reset(unsigned* count, int n) {
+// The n counters made whole for the next launch (n = 0: some block may not be past them yet); and what a warp has in flight lands before
+// the block's shared memory goes away.
+__device__ __noinline__ void tok_unwind(unsigned* count, int n, uint64_t* full, int got, int asked) {
     for (int i = threadIdx.x; i < n; i += kTokThreads) count[i] = 0u;
-}
-// what a warp has in flight lands before the block's shared memory goes away
-__device__ __noinline__ void tok_drain(uint64_t* full, int got, int asked) {
     for (; got < asked; ++got) mbar_wait(&full[got & 1], (got >> 1) & 1);
 }
 
@@ -521,7 +519,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
 
     // ---------------------------------------------------------------- phase 2: q8_1(h), down, combine
     if (done) {
-        const unsigned lost = tid == 0 ? __ldcg(A.sync + 16) : 0u;   // (asked for ahead of h: both arrive together)
+        const unsigned lost = tid == 0 ? __ldcg(A.sync + kTokMark) : 0u;   // (asked for ahead of h: both arrive together)
         const int nb_r = n_ff / 32, total_r = nv * nb_r, b_s = has_sh ? A.sh_lo / 32 : 0, nb_s = has_sh ? (A.sh_hi - A.sh_lo) / 32 : 0;
         const int xb2 = A.d_type == MAYA_Q4_K || A.d_type == MAYA_Q5_K ? 2 : 1;
         for (int i = tid; i < 2 * (total_r + nb_s); i += kTokThreads) {          // half a block each, its scale or its sum
@@ -537,10 +535,8 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             *(uint4*) (col + (two ? tok_piece<2>(n, blk, hf) : tok_piece<1>(n, blk, hf))) = v;
             *(uint32_t*) (col + (two ? tok_scale<2>(n, blk) : tok_scale<1>(n, blk)) + hf * n * 4) = ds;
         }
-        done = __syncthreads_or(lost == mark ? 1 : 0) == 0;         // no block gave up
-    }
-    if (done) {
-        const int nb_r = n_ff / 32, nb_s = has_sh ? (A.sh_hi - A.sh_lo) / 32 : 0;
+        if (tid == 0) sh.lost = lost == mark;            // a block gave up: looked at below, before anything is written
+        __syncthreads();
         if (SH) {                                        // the shared expert's rows, by the warps that have an item less (in the loop
                                                          // below, spread among the others, this phase took 21.1 us instead of 18.6)
             const TokCol H{cols + nv * tok_col_bytes(nb_r), nb_s};
@@ -592,7 +588,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             MAYA_TOK_DOWN(MAYA_IQ2_S) MAYA_TOK_DOWN(MAYA_IQ3_S) MAYA_TOK_DOWN(MAYA_IQ3_XXS) MAYA_TOK_DOWN(MAYA_IQ2_XXS) MAYA_TOK_DOWN(MAYA_IQ1_S)
         }
 #undef MAYA_TOK_DOWN
-        done = __syncthreads_or(ok ? 0 : 1) == 0;
+        done = __syncthreads_or(ok && sh.lost == 0 ? 0 : 1) == 0;
         if (!done && tid == 0) atomicExch(&A.sync[2], 1u);
         if (done && tid < nrows) {
             float m = 0.0f;
@@ -601,9 +597,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             A.out[o0 + tid] = __fadd_rn(m, has_sh ? sh.part[tid][k] : 0.0f);
         }
     }
-    if (met && !done)                                    // every block is past its counters: whole again for the next launch
-        tok_reset(A.unit_count, (MAYA_MAX_K + 1) * nblk_h);
-    if (got < asked) tok_drain(sh.full[warp], got, asked);       // (nothing in flight, unless a wait ran out)
+    if (!done) tok_unwind(A.unit_count, met ? (MAYA_MAX_K + 1) * nblk_h : 0, sh.full[warp], got, asked);
     stamp(A.sync, 4);
     __syncthreads();
     if (A.hc.R_new != nullptr && done) hc_post_rows(A.out, A.hc, n_embd, o0, o1, tid, kTokThreads);
