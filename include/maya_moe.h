@@ -315,13 +315,13 @@ typedef struct maya_moe_layer {
     int expert_lo, expert_hi;    /* this rank's experts [lo, hi); others contribute nothing (expert-parallel) */
     int shared_here;             /* non-zero: this rank adds the shared expert */
     int staged;                  /* non-zero: run one token through the staged kernels (routing with q8_1, gate/up, down, combine
-                                    as separate launches) instead of the single fused kernel; same bits either way */
+                                    as separate launches) instead of one of the one-launch kernels; same bits either way */
     int sh_lo, sh_hi;            /* with shared_here: this rank's slice [sh_lo, sh_hi) of the shared expert's FFN width
                                     (multiples of 32; 0, 0 = all of it): its gate/up rows and the same columns of the down
                                     rows, so that the ranks' partial outputs add up to the shared expert's output (the
                                     width-sliced placement; summed in another order than on one rank, so equal to it
-                                    only to rounding).  A proper slice needs the single fused kernel (one token, Q8_0
-                                    shared expert): otherwise the call is refused */
+                                    only to rounding).  A proper slice needs one token, a Q8_0 shared expert and routed experts of
+                                    one core type: otherwise the call is refused */
     int router;                  /* 0: softmax routing (router_top10); 1: sigmoid routing (router_sigmoid.hpp:27,
                                     glmf::moe_route's arithmetic, glm_fast.hpp:426) with the three fields below */
     const float* router_bias;    /* sigmoid: [n_expert] added to the scores for the SELECTION only; NULL: none */
@@ -341,7 +341,7 @@ typedef struct maya_moe_layer {
 MAYA_API size_t maya_moe_layer_scratch_bytes(const maya_moe_layer* L, int n_tokens);
 /* Reads the sticky error word of a layer scratch (synchronises the stream first). 0 = no error. */
 MAYA_API int maya_moe_layer_error(const maya_moe_layer* L, int n_tokens, const void* scratch, void* stream);
-/* Diagnostic: block 0's wall-clock stamps (ns, %globaltimer) of the last fused single-token launch on this scratch:
+/* Diagnostic: block 0's wall-clock stamps (ns, %globaltimer) of the last one-launch token (fused or token kernel) on this scratch:
  * start, end of routing/quantizing, end of its gate/up work, past the grid barrier, end of down + combine, end of the
  * cross-rank sum (= the previous stamp without one).  Synchronises the stream. */
 MAYA_API int maya_moe_layer_phase_ns(const maya_moe_layer* L, const void* scratch, void* stream, unsigned long long* out6);

@@ -50,8 +50,8 @@ bool token_takes(const maya_moe_layer& L, const FusedArgs& F, int sms) {
 // second; the fused kernel is through with its set-up sooner, has 32 warps to wait for a shared expert's rows with, and handles no stages.
 // So the lines lie at the routed bytes a token reads, and where rows leave stages half empty or the shared expert is much of the
 // work.  From 925 timed layers of 1024 .. 8192 x 512 .. 3072, 1 to 8 experts a token, half of them with a shared expert, as three layers in
-// turn and as so many that no row stays in L2: by this rule none is more than 4 % (5 % IQ2_S) slower than on the fused kernel, 11 more
-// than 2 %; 1.4 % (IQ2_S, Q8_0 with shared) to 11 % (Q4_K) faster on average.  (us fused / token kernel, 148 SMs, three layers in turn)
+// turn and as so many that no row stays in L2: by this rule none is more than 5 % slower than on the fused kernel, 13 more than 2 %
+// (seven of them IQ2_S, which out of HBM are the faster); 1.4 % (IQ2_S) to 9 % (Q4_K) faster on average.  (us fused / token kernel, 148 SMs, three layers in turn)
 bool token_better(int type, const FusedArgs& A, int sms) {
     const bool sh = A.shared != nullptr;
     const int width = A.sh_hi - A.sh_lo;

@@ -54,7 +54,8 @@ template<int T, int SPLIT = 1> struct WGeo : RowGeo<T> {
     static constexpr int stage = rw / SPLIT * RowGeo<T>::pitch;                                 // a warp's stage
     static constexpr int tab = RowTab<T, false>::bytes;
     // What a warp's four rows cost against nc columns, in units of 30 cycles, fitted to clock stamps of 16-token windows
-    // (Q8_0, Q4_K, IQ2_S, IQ3_S, IQ3_XXS, IQ4_XS; the other four types' are estimates without stamps): per 32
+    // (Q8_0, Q4_K, IQ2_S, IQ3_S, IQ3_XXS, IQ4_XS; the other four types' are estimates without stamps) - those of the codebook types before
+    // maya_rows.cuh's decoders, with which IQ2_S and IQ3_S rows cost about a tenth less; not fitted again since: per 32
     // calls of a row the decoding (for Q8_0: waiting for its bytes) and every column's dot, and every column's sums at the end.
     // A share that is off by a tenth is a tenth of the launch: with costs counted in instructions instead the slowest of 148
     // blocks took 27 % longer than the mean.
@@ -65,7 +66,7 @@ template<int T, int SPLIT = 1> struct WGeo : RowGeo<T> {
     static constexpr int job_cost = 350;                     // a block's change of job: its columns, and code it has not run
     __device__ __forceinline__ static int cost(int nc, int n_in) {
         if (nc > 4) nc = (nc + 1) & ~1;          // dotted as six, as eight
-        const int spilled = T == MAYA_IQ2_S && nc == 8 ? 60 : 0;
+        const int spilled = T == MAYA_IQ2_S && nc == 8 ? 60 : 0;     // (of the former decoder: now only beside a shared expert)
         return (dec_cost + nc * col_cost + spilled) * ((n_in / qk * cpb + 31) / 32) + nc * sum_cost;
     }
 };
