@@ -42,6 +42,7 @@ struct TokArgs : FusedArgs {
     size_t up_off, down_off;   // byte offsets of the up and of the down rows in a routed blob
     unsigned* unit_count;      // scratch [(MAYA_MAX_K + 1) * blocks of h]: items done of units that two blocks share, modulo 16
     unsigned polls;            // looks at a row's copy before a warp gives up
+    unsigned drain_polls;      // and, at the end, at the copies still in flight
     int stage, tab, cols;      // bytes of a ring stage, of the codebook, of the activation columns
     int units;                 // units of h a block may work on
 };

@@ -84,6 +84,7 @@ int token_layer(const maya_moe_layer& L, const FusedArgs& F, unsigned* unit_coun
     TokArgs A = token_args(L, F);
     A.unit_count = unit_count;
     A.polls = polls;
+    A.drain_polls = kMbarPolls;
     switch (L.gu_type) {
         case MAYA_Q8_0: return token_by_type<MAYA_Q8_0>(A, s);
         case MAYA_Q4_K: return token_by_type<MAYA_Q4_K>(A, s);

@@ -28,7 +28,8 @@
 // Every wait is bounded.  A warp whose copies never land asks for nothing more; its block says so in the error word and, with the
 // launch's mark, in sync[kTokMark], still meets the others at the grid barrier, and leaves after the copies in flight have had a bounded
 // time.  The other blocks ask for the mark behind the barrier, where the h that they read may be incomplete, and look at it where they
-// vote on their own rows (a vote of its own cost 1 %): none writes `out` or the residual stack, and the counters of split units, some of which stay short of a launch's 16, are set to zero for the next launch.
+// vote on their own rows (a vote of its own cost 1 %): none writes `out` or the residual stack.  The counters of split units, some of
+// which stay short of a launch's 16, are set to zero by the block that gave up.
 #pragma once
 
 #include "maya_fused_args.cuh"
@@ -205,11 +206,9 @@ __device__ __noinline__ void tok_gave_up(unsigned* sync, unsigned mark) {
     atomicExch(&sync[2], 1u);
     atomicExch(&sync[kTokMark], mark);
 }
-// The n counters made whole for the next launch (n = 0: some block may not be past them yet); and what a warp has in flight lands before
-// the block's shared memory goes away.
-__device__ __noinline__ void tok_unwind(unsigned* count, int n, uint64_t* full, int got, int asked) {
+// The n counters made whole for the next launch.  (Every block is past them.)
+__device__ __noinline__ void tok_reset(unsigned* count, int n) {
     for (int i = threadIdx.x; i < n; i += kTokThreads) count[i] = 0u;
-    for (; got < asked; ++got) mbar_wait(&full[got & 1], (got >> 1) & 1);
 }
 
 // T: gate/up type; SH: with a Q8_0 shared expert.
@@ -516,6 +515,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     const bool met = grid_barrier(A.sync, sh.epoch, &sh.bar_ok);
     stamp(A.sync, 3);
     bool done = ok && met;
+    if (!ok && met) tok_reset(A.unit_count, (MAYA_MAX_K + 1) * nblk_h);
 
     // ---------------------------------------------------------------- phase 2: q8_1(h), down, combine
     if (done) {
@@ -597,7 +597,8 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
             A.out[o0 + tid] = __fadd_rn(m, has_sh ? sh.part[tid][k] : 0.0f);
         }
     }
-    if (!done) tok_unwind(A.unit_count, met ? (MAYA_MAX_K + 1) * nblk_h : 0, sh.full[warp], got, asked);
+    // what a warp has in flight lands before the block's shared memory goes away (nothing, unless a wait ran out); A.polls may be few
+    for (; got < asked; ++got) mbar_wait(&sh.full[warp][got & 1], (got >> 1) & 1, A.drain_polls);
     stamp(A.sync, 4);
     __syncthreads();
     if (A.hc.R_new != nullptr && done) hc_post_rows(A.out, A.hc, n_embd, o0, o1, tid, kTokThreads);
