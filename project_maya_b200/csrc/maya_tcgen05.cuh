@@ -55,16 +55,33 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
 // Tiled TMA load of a 3-d box (plain: this block only, no multicast) from the tensor described by `map` (a
 // CUtensorMap in kernel-parameter or global memory) into shared memory; completion is counted in bytes on `bar`.
 // c0 * element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_3d(void* dst_smem, const void* map, uint64_t* bar, int c0, int c1, int c2) {
+// by one elected lane of a CONVERGED warp, every operand warp-uniform (they then stay in uniform registers, where the copy wants
+// them: a lane of its own in a divergent branch took 400 to 500 cycles a tile): so many bytes expected on `bar`, and a box that brings them
+__device__ __forceinline__ void tma_expect_load_3d(uint32_t dst_smem, const void* map, uint32_t bar, uint32_t bytes, int c0, int c1, int c2) {
+    __syncwarp();
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-        ::"r"(smem_u32(dst_smem)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %6;\n\t"
+        "@e cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+        ::"r"(dst_smem), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(bytes)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(void* dst_smem, const void* map, uint64_t* bar, int c0, int c1) {
+__device__ __forceinline__ void tma_expect_load_2d(uint32_t dst_smem, const void* map, uint32_t bar, uint32_t bytes, int c0, int c1) {
+    __syncwarp();
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst_smem)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], %5;\n\t"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+        ::"r"(dst_smem), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(bytes)
+        : "memory");
+}
+// the same without the expectation, for a second box on the same barrier
+__device__ __forceinline__ void tma_load_2d_elect(uint32_t dst_smem, const void* map, uint32_t bar, int c0, int c1) {
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+        ::"r"(dst_smem), "l"(map), "r"(bar), "r"(c0), "r"(c1)
         : "memory");
 }
 // shared -> global bulk copy (16-byte aligned, size % 16 == 0), tracked by this thread's bulk groups
@@ -84,6 +101,9 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool cond) {
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_addr(uint32_t bar_smem) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_smem) : "memory");
 }
 
 // The products of 64 K-values (four K = 16 steps) into one accumulator and the commit that follows them, issued by one elected

@@ -14,19 +14,29 @@
 // weights are the A operand and live in tensor memory too (lane = weight row, the layout a thread-per-row expansion
 // produces by itself), so shared memory carries only raw blocks and activations: an SM's 128 bytes/clock of shared
 // memory cannot feed two f16 operands of M = N = 128 products at the tensor core's rate.  Warp roles:
-//   warp 16     one lane: TMA loads of raw weight blocks, 64 rows x 256 K-values a "unit", into a ring of units;
-//   warp 18     one lane: TMA loads of activation tiles, 128 (+ 32) rows x 64 K-values, in the 128-byte swizzle layout
+//   warp 16     TMA loads of raw weight blocks, 64 rows x 256 K-values a "unit", into a ring of units;
+//   warp 18     TMA loads of activation tiles, 128 (+ 32) or 32 rows x 64 K-values, in the 128-byte swizzle layout
 //               the tensor core reads at full rate;
-//   warps 0..15 two teams of 8 warps that take alternate K steps; in a team one thread per weight row expands 32
-//               K-values of the row per step (packed half2 arithmetic: Q8_0 w = q * d; Q4_K w = fma(q, d * sc,
-//               -(dmin * m))) and tcgen05.st-s them into the row's lane;
+//   warps 0..15 two teams of 8 warps that take alternate K steps (i-quants: alternate blocks, whose steps alternate in the products'
+//               order); in a team one thread per weight row expands 32 K-values of the row per step (packed half2 arithmetic:
+//               Q8_0 w = q * d; Q4_K w = fma(q, d * sc, -(dmin * m))) and tcgen05.st-s them into the row's lane;
 //   warps 17,19 one accumulator each: two tcgen05.mma per step (2 K = 16 halves, A from tensor memory, B from shared
 //               memory), one commit per two steps -> the steps' buffers are free (the warp cannot issue products as fast as
 //               the tensor core retires them unless their operands stay in uniform registers: see there);
 //   warps 0..15 afterwards: the epilogue - tcgen05.ld (lane = weight row, column = activation row), SwiGLU, optional
 //               q8_1 rounding of h for the next product; f32 results leave through shared memory, one bulk copy per activation row.
 // Which expert and which 160-row group of it a block handles is found on the device from `bounds`; no count travels
-// to the host.  Every mbarrier wait is bounded: a wait that runs out sets the error word, the roles stop, copies in
+// to the host.
+//
+// What bounds it: for groups of many rows the board's power limit and the expansion, for
+// groups of few rows the expansion alone, 4 instructions a weight.  That holds only while no waiting role is in the way: clock stamps of 64 tokens of
+// IQ3_S showed finished weights waiting 3000 cycles - the activation loader, one lane in a divergent branch, took 540 cycles a tile
+// (every operand of a copy crossed into a uniform register), longer than the expansion.  Now both loaders walk their loops as whole
+// warps and an elected lane copies, the role's number is warp-uniform to the compiler (an issuing warp's products 137 -> 47 cycles), the
+// stages fill tensor memory, and a stage is asked for before the expansion that goes there.  us a layer, before and after: 64 tokens of IQ3_S 463 / 385,
+// 777 of IQ2_S with a shared expert 1262 / 1165, 4096 of Q8_0 / Q4_K 3499 / 3190, 60 of Q8_0 236 / 200, 100 of Q4_K 265 / 245.
+//
+// Every mbarrier wait is bounded: a wait that runs out sets the error word, the roles stop, copies in
 // flight are waited for (bounded), tensor memory is freed and the block returns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -35,8 +45,10 @@
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
+#include <utility>
 
 #include "maya_internal.cuh"
+#include "maya_rows.cuh"
 #include "maya_tcgen05.cuh"
 
 namespace maya {
@@ -45,14 +57,13 @@ namespace {
 constexpr int TM = 256;                 // weight rows of a block
 constexpr int TN = 160;                 // most activation rows of a block
 constexpr int BK = 32;                  // K values of one step
-constexpr int kSt = 3;                  // stages of expanded weights (the A operand, in tensor memory), 64 K-values each
+constexpr int kMaxSt = 7;               // most stages of expanded weights (the A operand, in tensor memory), 64 K-values each
+constexpr int kMaxBSt = 8;              // most activation tiles (64 K-values) in flight
 constexpr int kUnitRows = 64;           // weight rows of one raw unit
 constexpr int kDqWarps = 16;            // two teams of 8
 constexpr int kMmqThreads = (kDqWarps + 4) * 32;   // + raw-unit loader, issuer of accumulator 0, activation loader, issuer of accumulator 1
 constexpr int kBBox = 128 * 64 * 2;     // 16 KB: 128 activation rows x 64 K-values, 128-byte swizzle
 constexpr int kBStage = kBBox + 32 * 64 * 2;   // + the 32-row box of a block with more than 128 rows: 20 KB
-constexpr uint32_t kAccCols = TN;       // tensor-memory columns: accumulator 0 at 0, accumulator 1 at 160,
-constexpr uint32_t kACol = 2 * TN;      // the A operand's 3 stages from 320: per stage 32 columns for each accumulator
 constexpr int kMaxUnits = 16;
 constexpr int kDone = 16;               // ring of "pair of K steps consumed" barriers (one tcgen05.commit per pair: a commit
                                         // costs the tensor pipe about as much as a product)
@@ -66,8 +77,7 @@ template<int T> constexpr int kWin = T == MAYA_IQ2_S ? 96 : 128;
 template<int T> constexpr int kRawRow = T == MAYA_Q4_K ? 144 : T == MAYA_Q8_0 ? 272 : T == MAYA_IQ2_S ? 112 : 144;
 template<int T> constexpr int kUnitBytes = kUnitRows * kRawRow<T>;
 template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 10 : T == MAYA_Q8_0 ? 8 : T == MAYA_IQ2_S ? 11 : 9;   // raw units in flight
-template<int T> constexpr int kBStages = T == MAYA_Q4_K ? 6 : 4;            // activation tiles (64 K-values) in flight
-template<int T> constexpr int kBRing = kBStages<T> * kBStage;
+template<int T> constexpr int kBRing = (T == MAYA_Q4_K ? 6 : 4) * kBStage;    // activation tiles (64 K-values) in flight
 // i-quants: the codebook as f16 (IQ2_S 1024 entries of 8 values, IQ3_S 512 of 4), kept in kCopies copies that lie side by
 // side in every entry - lane l reads copy l % kCopies - so that a warp's 32 random entries spread over the banks: sixteen
 // 8-byte copies are free of conflicts, four 16-byte copies cost about 8 wavefronts a look-up where one costs 11.  (The
@@ -230,59 +240,54 @@ template<int BYTE> __device__ __forceinline__ uint32_t win_u32(const uint32_t* w
     if constexpr (r == 0) return w[i];
     else return __byte_perm(w[i], w[i + 1], 0x5432);
 }
-// bytes {B, B + 1, C, C + 1} (B and C even)
-template<int B, int C> __device__ __forceinline__ uint32_t win_two16(const uint32_t* w) {
-    return __byte_perm(w[B / 4], w[C / 4], (B % 4) | (B % 4 + 1) << 4 | (C % 4 + 4) << 8 | (C % 4 + 5) << 12);
+// the words at BYTE, BYTE + 4, ...
+template<int BYTE, int... I> __device__ __forceinline__ void win_words(const uint32_t* w, uint32_t* dst, std::integer_sequence<int, I...>) {
+    ((dst[I] = win_u32<BYTE + 4 * I>(w)), ...);
 }
-template<int BYTE> __device__ __forceinline__ float win_f16(const uint32_t* w) {
-    return __half2float(__ushort_as_half((unsigned short) ((w[BYTE / 4] >> (8 * (BYTE % 4))) & 0xFFFF)));
-}
-// The fields of the four sub-blocks of 32 values a team expands of a block: pairs TEAM and TEAM + 2, i.e. sub-blocks
-// 2 TEAM + {0, 1, 4, 5}.  q: codebook index bytes (one word a sub-block for IQ2_S, two for IQ3_S); sg: sign bytes; byte j of
-// qh: sub-block j's high index bits; sc: scale bytes, IQ2_S byte j = sub-block j's, IQ3_S byte j = pair j's.
+// A block's fields.  q: codebook index bytes (a word a sub-block of 32 values for IQ2_S, two for IQ3_S); sg: a word of sign bits
+// a sub-block; byte j of qh: sub-block j's high index bits; sc: scales, IQ2_S byte j = sub-block j's two, IQ3_S nibble j = sub-block j's.
 template<int T> struct IqFields {
-    uint32_t q[T == MAYA_IQ2_S ? 4 : 8], sg[4], qh, sc;
-    float d;
+    uint32_t q[T == MAYA_IQ2_S ? 8 : 16], sg[8], qh[2], sc[T == MAYA_IQ2_S ? 2 : 1], d2;     // d2: the block's scale, twice
 };
-template<int T, int OFF, int TEAM> __device__ __forceinline__ void iq_fields(const uint32_t* w, IqFields<T>& F) {
-    constexpr int a = 2 * TEAM, c = a + 4;
-    F.d = win_f16<OFF>(w);
-    F.qh = win_two16<OFF + 66 + a, OFF + 66 + c>(w);
-    if constexpr (T == MAYA_IQ2_S) {
-        F.q[0] = win_u32<OFF + 2 + 4 * a>(w); F.q[1] = win_u32<OFF + 6 + 4 * a>(w);
-        F.q[2] = win_u32<OFF + 2 + 4 * c>(w); F.q[3] = win_u32<OFF + 6 + 4 * c>(w);
-        F.sg[0] = win_u32<OFF + 34 + 4 * a>(w); F.sg[1] = win_u32<OFF + 38 + 4 * a>(w);
-        F.sg[2] = win_u32<OFF + 34 + 4 * c>(w); F.sg[3] = win_u32<OFF + 38 + 4 * c>(w);
-        F.sc = win_two16<OFF + 74 + a, OFF + 74 + c>(w);
-    } else {
-        F.q[0] = win_u32<OFF + 2 + 8 * a>(w); F.q[1] = win_u32<OFF + 6 + 8 * a>(w);
-        F.q[2] = win_u32<OFF + 10 + 8 * a>(w); F.q[3] = win_u32<OFF + 14 + 8 * a>(w);
-        F.q[4] = win_u32<OFF + 2 + 8 * c>(w); F.q[5] = win_u32<OFF + 6 + 8 * c>(w);
-        F.q[6] = win_u32<OFF + 10 + 8 * c>(w); F.q[7] = win_u32<OFF + 14 + 8 * c>(w);
-        F.sg[0] = win_u32<OFF + 74 + 4 * a>(w); F.sg[1] = win_u32<OFF + 78 + 4 * a>(w);
-        F.sg[2] = win_u32<OFF + 74 + 4 * c>(w); F.sg[3] = win_u32<OFF + 78 + 4 * c>(w);
-        // the block's four scale bytes lie side by side: pair TEAM's and pair TEAM + 2's
-        F.sc = __byte_perm(win_u32<OFF + 106>(w), 0, TEAM == 0 ? 0x4420 : 0x4431);
-    }
+template<int T, int OFF> __device__ __forceinline__ void iq_fields(const uint32_t* w, IqFields<T>& F) {
+    F.d2 = __byte_perm(w[OFF / 4], 0, OFF % 4 == 0 ? 0x1010 : 0x3232);
+    win_words<OFF + 2>(w, F.q, std::make_integer_sequence<int, T == MAYA_IQ2_S ? 8 : 16>{});
+    win_words<OFF + (T == MAYA_IQ2_S ? 34 : 74)>(w, F.sg, std::make_integer_sequence<int, 8>{});
+    win_words<OFF + 66>(w, F.qh, std::make_integer_sequence<int, 2>{});
+    win_words<OFF + (T == MAYA_IQ2_S ? 74 : 106)>(w, F.sc, std::make_integer_sequence<int, T == MAYA_IQ2_S ? 2 : 1>{});
 }
-// Sub-block J's codebook values, unsigned f16 pairs -> o[16].  `tab`: this lane's copy of the codebook.
-template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ2_S>& F, const uint4* tab, uint32_t* o) {
-    const uint32_t qh = byte_of(F.qh, J);
-    // byte l of hw = bits 2l, 2l + 1 of qh: an entry's index is one byte permute {qs byte l, hw byte l, 0, 0}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+// Sub-block J's codebook values, unsigned f16 pairs -> o[16].  tab: shared-memory address of this lane's copy of the codebook; f: the
+// entries' distance twice, as dp2a takes it (an index's 16 bits times the distance plus the base are one instruction).
+template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ2_S>& F, uint32_t tab, uint32_t f, uint32_t* o) {
+    const uint32_t qh = byte_of(F.qh[J / 4], J % 4);
+    // byte l of hw = bits 2l, 2l + 1 of qh: an entry's high index bits
     const uint32_t hw = ((qh & 0x33u) * 0x1001u + (qh & 0xCCu) * 0x40040u) & 0x03030303u;
+    const uint32_t p0 = prmt_raw(F.q[J], hw, 0x5140u), p1 = prmt_raw(F.q[J], hw, 0x7362u);      // the indices, two to a word
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-        const uint4 g = tab[prmt_raw(F.q[J], hw, 0xCC00u + ((4 + l) << 4) + l) * kCopies<MAYA_IQ2_S>];
+        const uint4 g = lds128((l & 1) ? dp2a_high(l < 2 ? p0 : p1, f, tab) : dp2a_low(l < 2 ? p0 : p1, f, tab));
         o[4 * l] = g.x; o[4 * l + 1] = g.y; o[4 * l + 2] = g.z; o[4 * l + 3] = g.w;
     }
 }
-template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ3_S>& F, const uint2* tab, uint32_t* o) {
-    const uint32_t qh = byte_of(F.qh, J);
+template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ3_S>& F, uint32_t tab, uint32_t f, uint32_t* o) {
+    const uint32_t qh = byte_of(F.qh[J / 4], J % 4);
     // byte l of h0 / h1 = bit l / 4 + l of qh, the ninth index bit of entry l / 4 + l
     const uint32_t h0 = ((qh & 15u) * 0x204081u) & 0x01010101u, h1 = ((qh >> 4) * 0x204081u) & 0x01010101u;
+    const uint32_t p[4] = {prmt_raw(F.q[2 * J], h0, 0x5140u), prmt_raw(F.q[2 * J], h0, 0x7362u), prmt_raw(F.q[2 * J + 1], h1, 0x5140u),
+                           prmt_raw(F.q[2 * J + 1], h1, 0x7362u)};
 #pragma unroll
     for (int l = 0; l < 8; ++l) {
-        const uint2 g = tab[prmt_raw(F.q[2 * J + l / 4], l < 4 ? h0 : h1, 0xCC00u + ((4 + l % 4) << 4) + l % 4) * kCopies<MAYA_IQ3_S>];
+        const uint2 g = lds64((l & 1) ? dp2a_high(p[l / 2], f, tab) : dp2a_low(p[l / 2], f, tab));
         o[2 * l] = g.x; o[2 * l + 1] = g.y;
     }
 }
@@ -294,20 +299,36 @@ __device__ __forceinline__ void iq_eight(uint32_t s, __half2 dl, uint32_t* r) {
     for (int p = 0; p < 4; ++p)
         r[p] = h2_bits(__hmul2(bits_h2(r[p]), dl)) ^ ((s * ((1u << (15 - 2 * p)) + (1u << (30 - 2 * p)))) & 0x80008000u);
 }
-// Sub-block J's values -> weights, in place.
-// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; dl = f16(d (2 ls + 1) / 8).
-template<int J> __device__ __forceinline__ void iq_finish(const IqFields<MAYA_IQ2_S>& F, uint32_t* o) {
-    const uint32_t sc = byte_of(F.sc, J);
-    const __half2 dl0 = __float2half2_rn(F.d * (float) (2 * (sc & 15) + 1) * 0.125f), dl1 = __float2half2_rn(F.d * (float) (2 * (sc >> 4) + 1) * 0.125f);
+// A byte's two scale nibbles (n0 low) -> (f16 scale times a (2 n0 + 1), and times a (2 n1 + 1)), a a power of two: the factors are exact
+// and each product is rounded once, as f16 of the f32 product is.
+template<int T> __device__ __forceinline__ __half2 iq_scales(uint32_t word, int byte, uint32_t d2) {
+    const uint32_t z = (__byte_perm(word, 0, byte | 0x40 | byte << 8 | 0x4000) & 0x00F0000Fu) | 0x64006400u;     // 1024 + n0, 1024 + 16 n1
+    const __half2 n = T == MAYA_IQ2_S ? __hfma2(bits_h2(z), __floats2half2_rn(0.25f, 0.015625f), __floats2half2_rn(-255.875f, -15.875f))
+                                      : __hfma2(bits_h2(z), __floats2half2_rn(2.0f, 0.125f), __floats2half2_rn(-2047.0f, -127.0f));
+    return __hmul2(bits_h2(d2), n);
+}
+// Sub-blocks J and J + 1 (J even): values -> weights, in place; `mid` runs when the first is done.
+// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; the factor is f16(d (2 ls + 1) / 8).
+template<int J, class Mid> __device__ __forceinline__ void iq_finish2(const IqFields<MAYA_IQ2_S>& F, uint32_t* o, Mid mid) {
 #pragma unroll
-    for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J], l), l < 2 ? dl0 : dl1, o + 4 * l);
+    for (int h = 0; h < 2; ++h) {
+        const __half2 dl = iq_scales<MAYA_IQ2_S>(F.sc[J / 4], (J + h) % 4, F.d2);
+        const __half2 dl0 = __low2half2(dl), dl1 = __high2half2(dl);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J + h], l), l < 2 ? dl0 : dl1, o + 16 * h + 4 * l);
+        if (h == 0) mid();
+    }
 }
 // IQ3_S (ggml dequantize_row_iq3_s): y = d (1 + 2 scale) * grid[qs | qh bit] * sign.
-template<int J> __device__ __forceinline__ void iq_finish(const IqFields<MAYA_IQ3_S>& F, uint32_t* o) {
-    const uint32_t nib = (F.sc >> (8 * (J / 2) + 4 * (J % 2))) & 15u;
-    const __half2 db = __float2half2_rn(F.d * (float) (1 + 2 * nib));
+template<int J, class Mid> __device__ __forceinline__ void iq_finish2(const IqFields<MAYA_IQ3_S>& F, uint32_t* o, Mid mid) {
+    const __half2 db = iq_scales<MAYA_IQ3_S>(F.sc[0], J / 2, F.d2);
 #pragma unroll
-    for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J], l), db, o + 4 * l);
+    for (int h = 0; h < 2; ++h) {
+        const __half2 dl = h == 0 ? __low2half2(db) : __high2half2(db);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J + h], l), dl, o + 16 * h + 4 * l);
+        if (h == 0) mid();
+    }
 }
 
 // A block works on tile after tile (see mmq_kernel): what the roles share of one of them.  e < 0: no tile left.
@@ -315,8 +336,29 @@ struct TileInfo { int e, row0, nrows, m0, lin; };     // lin: its place in the l
 constexpr int kTiles = 8;            // ring of tile entries: the raw-unit loader, which makes them, is at most kMaxUnits / 4 + 1
                                      // tiles ahead of the slowest reader (it waits for every unit to be read)
 
+// How a tile of `nrows` activation rows divides tensor memory and the activation ring.  Two accumulators of as many columns as
+// there are rows, in steps of 32; what is left of the 512 holds stages of expanded weights, 32 columns for each accumulator - three
+// beside 160 rows, seven beside 32: with three, the two teams of expanding warps waited for each other, since a team takes a block's
+// fields out of its window (400 to 600 cycles) while the other one's pairs need the stages in between.  An activation tile is a 128-row
+// box (and a 32-row box behind it), or just the latter.
+struct TileGeo {
+    uint32_t acc;                    // columns of an accumulator: accumulator 0 at 0, accumulator 1 at acc, the stages from 2 acc
+    int st, bst;                     // stages of expanded weights, of activations
+    uint32_t bbytes;                 // bytes of the latter
+};
+template<int T> __device__ __forceinline__ TileGeo tile_geo(int nrows) {
+    const int q = (max(nrows, 1) + 31) >> 5;
+    TileGeo g;
+    g.acc = 32u * (uint32_t) q;
+    g.st = kMaxSt + 1 - q;
+    g.bbytes = q == 1 ? 32 * 128 : q <= 4 ? kBBox : kBStage;
+    g.bst = q == 1 ? kMaxBSt : min(kMaxBSt, q <= 4 ? kBRing<T> / kBBox : kBRing<T> / kBStage);
+    return g;
+}
+static_assert(2 * TN + 64 * (kMaxSt + 1 - TN / 32) <= 512 && 64 + 64 * kMaxSt <= 512 && kMaxBSt * 32 * 128 <= kBRing<MAYA_Q8_0>, "tile_geo");
+
 struct Pipe {                       // static shared memory of a block
-    uint64_t a_full[kSt], b_full[6];
+    uint64_t a_full[kMaxSt], b_full[kMaxBSt];
     uint64_t done[kDone];            // done[p % kDone]: the products of K-step pair p (64 K-values) have completed
     uint64_t raw_full[kMaxUnits], raw_empty[kMaxUnits];
     uint64_t tile_full[kTiles];      // tile entry written
@@ -329,15 +371,17 @@ struct Pipe {                       // static shared memory of a block
 };
 
 __device__ __forceinline__ bool failed(const Pipe& P) { return *(volatile const int*) &P.fail != 0; }
-// Bounded wait; false when this wait ran out (the block's failure flag is then set) or another role has failed.
-// (try_wait with a suspend-time hint, so that the waiting single-lane roles poll less, changed nothing when only the
-// loaders used it and cost 0.7 % when the issuers and the expanding warps did.)
+// Bounded wait of a whole warp; false when it ran out (the block's failure flag is then set) or another role has failed.  The lanes
+// vote on every look - a look may find a barrier's phase ended for some of them and not yet for the others - so that they leave
+// together: what follows (tensor-memory stores, elected copies and products) needs the warp converged.
+// (try_wait with a suspend-time hint, so that the waiting roles poll less: 1 to 7 % slower, longest when all roles used it; four looks
+// between two counts of the loop 5 to 10 % slower.)
 __device__ __forceinline__ bool wait_or_fail(Pipe& P, uint64_t* bar, uint32_t parity) {
     for (unsigned i = 0; i < (1u << 21); ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
         if (i > 4096) {                          // try_wait itself suspends the thread for a while; back off only late
             __nanosleep(64);
-            if ((i & 255) == 0 && failed(P)) return false;
+            if ((i & 255) == 0 && __any_sync(0xFFFFFFFFu, failed(P))) return false;
         }
     }
     *(volatile int*) &P.fail = 1;
@@ -382,8 +426,8 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
            const __grid_constant__ CUtensorMap tm_x32, const MmqArgs A) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ Pipe P;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int NU = kUnits<T>, NB = kBStages<T>;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
+    constexpr int NU = kUnits<T>;
     const int nkt = A.w_cols / BK, nkb = A.w_cols / 256;
     // Q4_K: after every 8 blocks of K (32 pairs of K steps) one more pair carries the sum correction of those blocks' 64
     // groups - A = the groups' constant terms -dmin * m, B = the tail of the activation image (see xq_tail); the last pair
@@ -400,10 +444,10 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
 
     uint8_t* const raw = smem + kBRing<T>;
     if (tid == 0) {
-        for (int s = 0; s < kSt; ++s) mbar_init(&P.a_full[s], 8);
-        for (int s = 0; s < NB; ++s) mbar_init(&P.b_full[s], 1);
+        for (int s = 0; s < kMaxSt; ++s) mbar_init(&P.a_full[s], 8);
+        for (int s = 0; s < kMaxBSt; ++s) mbar_init(&P.b_full[s], 1);
         for (int s = 0; s < kDone; ++s) mbar_init(&P.done[s], 2);      // both issuers commit
-        for (int u = 0; u < NU; ++u) { mbar_init(&P.raw_full[u], 1); mbar_init(&P.raw_empty[u], 4); }
+        for (int u = 0; u < NU; ++u) { mbar_init(&P.raw_full[u], 1); mbar_init(&P.raw_empty[u], kIq<T> ? 2 : 4); }
         for (int i = 0; i < kTiles; ++i) mbar_init(&P.tile_full[i], 1);
         mbar_init(&P.final, 2);
         mbar_init(&P.acc_free, kDqWarps);
@@ -452,50 +496,67 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         const int slab = row >> 6;
         const uint8_t* const rbase = raw + (size_t) (row & 63) * kRawRow<T>;
         // rows 0..127 feed accumulator 0, rows 128..255 accumulator 1; a warp reaches the 32 lanes of its quadrant
-        const uint32_t a_lane = tmem + ((uint32_t) (32 * (w8 & 3)) << 16) + kACol + (w8 >> 2) * 32;
-        // the stage of pair kp (counted over the block's tiles) is free: it was last read by pair kp - kSt
-        auto acquire = [&](int kp) -> bool {
-            if (kp >= kSt) {
-                const int pp = kp - kSt;
-                if (!wait_or_fail(P, &P.done[pp & (kDone - 1)], (pp / kDone) & 1)) return false;
-                tc_fence_after();
+        const uint32_t a_lane = tmem + ((uint32_t) (32 * (w8 & 3)) << 16) + (w8 >> 2) * 32;
+        const uint32_t afull0 = smem_u32(&P.a_full[0]), done0 = smem_u32(&P.done[0]);
+        // The team's next pair of the tile, its stage and that stage's place in tensor memory.  (A tile's stages start at 0: every product
+        // of the tile before it has completed.)
+        int seq = 0, st = 0, n_st = 0, kp0 = 0;          // kp0: pairs of the tiles before this one
+        uint32_t a_at = 0;
+        auto ahead = [&](int d) {                        // d <= 3
+            seq += d;
+            st += d;
+            if (st >= n_st) st -= n_st;
+        };
+        // The stage is free when pair seq - n_st, which read it last, has completed.  look(): whether it is, asked before the expansion so
+        // that the answer is there behind it; acquire(): now (the warp is then converged, as the stores need it).
+        auto look = [&]() -> bool {
+            if (seq < n_st) return true;
+            const unsigned pp = (unsigned) (kp0 + seq - n_st);
+            return mbar_test_wait_addr(done0 + 8 * (pp & (kDone - 1)), (pp / kDone) & 1u);
+        };
+        auto acquire = [&](bool seen) -> bool {
+            if (!__all_sync(0xFFFFFFFFu, seen)) {
+                const unsigned pp = (unsigned) (kp0 + seq - n_st);
+                if (!wait_or_fail(P, &P.done[pp & (kDone - 1)], (pp / kDone) & 1u)) return false;
             }
+            tc_fence_after();
+            __syncwarp();
             return true;
         };
-        auto release = [&](int kp) {
+        auto release = [&] {
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&P.a_full[kp % kSt]);
+            if (lane == 0) mbar_arrive_addr(afull0 + 8 * st);
         };
-        auto put = [&](int kp, const uint32_t (&o)[32]) -> bool {   // the row's 64 values of pair kp -> its lane
-            if (!acquire(kp)) return false;
-            tmem_st32(a_lane + (kp % kSt) * 64, o);
-            release(kp);
-            return true;
-        };
-        // i-quants: this lane's copy of the codebook
-        using Entry = std::conditional_t<T == MAYA_IQ2_S, uint4, uint2>;
-        [[maybe_unused]] const Entry* const tab = (const Entry*) (smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) : 0);
+        // i-quants: this lane's copy of the codebook, and the entries' distance
+        constexpr uint32_t kEnt = kIq<T> ? kCopies<T> * (T == MAYA_IQ2_S ? 16 : 8) : 0;
+        [[maybe_unused]] const uint32_t tab = smem_u32(smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) * (T == MAYA_IQ2_S ? 16 : 8) : 0);
+        [[maybe_unused]] const uint32_t tab_f = kEnt | kEnt << 24;
         [[maybe_unused]] uint4 corr[8];      // Q4_K: the constant terms of the current 8-block chunk (indexed by kb: local memory)
         // A pair's two halves of 32 K-values: the first half's tensor-memory store is under way while the second half is
         // expanded (the store, its wait and the hand-off were a serial tail of every pair).
-        auto st_half = [&](int kp, int h, const uint32_t* o16) {
-            tmem_st16(a_lane + (kp % kSt) * 64 + 16 * h, *(const uint32_t(*)[16]) o16);
-        };
-        int kp0 = 0, u0 = 0;                 // pairs and raw units of the tiles before this one
-        for (int t = 0;; ++t, kp0 += npairs, u0 += 4 * nkb) {
+        auto st_half = [&](int h, const uint32_t* o16) { tmem_st16(a_at + 64 * st + 16 * h, *(const uint32_t(*)[16]) o16); };
+        // the raw unit of this warp's rows in the next block it expands, and its barrier's phase
+        int slot = slab + (kIq<T> ? 4 * team : 0);
+        uint32_t raw_phase = 0;
+        for (int t = 0;; ++t, kp0 += npairs) {
         TileInfo ti;
         bool ok = tile_of(t, ti);
         if (named_bar_or(3, kDqWarps * 32, !ok) || ti.e < 0) break;      // the same for every expanding warp
         const int nrows = ti.nrows, row0 = ti.row0, m0 = ti.m0;
+        const TileGeo geo = tile_geo<T>(nrows);
+        seq = st = team;
+        n_st = geo.st;
+        a_at = a_lane + 2 * geo.acc;
 #ifdef MAYA_MMQ_STAMPS
         long long* const stamps = tid == 0 && ok ? stamps_of(ti.lin) : nullptr;
         if (stamps) { stamps[0] = clock64(); stamps[14] = nrows; stamps[15] = npairs; }
 #endif
-        for (int kb = 0; kb < nkb && ok; ++kb) {
-            const int u = u0 + kb * 4 + slab, slot = u % NU;
-            if (!wait_or_fail(P, &P.raw_full[slot], (u / NU) & 1)) { ok = false; break; }
+        // i-quants: a team expands every other block whole - its fields are taken out of the window once - and the pairs of a block
+        // and the next one's alternate (see pair_block).  The other types: both teams work on a block, on alternate pairs.
+        for (int kb = kIq<T> ? team : 0; kb < nkb && ok; kb += kIq<T> ? 2 : 1) {
+            if (!wait_or_fail(P, &P.raw_full[slot], raw_phase)) { ok = false; break; }
             const uint8_t* rrow = rbase + (size_t) slot * kUnitBytes<T>;
             uint32_t o[32];
             if constexpr (kIq<T>) {
@@ -507,26 +568,43 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     wv[4 * i] = v.x; wv[4 * i + 1] = v.y; wv[4 * i + 2] = v.z; wv[4 * i + 3] = v.w;
                 }
                 IqFields<T> F;
-#define MAYA_IQ_FIELDS(OFF) case OFF: if (team == 0) iq_fields<T, OFF, 0>(wv, F); else iq_fields<T, OFF, 1>(wv, F); break;
-                switch ((kb * kBlkBytes<T>) & 15) {      // where the block starts in its window: period 8 in kb
-                    MAYA_IQ_FIELDS(0) MAYA_IQ_FIELDS(2) MAYA_IQ_FIELDS(4) MAYA_IQ_FIELDS(6)
-                    MAYA_IQ_FIELDS(8) MAYA_IQ_FIELDS(10) MAYA_IQ_FIELDS(12)
-                    default: if (team == 0) iq_fields<T, 14, 0>(wv, F); else iq_fields<T, 14, 1>(wv, F); break;
+                // where the block starts in its window: period 8 in kb, a multiple of 4 for every other block
+                switch ((kb * kBlkBytes<T>) & 15) {
+                    case 0: iq_fields<T, 0>(wv, F); break;
+                    case 2: iq_fields<T, 2>(wv, F); break;
+                    case 4: iq_fields<T, 4>(wv, F); break;
+                    case 6: iq_fields<T, 6>(wv, F); break;
+                    case 8: iq_fields<T, 8>(wv, F); break;
+                    case 10: iq_fields<T, 10>(wv, F); break;
+                    case 12: iq_fields<T, 12>(wv, F); break;
+                    default: iq_fields<T, 14>(wv, F);
                 }
-#undef MAYA_IQ_FIELDS
-                auto pair = [&](auto i, int kp) {        // both sub-blocks' look-ups are under way before the first is finished
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&P.raw_empty[slot]);      // its two warps have read the unit
+                // Both sub-blocks' look-ups are under way before the first is finished, and the next pair's before this one's stores
+                // are waited for.
+                iq_lookup<0>(F, tab, tab_f, o);
+                iq_lookup<1>(F, tab, tab_f, o + 16);
+                auto pair = [&](auto i) {
                     constexpr int J = 2 * decltype(i)::value;
-                    iq_lookup<J>(F, tab, o);
-                    iq_lookup<J + 1>(F, tab, o + 16);
-                    iq_finish<J>(F, o);
-                    if (!acquire(kp)) return false;
-                    st_half(kp, 0, o);
-                    iq_finish<J + 1>(F, o + 16);
-                    st_half(kp, 1, o + 16);
-                    release(kp);
+                    const bool seen = look();
+                    bool got = true;
+                    iq_finish2<J>(F, o, [&] {
+                        got = acquire(seen);
+                        if (got) st_half(0, o);
+                    });
+                    if (!got) return false;
+                    st_half(1, o + 16);
+                    if constexpr (J < 6) {
+                        iq_lookup<J + 2>(F, tab, tab_f, o);
+                        iq_lookup<J + 3>(F, tab, tab_f, o + 16);
+                    }
+                    release();
+                    ahead(2);
                     return true;
                 };
-                ok = pair(std::integral_constant<int, 0>{}, kp0 + kb * 4 + team) && pair(std::integral_constant<int, 1>{}, kp0 + kb * 4 + team + 2);
+                ok = pair(std::integral_constant<int, 0>{}) && pair(std::integral_constant<int, 1>{}) && pair(std::integral_constant<int, 2>{}) &&
+                     pair(std::integral_constant<int, 3>{});
             } else if constexpr (T == MAYA_Q4_K) {
                 Q4Scales S;
                 q4k_scales(*(const uint4*) rrow, S);
@@ -538,32 +616,48 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 for (int i = 0; i < 2; ++i) {        // the 64 values of quant pair p: low nibbles, then high nibbles
                     const int p = 2 * i + team;
                     const uint4 qa = *(const uint4*) (rrow + 16 + 32 * p), qb = *(const uint4*) (rrow + 32 + 32 * p);
-                    const int kp = kp0 + kb * 4 + chunk + p, sb0 = 4 * i + 2 * team;
+                    const int sb0 = 4 * i + 2 * team;
+                    const bool seen = look();
                     q4k_stage(qa, qb, 0, S.dl[sb0], S.nml[sb0], o);
-                    if (!acquire(kp)) { ok = false; break; }
-                    st_half(kp, 0, o);
+                    if (!acquire(seen)) { ok = false; break; }
+                    st_half(0, o);
                     q4k_stage(qa, qb, 1, S.dl[sb0 + 1], S.nml[sb0 + 1], o + 16);
-                    st_half(kp, 1, o + 16);
-                    release(kp);
+                    st_half(1, o + 16);
+                    release();
+                    if (i == 0) ahead(2);
                 }
-                if (ok && (chunk & 1) == team && ((kb & 7) == 7 || kb == nkb - 1)) {      // the chunk's correction pair
+                // the chunk's correction pair stands behind its last pair, team 1's
+                const bool last = (kb & 7) == 7 || kb == nkb - 1;
+                if (!last) {
+                    ahead(2);
+                } else if (ok && (chunk & 1) == team) {
+                    ahead(2 - team);
 #pragma unroll
                     for (int b = 0; b < 8; ++b) {
                         const uint4 c = b <= (kb & 7) ? corr[b] : make_uint4(0u, 0u, 0u, 0u);
                         o[4 * b] = c.x; o[4 * b + 1] = c.y; o[4 * b + 2] = c.z; o[4 * b + 3] = c.w;
                     }
-                    ok = put(kp0 + kb * 4 + chunk + 4, o);
+                    ok = acquire(look());
+                    if (ok) {
+                        tmem_st32(a_at + 64 * st, o);
+                        release();
+                    }
+                    ahead(1 + team);
+                } else {
+                    ahead(3);
                 }
             } else {
 #define MAYA_Q80_PAIR(PP)                                                                      \
     if (ok) {                                                                                  \
+        const bool seen = look();                                                              \
         q80_stage<2 * (PP)>(rrow, o);                                                          \
-        ok = acquire(kp0 + kb * 4 + (PP));                                                           \
+        ok = acquire(seen);                                                                    \
         if (ok) {                                                                              \
-            st_half(kp0 + kb * 4 + (PP), 0, o);                                                      \
+            st_half(0, o);                                                                     \
             q80_stage<2 * (PP) + 1>(rrow, o + 16);                                             \
-            st_half(kp0 + kb * 4 + (PP), 1, o + 16);                                                 \
-            release(kp0 + kb * 4 + (PP));                                                            \
+            st_half(1, o + 16);                                                                \
+            release();                                                                         \
+            ahead(2);                                                                          \
         }                                                                                      \
     }
                 if (team == 0) { MAYA_Q80_PAIR(0) MAYA_Q80_PAIR(2) }
@@ -571,8 +665,12 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
 #undef MAYA_Q80_PAIR
             }
             if (!ok) break;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&P.raw_empty[slot]);      // 4 warps read a unit; after the 4th it may be overwritten
+            if constexpr (!kIq<T>) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&P.raw_empty[slot]);      // 4 warps read a unit; after the 4th it may be overwritten
+            }
+            slot += kIq<T> ? 8 : 4;
+            if (slot >= NU) { slot -= NU; raw_phase ^= 1u; }
         }
         // ------------------------------------------------------------ write-back
         if (ok && !wait_or_fail(P, &P.final, t & 1)) ok = false;
@@ -610,7 +708,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     const int col0 = 8 * c;
                     float v[8], up[8];
                     tmem_ld8(lane_base + col0, v);
-                    tmem_ld8(lane_base + kAccCols + col0, up);
+                    tmem_ld8(lane_base + geo.acc + col0, up);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         if (col0 + j < nrows) b32[(col0 + j) * 128 + mcol] = swiglu(v[j], up[j], A.limit);   // uniform in the warp
@@ -664,7 +762,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                     for (int c = grp; c < nchunk; c += 2) {
                         const int col0 = 16 * c;
                         float v[16];
-                        tmem_ld16(lane_base + acc * kAccCols + col0, v);
+                        tmem_ld16(lane_base + acc * geo.acc + col0, v);
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
                             if (col0 + j < nrows) buf[(col0 + j) * TM + mcol] = v[j];
@@ -689,13 +787,15 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
 #endif
         }
     } else if (warp == kDqWarps) {
-        // ------------------------------------------------------------ the tile list, and raw weight units (one lane)
-        int u0 = 0, prev_rows = 0;           // raw units of the tiles before this one; rows of the tile before this one
+        // ------------------------------------------------------------ the tile list, and raw weight units (one warp)
+        const uint32_t raw0 = smem_u32(raw), rawfull0 = smem_u32(&P.raw_full[0]);
+        int slot = 0, prev_rows = 0;         // the next raw unit's place; rows of the tile before this one
+        uint32_t raw_phase = 1;              // of the barrier that says the place is free: at once the first time round
         // In a chain the tiles are taken as blocks get to them (blocks of the next product start where this one's have run out of
         // tiles), a tile ahead of its use; else block b's are b, b + grid, ...
         int claimed = (int) blockIdx.x;
         if (A.claim != nullptr && lane == 0) claimed = (int) atomicAdd(A.claim, 1u);
-        for (int t = 0;; ++t, u0 += 4 * nkb) {
+        for (int t = 0;; ++t) {
             // Which (matrix, 160-row group) is this tile's: the warp scans the per-matrix group counts - each lane the counts
             // of a run of consecutive matrices, an exclusive warp scan of the runs' sums, then the lane whose run holds the
             // wanted group walks it - 1024 matrices a round.
@@ -739,37 +839,36 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             }
             const int m0 = (lin % nslab) * kSlab;
             bool ok = true;
-            if (lane == 0) {
+            {
                 claimed = lin + (int) gridDim.x;
-                if (A.claim != nullptr && found_e >= 0) claimed = (int) atomicAdd(A.claim, 1u);
+                if (A.claim != nullptr && found_e >= 0 && lane == 0) claimed = (int) atomicAdd(A.claim, 1u);
                 // Entry t % kTiles was read by every role before tile t - kTiles ended.  The write-back of the tile two before
                 // this one has to be over in any case (so that a barrier's phase is never two behind), that of the tile before
                 // only where it stretches into the raw ring.
                 if (t >= 2) ok = wait_or_fail(P, &P.stg_free[t & 1], ((t - 2) >> 1) & 1);
-                P.tile[t % kTiles] = TileInfo{found_e, row0, nrows, m0, lin};
-                mbar_arrive(&P.tile_full[t % kTiles]);
+                if (lane == 0) {
+                    P.tile[t % kTiles] = TileInfo{found_e, row0, nrows, m0, lin};
+                    mbar_arrive(&P.tile_full[t % kTiles]);
+                }
+                __syncwarp();
                 if (found_e >= 0) {
                     if (ok && t >= 1 && staging_bytes<GLU>(prev_rows) > kBRing<T>)
                         ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
-                    int issued = u0;
                     for (int kb = 0; kb < nkb && ok; ++kb) {
                         for (int sl = 0; sl < 4; ++sl) {
-                            const int u = u0 + kb * 4 + sl, slot = u % NU;
-                            if (u >= NU && !wait_or_fail(P, &P.raw_empty[slot], ((u / NU) - 1) & 1)) { ok = false; break; }
+                            if (!wait_or_fail(P, &P.raw_empty[slot], raw_phase)) { ok = false; break; }
                             const int wrow = GLU ? (sl < 2 ? m0 + 64 * sl : A.w_rows + m0 + 64 * (sl - 2)) : m0 + 64 * sl;
-                            mbar_expect_tx(&P.raw_full[slot], kUnitBytes<T>);
                             // x: the block's 32-bit words (k-quants), or the 16-byte aligned byte offset of the window around the
                             // i-quant block (the box is then 112 / 144 bytes of each row; past the row's end it reads as zeros)
                             const int x0 = kIq<T> ? (int) (((size_t) kb * kBlkBytes<T>) & ~(size_t) 15) : kb * (kRawRow<T> / 4);
-                            tma_load_3d(raw + (size_t) slot * kUnitBytes<T>, &tm_w, &P.raw_full[slot], x0, wrow, found_e);
-                            issued = u + 1;
+                            tma_expect_load_3d(raw0 + slot * kUnitBytes<T>, &tm_w, rawfull0 + 8 * slot, kUnitBytes<T>, x0, wrow, found_e);
+                            if (++slot == NU) { slot = 0; raw_phase ^= 1u; }
                         }
                     }
-                    if (!ok)                                     // let the copies in flight land before the block ends
-                        for (int u = max(0, issued - NU); u < issued; ++u) wait_or_fail(P, &P.raw_full[u % NU], (u / NU) & 1);
+                    if (!ok)                                     // let the copies in flight land before the block ends: a place's last one
+                        for (int i = 0; i < NU; ++i) wait_or_fail(P, &P.raw_full[i], i < slot ? raw_phase ^ 1u : raw_phase);
                 }
             }
-            ok = __shfl_sync(0xFFFFFFFFu, ok ? 1 : 0, 0) != 0;
             if (!ok || found_e < 0) break;
             prev_rows = nrows;
         }
@@ -788,30 +887,31 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         const int my = warp == kDqWarps + 1 ? 0 : 1;
         const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
         const uint64_t bdesc0 = smem_desc_sw128(smem_u32(smem));
-        const uint32_t b_hi = (uint32_t) (bdesc0 >> 32), b_lo0 = (uint32_t) bdesc0, b_lo_end = b_lo0 + NB * (kBStage >> 4);
-        const uint32_t a0 = tm + kACol + my * 32, a_end = a0 + kSt * 64, d0 = tm + my * kAccCols;
+        const uint32_t b_hi = (uint32_t) (bdesc0 >> 32), b_lo0 = (uint32_t) bdesc0;
         const uint32_t bfull0 = smem_u32(&P.b_full[0]), afull0 = smem_u32(&P.a_full[0]), done0 = smem_u32(&P.done[0]);
-        uint32_t b_lo = b_lo0, at = a0, bfull = bfull0, afull = afull0;   // of the next pair of K steps
-        uint32_t ph_a = 0, ph_b = 0, done_at = 0;    // the barriers' phases; the next pair's place in the ring of done barriers
+        uint32_t ph_a = 0, ph_b = 0, done_at = 0;    // the barriers' phases, a bit each; the next pair's place in the ring of done barriers
         for (int t = 0;; ++t) {
             TileInfo ti;
             bool ok = tile_of(t, ti);
-            if (!__all_sync(0xFFFFFFFFu, ok)) break;
+            if (!ok) break;
             const int n_rows = __shfl_sync(0xFFFFFFFFu, ti.nrows, 0);
             if (__shfl_sync(0xFFFFFFFFu, ti.e, 0) < 0) break;
             if (t > 0) {                             // the accumulators still hold the tile before until its write-back has read them
                 ok = wait_or_fail(P, &P.acc_free, (t - 1) & 1);
-                if (!__all_sync(0xFFFFFFFFu, ok)) break;
+                if (!ok) break;
                 tc_fence_after();
             }
             const int n_mma = max(16, (n_rows + 15) & ~15);
             const uint32_t idesc = (1u << 4) | ((uint32_t) (n_mma >> 3) << 17) | ((uint32_t) (128 >> 4) << 24);
+            const TileGeo geo = tile_geo<T>(n_rows);
+            const uint32_t a0 = tm + 2 * geo.acc + my * 32, d0 = tm + my * geo.acc, b_step = geo.bbytes >> 4;
             uint32_t first = 0;                      // 0: the first product overwrites
+            uint32_t b_lo = b_lo0, at = a0, sa = 0, sb = 0;       // the next pair's place in the activation ring and in tensor memory, its stages
             for (int kp = 0; kp < npairs; ++kp) {
-                const bool rb = mbar_test_wait_addr(bfull, ph_b), ra = mbar_test_wait_addr(afull, ph_a);
+                const uint32_t pa = (ph_a >> sa) & 1u, pb = (ph_b >> sb) & 1u;
+                const bool rb = mbar_test_wait_addr(bfull0 + 8 * sb, pb), ra = mbar_test_wait_addr(afull0 + 8 * sa, pa);
                 if (!__all_sync(0xFFFFFFFFu, rb && ra)) {        // not there yet: the bounded waits
-                    const bool got = wait_or_fail(P, &P.b_full[(bfull - bfull0) >> 3], ph_b) && wait_or_fail(P, &P.a_full[(afull - afull0) >> 3], ph_a);
-                    if (!__all_sync(0xFFFFFFFFu, got)) { ok = false; break; }
+                    if (!wait_or_fail(P, &P.b_full[sb], pb) || !wait_or_fail(P, &P.a_full[sa], pa)) { ok = false; break; }
                 }
                 tc_fence_after();
 #ifdef MAYA_MMQ_STAMPS
@@ -820,10 +920,12 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 mma_f16_ts_x4_commit(d0, at, b_lo, b_hi, idesc, first, done0 + done_at);
                 first = 1;
                 done_at = (done_at + 8) & (8 * kDone - 1);
-                at += 64; afull += 8;
-                if (at == a_end) { at = a0; afull = afull0; ph_a ^= 1; }
-                b_lo += kBStage >> 4; bfull += 8;
-                if (b_lo == b_lo_end) { b_lo = b_lo0; bfull = bfull0; ph_b ^= 1; }
+                ph_a ^= 1u << sa;
+                ph_b ^= 1u << sb;
+                at += 64;
+                if (++sa == (uint32_t) geo.st) { sa = 0; at = a0; }
+                b_lo += b_step;
+                if (++sb == (uint32_t) geo.bst) { sb = 0; b_lo = b_lo0; }
             }
 #ifdef MAYA_MMQ_STAMPS
             if (my == 0 && lane == 0 && stamps_of(ti.lin)) stamps_of(ti.lin)[3] = clock64();                      // the last product issued
@@ -832,62 +934,68 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             mma_commit_elect(smem_u32(&P.final));
         }
     } else if (warp == kDqWarps + 2) {
-        // ------------------------------------------------------------ activation tiles (one lane)
-        if (lane == 0) {
-            const int nmain = nkt / 2;
-            int p0 = 0, issued = 0;                  // pairs of the tiles before this one; tiles of activations asked for
-            bool ok = true;
-            unsigned* counter = nullptr;             // gate/up in a chain: the counter of the tile before's rows, not counted yet
-            unsigned written = 0;
-            auto count_rows = [&] {
-                if (counter != nullptr) red_release(counter, written);
-                counter = nullptr;
-            };
-            for (int t = 0;; ++t, p0 += npairs) {
-                TileInfo ti;
-                ok = tile_of(t, ti);
-                // the write-back of the tile before uses the activation ring
-                if (ok && t > 0) ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
-                if (!ok || ti.e < 0) {
-                    if (ok) count_rows();
-                    break;
-                }
-                if (!GLU && A.ready != nullptr) {
-                    unsigned* const r = A.ready + 2 * (ti.lin / nslab);
-                    ok = wait_rows(P, r, (unsigned) (ti.nrows * A.ready_slabs));
-                    if (!ok) break;
-                    if (atomicAdd(r + 1, 1u) == (unsigned) nslab - 1u) { r[0] = 0u; r[1] = 0u; }     // the group's last tile to wait
-                }
-                const bool big = ti.nrows > 128;     // the activation tile is a 128-row box and a 32-row box
-                const uint32_t tx_bytes = big ? kBStage : kBBox;
-                for (int kb2 = 0; kb2 < npairs && ok; ++kb2) {
-                    const int pg = p0 + kb2, sb = pg % NB;
-                    // the pair's 64 K-values in the image: K values in order, and after every 32 pairs (or at the end) the
-                    // chunk's 64 corrections from the tail behind the row's K values
-                    int xcol;
-                    if (ntp == 0) xcol = kb2 * 64;
-                    else {
-                        const int c = kb2 / 33, r = kb2 - c * 33;
-                        const bool is_corr = r == 32 || kb2 == nmain + ntp - 1;
-                        xcol = is_corr ? A.w_cols + 64 * c : (kb2 - c) * 64;
-                    }
-                    if (pg >= NB) {                          // the slot was last read by pair pg - NB
-                        const int pp = pg - NB;
-                        if (!wait_or_fail(P, &P.done[pp % kDone], (pp / kDone) & 1)) { ok = false; break; }
-                    }
-                    uint8_t* bt = smem + (size_t) sb * kBStage;
-                    mbar_expect_tx(&P.b_full[sb], tx_bytes);
-                    tma_load_2d(bt, &tm_x, &P.b_full[sb], xcol, ti.row0);
-                    if (big) tma_load_2d(bt + kBBox, &tm_x32, &P.b_full[sb], xcol, ti.row0 + 128);
-                    issued = pg + 1;
-                    if (kb2 == min(NB, npairs) - 1) count_rows();        // behind the loads the expansion waits for
-                }
-                if (!ok) break;
-                if (GLU && A.ready != nullptr) { counter = A.ready + 2 * (ti.lin / nslab); written = (unsigned) ti.nrows; }
+        // ------------------------------------------------------------ activation tiles (one warp)
+        const int nmain = nkt / 2;
+        const uint32_t ring0 = smem_u32(smem), bfull0 = smem_u32(&P.b_full[0]);
+        int p0 = 0;                                  // pairs of the tiles before this one
+        uint32_t phases = 0;                         // a bit a place of the ring: the phase its next load ends
+        bool ok = true;
+        unsigned* counter = nullptr;                 // gate/up in a chain: the counter of the tile before's rows, not counted yet
+        unsigned written = 0;
+        auto count_rows = [&] {
+            if (counter != nullptr && lane == 0) red_release(counter, written);
+            counter = nullptr;
+            __syncwarp();
+        };
+        for (int t = 0;; ++t, p0 += npairs) {
+            TileInfo ti;
+            ok = tile_of(t, ti);
+            // the write-back of the tile before uses the activation ring
+            if (ok && t > 0) ok = wait_or_fail(P, &P.stg_free[(t - 1) & 1], ((t - 1) >> 1) & 1);
+            const int e = __shfl_sync(0xFFFFFFFFu, ti.e, 0), nrows = __shfl_sync(0xFFFFFFFFu, ti.nrows, 0);
+            const int row0 = __shfl_sync(0xFFFFFFFFu, ti.row0, 0), lin = __shfl_sync(0xFFFFFFFFu, ti.lin, 0);
+            if (!ok || e < 0) {
+                if (ok) count_rows();
+                break;
             }
-            if (!ok)                                         // let the copies in flight land before the block ends
-                for (int pg = max(0, issued - NB); pg < issued; ++pg) wait_or_fail(P, &P.b_full[pg % NB], (pg / NB) & 1);
+            if (!GLU && A.ready != nullptr) {
+                unsigned* const r = A.ready + 2 * (lin / nslab);
+                ok = __all_sync(0xFFFFFFFFu, wait_rows(P, r, (unsigned) (nrows * A.ready_slabs)));
+                if (!ok) break;
+                if (lane == 0 && atomicAdd(r + 1, 1u) == (unsigned) nslab - 1u) { r[0] = 0u; r[1] = 0u; }      // the group's last tile to wait
+                __syncwarp();
+            }
+            const TileGeo geo = tile_geo<T>(nrows);
+            int sb = 0;
+            for (int kb2 = 0; kb2 < npairs; ++kb2) {
+                // the pair's 64 K-values in the image: K values in order, and after every 32 pairs (or at the end) the
+                // chunk's 64 corrections from the tail behind the row's K values
+                int xcol;
+                if constexpr (kIq<T>) {
+                    xcol = ((kb2 >> 3) * 2 + (kb2 & 1)) * 256 + ((kb2 >> 1) & 3) * 64;
+                } else if (ntp == 0) {
+                    xcol = kb2 * 64;
+                } else {
+                    const int c = kb2 / 33, r = kb2 - c * 33;
+                    const bool is_corr = r == 32 || kb2 == nmain + ntp - 1;
+                    xcol = is_corr ? A.w_cols + 64 * c : (kb2 - c) * 64;
+                }
+                if (kb2 >= geo.bst) {                // the place was last read by pair kb2 - bst
+                    const unsigned pp = (unsigned) (p0 + kb2 - geo.bst);
+                    if (!wait_or_fail(P, &P.done[pp % kDone], (pp / kDone) & 1u)) { ok = false; break; }
+                }
+                const uint32_t dst = ring0 + (uint32_t) sb * geo.bbytes, bar = bfull0 + 8 * sb;
+                tma_expect_load_2d(dst, geo.bbytes < kBBox ? &tm_x32 : &tm_x, bar, geo.bbytes, xcol, row0);
+                if (geo.bbytes > kBBox) tma_load_2d_elect(dst + kBBox, &tm_x32, bar, xcol, row0 + 128);
+                phases ^= 1u << sb;
+                if (++sb == geo.bst) sb = 0;
+                if (kb2 == min(geo.bst, npairs) - 1) count_rows();       // behind the loads the expansion waits for
+            }
+            if (!ok) break;
+            if (GLU && A.ready != nullptr) { counter = A.ready + 2 * (lin / nslab); written = (unsigned) nrows; }
         }
+        if (!ok)                                     // let the copies in flight land before the block ends: a place's last one
+            for (int i = 0; i < kMaxBSt; ++i) wait_or_fail(P, &P.b_full[i], ((phases >> i) & 1u) ^ 1u);
     }
     tc_fence_before();
     __syncthreads();

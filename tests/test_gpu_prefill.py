@@ -257,6 +257,33 @@ def test_tall_groups_equal_short_groups_bitwise(T, api, t, rows):
     assert T.equal(got[:, half:], run(image[:, half:].contiguous(), rows - half))
 
 
+@pytest.mark.parametrize("t,cols", [(H.Q4_K, 256), (H.Q4_K, 1792), (H.Q4_K, 2304), (H.Q8_0, 256), (H.Q8_0, 768), (H.IQ2_S, 4096), (H.IQ3_S, 2048)])
+def test_tiles_of_every_height_one_after_another_bitwise(T, api, t, cols):
+    """A tile's rows decide how tensor memory and the activation ring are divided.  Blocks that take tiles of every division in turn
+    (heights at both edges of each, more tiles than SMs; K of less than a ring, and Q4_K chunks of 1, 7 and 8 + 1 blocks): the bits of
+    the same rows in groups of at most 16, which all have one division."""
+    w_rows, heights = 512, [1, 160, 33, 32, 129, 64, 97, 65, 128, 96, 16, 17] * 8
+    w1 = synth_matrices(T, api, t, 4, w_rows, cols, 61)
+    w = w1[T.arange(len(heights), device="cuda") % 4].contiguous()
+    total = sum(heights)
+    xq = api.mmq_quantize(dev(T, H.rng_for("heights", t, cols).standard_normal((total, cols)).astype(np.float32)), None, t)
+
+    def run(mats, counts):
+        out = T.full((total, w_rows), 7.0, dtype=T.float32, device="cuda")
+        err = T.zeros(1, dtype=T.int32, device="cuda")
+        bounds = dev(T, np.concatenate([[0], np.cumsum(counts)]).astype(np.int32))
+        api.mmq_run(api.mmq_product(mats, t, w_rows, cols, mats.shape[1], len(counts), xq, bounds, None, total, out, w_rows, error=err))
+        T.cuda.synchronize()
+        assert int(err.item()) == 0
+        return out
+
+    short = [(g % 4, min(16, h - at)) for g, h in enumerate(heights) for at in range(0, h, 16)]
+    want = run(w1[T.tensor([e for e, _ in short], device="cuda")].contiguous(), [n for _, n in short])
+    got = run(w, heights)
+    assert T.isfinite(got).all() and float(got.abs().max()) > 0.1
+    assert T.equal(got, want)
+
+
 @pytest.mark.parametrize("ta,tb,counts,n_ff", [
     (H.Q8_0, H.Q4_K, [1, 0, 161, 7, 320, 33], 256),                                       # fewer tiles than blocks, remainders of 160 rows
     (H.IQ2_S, H.IQ3_S, [5] * 24 + [0] * 3 + [170] * 3, 2048),                             # several rounds of tiles
