@@ -73,7 +73,7 @@ template<int T, int SPLIT = 1> struct WGeo : RowGeo<T> {
 using WShGeo = WGeo<MAYA_Q8_0, 2>;           // the shared expert's rows: a stage no larger than the 2-bit types'
 
 // what differs between the routed experts' jobs and the shared one's
-struct WKind { int n_in, nunit, nseg, bytes, pitch, split; size_t rb, up, off; };
+struct WKind { int n_in, nunit, nseg, bytes, pitch; size_t rb, up, off; };
 struct WJob { unsigned long long ptr; int e0, nc, shared, per; };     // per: cost of one unit
 struct WShared {
     uint64_t full[16][kWStages];
@@ -181,7 +181,6 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             k.nunit = UP ? ff / 32 : A.n_embd / RW;
             k.nseg = warp ? (k.n_in + GS::vals - 1) / GS::vals : (k.n_in + G::vals - 1) / G::vals;
             k.bytes = warp ? GS::bytes : G::bytes;
-            k.split = warp ? GS::split : 1;
             k.pitch = warp ? GS::pitch : G::pitch;
             k.rb = row_bytes(warp ? (int) MAYA_Q8_0 : T, k.n_in);
             k.up = warp ? (size_t) A.n_ff_sh * k.rb : A.up_off;
@@ -288,16 +287,20 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         const WJob& J = sh.job[pj];
         const WKind& k = sh.kind[SH ? J.shared : 0];
         __syncwarp();                                            // every lane has read the stage's last bytes
-        const uint32_t at = (uint32_t) (ps * k.bytes), len = min((uint32_t) k.bytes, (uint32_t) k.rb - at);
+        // Beside a shared expert which of two constants each: looked up, and with a division for the rows of a stage, they cost two-token windows
+        // 2 to 6 % (6144 x 2048 IQ2_S with 2048 shared 130.0 / 124.4 us).  Without one they are looked up: as constants 4 % slower on Q8_0.
+        const bool js = SH && J.shared;
+        const int seg_bytes = SH ? (js ? GS::bytes : G::bytes) : k.bytes, pitch = SH ? (js ? GS::pitch : G::pitch) : k.pitch, split = js ? GS::split : 1;
+        const uint32_t at = (uint32_t) (ps * seg_bytes), len = min((uint32_t) seg_bytes, (uint32_t) k.rb - at);
         const uint32_t pstage = asked & 1u, dst = ring + pstage * kStage;
-        const int rows = SH ? RW / k.split : RW, first = SH ? pq * rows : 0;      // the stage's rows
-        if ((J.ptr & 15ull) == 0 && (!A.plain || (SH && J.shared))) {
+        const int rows = js ? RW / GS::split : RW, first = js ? pq * rows : 0;      // the stage's rows
+        if ((J.ptr & 15ull) == 0 && (!A.plain || js)) {
             if (lane < rows) {
                 const uint8_t* src = row_ptr(J.ptr, k, pc, first + lane) + at;
                 const uint32_t off = (uint32_t) (uintptr_t) src & 15u, bytes = (off + len + 15u) & ~15u;
                 fence_proxy_async();
                 mbar_expect_tx(&sh.full[warp][pstage], bytes);
-                bulk_load(s_raw + dst + lane * k.pitch, src - off, bytes, &sh.full[warp][pstage]);
+                bulk_load(s_raw + dst + lane * pitch, src - off, bytes, &sh.full[warp][pstage]);
             } else if (SH && lane < RW) {
                 mbar_arrive_one(&sh.full[warp][pstage]);
             }
@@ -305,13 +308,13 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             for (int r = 0; r < rows; ++r) {
                 const uint8_t* src = row_ptr(J.ptr, k, pc, first + r) + at;
                 const uint32_t off = (uint32_t) (uintptr_t) src & 15u;
-                for (uint32_t i = 2 * lane; i < len; i += 64) *(uint16_t*) (s_raw + dst + r * k.pitch + off + i) = *(const uint16_t*) (src + i);
+                for (uint32_t i = 2 * lane; i < len; i += 64) *(uint16_t*) (s_raw + dst + r * pitch + off + i) = *(const uint16_t*) (src + i);
             }
             __syncwarp();
             if (lane < RW) mbar_arrive_one(&sh.full[warp][pstage]);
         }
         asked = (asked + 1) & 3u;
-        if (SH && ++pq < k.split) return;
+        if (SH && ++pq < split) return;
         pq = 0;
         if (++ps == k.nseg) {
             ps = 0;
