@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid == 0) {
         sh.epoch = *(volatile unsigned*) &A.sync[1];
+        block_started(A.sync);
         sh.ar_seq = ar_seq_begin(A.ar, A.ar_seq);
     }
     stamp(A.sync, 0);
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     stamp(A.sync, 5);
     // the launch's last word: the next launch on this scratch (stream-ordered) starts a new epoch
     if (blockIdx.x == 0 && tid == 0) {
-        *(volatile unsigned*) &A.sync[1] = sh.epoch + 1u;
+        launch_ends(A.sync, sh.epoch);
         if (A.ar.nm >= 2 && A.ar_seq == 0u && A.ar.seq_counter != nullptr) *(volatile unsigned*) A.ar.seq_counter = sh.ar_seq;
     }
 }
@@ -448,7 +449,7 @@ int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
     if (A.ar.nm >= 2 && grid > MAYA_PEER_AR_BLOCKS) return refuse(MAYA_ERR_LIMIT);
     FusedArgs args = A;
     void* params[] = {&args};
-    return launch_cooperative<moe_layer_t1_kernel<T, TS, RT, HV>>(dim3(grid), dim3(kFusedThreads), params, smem, s, "moe_layer_t1");
+    return launch_cooperative<moe_layer_t1_kernel<T, TS, RT, HV>>(dim3(grid), dim3(kFusedThreads), params, smem, s, A.ar.nm >= 2, "moe_layer_t1");
 }
 
 // Units of one routed expert + the shared expert's: when even twice that many fit the grid, a rank with few local experts (or a

@@ -250,7 +250,10 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
         RowTab<T, true>::fill(s_tab, t2, kTokThreads - kRouteThreads);
     }
     grid_dependency_wait();
-    if (tid == 0) sh.epoch = *(volatile unsigned*) &A.sync[1];
+    if (tid == 0) {
+        sh.epoch = *(volatile unsigned*) &A.sync[1];
+        block_started(A.sync);
+    }
     stamp(A.sync, 0);
 
     // ---------------------------------------------------------------- phase 0
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     __syncthreads();
     if (A.hc.R_new != nullptr && done) hc_post_rows(A.out, A.hc, n_embd, o0, o1, tid, kTokThreads);
     stamp(A.sync, 5);
-    if (blockIdx.x == 0 && tid == 0) *(volatile unsigned*) &A.sync[1] = sh.epoch + 1u;       // the next launch's epoch
+    if (blockIdx.x == 0 && tid == 0) launch_ends(A.sync, sh.epoch);
 }
 
 template<int T, bool SH> int launch_token(TokArgs A, cudaStream_t s) {
@@ -613,7 +616,7 @@ template<int T, bool SH> int launch_token(TokArgs A, cudaStream_t s) {
     if (smem == 0) return kNotHere;
     if (!smem_limit.raise((const void*) token_kernel<T, SH>, kTokMostSmem)) return note_launch("token smem attribute");
     void* params[] = {&A};
-    return launch_cooperative<token_kernel<T, SH>>(dim3(grid), dim3(kTokThreads), params, smem, s, "moe_token");
+    return launch_cooperative<token_kernel<T, SH>>(dim3(grid), dim3(kTokThreads), params, smem, s, false, "moe_token");
 }
 
 }  // namespace

@@ -511,6 +511,37 @@ def test_window_combine_carries_the_cross_rank_sum(T, api, oracle):
         assert out.cpu().numpy().tobytes() == want.tobytes(), f"rank {r}"
 
 
+@pytest.mark.parametrize("kernel", ["LAYER_FUSED", "LAYER_TOKEN"])
+def test_single_tokens_on_several_streams_at_once(T, api, kernel):
+    """Launches on the legacy default stream are not cooperative, those on other streams are: hundreds of both in flight together, a layer
+    and a scratch a stream, and a captured one replayed between them - every output the same bits, no wait ran out."""
+    cfg = dict(n_embd=2304, n_ff=768, n_expert=8, k=4, gu_type=H.Q4_K, d_type=H.Q4_K)
+    lc, experts, _ = synth_layer(T, api, cfg, 8, seed=3)
+    logits, x = dev(T, H.router_logits("streams", 1, 8, None)), dev(T, H.activations("streams", 1, 2304, "f32"))
+    want = api.MoeLayer(lc, experts).forward_checked(logits, x, getattr(api, kernel))[2]
+    side = [T.cuda.Stream(), T.cuda.Stream()]
+    streams = [T.cuda.default_stream(), *side]
+    layers = [api.MoeLayer(lc, experts) for _ in range(4)]
+    T.cuda.synchronize()
+    with T.cuda.stream(side[0]):
+        layers[3].forward_checked(logits, x, getattr(api, kernel))
+    side[0].synchronize()
+    graph = T.cuda.CUDAGraph()
+    with T.cuda.graph(graph, stream=side[0]):
+        replayed = layers[3].forward_checked(logits, x, getattr(api, kernel))[2]
+    outs = []
+    for i in range(100):
+        for s, layer in zip(streams, layers):
+            with T.cuda.stream(s):
+                outs.append(layer.forward_checked(logits, x, getattr(api, kernel))[2])
+        if i % 10 == 0:
+            with T.cuda.stream(side[1]):
+                graph.replay()
+    T.cuda.synchronize()
+    assert all(layer.error() == 0 for layer in layers)
+    assert all(T.equal(o, want) for o in [*outs, replayed])
+
+
 def test_fused_layer_barrier_times_out_and_reports(T, api):
     """The fused kernel's one wait on other blocks is bounded: with the scratch's epoch word set ahead of its arrival
     counter (a state no launch leaves behind) the grid barrier can never be satisfied; the call still returns after the
