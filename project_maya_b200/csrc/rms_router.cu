@@ -14,7 +14,8 @@
 // launch, one round trip for h, one for the router rows.  So the rows are asked into L2 before the wait on the launch in
 // front and into registers before the norm's reduction, 16 bytes a lane; and a block takes only as many experts as leave
 // one block an SM (its eight warps split between them), where one warp per expert kept 32 of 148 SMs busy with a chain
-// of dependent 2-byte loads: 19.7 us a call at that size, about 7 us now.
+// of dependent 2-byte loads: 19.7 us a call at that size, 5.4 so.  The norm's weights come with the same round trip as h, in registers, where
+// they were a third one behind the reduction: 4.4 us (64 experts of 2048 3.1 / 2.7, 512 of 7168 8.8 / 7.4; calls in a row in a graph).
 //
 // A logit is an f32 sum whose order - and with it its last bits - depends on how many warps share a row (8, 4, 2 or 1, by the
 // number of experts and SMs) and on whether the 16-byte form runs (alignment): equal to rounding, not bit for bit, between calls
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(kRmsThreads) rms_router_kernel(const float* __
     grid_launch_dependents();
     for (size_t b = (size_t) tid * 128; b < ne * rb; b += kRmsThreads * 128)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(router + (size_t) e0 * rb + b));
+    for (int e = tid * 32; e < n; e += kRmsThreads * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + e));
     grid_dependency_wait();
 
     // the block's warps split evenly over its experts (epb divides kRmsWarps): expert e0 + warp / wpe, part warp % wpe
@@ -76,7 +78,14 @@ __global__ void __launch_bounds__(kRmsThreads) rms_router_kernel(const float* __
         }
     }
     float ss = 0.0f;
+    float4 wr[kAhead];
     if constexpr (VEC) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int e = (tid + i * kRmsThreads) * 4;
+            wr[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (e < n) wr[i] = *(const float4*) (w + e);
+        }
 #pragma unroll 4
         for (int e = tid * 4; e < n; e += kRmsThreads * 4) {
             float4 t = *(const float4*) (h + e);
@@ -103,16 +112,19 @@ __global__ void __launch_bounds__(kRmsThreads) rms_router_kernel(const float* __
     for (int i = 0; i < kRmsWarps; ++i) tot += sred[i];
     const float inv = rsqrtf(tot / (float) n + eps);
     if constexpr (VEC) {                                  // a thread scales the values it added itself
-#pragma unroll 4
-        for (int e = tid * 4; e < n; e += kRmsThreads * 4) {
-            const float4 t = *(const float4*) (xs + e), wv = *(const float4*) (w + e);
+        auto scale = [&](int e, const float4 wv) {
+            const float4 t = *(const float4*) (xs + e);
             const float4 xv = make_float4(t.x * inv * wv.x, t.y * inv * wv.y, t.z * inv * wv.z, t.w * inv * wv.w);
             *(float4*) (xs + e) = xv;
             if (blockIdx.x == 0) {
                 *(float4*) (x_out + e) = xv;
                 if (h_out != nullptr) *(float4*) (h_out + e) = t;
             }
-        }
+        };
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i)
+            if ((tid + i * kRmsThreads) * 4 < n) scale((tid + i * kRmsThreads) * 4, wr[i]);
+        for (int e = (tid + kAhead * kRmsThreads) * 4; e < n; e += kRmsThreads * 4) scale(e, *(const float4*) (w + e));
     } else {
         for (int e = tid; e < n; e += kRmsThreads) {
             const float t = xs[e], xv = t * inv * w[e];
