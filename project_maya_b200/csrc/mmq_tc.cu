@@ -169,24 +169,17 @@ __device__ __forceinline__ __half q8_1_round8(const float (&v)[8], uint32_t (&o)
     return __float2half_rn(__half2float(__float2half_rn(__fadd_rn(s0, s1))) - bsum);
 }
 
-// ---- Q4_K: the 16-byte header of a 144-byte block -> d * sc and -(dmin * m) of its 8 sub-blocks, as half2 pairs
-struct Q4Scales { __half2 dl[8], nml[8]; };
-__device__ __forceinline__ void q4k_scales(const uint4 hdr, Q4Scales& S) {
-    const __half2 dd = bits_h2(hdr.x);
-    const __half2 d2 = __low2half2(dd), m2 = __high2half2(dd);
-    const uint32_t s[3] = {hdr.y, hdr.z, hdr.w};
-    auto byte = [&](int i) -> uint32_t { return (s[i >> 2] >> (8 * (i & 3))) & 0xFF; };
-    const __half2 k1024 = __float2half2_rn(1024.0f);
-#pragma unroll
-    for (int sb = 0; sb < 8; ++sb) {
-        uint32_t sc, mn;
-        if (sb < 4) { sc = byte(sb) & 63; mn = byte(sb + 4) & 63; }
-        else { sc = (byte(sb + 4) & 0x0F) | ((byte(sb - 4) >> 6) << 4); mn = (byte(sb + 4) >> 4) | ((byte(sb) >> 6) << 4); }
-        const __half2 sc2 = __hsub2(bits_h2(0x64006400u | sc | (sc << 16)), k1024);      // exact
-        const __half2 mn2 = __hsub2(bits_h2(0x64006400u | mn | (mn << 16)), k1024);
-        S.dl[sb] = __hmul2(d2, sc2);
-        S.nml[sb] = __hneg2(__hmul2(m2, mn2));
-    }
+// ---- Q4_K: of a 144-byte block's 16-byte header, d * sc and -(dmin * m) of sub-blocks 2 (2 i + t) and 2 (2 i + t) + 1, i = 0 or 1, as a half2
+// each.  y, z, w: the header's scale words, shifted so that their low 16 bits are columns 2 t and 2 t + 1.  (Two sub-blocks at a time and only those a
+// team expands: all eight one by one, in an array the team indexed, took four times the instructions and local memory.)
+__device__ __forceinline__ __half2 q4k_pair(uint32_t two_bytes, __half2 factor) {
+    return __hmul2(factor, __hsub2(bytes01_plus1024(two_bytes), __float2half2_rn(1024.0f)));      // the difference is exact
+}
+__device__ __forceinline__ __half2 q4k_scale(int i, uint32_t y, uint32_t w, __half2 d2) {
+    return q4k_pair(i == 0 ? y & 0x3F3Fu : (w & 0x0F0Fu) | ((y >> 2) & 0x3030u), d2);
+}
+__device__ __forceinline__ __half2 q4k_min(int i, uint32_t z, uint32_t w, __half2 m2) {
+    return __hneg2(q4k_pair(i == 0 ? z & 0x3F3Fu : ((w >> 4) & 0x0F0Fu) | ((z >> 2) & 0x3030u), m2));
 }
 // 32 weights of sub-block (2p + hi) from the 32 quant bytes of pair p
 __device__ __forceinline__ void q4k_stage(const uint4 qa, const uint4 qb, int hi, __half2 dl, __half2 nml, uint32_t* r) {
@@ -606,22 +599,29 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 ok = pair(std::integral_constant<int, 0>{}) && pair(std::integral_constant<int, 1>{}) && pair(std::integral_constant<int, 2>{}) &&
                      pair(std::integral_constant<int, 3>{});
             } else if constexpr (T == MAYA_Q4_K) {
-                Q4Scales S;
-                q4k_scales(*(const uint4*) rrow, S);
-                const int chunk = kb >> 3;           // the team that owns the chunk's correction pair keeps the constant terms
-                if ((chunk & 1) == team)
-                    corr[kb & 7] = make_uint4(h2_bits(__lows2half2(S.nml[0], S.nml[1])), h2_bits(__lows2half2(S.nml[2], S.nml[3])),
-                                              h2_bits(__lows2half2(S.nml[4], S.nml[5])), h2_bits(__lows2half2(S.nml[6], S.nml[7])));
+                const uint4 hdr = *(const uint4*) rrow;
+                const __half2 d2 = __low2half2(bits_h2(hdr.x)), m2 = __high2half2(bits_h2(hdr.x));
+                const int mine = 16 * team, chunk = kb >> 3;     // the team that owns the chunk's correction pair keeps the constant terms
+                __half2 nml[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) nml[i] = q4k_min(i, hdr.z >> mine, hdr.w >> mine, m2);
+                if ((chunk & 1) == team) {
+                    const int other = 16 - mine;
+                    uint32_t own[2], oth[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) { own[i] = h2_bits(nml[i]); oth[i] = h2_bits(q4k_min(i, hdr.z >> other, hdr.w >> other, m2)); }
+                    corr[kb & 7] = team == 0 ? make_uint4(own[0], oth[0], own[1], oth[1]) : make_uint4(oth[0], own[0], oth[1], own[1]);
+                }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {        // the 64 values of quant pair p: low nibbles, then high nibbles
                     const int p = 2 * i + team;
                     const uint4 qa = *(const uint4*) (rrow + 16 + 32 * p), qb = *(const uint4*) (rrow + 32 + 32 * p);
-                    const int sb0 = 4 * i + 2 * team;
+                    const __half2 dl = q4k_scale(i, hdr.y >> mine, hdr.w >> mine, d2);
                     const bool seen = look();
-                    q4k_stage(qa, qb, 0, S.dl[sb0], S.nml[sb0], o);
+                    q4k_stage(qa, qb, 0, __low2half2(dl), __low2half2(nml[i]), o);
                     if (!acquire(seen)) { ok = false; break; }
                     st_half(0, o);
-                    q4k_stage(qa, qb, 1, S.dl[sb0 + 1], S.nml[sb0 + 1], o + 16);
+                    q4k_stage(qa, qb, 1, __high2half2(dl), __high2half2(nml[i]), o + 16);
                     st_half(1, o + 16);
                     release();
                     if (i == 0) ahead(2);
