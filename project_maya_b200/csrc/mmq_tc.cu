@@ -76,8 +76,12 @@ template<int T> constexpr int kBlkBytes = T == MAYA_IQ2_S ? 82 : T == MAYA_IQ3_S
 template<int T> constexpr int kWin = T == MAYA_IQ2_S ? 96 : 128;
 template<int T> constexpr int kRawRow = T == MAYA_Q4_K ? 144 : T == MAYA_Q8_0 ? 272 : T == MAYA_IQ2_S ? 112 : 144;
 template<int T> constexpr int kUnitBytes = kUnitRows * kRawRow<T>;
-template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 10 : T == MAYA_Q8_0 ? 8 : T == MAYA_IQ2_S ? 11 : 9;   // raw units in flight
-template<int T> constexpr int kBRing = (T == MAYA_Q4_K ? 6 : 4) * kBStage;    // activation tiles (64 K-values) in flight
+// Raw units in flight: whole rounds of what the expanding warps take - 4 a block of K, i-quants 8, two blocks - so that a place of the ring is
+// always the same warps' and each of them waits for every one of its phases.  A wait names a phase by its parity alone: a warp that came
+// to a place other warps had filled the round before (rings of 9, 10 and 11 units) and was a block ahead of them, as seven stages let it be, took a unit
+// that had not even been asked for.  A load that came 2.6 us late was enough.
+template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 12 : 8;
+template<int T> constexpr int kBRing = (T == MAYA_Q4_K ? 5 : 4) * kBStage;    // activation tiles (64 K-values) in flight
 // i-quants: the codebook as f16 (IQ2_S 1024 entries of 8 values, IQ3_S 512 of 4), kept in kCopies copies that lie side by
 // side in every entry - lane l reads copy l % kCopies - so that a warp's 32 random entries spread over the banks: sixteen
 // 8-byte copies are free of conflicts, four 16-byte copies cost about 8 wavefronts a look-up where one costs 11.  (The
@@ -88,8 +92,8 @@ template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 16 * kCopies<
 // the codebook lies behind the rings - and behind a finished tile, which takes their place: 160 rows of 256 f32 values
 template<int T> constexpr int kTabOff = kBRing<T> + kUnits<T> * kUnitBytes<T> > TN * TM * 4 ? kBRing<T> + kUnits<T> * kUnitBytes<T> : TN * TM * 4;
 template<int T> constexpr size_t kSmemBytes = (size_t) kTabOff<T> + kTabBytes<T>;
-static_assert(kUnits<MAYA_Q4_K> <= kMaxUnits && kUnits<MAYA_Q8_0> <= kMaxUnits && kUnits<MAYA_IQ2_S> <= kMaxUnits &&
-              kUnits<MAYA_IQ3_S> <= kMaxUnits, "one mbarrier pair per raw unit");
+template<int T> constexpr bool kUnitsFit = kUnits<T> <= kMaxUnits && kUnits<T> % (kIq<T> ? 8 : 4) == 0 && kSmemBytes<T> <= 227 * 1024 - 1024;
+static_assert(kUnitsFit<MAYA_Q4_K> && kUnitsFit<MAYA_Q8_0> && kUnitsFit<MAYA_IQ2_S> && kUnitsFit<MAYA_IQ3_S>, "the ring of raw units");
 
 // The activation image: a row is its w_cols f16 values d * q, then one f16 per 32 values - the group's SUM CORRECTION
 // xa = f16(sum of the unquantized values) - sum of the row's stored d * q values - padded with zeros to a multiple of 64.  llama.cpp's
@@ -530,7 +534,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         // A pair's two halves of 32 K-values: the first half's tensor-memory store is under way while the second half is
         // expanded (the store, its wait and the hand-off were a serial tail of every pair).
         auto st_half = [&](int h, const uint32_t* o16) { tmem_st16(a_at + 64 * st + 16 * h, *(const uint32_t(*)[16]) o16); };
-        // the raw unit of this warp's rows in the next block it expands, and its barrier's phase
+        // the place of the raw unit of this warp's rows in the next block it expands (i-quants: always the same), and its barrier's phase
         int slot = slab + (kIq<T> ? 4 * team : 0);
         uint32_t raw_phase = 0;
         for (int t = 0;; ++t, kp0 += npairs) {
@@ -669,8 +673,8 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&P.raw_empty[slot]);      // 4 warps read a unit; after the 4th it may be overwritten
             }
-            slot += kIq<T> ? 8 : 4;
-            if (slot >= NU) { slot -= NU; raw_phase ^= 1u; }
+            if constexpr (!kIq<T>) slot += 4;
+            if (kIq<T> || slot >= NU) { if constexpr (!kIq<T>) slot -= NU; raw_phase ^= 1u; }
         }
         // ------------------------------------------------------------ write-back
         if (ok && !wait_or_fail(P, &P.final, t & 1)) ok = false;
