@@ -564,10 +564,14 @@ class MoePrefill:
         quant_routed = lib.maya_mmq_quantize_routed_bf16 if x.dtype == torch.bfloat16 else lib.maya_mmq_quantize_routed
         ids, w = self.ids[:T], self.weights[:T]
         _check("router_top10", lib.maya_router_top10(_ptr(logits), T, E, k, _ptr(ids), _ptr(w), s))
-        _check("expert_count", lib.maya_expert_count(_ptr(ids), n, E, _ptr(self.counts), _ptr(self.rank), s))
-        _check("expert_bounds", lib.maya_expert_bounds(_ptr(self.counts), E, _ptr(self.bounds), s))
-        _check("expert_scatter", lib.maya_expert_scatter(_ptr(ids), _ptr(self.rank), _ptr(self.bounds), n, k,
-                                                         _ptr(self.row_tok), _ptr(self.pos), s))
+        if n <= 4096 and E <= 1024:  # one block does it all: 20 tokens of top 8 109.6 / 107.0 us a layer, 300 135.9 / 134.3; 2000 over 512 experts 457 / 466
+            _check("expert_group", lib.maya_expert_group(_ptr(ids), n, k, E, _ptr(self.rank), _ptr(self.bounds), _ptr(self.row_tok),
+                                                         _ptr(self.pos), s))
+        else:
+            _check("expert_count", lib.maya_expert_count(_ptr(ids), n, E, _ptr(self.counts), _ptr(self.rank), s))
+            _check("expert_bounds", lib.maya_expert_bounds(_ptr(self.counts), E, _ptr(self.bounds), s))
+            _check("expert_scatter", lib.maya_expert_scatter(_ptr(ids), _ptr(self.rank), _ptr(self.bounds), n, k,
+                                                             _ptr(self.row_tok), _ptr(self.pos), s))
         qtype = self.pools[0][0] if self.pools else cfg.gu_type
         # each token rounded once, its image stored to its k sorted rows (the bytes quant(x, row_tok, ...) would write)
         _check("mmq_quantize_routed", quant_routed(_ptr(x), _ptr(self.pos), k, _ptr(self.xq), qtype, H, x.stride(0), T, s))

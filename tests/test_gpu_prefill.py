@@ -590,6 +590,28 @@ def test_expert_group_is_the_stable_sort_by_expert(T, api, n_tok, k, E):
     assert np.array_equal(pos.cpu().numpy(), want_pos)
 
 
+@pytest.mark.parametrize("n_tok,k,E", [(1, 1, 1), (1, 8, 256), (129, 1, 3), (37, 7, 16), (300, 5, 1024), (127, 8, 1000), (4096, 8, 256)])
+def test_grouping_in_one_launch_equals_three(T, api, lib, n_tok, k, E):
+    """maya_expert_group against expert_count, expert_bounds and expert_scatter (the test above pins those): one warp's pairs and
+    all 32 warps', remainders of 32, one expert and as many as it takes, everything routed to one of many; more are refused."""
+    for spread in (E, 1):
+        ids = dev(T, H.rng_for("group1", n_tok, k, E).integers(0, spread, (n_tok, k)).astype(np.int32))
+        n = n_tok * k
+        counts, rank, row_tok, pos = (T.full((m,), -5, dtype=T.int32, device="cuda") for m in (E, n, n, n))
+        bounds = T.full((E + 1,), -5, dtype=T.int32, device="cuda")
+        p = lambda *ts: [t.data_ptr() for t in ts]  # noqa: E731
+        assert lib.maya_expert_count(*p(ids), n, E, *p(counts, rank), None) == 0
+        assert lib.maya_expert_bounds(*p(counts), E, *p(bounds), None) == 0
+        assert lib.maya_expert_scatter(*p(ids, rank, bounds), n, k, *p(row_tok, pos), None) == 0
+        rank1, row_tok1, pos1 = (T.full((n,), -5, dtype=T.int32, device="cuda") for _ in range(3))
+        bounds1 = T.full((E + 1,), -5, dtype=T.int32, device="cuda")
+        for _ in range(2):
+            assert lib.maya_expert_group(*p(ids), n, k, E, *p(rank1, bounds1, row_tok1, pos1), None) == 0
+        T.cuda.synchronize()
+        assert T.equal(bounds1, bounds) and T.equal(row_tok1, row_tok) and T.equal(pos1, pos)
+    assert lib.maya_expert_group(*p(ids), n, k, 1025, *p(rank1, bounds1, row_tok1, pos1), None) == -4
+
+
 @pytest.mark.parametrize("cols", [256, 1536, 96])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_routed_quantizer_writes_the_gathered_image(T, api, cols, dtype):
