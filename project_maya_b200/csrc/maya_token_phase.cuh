@@ -111,7 +111,7 @@ inline bool plain_launch_is_safe(cudaStream_t s) {
     return v == 1;
 }
 template<auto Kernel>
-int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, bool ranks, const char* what) {
+int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what, bool ranks = false) {
     static std::atomic<int> pdl{-1};           // for this kernel: the attribute is in use (1), was refused by the driver (0), has not been tried (-1)
     const void* const kernel = (const void*) Kernel;
     if (pdl.load() != 0) {

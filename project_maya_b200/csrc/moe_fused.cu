@@ -449,7 +449,7 @@ int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
     if (A.ar.nm >= 2 && grid > MAYA_PEER_AR_BLOCKS) return refuse(MAYA_ERR_LIMIT);
     FusedArgs args = A;
     void* params[] = {&args};
-    return launch_cooperative<moe_layer_t1_kernel<T, TS, RT, HV>>(dim3(grid), dim3(kFusedThreads), params, smem, s, A.ar.nm >= 2, "moe_layer_t1");
+    return launch_cooperative<moe_layer_t1_kernel<T, TS, RT, HV>>(dim3(grid), dim3(kFusedThreads), params, smem, s, "moe_layer_t1", A.ar.nm >= 2);
 }
 
 // Units of one routed expert + the shared expert's: when even twice that many fit the grid, a rank with few local experts (or a

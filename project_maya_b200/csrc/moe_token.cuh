@@ -616,7 +616,7 @@ template<int T, bool SH> int launch_token(TokArgs A, cudaStream_t s) {
     if (smem == 0) return kNotHere;
     if (!smem_limit.raise((const void*) token_kernel<T, SH>, kTokMostSmem)) return note_launch("token smem attribute");
     void* params[] = {&A};
-    return launch_cooperative<token_kernel<T, SH>>(dim3(grid), dim3(kTokThreads), params, smem, s, false, "moe_token");
+    return launch_cooperative<token_kernel<T, SH>>(dim3(grid), dim3(kTokThreads), params, smem, s, "moe_token");
 }
 
 }  // namespace
