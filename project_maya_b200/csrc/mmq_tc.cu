@@ -82,13 +82,13 @@ template<int T> constexpr int kUnitBytes = kUnitRows * kRawRow<T>;
 // that had not even been asked for.  A load that came 2.6 us late was enough.
 template<int T> constexpr int kUnits = T == MAYA_Q4_K ? 12 : 8;
 template<int T> constexpr int kBRing = (T == MAYA_Q4_K ? 5 : 4) * kBStage;    // activation tiles (64 K-values) in flight
-// i-quants: the codebook as f16 (IQ2_S 1024 entries of 8 values, IQ3_S 512 of 4), kept in kCopies copies that lie side by
-// side in every entry - lane l reads copy l % kCopies - so that a warp's 32 random entries spread over the banks: sixteen
-// 8-byte copies are free of conflicts, four 16-byte copies cost about 8 wavefronts a look-up where one costs 11.  (The
-// codebook as bytes takes a quarter of the wavefronts' width but one byte permute more for every two weights; the expansion
-// is bound by those instructions: 64 tokens of IQ3_S 553 -> 475 us, 777 of IQ2_S 1436 -> 1316.)
-template<int T> constexpr int kCopies = T == MAYA_IQ2_S ? 4 : T == MAYA_IQ3_S ? 16 : 0;
-template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 16 * kCopies<T> : T == MAYA_IQ3_S ? 512 * 8 * kCopies<T> : 0;
+// i-quants: the codebook, 64 KB of it, in kCopies copies that lie side by side in every entry - lane l reads copy l % kCopies - so that a warp's
+// random entries spread over the banks.  Both have 8-byte entries: IQ3_S's 512 are four values as f16, sixteen copies, free of conflicts; IQ2_S's 1024 are
+// byte selectors of eight values, eight copies (see iq_lookup).  (As f16, 16 bytes in four copies, IQ2_S's look-ups held the shared-memory pipe for
+// eight wavefronts each, nine tenths of the time.  As bytes a codebook takes one byte permute more for every two weights, and the expansion is bound by
+// instructions: 64 tokens of IQ3_S 553 -> 475 us.)
+template<int T> constexpr int kCopies = T == MAYA_IQ2_S ? 8 : T == MAYA_IQ3_S ? 16 : 0;
+template<int T> constexpr int kTabBytes = T == MAYA_IQ2_S ? 1024 * 8 * kCopies<T> : T == MAYA_IQ3_S ? 512 * 8 * kCopies<T> : 0;
 // the codebook lies behind the rings - and behind a finished tile, which takes their place: 160 rows of 256 f32 values
 template<int T> constexpr int kTabOff = kBRing<T> + kUnits<T> * kUnitBytes<T> > TN * TM * 4 ? kBRing<T> + kUnits<T> * kUnitBytes<T> : TN * TM * 4;
 template<int T> constexpr size_t kSmemBytes = (size_t) kTabOff<T> + kTabBytes<T>;
@@ -253,18 +253,15 @@ template<int T, int OFF> __device__ __forceinline__ void iq_fields(const uint32_
     win_words<OFF + 66>(w, F.qh, std::make_integer_sequence<int, 2>{});
     win_words<OFF + (T == MAYA_IQ2_S ? 74 : 106)>(w, F.sc, std::make_integer_sequence<int, T == MAYA_IQ2_S ? 2 : 1>{});
 }
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
 __device__ __forceinline__ uint2 lds64(uint32_t a) {
     uint2 v;
     asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
     return v;
 }
-// Sub-block J's codebook values, unsigned f16 pairs -> o[16].  tab: shared-memory address of this lane's copy of the codebook; f: the
-// entries' distance twice, as dp2a takes it (an index's 16 bits times the distance plus the base are one instruction).
+// Sub-block J's look-ups -> o[16], 8 bytes an entry.  tab: shared-memory address of this lane's copy of the codebook; f: the entries' distance
+// twice, as dp2a takes it (an index's 16 bits times the distance plus the base are one instruction).
+// IQ2_S: the magnitudes are 8, 25 and 43, so a sub-block's half has three weights but for the signs, and an entry is four byte selectors of 16 bits,
+// two to a word, each picking two of them: o[2 l], o[2 l + 1] the words of entry l.
 template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ2_S>& F, uint32_t tab, uint32_t f, uint32_t* o) {
     const uint32_t qh = byte_of(F.qh[J / 4], J % 4);
     // byte l of hw = bits 2l, 2l + 1 of qh: an entry's high index bits
@@ -272,10 +269,15 @@ template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ
     const uint32_t p0 = prmt_raw(F.q[J], hw, 0x5140u), p1 = prmt_raw(F.q[J], hw, 0x7362u);      // the indices, two to a word
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
-        const uint4 g = lds128((l & 1) ? dp2a_high(l < 2 ? p0 : p1, f, tab) : dp2a_low(l < 2 ? p0 : p1, f, tab));
-        o[4 * l] = g.x; o[4 * l + 1] = g.y; o[4 * l + 2] = g.z; o[4 * l + 3] = g.w;
+        const uint2 g = lds64((l & 1) ? dp2a_high(l < 2 ? p0 : p1, f, tab) : dp2a_low(l < 2 ? p0 : p1, f, tab));
+        o[2 * l] = g.x; o[2 * l + 1] = g.y;
     }
 }
+__device__ __forceinline__ uint32_t iq2s_select(uint32_t four) {             // four codebook bytes, 0x08, 0x19 or 0x2b: value i's bytes 2 c, 2 c + 1
+    const uint32_t c = (four >> 4) & 0x03030303u;
+    return c << 1 | c << 5 | 0x10101010u;
+}
+// IQ3_S: the entry's four values as f16.
 template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ3_S>& F, uint32_t tab, uint32_t f, uint32_t* o) {
     const uint32_t qh = byte_of(F.qh[J / 4], J % 4);
     // byte l of h0 / h1 = bit l / 4 + l of qh, the ninth index bit of entry l / 4 + l
@@ -288,13 +290,13 @@ template<int J> __device__ __forceinline__ void iq_lookup(const IqFields<MAYA_IQ
         o[2 * l] = g.x; o[2 * l + 1] = g.y;
     }
 }
-// Eight values in place: times dl (one f16 rounding), then the signs.  Pair p's signs from sign byte s: s * (2^(15 - 2p) +
-// 2^(30 - 2p)) has them at bits 15 and 31 (the two shifted copies of the 8 bits do not meet), and one three-input operation
-// masks them out and flips the signs.
+// Pair p's signs from sign byte s: s * (2^(15 - 2p) + 2^(30 - 2p)) has them at bits 15 and 31 (the two shifted copies of the 8 bits do not meet);
+// masked out and the signs flipped by one three-input operation.
+__device__ __forceinline__ uint32_t iq_signs(uint32_t s, int p) { return (s * ((1u << (15 - 2 * p)) + (1u << (30 - 2 * p)))) & 0x80008000u; }
+// Eight values in place: times dl (one f16 rounding), then the signs.
 __device__ __forceinline__ void iq_eight(uint32_t s, __half2 dl, uint32_t* r) {
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
-        r[p] = h2_bits(__hmul2(bits_h2(r[p]), dl)) ^ ((s * ((1u << (15 - 2 * p)) + (1u << (30 - 2 * p)))) & 0x80008000u);
+    for (int p = 0; p < 4; ++p) r[p] = h2_bits(__hmul2(bits_h2(r[p]), dl)) ^ iq_signs(s, p);
 }
 // A byte's two scale nibbles (n0 low) -> (f16 scale times a (2 n0 + 1), and times a (2 n1 + 1)), a a power of two: the factors are exact
 // and each product is rounded once, as f16 of the f32 product is.
@@ -304,15 +306,27 @@ template<int T> __device__ __forceinline__ __half2 iq_scales(uint32_t word, int 
                                       : __hfma2(bits_h2(z), __floats2half2_rn(2.0f, 0.125f), __floats2half2_rn(-2047.0f, -127.0f));
     return __hmul2(bits_h2(d2), n);
 }
-// Sub-blocks J and J + 1 (J even): values -> weights, in place; `mid` runs when the first is done.
-// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; the factor is f16(d (2 ls + 1) / 8).
+// Sub-blocks J and J + 1 (J even): look-ups -> weights, in place; `mid` runs when the first is done.
+// IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; the factor is f16(d (2 ls + 1) / 8), and the three
+// products by it are rounded once, as every weight's own would be.  (A selector's upper half is brought down by a dp2a: the byte permutes fill the integer pipe,
+// and with a shift there 3000 tokens of 4096 x 2048 took 1445 us, so 1416, with f16 entries 1561; 777 of 6144 x 2048 1138, 1108, 1184.)
 template<int J, class Mid> __device__ __forceinline__ void iq_finish2(const IqFields<MAYA_IQ2_S>& F, uint32_t* o, Mid mid) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const __half2 dl = iq_scales<MAYA_IQ2_S>(F.sc[J / 4], (J + h) % 4, F.d2);
-        const __half2 dl0 = __low2half2(dl), dl1 = __high2half2(dl);
+        uint32_t* const r = o + 16 * h;
+        uint32_t sel[8];
 #pragma unroll
-        for (int l = 0; l < 4; ++l) iq_eight(byte_of(F.sg[J + h], l), l < 2 ? dl0 : dl1, o + 16 * h + 4 * l);
+        for (int i = 0; i < 8; ++i) sel[i] = r[i];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const __half2 d = l < 2 ? __low2half2(dl) : __high2half2(dl);
+            const uint32_t a = h2_bits(__hmul2(d, __floats2half2_rn(8.0f, 25.0f))), b = h2_bits(__hmul2(d, __floats2half2_rn(43.0f, 43.0f)));
+            const uint32_t s = byte_of(F.sg[J + h], l);
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+                r[4 * l + p] = prmt_raw(a, b, (p & 1) ? dp2a_high(sel[2 * l + p / 2], 1u << 24, 0u) : sel[2 * l + p / 2]) ^ iq_signs(s, p);
+        }
         if (h == 0) mid();
     }
 }
@@ -482,10 +496,14 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 return make_uint2(h2_bits(__hsub2(bytes01_plus1024(g), k1024)), h2_bits(__hsub2(bytes23_plus1024(g), k1024)));
             };
             uint2* const grid = (uint2*) (smem + kTabOff<T>);
-            constexpr int W = T == MAYA_IQ2_S ? 2 : 1;                   // four-value words of an entry
             for (int i = tid; i < kTabBytes<T> / 8; i += kDqWarps * 32) {
-                const int e = i / (W * kCopies<T>), h = i % W;
-                grid[i] = wide(T == MAYA_IQ2_S ? ((const uint32_t*) g_iq2s_grid)[2 * e + h] : g_iq3s_grid[e]);
+                const int e = i / kCopies<T>;
+                if constexpr (T == MAYA_IQ2_S) {
+                    const uint2 g = ((const uint2*) g_iq2s_grid)[e];
+                    grid[i] = make_uint2(iq2s_select(g.x), iq2s_select(g.y));
+                } else {
+                    grid[i] = wide(g_iq3s_grid[e]);
+                }
             }
             named_bar_sync(2, kDqWarps * 32);
         }
@@ -527,8 +545,8 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
             if (lane == 0) mbar_arrive_addr(afull0 + 8 * st);
         };
         // i-quants: this lane's copy of the codebook, and the entries' distance
-        constexpr uint32_t kEnt = kIq<T> ? kCopies<T> * (T == MAYA_IQ2_S ? 16 : 8) : 0;
-        [[maybe_unused]] const uint32_t tab = smem_u32(smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) * (T == MAYA_IQ2_S ? 16 : 8) : 0);
+        constexpr uint32_t kEnt = kCopies<T> * 8;
+        [[maybe_unused]] const uint32_t tab = smem_u32(smem + kTabOff<T>) + (kIq<T> ? lane % (kIq<T> ? kCopies<T> : 1) * 8 : 0);
         [[maybe_unused]] const uint32_t tab_f = kEnt | kEnt << 24;
         [[maybe_unused]] uint4 corr[8];      // Q4_K: the constant terms of the current 8-block chunk (indexed by kb: local memory)
         // A pair's two halves of 32 K-values: the first half's tensor-memory store is under way while the second half is
