@@ -158,10 +158,21 @@ __device__ __forceinline__ void select_rank(uint32_t order, float p, int n_exper
     Sync::sync();
 }
 
+// The weight of selected expert i from the values it was selected with, sh.val, in selection order: divided in double by max(their sum, 2^-14)
+// (RT 1: if norm_w, and times w_scale).
+template<int RT> __device__ __forceinline__ float route_weight(const RouterShared& sh, int k, int i, float w_scale, int norm_w) {
+    double s = 0.0;
+    for (int j = 0; j < k; ++j) s += (double) sh.val[j];
+    const double sc = fmax(s, 6.103515625e-05);   // 2^-14
+    if constexpr (RT == 0) return (float) ((double) sh.val[i] / sc);
+    const float v = sh.val[i];
+    return (norm_w ? (float) ((double) v / sc) : v) * w_scale;
+}
+
 // One token's softmax routing by the calling thread group.  l: n_expert logits; s_ex: n_expert doubles of shared
 // memory, 16-byte aligned.  On return (after the group's last sync) sh.ids[0..k) hold the ids and sh.val[0..k) the
-// renormalised weights.
-template<int PER, class Sync>
+// renormalised weights - with LATER the values they are made of (route_weight).
+template<int PER, class Sync, bool LATER = false>
 __device__ __forceinline__ void route_softmax(const float* __restrict__ l, int n_expert, int k, int tid, int nt,
                                               double* s_ex, RouterShared& sh) {
     const int nw = nt >> 5;
@@ -215,22 +226,20 @@ __device__ __forceinline__ void route_softmax(const float* __restrict__ l, int n
     }
     if constexpr (PER == 1) select_rank<Sync>(order[0], p[0], n_expert, k, tid, (unsigned long long*) s_ex, sh);
     else select_topk<PER, Sync>(order, p, n_expert, k, tid, nt, sh);
-    // weights renormalised in double by max(their sum in selection order, 2^-14): every thread adds, k threads divide
-    double s = 0.0;
-    for (int i = 0; i < k; ++i) s += (double) sh.val[i];
-    const double sc = fmax(s, 6.103515625e-05);   // 2^-14
-    const float mine = tid < k ? (float) ((double) sh.val[tid] / sc) : 0.0f;
-    Sync::sync();
-    if (tid < k) sh.val[tid] = mine;
-    Sync::sync();
+    if constexpr (!LATER) {
+        const float mine = tid < k ? route_weight<0>(sh, k, tid, 1.0f, 1) : 0.0f;
+        Sync::sync();
+        if (tid < k) sh.val[tid] = mine;
+        Sync::sync();
+    }
 }
 
 // One token's sigmoid routing (router_sigmoid.cu:29-74, glm_batch.cu:2063-2100): p = sigmoid(logit) in FP32, selection on
 // p + bias (bias NULL: none), the stable descending top-k, weights from the unbiased p - divided in double by
-// max(their sum, 2^-14) when norm_w - times w_scale.  On return sh.ids[0..k) / sh.val[0..k) hold ids and final weights.
+// max(their sum, 2^-14) when norm_w - times w_scale.  On return sh.ids[0..k) / sh.val[0..k) hold ids and final weights (LATER: as above).
 // s_keys: n_expert 64-bit words of shared memory, 16-byte aligned (one expert per thread: selection by rank, one pass instead of
 // k rounds of arg-max with two barriers each).
-template<int PER, class Sync>
+template<int PER, class Sync, bool LATER = false>
 __device__ __forceinline__ void route_sigmoid(const float* __restrict__ l, const float* __restrict__ bias, int n_expert, int k,
                                               float w_scale, int norm_w, int tid, int nt, double* s_keys, RouterShared& sh) {
     float p[PER];
@@ -247,14 +256,12 @@ __device__ __forceinline__ void route_sigmoid(const float* __restrict__ l, const
     }
     if constexpr (PER == 1) select_rank<Sync>(order[0], p[0], n_expert, k, tid, (unsigned long long*) s_keys, sh);
     else select_topk<PER, Sync>(order, p, n_expert, k, tid, nt, sh);
-    double s = 0.0;                                              // every thread adds, k threads divide
-    for (int i = 0; i < k; ++i) s += (double) sh.val[i];
-    const double sc = fmax(s, 6.103515625e-05);
-    float mine = tid < k ? sh.val[tid] : 0.0f;
-    if (norm_w) mine = (float) ((double) mine / sc);
-    Sync::sync();
-    if (tid < k) sh.val[tid] = mine * w_scale;
-    Sync::sync();
+    if constexpr (!LATER) {
+        const float mine = tid < k ? route_weight<1>(sh, k, tid, w_scale, norm_w) : 0.0f;
+        Sync::sync();
+        if (tid < k) sh.val[tid] = mine;
+        Sync::sync();
+    }
 }
 
 }  // namespace maya

@@ -267,16 +267,14 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
         else route_token<0>(A.logits, nullptr, A.n_expert, k, 0.0f, 0, tid, s_ex, &sh.route);
         if (tid < k) {
             const int e = sh.route.ids[tid];
-            sh.w[tid] = sh.route.val[tid];
             sh.ptr[tid] = (e >= A.expert_lo && e < A.expert_hi) ? (unsigned long long) (A.experts + (size_t) e * A.expert_stride) : 0ull;
-            if (blockIdx.x == 0) { A.ids[tid] = e; A.weights[tid] = sh.route.val[tid]; }
+            if (blockIdx.x == 0) A.ids[tid] = e;
         }
         NamedSync<1, kRouteThreads>::sync();
-        if (tid == 0) {                                  // the entries that are this rank's
-            int nv = 0;
-            for (int i = 0; i < k; ++i)
-                if (sh.ptr[i] != 0ull) sh.ve[nv++] = i;
-            sh.nv = nv;
+        if (tid < 32) {                                  // the entries that are this rank's
+            const unsigned here = __ballot_sync(0xffffffffu, tid < k && sh.ptr[tid] != 0ull);
+            if (here >> tid & 1u) sh.ve[__popc(here & ((1u << tid) - 1u))] = tid;
+            if (tid == 0) sh.nv = __popc(here);
         }
     } else {
         constexpr int NW2 = kTokWarps - kRouteThreads / 32;
@@ -515,7 +513,11 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     if (!ok && tid == 0) tok_gave_up(A.sync, mark);
     if (A.d_type != T) tok_fill(A.d_type, s_tab, tid);
     stamp(A.sync, 2);
-    const bool met = grid_barrier(A.sync, sh.epoch, &sh.bar_ok);
+    const bool met = grid_barrier(A.sync, sh.epoch, &sh.bar_ok, [&](int i) {
+        if (i >= k) return;
+        sh.w[i] = A.router == 1 ? route_weight<1>(sh.route, k, i, A.router_w_scale, A.router_norm_w) : route_weight<0>(sh.route, k, i, 0.0f, 0);
+        if (blockIdx.x == 0) A.weights[i] = sh.w[i];
+    });
     stamp(A.sync, 3);
     bool done = ok && met;
     if (!ok && met) tok_reset(A.unit_count, (MAYA_MAX_K + 1) * nblk_h);
