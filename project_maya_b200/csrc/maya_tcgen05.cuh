@@ -52,11 +52,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
     return (uint64_t) ((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t) (1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// Tiled TMA load of a 3-d box (plain: this block only, no multicast) from the tensor described by `map` (a
-// CUtensorMap in kernel-parameter or global memory) into shared memory; completion is counted in bytes on `bar`.
-// c0 * element size must be a multiple of 16 bytes.
-// by one elected lane of a CONVERGED warp, every operand warp-uniform (they then stay in uniform registers, where the copy wants
-// them: a lane of its own in a divergent branch took 400 to 500 cycles a tile): so many bytes expected on `bar`, and a box that brings them
+// Tiled TMA load of a 3-d box (plain: this block only, no multicast) from the tensor described by `map` (a CUtensorMap in
+// kernel-parameter or global memory) into shared memory; `bytes` are expected on `bar`, where completion is counted.
+// c0 * element size must be a multiple of 16 bytes.  Called by a converged warp with warp-uniform operands, one elected lane
+// copies: the operands stay in the uniform registers that the copy wants (a lane of its own in a divergent branch took 400 to 500
+// cycles a tile).
 __device__ __forceinline__ void tma_expect_load_3d(uint32_t dst_smem, const void* map, uint32_t bar, uint32_t bytes, int c0, int c1, int c2) {
     __syncwarp();
     asm volatile(

@@ -31,7 +31,8 @@ __device__ __forceinline__ void stamp(unsigned* sync, int i) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile unsigned long long*) &sync[4 + 2 * i] = global_ns();
 }
 
-// One thread a block, behind the wait for the launch in front; and block 0's last word, which every other block's comes before.
+// One thread a block of a launch that is not cooperative, behind the wait for the launch in front (all of them at once on one word cost the
+// fused kernel 3.6 us a token in a graph: 63.4 / 59.9); and block 0's last word, which every other block's comes before.
 __device__ __forceinline__ void block_started(unsigned* sync) { atomicAdd(&sync[kSyncStarted], 1u); }
 __device__ __forceinline__ void launch_ends(unsigned* sync, unsigned epoch) {
     *(volatile unsigned*) &sync[kSyncStarted] = 0u;
@@ -39,7 +40,7 @@ __device__ __forceinline__ void launch_ends(unsigned* sync, unsigned epoch) {
 }
 // All blocks of the grid meet here.  false in EVERY thread of the block when the wait ran out: thread 0 leaves the outcome in shared
 // memory before the closing barrier.  meanwhile(lane): what the second warp does while the first one's thread 0 waits.
-template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned epoch, int* s_ok, Meanwhile meanwhile) {
+template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned epoch, bool plain, int* s_ok, Meanwhile meanwhile) {
     __syncthreads();
     if (threadIdx.x >= 32 && threadIdx.x < 64) meanwhile((int) threadIdx.x - 32);
     if (threadIdx.x == 0) {
@@ -53,7 +54,7 @@ template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned*
             if (global_ns() - t0 > kBarrierTimeoutNs) {
                 // a block that has not started: other work of this GPU has its SM still.  (Not once a block has given up: block 0's last word
                 // may be written.)
-                if (*(volatile unsigned*) &sync[2] == 0u && *(volatile unsigned*) &sync[kSyncStarted] < gridDim.x && ++waits < kStartWaits) {
+                if (plain && *(volatile unsigned*) &sync[2] == 0u && *(volatile unsigned*) &sync[kSyncStarted] < gridDim.x && ++waits < kStartWaits) {
                     t0 = global_ns();
                     continue;
                 }
@@ -70,10 +71,11 @@ template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned*
     return *s_ok != 0;
 }
 
-// The token's routing by the block's first kRouteThreads threads - which experts, and the values their weights are made of (route_weight: a
-// sum and a division in double, not needed before the combine: made while the grid barrier is waited for, where the first rows waited for
-// them; 2048 x 1024 Q4_K 18.0 / 17.4 us a token, two layers of IQ3_S with producer 132.8 / 129.2) - as a function of its own: run once a launch, it is
-// kept out of the kernel's register allocation and instruction scheduling (which proved sensitive to what phase 0 holds).
+// The token's routing by the block's first kRouteThreads threads: which experts, and the values their weights are made of.  The weights
+// themselves (route_weight: a sum and a division in double) are not needed before the combine and are made while the grid barrier is
+// waited for; made here the first rows waited for them (2048 x 1024 Q4_K 18.0 / 17.4 us a token, two layers of IQ3_S with producer
+// 132.8 / 129.2).  A function of its own: run once a launch, it is kept out of the kernel's register allocation and instruction
+// scheduling (which proved sensitive to what phase 0 holds).
 template<int RT>
 __device__ __noinline__ void route_token(const float* logits, const float* bias, int n_expert, int k, float w_scale, int norm_w,
                                          int tid, double* s_ex, RouterShared* route) {
@@ -114,7 +116,7 @@ inline bool plain_launch_is_safe(cudaStream_t s) {
     return v == 1;
 }
 template<auto Kernel>
-int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what, bool ranks = false) {
+int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what, bool plain = false) {
     static std::atomic<int> pdl{-1};           // for this kernel: the attribute is in use (1), was refused by the driver (0), has not been tried (-1)
     const void* const kernel = (const void*) Kernel;
     if (pdl.load() != 0) {
@@ -129,7 +131,7 @@ int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaSt
         at[1].id = cudaLaunchAttributeCooperative;
         at[1].val.cooperative = 1;
         cfg.attrs = at;
-        cfg.numAttrs = !ranks && plain_launch_is_safe(s) ? 1 : 2;
+        cfg.numAttrs = plain ? 1 : 2;
         const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, params);
         if (e == cudaSuccess) { pdl.store(1); return note_launch(what); }
         // only "this attribute / combination is not supported" turns the attribute off; any other failure is the launch's

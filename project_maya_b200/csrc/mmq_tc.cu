@@ -28,13 +28,14 @@
 // Which expert and which 160-row group of it a block handles is found on the device from `bounds`; no count travels
 // to the host.
 //
-// What bounds it: for groups of many rows the board's power limit and the expansion, for
-// groups of few rows the expansion alone, 4 instructions a weight.  That holds only while no waiting role is in the way: clock stamps of 64 tokens of
-// IQ3_S showed finished weights waiting 3000 cycles - the activation loader, one lane in a divergent branch, took 540 cycles a tile
-// (every operand of a copy crossed into a uniform register), longer than the expansion.  Now both loaders walk their loops as whole
-// warps and an elected lane copies, the role's number is warp-uniform to the compiler (an issuing warp's products 137 -> 47 cycles), the
-// stages fill tensor memory, and a stage is asked for before the expansion that goes there.  us a layer, before and after: 64 tokens of IQ3_S 463 / 385,
-// 777 of IQ2_S with a shared expert 1262 / 1165, 4096 of Q8_0 / Q4_K 3499 / 3190, 60 of Q8_0 236 / 200, 100 of Q4_K 265 / 245.
+// What bounds it: for groups of many rows the board's power limit and the expansion, for groups of few rows the expansion alone,
+// 4 instructions a weight.  That holds only while no waiting role is in the way: clock stamps of 64 tokens of IQ3_S showed finished
+// weights waiting 3000 cycles - the activation loader, one lane in a divergent branch, took 540 cycles a tile (every operand of a copy
+// crossed into a uniform register), longer than the expansion.  Now both loaders walk their loops as whole warps and an elected lane
+// copies, the role's number is warp-uniform to the compiler (an issuing warp's products 137 -> 47 cycles), the stages fill tensor
+// memory, and a stage is asked for before the expansion that goes there.  us a layer, before and after: 64 tokens of IQ3_S 463 / 385,
+// 777 of IQ2_S with a shared expert 1262 / 1165, 4096 of Q8_0 / Q4_K 3499 / 3190, 60 of Q8_0 236 / 200, 100 of Q4_K 265 / 245.  Then the
+// expansions themselves: Q4_K's header two sub-blocks at a time (100 of Q4_K 218), IQ2_S's codebook of byte selectors (777 of IQ2_S 1184 / 1108).
 //
 // Every mbarrier wait is bounded: a wait that runs out sets the error word, the roles stop, copies in
 // flight are waited for (bounded), tensor memory is freed and the block returns.
