@@ -17,8 +17,8 @@
 //   warp 16     TMA loads of raw weight blocks, 64 rows x 256 K-values a "unit", into a ring of units;
 //   warp 18     TMA loads of activation tiles, 128 (+ 32) or 32 rows x 64 K-values, in the 128-byte swizzle layout
 //               the tensor core reads at full rate;
-//   warps 0..15 two teams of 8 warps that take alternate K steps (i-quants: alternate blocks, whose steps alternate in the products'
-//               order); in a team one thread per weight row expands 32 K-values of the row per step (packed half2 arithmetic:
+//   warps 0..15 two teams of 8 warps that take alternate K steps (i-quants: alternate blocks of 256 K-values); in a team one thread
+//               per weight row expands 32 K-values of the row per step (packed half2 arithmetic:
 //               Q8_0 w = q * d; Q4_K w = fma(q, d * sc, -(dmin * m))) and tcgen05.st-s them into the row's lane;
 //   warps 17,19 one accumulator each: two tcgen05.mma per step (2 K = 16 halves, A from tensor memory, B from shared
 //               memory), one commit per two steps -> the steps' buffers are free (the warp cannot issue products as fast as
@@ -518,10 +518,11 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         // of the tile before it has completed.)
         int seq = 0, st = 0, n_st = 0, kp0 = 0;          // kp0: pairs of the tiles before this one
         uint32_t a_at = 0;
-        auto ahead = [&](int d) {                        // d <= 3
+        auto ahead = [&](int d) {                        // d <= 4
             seq += d;
             st += d;
             if (st >= n_st) st -= n_st;
+            if (kIq<T> && st >= n_st) st -= n_st;        // there are at least three
         };
         // The stage is free when pair seq - n_st, which read it last, has completed.  look(): whether it is, asked before the expansion so
         // that the answer is there behind it; acquire(): now (the warp is then converged, as the stores need it).
@@ -562,15 +563,17 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
         if (named_bar_or(3, kDqWarps * 32, !ok) || ti.e < 0) break;      // the same for every expanding warp
         const int nrows = ti.nrows, row0 = ti.row0, m0 = ti.m0;
         const TileGeo geo = tile_geo<T>(nrows);
-        seq = st = team;
+        seq = st = 0;
         n_st = geo.st;
+        ahead(kIq<T> ? 4 * team : team);
         a_at = a_lane + 2 * geo.acc;
 #ifdef MAYA_MMQ_STAMPS
         long long* const stamps = tid == 0 && ok ? stamps_of(ti.lin) : nullptr;
         if (stamps) { stamps[0] = clock64(); stamps[14] = nrows; stamps[15] = npairs; }
 #endif
-        // i-quants: a team expands every other block whole - its fields are taken out of the window once - and the pairs of a block
-        // and the next one's alternate (see pair_block).  The other types: both teams work on a block, on alternate pairs.
+        // i-quants: a team expands every other block whole - its fields are taken out of the window once.  The products take the pairs in
+        // K's order all the same (the accumulator's sums are f32: another order is another result): a team's four pairs wait in the stages
+        // while the other team's are taken.  The other types: both teams work on a block, on alternate pairs.
         for (int kb = kIq<T> ? team : 0; kb < nkb && ok; kb += kIq<T> ? 2 : 1) {
             if (!wait_or_fail(P, &P.raw_full[slot], raw_phase)) { ok = false; break; }
             const uint8_t* rrow = rbase + (size_t) slot * kUnitBytes<T>;
@@ -616,11 +619,12 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                         iq_lookup<J + 3>(F, tab, tab_f, o + 16);
                     }
                     release();
-                    ahead(2);
+                    ahead(1);
                     return true;
                 };
                 ok = pair(std::integral_constant<int, 0>{}) && pair(std::integral_constant<int, 1>{}) && pair(std::integral_constant<int, 2>{}) &&
                      pair(std::integral_constant<int, 3>{});
+                ahead(4);
             } else if constexpr (T == MAYA_Q4_K) {
                 const uint4 hdr = *(const uint4*) rrow;
                 const __half2 d2 = __low2half2(bits_h2(hdr.x)), m2 = __high2half2(bits_h2(hdr.x));
@@ -994,9 +998,7 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                 // the pair's 64 K-values in the image: K values in order, and after every 32 pairs (or at the end) the
                 // chunk's 64 corrections from the tail behind the row's K values
                 int xcol;
-                if constexpr (kIq<T>) {
-                    xcol = ((kb2 >> 3) * 2 + (kb2 & 1)) * 256 + ((kb2 >> 1) & 3) * 64;
-                } else if (ntp == 0) {
+                if (ntp == 0) {
                     xcol = kb2 * 64;
                 } else {
                     const int c = kb2 / 33, r = kb2 - c * 33;

@@ -284,6 +284,43 @@ def test_tiles_of_every_height_one_after_another_bitwise(T, api, t, cols):
     assert T.equal(got, want)
 
 
+@pytest.mark.parametrize("t", [H.Q4_K, H.Q8_0, H.IQ2_S, H.IQ3_S])
+@pytest.mark.parametrize("copies", [1, 2, 3, 4, 5])
+def test_k_values_are_added_in_order(T, api, t, copies):
+    """The f32 sums run over K from its start to its end, 64 values after 64, at every division of tensor memory.  Row r has X at the first of
+    the 64 values r, Y at those of r + 1 and -X at those of r + 2, and all weights are one w: X w + Y w is X w in f32 (Y / X = 2^-29, of the
+    same sign, so that it is lost whether the sum is rounded or cut off), and the row's result is 0.  Were r + 1 added before r or
+    behind r + 2, Y w would be left."""
+    cols, w_rows = 2048, 256
+    if t == H.Q8_0:           # d = 0.5, q = 3
+        block = np.concatenate([np.array([0.5], np.float16).view(np.uint8), np.full(32, 3, np.uint8)])
+    elif t == H.Q4_K:         # d = 0.5, dmin = 0, every scale 1 and minimum 0, every q 3
+        block = np.concatenate([np.array([0.5, 0.0], np.float16).view(np.uint8), np.array([1, 1, 1, 1, 0, 0, 0, 0, 1, 1, 1, 1], np.uint8), np.full(128, 0x33, np.uint8)])
+    else:                     # d = 0.5, every index 0, no signs, every scale 1
+        block = np.zeros(82 if t == H.IQ2_S else 110, np.uint8)
+        block[:2] = np.array([0.5], np.float16).view(np.uint8)
+        block[-8 if t == H.IQ2_S else -4:] = 0x11
+    w = dev(T, np.tile(np.tile(block, H.row_bytes(t, cols) // len(block)), w_rows)[None])
+    rows = cols // 64 - 2
+    x = np.zeros((rows, cols), np.float32)
+    for r in range(rows):
+        x[r, 64 * r], x[r, 64 * r + 64], x[r, 64 * r + 128] = 2.0 ** 14, 2.0 ** -15, -2.0 ** 14
+    x = np.tile(x, (copies, 1))
+    n = len(x)
+
+    def run(values):
+        out = T.full((n, w_rows), 7.0, dtype=T.float32, device="cuda")
+        xq = api.mmq_quantize(dev(T, values), None, t)
+        api.mmq_run(api.mmq_product(w, t, w_rows, cols, w.shape[1], 1, xq, dev(T, np.array([0, n], np.int32)), None, n, out, w_rows))
+        T.cuda.synchronize()
+        return out.cpu().numpy()
+
+    small = x.copy()
+    small[np.abs(x) > 1.0] = 0.0
+    assert (run(small) != 0).all()
+    np.testing.assert_array_equal(run(x), 0.0)
+
+
 @pytest.mark.parametrize("ta,tb,counts,n_ff", [
     (H.Q8_0, H.Q4_K, [1, 0, 161, 7, 320, 33], 256),                                       # fewer tiles than blocks, remainders of 160 rows
     (H.IQ2_S, H.IQ3_S, [5] * 24 + [0] * 3 + [170] * 3, 2048),                             # several rounds of tiles
