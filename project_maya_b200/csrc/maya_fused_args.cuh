@@ -32,8 +32,7 @@ struct FusedArgs {
     int ar_rank;
     unsigned ar_seq;
     maya_hc_post_args hc;      // hc.R_new != NULL: the hyper-connection write of `out` into the residual stack, last
-    bool plain;                // launched without the cooperative attribute: blocks count themselves as started
-    unsigned* sync;            // scratch: [0] arrivals, [1] epoch, [2] error, [4..15] block 0's phase time stamps (ns), [16] blocks started, [kTokMark] the mark
+    unsigned* sync;            // scratch: [0] arrivals, [1] epoch, [2] error, [4..15] block 0's phase time stamps (ns), [kTokMark] the mark
                                // of the last launch in which a block of the token kernel gave up
 };
 

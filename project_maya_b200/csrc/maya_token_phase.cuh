@@ -10,9 +10,7 @@ namespace {
 
 constexpr int kRouteThreads = 256;
 constexpr int kMaxSliceRows = 96;          // output rows a block may own (n_embd / grid rounded up)
-constexpr unsigned long long kBarrierTimeoutNs = 1000000000ull;   // the grid barrier gives up after a second ...
-constexpr int kStartWaits = 30;            // ... or as many, while some block of the grid has not started (see launch_cooperative)
-constexpr int kSyncStarted = 16;           // scratch word: blocks of this launch that have started; 0 between launches
+constexpr unsigned long long kBarrierTimeoutNs = 1000000000ull;   // the grid barrier gives up after a second
 
 // balanced contiguous split of n rows over nb blocks
 __device__ __forceinline__ void slice(int n, int nb, int b, int& r0, int& r1) {
@@ -31,16 +29,9 @@ __device__ __forceinline__ void stamp(unsigned* sync, int i) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile unsigned long long*) &sync[4 + 2 * i] = global_ns();
 }
 
-// One thread a block of a launch that is not cooperative, behind the wait for the launch in front (all of them at once on one word cost the
-// fused kernel 3.6 us a token in a graph: 63.4 / 59.9); and block 0's last word, which every other block's comes before.
-__device__ __forceinline__ void block_started(unsigned* sync) { atomicAdd(&sync[kSyncStarted], 1u); }
-__device__ __forceinline__ void launch_ends(unsigned* sync, unsigned epoch) {
-    *(volatile unsigned*) &sync[kSyncStarted] = 0u;
-    *(volatile unsigned*) &sync[1] = epoch + 1u;
-}
-// All blocks of the grid meet here.  false in EVERY thread of the block when the wait ran out: thread 0 leaves the outcome in shared
-// memory before the closing barrier.  meanwhile(lane): what the second warp does while the first one's thread 0 waits.
-template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned epoch, bool plain, int* s_ok, Meanwhile meanwhile) {
+// All blocks of the (cooperative) grid meet here.  false in EVERY thread of the block when the wait ran out: thread 0
+// leaves the outcome in shared memory before the closing barrier.  meanwhile(lane): what the second warp does while the first one's thread 0 waits.
+template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned* sync, unsigned epoch, int* s_ok, Meanwhile meanwhile) {
     __syncthreads();
     if (threadIdx.x >= 32 && threadIdx.x < 64) meanwhile((int) threadIdx.x - 32);
     if (threadIdx.x == 0) {
@@ -48,20 +39,9 @@ template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned*
         __threadfence();
         atomicAdd(&sync[0], 1u);
         const unsigned target = (epoch + 1u) * gridDim.x;
-        unsigned long long t0 = global_ns();
-        int waits = 0;
+        const unsigned long long t0 = global_ns();
         while ((int) (*(volatile unsigned*) &sync[0] - target) < 0) {
-            if (global_ns() - t0 > kBarrierTimeoutNs) {
-                // a block that has not started: other work of this GPU has its SM still.  (Not once a block has given up: block 0's last word
-                // may be written.)
-                if (plain && *(volatile unsigned*) &sync[2] == 0u && *(volatile unsigned*) &sync[kSyncStarted] < gridDim.x && ++waits < kStartWaits) {
-                    t0 = global_ns();
-                    continue;
-                }
-                ok = 0;
-                atomicExch(&sync[2], 1u);
-                break;
-            }
+            if (global_ns() - t0 > kBarrierTimeoutNs) { ok = 0; atomicExch(&sync[2], 1u); break; }
             __nanosleep(20);
         }
         __threadfence();
@@ -94,29 +74,13 @@ __device__ __noinline__ void route_token(const float* logits, const float* bias,
     }
 }
 
-// A launch whose blocks wait for one another, with every block resident, and programmatically serialized after the launch in front
-// of it: its set-up then overlaps that launch's tail.
-//
-// On the legacy default stream without the cooperative attribute.  There are as many blocks as SMs, and a block takes most of an SM: they
-// are all resident as soon as nothing else holds an SM for good.  Only another launch of this kind could, half resident itself; but
-// the legacy stream's launches follow one another, and all others are cooperative, which start with their whole grid or not at all.  In a stream
-// a cooperative launch gives up the overlap: it starts 2 to 3 us after the launch in front has ended, at the next multiple of 2.05 us
-// (in a graph it keeps it).  us a token, launched one by one, cooperative / so: 2048 x 1024 Q4_K 20.5 / 18.4, 1536 24.6 / 21.8, 2048
-// 26.7 / 23.7.  A server of several processes (MPS) shares the SMs out by rules of its own: cooperative there.  nm >= 2 ranks: cooperative.
-inline bool plain_launch_is_safe(cudaStream_t s) {
-    if (s != nullptr && s != cudaStreamLegacy) return false;
-    static std::atomic<int> mps[64];           // a device: not asked yet (0), no (1), yes (2)
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return false;
-    if ((v = mps[dev].load()) == 0) {
-        int on = 1;
-        v = cudaDeviceGetAttribute(&on, cudaDevAttrMpsEnabled, dev) == cudaSuccess && on == 0 ? 1 : 2;
-        mps[dev].store(v);
-    }
-    return v == 1;
-}
+// A cooperative launch (the grid barrier needs every block resident) and, where the driver accepts the attribute,
+// programmatically serialized after the launch in front of it: its set-up then overlaps that launch's tail.  (In a stream a cooperative
+// launch gives up the overlap - it starts 2 to 3 us after the launch in front has ended - in a graph it keeps it.  An ordinary
+// launch would keep it there too, but starts with the blocks that fit: they hold their SMs and wait, and a launch on another stream whose
+// own blocks wait for one another, NCCL's say, may have the others and wait for these.)
 template<auto Kernel>
-int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what, bool plain = false) {
+int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s, const char* what) {
     static std::atomic<int> pdl{-1};           // for this kernel: the attribute is in use (1), was refused by the driver (0), has not been tried (-1)
     const void* const kernel = (const void*) Kernel;
     if (pdl.load() != 0) {
@@ -126,12 +90,12 @@ int launch_cooperative(dim3 grid, dim3 block, void** params, size_t smem, cudaSt
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        at[1].id = cudaLaunchAttributeCooperative;
-        at[1].val.cooperative = 1;
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
-        cfg.numAttrs = plain ? 1 : 2;
+        cfg.numAttrs = 2;
         const cudaError_t e = cudaLaunchKernelExC(&cfg, kernel, params);
         if (e == cudaSuccess) { pdl.store(1); return note_launch(what); }
         // only "this attribute / combination is not supported" turns the attribute off; any other failure is the launch's

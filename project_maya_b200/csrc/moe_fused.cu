@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid == 0) {
         sh.epoch = *(volatile unsigned*) &A.sync[1];
-        if (A.plain) block_started(A.sync);
         sh.ar_seq = ar_seq_begin(A.ar, A.ar_seq);
     }
     stamp(A.sync, 0);
@@ -309,7 +308,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     if constexpr (TS != 0) ds = shape(calls_per_row<TS>(has_sh ? A.sh_hi - A.sh_lo : n_ff));
     __syncthreads();
     stamp(A.sync, 2);
-    const bool ok = grid_barrier(A.sync, sh.epoch, A.plain, &sh.bar_ok, [&](int i) {
+    const bool ok = grid_barrier(A.sync, sh.epoch, &sh.bar_ok, [&](int i) {
         if (i >= k) return;
         sh.w[i] = route_weight<RT>(sh.route, k, i, A.router_w_scale, A.router_norm_w);
         if (blockIdx.x == 0) A.weights[i] = sh.w[i];
@@ -424,7 +423,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     stamp(A.sync, 5);
     // the launch's last word: the next launch on this scratch (stream-ordered) starts a new epoch
     if (blockIdx.x == 0 && tid == 0) {
-        launch_ends(A.sync, sh.epoch);
+        *(volatile unsigned*) &A.sync[1] = sh.epoch + 1u;
         if (A.ar.nm >= 2 && A.ar_seq == 0u && A.ar.seq_counter != nullptr) *(volatile unsigned*) A.ar.seq_counter = sh.ar_seq;
     }
 }
@@ -450,9 +449,8 @@ int launch_fused_rt(const FusedArgs& A, cudaStream_t s) {
     if (4 * ((A.n_embd / 4 + grid - 1) / grid) > kMaxSliceRows || A.n_embd % 4) return refuse(MAYA_ERR_LIMIT);
     if (A.ar.nm >= 2 && grid > MAYA_PEER_AR_BLOCKS) return refuse(MAYA_ERR_LIMIT);
     FusedArgs args = A;
-    args.plain = A.ar.nm < 2 && plain_launch_is_safe(s);
     void* params[] = {&args};
-    return launch_cooperative<moe_layer_t1_kernel<T, TS, RT, HV>>(dim3(grid), dim3(kFusedThreads), params, smem, s, "moe_layer_t1", args.plain);
+    return launch_cooperative<moe_layer_t1_kernel<T, TS, RT, HV>>(dim3(grid), dim3(kFusedThreads), params, smem, s, "moe_layer_t1");
 }
 
 // Units of one routed expert + the shared expert's: when even twice that many fit the grid, a rank with few local experts (or a

@@ -30,7 +30,7 @@ struct Scratch {
     float* h;                    // the fused single-token kernel's h: q8_1 image, shared-unit halves, counters
     unsigned* unit_count;        // the token kernel's counters of units that two blocks share (zero before first use)
     unsigned* sync;              // [33]: the fused and the token kernel's barrier counter, epoch, [2] error word (also the window kernels'); [3] prep_kernel's ticket;
-                                 // stamps; [16] blocks started; [32] the token kernel's mark of a launch that gave up (zero before first use)
+                                 // stamps; [32] the token kernel's mark of a launch that gave up (zero before first use)
     size_t bytes;
 };
 

@@ -250,10 +250,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
         RowTab<T, true>::fill(s_tab, t2, kTokThreads - kRouteThreads);
     }
     grid_dependency_wait();
-    if (tid == 0) {
-        sh.epoch = *(volatile unsigned*) &A.sync[1];
-        if (A.plain) block_started(A.sync);
-    }
+    if (tid == 0) sh.epoch = *(volatile unsigned*) &A.sync[1];
     stamp(A.sync, 0);
 
     // ---------------------------------------------------------------- phase 0
@@ -513,7 +510,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     if (!ok && tid == 0) tok_gave_up(A.sync, mark);
     if (A.d_type != T) tok_fill(A.d_type, s_tab, tid);
     stamp(A.sync, 2);
-    const bool met = grid_barrier(A.sync, sh.epoch, A.plain, &sh.bar_ok, [&](int i) {
+    const bool met = grid_barrier(A.sync, sh.epoch, &sh.bar_ok, [&](int i) {
         if (i >= k) return;
         sh.w[i] = A.router == 1 ? route_weight<1>(sh.route, k, i, A.router_w_scale, A.router_norm_w) : route_weight<0>(sh.route, k, i, 0.0f, 0);
         if (blockIdx.x == 0) A.weights[i] = sh.w[i];
@@ -608,7 +605,7 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     __syncthreads();
     if (A.hc.R_new != nullptr && done) hc_post_rows(A.out, A.hc, n_embd, o0, o1, tid, kTokThreads);
     stamp(A.sync, 5);
-    if (blockIdx.x == 0 && tid == 0) launch_ends(A.sync, sh.epoch);
+    if (blockIdx.x == 0 && tid == 0) *(volatile unsigned*) &A.sync[1] = sh.epoch + 1u;       // the next launch's epoch
 }
 
 template<int T, bool SH> int launch_token(TokArgs A, cudaStream_t s) {
@@ -617,9 +614,8 @@ template<int T, bool SH> int launch_token(TokArgs A, cudaStream_t s) {
     const size_t smem = token_smem(T, A, grid);
     if (smem == 0) return kNotHere;
     if (!smem_limit.raise((const void*) token_kernel<T, SH>, kTokMostSmem)) return note_launch("token smem attribute");
-    A.plain = plain_launch_is_safe(s);
     void* params[] = {&A};
-    return launch_cooperative<token_kernel<T, SH>>(dim3(grid), dim3(kTokThreads), params, smem, s, "moe_token", A.plain);
+    return launch_cooperative<token_kernel<T, SH>>(dim3(grid), dim3(kTokThreads), params, smem, s, "moe_token");
 }
 
 }  // namespace

@@ -513,8 +513,8 @@ def test_window_combine_carries_the_cross_rank_sum(T, api, oracle):
 
 @pytest.mark.parametrize("kernel", ["LAYER_FUSED", "LAYER_TOKEN"])
 def test_single_tokens_on_several_streams_at_once(T, api, kernel):
-    """Launches on the legacy default stream are not cooperative, those on other streams are: hundreds of both in flight together, a layer
-    and a scratch a stream, and a captured one replayed between them - every output the same bits, no wait ran out."""
+    """Hundreds of launches on the legacy default stream and on others in flight together, a layer and a scratch a stream, and a captured
+    one replayed between them - every output the same bits, no wait ran out."""
     cfg = dict(n_embd=2304, n_ff=768, n_expert=8, k=4, gu_type=H.Q4_K, d_type=H.Q4_K)
     lc, experts, _ = synth_layer(T, api, cfg, 8, seed=3)
     logits, x = dev(T, H.router_logits("streams", 1, 8, None)), dev(T, H.activations("streams", 1, 2304, "f32"))
@@ -540,6 +540,40 @@ def test_single_tokens_on_several_streams_at_once(T, api, kernel):
     T.cuda.synchronize()
     assert all(layer.error() == 0 for layer in layers)
     assert all(T.equal(o, want) for o in [*outs, replayed])
+
+
+@pytest.mark.parametrize("kernel", ["LAYER_FUSED", "LAYER_TOKEN"])
+def test_single_token_starts_with_its_whole_grid_or_not_at_all(T, api, kernel):
+    """A launch whose blocks wait for one another must not hold SMs while some of its blocks cannot start: another launch of that kind could
+    have the SMs they need.  One block of a long product holds an SM (more shared memory than lies beside a block of the layer); on the
+    default stream the layer's first block, once it runs, does not wait that long at the grid barrier."""
+    cfg = dict(n_embd=2304, n_ff=768, n_expert=8, k=4, gu_type=H.Q4_K, d_type=H.Q4_K)
+    lc, experts, _ = synth_layer(T, api, cfg, 8, seed=3)
+    logits, x = dev(T, H.router_logits("whole", 1, 8, None)), dev(T, H.activations("whole", 1, 2304, "f32"))
+    layer = api.MoeLayer(lc, experts)
+    rows, cols = 256, 1 << 18
+    w = T.zeros((1, rows * H.row_bytes(H.Q8_0, cols)), dtype=T.uint8, device="cuda")
+    xq = api.mmq_quantize(T.ones((1, cols), device="cuda"), None, H.Q8_0)
+    out = T.empty((1, rows), dtype=T.float32, device="cuda")
+    product = api.mmq_product(w, H.Q8_0, rows, cols, w.shape[1], 1, xq, dev(T, np.array([0, 1], np.int32)), None, 1, out, rows)
+    side = T.cuda.Stream()
+    barrier, held = [], []
+    for i in range(4):
+        T.cuda.synchronize()
+        begin, end = T.cuda.Event(enable_timing=True), T.cuda.Event(enable_timing=True)
+        with T.cuda.stream(side):
+            begin.record()
+            api.mmq_run(product)
+            end.record()
+        layer.forward_checked(logits, x, getattr(api, kernel))
+        T.cuda.synchronize()
+        ns = layer.phase_ns()
+        if i > 0:
+            barrier.append(ns[3] - ns[2])
+            held.append(begin.elapsed_time(end) * 1e6)
+    assert layer.error() == 0
+    assert min(held) > 4e5, "the product is over too soon for this test"
+    assert max(barrier) < 1e5, f"{max(barrier)} ns at the barrier"
 
 
 def test_fused_layer_barrier_times_out_and_reports(T, api):
