@@ -51,26 +51,27 @@ template<class Meanwhile> __device__ __forceinline__ bool grid_barrier(unsigned*
     return *s_ok != 0;
 }
 
-// The token's routing by the block's first kRouteThreads threads: which experts, and the values their weights are made of.  The weights
-// themselves (route_weight: a sum and a division in double) are not needed before the combine and are made while the grid barrier is
-// waited for; made here the first rows waited for them (2048 x 1024 Q4_K 18.0 / 17.4 us a token, two layers of IQ3_S with producer
-// 132.8 / 129.2).  A function of its own: run once a launch, it is kept out of the kernel's register allocation and instruction
-// scheduling (which proved sensitive to what phase 0 holds).
-template<int RT>
+// The token's routing by the block's first kRouteThreads threads, as a function of its own: run once a launch, it is
+// kept out of the kernel's register allocation and instruction scheduling (which proved sensitive to what phase 0 holds).
+// LATER: which experts, and only the values their weights are made of.  The token kernel makes the weights (route_weight: a sum and a
+// division in double) while the grid barrier is waited for; made here its first rows waited for them (us a token in a graph, here / there:
+// 2048 x 1024 Q4_K 16.97 / 16.49, 2048 x 2048 24.12 / 23.69).  The fused kernel, whose body has no register to spare, has them made
+// here: there they cost it 0.3 us (6144 x 2048 IQ2_S with 2048 shared 59.54 / 59.86).
+template<int RT, bool LATER>
 __device__ __noinline__ void route_token(const float* logits, const float* bias, int n_expert, int k, float w_scale, int norm_w,
                                          int tid, double* s_ex, RouterShared* route) {
     using RS = NamedSync<1, kRouteThreads>;
     const int per = (n_expert + kRouteThreads - 1) / kRouteThreads;
     if constexpr (RT == 1) {
-        if (per <= 1) route_sigmoid<1, RS, true>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 2) route_sigmoid<2, RS, true>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 4) route_sigmoid<4, RS, true>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
-        else route_sigmoid<8, RS, true>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        if (per <= 1) route_sigmoid<1, RS, LATER>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        else if (per <= 2) route_sigmoid<2, RS, LATER>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        else if (per <= 4) route_sigmoid<4, RS, LATER>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
+        else route_sigmoid<8, RS, LATER>(logits, bias, n_expert, k, w_scale, norm_w, tid, kRouteThreads, s_ex, *route);
     } else {
-        if (per <= 1) route_softmax<1, RS, true>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 2) route_softmax<2, RS, true>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-        else if (per <= 4) route_softmax<4, RS, true>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
-        else route_softmax<8, RS, true>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
+        if (per <= 1) route_softmax<1, RS, LATER>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
+        else if (per <= 2) route_softmax<2, RS, LATER>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
+        else if (per <= 4) route_softmax<4, RS, LATER>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
+        else route_softmax<8, RS, LATER>(logits, n_expert, k, tid, kRouteThreads, s_ex, *route);
     }
 }
 

@@ -117,12 +117,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
 
     // ---------------------------------------------------------------- phase 0
     if (tid < kRouteThreads) {
-        route_token<RT>(A.logits, A.router_bias, A.n_expert, k, A.router_w_scale, A.router_norm_w, tid, s_ex, &sh.route);
+        route_token<RT, false>(A.logits, A.router_bias, A.n_expert, k, A.router_w_scale, A.router_norm_w, tid, s_ex, &sh.route);
         if (tid < k) {
             const int e = sh.route.ids[tid];
+            sh.w[tid] = sh.route.val[tid];
             sh.ptr[tid] = (e >= A.expert_lo && e < A.expert_hi)
                               ? (unsigned long long) (A.experts + (size_t) e * A.expert_stride) : 0ull;
-            if (blockIdx.x == 0) A.ids[tid] = e;
+            if (blockIdx.x == 0) { A.ids[tid] = e; A.weights[tid] = sh.route.val[tid]; }
         }
         if (tid == 0) sh.ptr[k] = has_sh ? (unsigned long long) A.shared : 0ull;
         NamedSync<1, kRouteThreads>::sync();
@@ -308,11 +309,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) moe_layer_t1_kernel(FusedArg
     if constexpr (TS != 0) ds = shape(calls_per_row<TS>(has_sh ? A.sh_hi - A.sh_lo : n_ff));
     __syncthreads();
     stamp(A.sync, 2);
-    const bool ok = grid_barrier(A.sync, sh.epoch, &sh.bar_ok, [&](int i) {
-        if (i >= k) return;
-        sh.w[i] = route_weight<RT>(sh.route, k, i, A.router_w_scale, A.router_norm_w);
-        if (blockIdx.x == 0) A.weights[i] = sh.w[i];
-    });
+    const bool ok = grid_barrier(A.sync, sh.epoch, &sh.bar_ok, [](int) {});
     stamp(A.sync, 3);
 
     // ---------------------------------------------------------------- phase 2: q8_1(h), down, combine

@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(kTokThreads, 1) token_kernel(const TokArgs A) 
     o1 *= 4;
     const int nrows = o1 - o0;
     if (tid < kRouteThreads) {
-        if (A.router == 1) route_token<1>(A.logits, A.router_bias, A.n_expert, k, A.router_w_scale, A.router_norm_w, tid, s_ex, &sh.route);
-        else route_token<0>(A.logits, nullptr, A.n_expert, k, 0.0f, 0, tid, s_ex, &sh.route);
+        if (A.router == 1) route_token<1, true>(A.logits, A.router_bias, A.n_expert, k, A.router_w_scale, A.router_norm_w, tid, s_ex, &sh.route);
+        else route_token<0, true>(A.logits, nullptr, A.n_expert, k, 0.0f, 0, tid, s_ex, &sh.route);
         if (tid < k) {
             const int e = sh.route.ids[tid];
             sh.ptr[tid] = (e >= A.expert_lo && e < A.expert_hi) ? (unsigned long long) (A.experts + (size_t) e * A.expert_stride) : 0ull;
