@@ -209,8 +209,10 @@ MAYA_API int maya_expert_bounds(const int* counts, int n_expert, int* bounds, vo
 /* glmb::expert_scatter (glm_batch.hpp:139): row = base[ids[i]] + rank[i]; row_tok[row] = i / k; pos[i] = row. */
 MAYA_API int maya_expert_scatter(const int* ids, const int* rank, const int* base, int n, int k, int* row_tok, int* pos,
                                  void* stream);
-/* The three in one launch, for up to 1024 experts (MAYA_ERR_LIMIT beyond): bounds [n_expert + 1], row_tok and pos [n] as above;
- * rank [n] is scratch. */
+/* The three in one launch, for up to 1024 experts (MAYA_ERR_LIMIT beyond): counts [n_expert] (NULL: not wanted), bounds [n_expert + 1],
+ * row_tok and pos [n] as above; rank [n] is scratch.  maya_expert_group: without the counts. */
+MAYA_API int maya_expert_group_counts(const int* ids, int n, int k, int n_expert, int* counts, int* rank, int* bounds, int* row_tok, int* pos,
+                                      void* stream);
 MAYA_API int maya_expert_group(const int* ids, int n, int k, int n_expert, int* rank, int* bounds, int* row_tok, int* pos, void* stream);
 /* glmb::swiglu_rows (glm_batch.hpp:141): h[r][c] = silu(min(gu[r][c], limit)) * clamp(gu[r][n_ff + c], +-limit) over
  * rows of [gate | up]; ld_h = h's row stride (0: n_ff); h may be gu with ld_h = 2 n_ff. */

@@ -99,6 +99,7 @@ _SIGNATURES = {
     "maya_moe_combine": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p]),
     "maya_expert_count": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "maya_expert_bounds": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),
+    "maya_expert_group_counts": (c_int, [c_void_p, c_int, c_int, c_int, *[c_void_p] * 6]),
     "maya_expert_group": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "maya_expert_scatter": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "maya_swiglu_rows": (c_int, [c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]),

@@ -565,8 +565,8 @@ class MoePrefill:
         ids, w = self.ids[:T], self.weights[:T]
         _check("router_top10", lib.maya_router_top10(_ptr(logits), T, E, k, _ptr(ids), _ptr(w), s))
         if n <= 4096 and E <= 1024:  # one block does it all: 20 tokens of top 8 109.6 / 107.0 us a layer, 300 135.9 / 134.3; 2000 over 512 experts 457 / 466
-            _check("expert_group", lib.maya_expert_group(_ptr(ids), n, k, E, _ptr(self.rank), _ptr(self.bounds), _ptr(self.row_tok),
-                                                         _ptr(self.pos), s))
+            _check("expert_group", lib.maya_expert_group_counts(_ptr(ids), n, k, E, _ptr(self.counts), _ptr(self.rank), _ptr(self.bounds),
+                                                                _ptr(self.row_tok), _ptr(self.pos), s))
         else:
             _check("expert_count", lib.maya_expert_count(_ptr(ids), n, E, _ptr(self.counts), _ptr(self.rank), s))
             _check("expert_bounds", lib.maya_expert_bounds(_ptr(self.counts), E, _ptr(self.bounds), s))

@@ -82,8 +82,9 @@ __global__ void __launch_bounds__(1024) expert_bounds_kernel(const int* __restri
 // in shared memory, 32 pairs a step - lanes with the same expert find one another with one match - then a thread an expert turns the warps'
 // counts into first ranks, a scan the totals into bounds, and every pair's row is bounds + first rank + rank.
 constexpr int kGroupExperts = 1024;
-__global__ void __launch_bounds__(1024) expert_group_kernel(const int* __restrict__ ids, int n, int k, int n_expert, int* __restrict__ rank,
-                                                            int* __restrict__ bounds, int* __restrict__ row_tok, int* __restrict__ pos) {
+__global__ void __launch_bounds__(1024) expert_group_kernel(const int* __restrict__ ids, int n, int k, int n_expert, int* __restrict__ counts,
+                                                            int* __restrict__ rank, int* __restrict__ bounds, int* __restrict__ row_tok,
+                                                            int* __restrict__ pos) {
     extern __shared__ int s_group[];                  // [32][n_expert] counts, then first ranks; [n_expert] bounds
     __shared__ int s_tot[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(1024) expert_group_kernel(const int* __restric
         s_base[tid] = incl - tot;
         bounds[tid + 1] = incl;
         if (tid == 0) bounds[0] = 0;
+        if (counts != nullptr) counts[tid] = tot;
     }
     __syncthreads();
     for (int i = i0 + lane; i < i1; i += 32) {
@@ -288,15 +290,19 @@ extern "C" int maya_expert_bounds(const int* counts, int n_expert, int* bounds, 
     launch_dependent(expert_bounds_kernel, dim3(1), dim3(1024), 0, as_stream(stream), counts, n_expert, bounds);
     return note_launch("expert_bounds");
 }
-extern "C" int maya_expert_group(const int* ids, int n, int k, int n_expert, int* rank, int* bounds, int* row_tok, int* pos, void* stream) {
+extern "C" int maya_expert_group_counts(const int* ids, int n, int k, int n_expert, int* counts, int* rank, int* bounds, int* row_tok, int* pos,
+                                        void* stream) {
     if (n_expert <= 0 || n < 0 || k <= 0 || !bounds || (n > 0 && (!ids || !rank || !row_tok || !pos))) return refuse(MAYA_ERR_ARG);
     if (n_expert > kGroupExperts) return refuse(MAYA_ERR_LIMIT);
     const size_t smem = 33 * (size_t) n_expert * sizeof(int);
     static SmemLimit smem_limit;
     if (smem > kSmemNoLimit && !smem_limit.raise((const void*) expert_group_kernel, 33 * (size_t) kGroupExperts * sizeof(int)))
         return note_launch("expert_group smem attribute");
-    launch_dependent(expert_group_kernel, dim3(1), dim3(1024), smem, as_stream(stream), ids, n, k, n_expert, rank, bounds, row_tok, pos);
+    launch_dependent(expert_group_kernel, dim3(1), dim3(1024), smem, as_stream(stream), ids, n, k, n_expert, counts, rank, bounds, row_tok, pos);
     return note_launch("expert_group");
+}
+extern "C" int maya_expert_group(const int* ids, int n, int k, int n_expert, int* rank, int* bounds, int* row_tok, int* pos, void* stream) {
+    return maya_expert_group_counts(ids, n, k, n_expert, nullptr, rank, bounds, row_tok, pos, stream);
 }
 extern "C" int maya_expert_scatter(const int* ids, const int* rank, const int* base, int n, int k, int* row_tok, int* pos,
                                    void* stream) {

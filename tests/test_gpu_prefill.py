@@ -627,6 +627,17 @@ def test_expert_group_is_the_stable_sort_by_expert(T, api, n_tok, k, E):
     assert np.array_equal(pos.cpu().numpy(), want_pos)
 
 
+@pytest.mark.parametrize("n_tok,k,E", [(1, 4, 8), (300, 8, 16), (512, 8, 16), (513, 8, 16)])
+def test_prefill_counts_each_experts_tokens(T, api, n_tok, k, E):
+    """MoePrefill.counts after a call, on both sides of the 4096 pairs up to which the rows are grouped in one launch."""
+    lc = api.MoeLayerConfig(256, 256, E, k, H.Q8_0, H.Q8_0)
+    layer = api.MoePrefill(lc, T.zeros((E, lc.blob_bytes), dtype=T.uint8, device="cuda"), max_tokens=n_tok)
+    layer.counts.fill_(-5)
+    ids = layer.forward(dev(T, H.router_logits("counts", n_tok, E, None)), dev(T, H.activations("counts", n_tok, 256, "f32")))[0]
+    T.cuda.synchronize()
+    assert T.equal(layer.counts, T.bincount(ids.flatten(), minlength=E).int())
+
+
 @pytest.mark.parametrize("n_tok,k,E", [(1, 1, 1), (1, 8, 256), (129, 1, 3), (37, 7, 16), (300, 5, 1024), (127, 8, 1000), (4096, 8, 256)])
 def test_grouping_in_one_launch_equals_three(T, api, lib, n_tok, k, E):
     """maya_expert_group against expert_count, expert_bounds and expert_scatter (the test above pins those): one warp's pairs and
