@@ -892,13 +892,14 @@ mmq_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUt
                             if (++slot == NU) { slot = 0; raw_phase ^= 1u; }
                         }
                     }
-                    if (!ok)                                     // let the copies in flight land before the block ends: a place's last one
-                        for (int i = 0; i < NU; ++i) wait_or_fail(P, &P.raw_full[i], i < slot ? raw_phase ^ 1u : raw_phase);
                 }
             }
             if (!ok || found_e < 0) break;
             prev_rows = nrows;
         }
+        // Let the copies in flight land before the block ends: a place's last one.  Also when all went well so far - the roles that
+        // would wait for them may still give up.
+        for (int i = 0; i < NU; ++i) wait_or_fail(P, &P.raw_full[i], i < slot ? raw_phase ^ 1u : raw_phase);
         if (A.claim != nullptr && lane == 0 && atomicAdd(A.claim + 1, 1u) == gridDim.x - 1u) {       // no block will claim again
             A.claim[0] = 0u;
             A.claim[1] = 0u;
