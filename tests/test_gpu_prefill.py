@@ -259,10 +259,13 @@ def test_tall_groups_equal_short_groups_bitwise(T, api, t, rows):
 
 @pytest.mark.parametrize("t,cols", [(H.Q4_K, 256), (H.Q4_K, 1792), (H.Q4_K, 2304), (H.Q8_0, 256), (H.Q8_0, 768), (H.IQ2_S, 4096), (H.IQ3_S, 2048)])
 def test_tiles_of_every_height_one_after_another_bitwise(T, api, t, cols):
-    """A tile's rows decide how tensor memory and the activation ring are divided.  Blocks that take tiles of every division in turn
-    (heights at both edges of each, more tiles than SMs; K of less than a ring, and Q4_K chunks of 1, 7 and 8 + 1 blocks): the bits of
-    the same rows in groups of at most 16, which all have one division."""
-    w_rows, heights = 512, [1, 160, 33, 32, 129, 64, 97, 65, 128, 96, 16, 17] * 8
+    """A tile's rows decide how tensor memory and the activation ring are divided.  Blocks that take ten tiles and more, every division behind
+    every other (heights at both edges of each; K of less than a ring, and Q4_K chunks of 1, 7 and 8 + 1 blocks), plain and with
+    SwiGLU and the rounding of h in the write-back: the bits of the same rows in groups of at most 16, which all have one division."""
+    w_rows, heights = 1024, [int(h) for h in H.rng_for("heights order").permutation([1, 160, 33, 32, 129, 64, 97, 65, 128, 96, 16, 17] * 31)]
+    sms, per_group = T.cuda.get_device_properties(0).multi_processor_count, w_rows // 256
+    division = np.repeat([(h + 31) // 32 for h in heights], per_group)               # of every tile; block b's are b, b + sms, ...
+    assert len(division) >= 10 * sms and len(set(zip(division, division[sms:]))) == 25
     w1 = synth_matrices(T, api, t, 4, w_rows, cols, 61)
     w = w1[T.arange(len(heights), device="cuda") % 4].contiguous()
     total = sum(heights)
@@ -273,15 +276,18 @@ def test_tiles_of_every_height_one_after_another_bitwise(T, api, t, cols):
         err = T.zeros(1, dtype=T.int32, device="cuda")
         bounds = dev(T, np.concatenate([[0], np.cumsum(counts)]).astype(np.int32))
         api.mmq_run(api.mmq_product(mats, t, w_rows, cols, mats.shape[1], len(counts), xq, bounds, None, total, out, w_rows, error=err))
+        n_ff = w_rows // 2
+        hq = T.zeros(api.mmq_q8_bytes(total, n_ff), dtype=T.uint8, device="cuda")
+        api.mmq_run_glu(api.mmq_product(mats, t, w_rows, cols, mats.shape[1], len(counts), xq, bounds, None, total, None, n_ff, error=err, xq_out=hq), 7.0)
         T.cuda.synchronize()
         assert int(err.item()) == 0
-        return out
+        return out, hq
 
     short = [(g % 4, min(16, h - at)) for g, h in enumerate(heights) for at in range(0, h, 16)]
-    want = run(w1[T.tensor([e for e, _ in short], device="cuda")].contiguous(), [n for _, n in short])
-    got = run(w, heights)
+    want, want_hq = run(w1[T.tensor([e for e, _ in short], device="cuda")].contiguous(), [n for _, n in short])
+    got, got_hq = run(w, heights)
     assert T.isfinite(got).all() and float(got.abs().max()) > 0.1
-    assert T.equal(got, want)
+    assert T.equal(got, want) and T.equal(got_hq, want_hq)
 
 
 @pytest.mark.parametrize("t", [H.Q4_K, H.Q8_0, H.IQ2_S, H.IQ3_S])
@@ -324,6 +330,7 @@ def test_k_values_are_added_in_order(T, api, t, copies):
 @pytest.mark.parametrize("ta,tb,counts,n_ff", [
     (H.Q8_0, H.Q4_K, [1, 0, 161, 7, 320, 33], 256),                                       # fewer tiles than blocks, remainders of 160 rows
     (H.IQ2_S, H.IQ3_S, [5] * 24 + [0] * 3 + [170] * 3, 2048),                             # several rounds of tiles
+    (H.IQ3_S, H.Q4_K, [97, 1, 160, 33, 16, 129, 64, 32, 65, 128, 17, 96] * 4, 2048),      # ten tiles a block, of every division
     (H.Q4_K, H.Q8_0, [0] * 6, 256)])                                                      # no rows at all in one pair
 def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
     """Two pairs of gate/up and down products in one chain, each down tile starting when its own rows of h are there: the bits
@@ -349,7 +356,7 @@ def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
     for gu, dn, _, _ in want:
         api.mmq_run_glu(gu, 7.0)
         api.mmq_run(dn)
-    counters = T.zeros(4096, dtype=T.uint8, device="cuda")
+    counters = T.zeros(max(4096, api._lib.load().maya_mmq_chain_bytes(sum(p["total"] for p in pairs), sum(p["n"] for p in pairs), 2)), dtype=T.uint8, device="cuda")
     for _ in range(2):
         got = [products(p) for p in pairs]
         api.mmq_run_chain([g[0] for g in got], [g[1] for g in got], 7.0, counters)
