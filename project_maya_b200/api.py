@@ -406,7 +406,6 @@ class MoeLayer:
                                  *((1, _ptr(sigmoid[0]), float(sigmoid[1]), int(bool(sigmoid[2]))) if sigmoid is not None else (0, None, 1.0, 0)),
                                  _ptr(cpu_part), _ptr(cpu_flag))
         self._keep = (sigmoid, cpu_part, cpu_flag)
-        self._one = (torch.empty((), dtype=torch.int32, device=experts.device), torch.empty((), dtype=torch.float32, device=experts.device))
         self._shapes = {}
         self.max_tokens = max_tokens
         nbytes = int(_lib.load().maya_moe_layer_scratch_bytes(C.byref(self.desc), max_tokens))
@@ -414,20 +413,23 @@ class MoeLayer:
             raise MayaError("moe_layer_scratch_bytes", -1)
         self.scratch = torch.zeros(nbytes, dtype=torch.uint8, device=experts.device)   # zeroed: holds a barrier counter
 
-    def _like(self, T):
-        """What a call's outputs look like (one value of memory each): torch.empty_like of these takes 1.3 us, torch.empty of a shape, a
-        type and a device 2.3."""
-        if T not in self._shapes:
-            i32, f32 = self._one
-            self._shapes[T] = (i32.expand(T, self.cfg.k), f32.expand(T, self.cfg.k), f32.expand(T, self.cfg.n_embd))
-        return self._shapes[T]
+    def _like(self, T, device):
+        """What a call's outputs look like (one value of memory each), on the logits' device: torch.empty_like of these takes 1.3 us,
+        torch.empty of a shape, a type and a device 2.3."""
+        like = self._shapes.get((T, device))
+        if like is None:
+            i32, f32 = torch.empty((), dtype=torch.int32, device=device), torch.empty((), dtype=torch.float32, device=device)
+            like = (i32.expand(T, self.cfg.k), f32.expand(T, self.cfg.k), f32.expand(T, self.cfg.n_embd))
+            if T <= self.max_tokens:             # more are refused: nothing to keep
+                self._shapes[T, device] = like
+        return like
 
     def forward(self, logits, x, ids=None, weights=None, out=None, stream=None, peer=None, hc=None):
         """hc = (R_old [T, 4, n_embd], post [T, 4], comb [T, 4, 4], R_new [T, 4, n_embd]): also write the block's output
         into the residual stack (glmf::hc_post) - in the layer kernel's epilogue for one token."""
         T = logits.shape[0]
         if ids is None or weights is None or out is None:
-            like = self._like(T)
+            like = self._like(T, logits.device)
             ids = ids if ids is not None else torch.empty_like(like[0], memory_format=torch.contiguous_format)
             weights = weights if weights is not None else torch.empty_like(like[1], memory_format=torch.contiguous_format)
             out = out if out is not None else torch.empty_like(like[2], memory_format=torch.contiguous_format)

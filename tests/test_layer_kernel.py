@@ -72,3 +72,35 @@ def test_what_the_token_kernel_leaves_to_others(lib):
     assert kernel(lib, desc(*mixed, n_ff_sh=1024, sh_lo=0, sh_hi=512)) == STAGED      # a slice beside two types: refused there
     assert kernel(lib, desc(H.Q4_K, H.Q4_K, 4096, 1536, 8, n_ff_sh=1024, sh_lo=0, sh_hi=512)) == TOKEN
     assert kernel(lib, desc(H.Q4_K, H.Q4_K, 4096, 1536, 9)) == -4
+
+
+def test_a_layers_outputs_lie_where_its_logits_do(monkeypatch):
+    """MoeLayer.forward with its library replaced: ids, weights and out are allocated on the logits' device, contiguous and anew at each
+    call, and a refused number of tokens leaves nothing behind."""
+    import torch
+
+    from project_maya_b200 import _lib, api
+
+    class Fake:
+        maya_row_bytes = staticmethod(lambda t, n: 144 * (n // 256))
+        maya_moe_layer_scratch_bytes = staticmethod(lambda *a: 64)
+        maya_moe_layer_decode = staticmethod(lambda L, logits, x, bf16, T, *a: 0 if T <= 4 else -4)
+
+    monkeypatch.setattr(_lib, "load", lambda: Fake)
+    monkeypatch.setattr(api, "_ptr", lambda t: None)             # (asks for CUDA tensors)
+    cfg = api.MoeLayerConfig(256, 256, 8, 3, H.Q4_K, H.Q4_K)
+    layer = api.MoeLayer(cfg, torch.empty((8, cfg.blob_bytes), dtype=torch.uint8, device="meta"), max_tokens=4)
+    kept = None
+    for T in (1, 4, 1):
+        for device in ("cpu", "meta"):
+            outs = layer.forward(torch.zeros((T, 8), device=device), torch.zeros((T, 256), device=device), stream=0)
+            assert [(tuple(o.shape), o.dtype, o.device.type, o.is_contiguous()) for o in outs] == [
+                ((T, 3), torch.int32, device, True), ((T, 3), torch.float32, device, True), ((T, 256), torch.float32, device, True)]
+            if device == "cpu":
+                assert kept is None or kept.data_ptr() != outs[2].data_ptr()
+                kept = outs[2]
+    held = len(layer._shapes)
+    for T in (5, 6, 7):
+        with pytest.raises(api.MayaError):
+            layer.forward(torch.zeros((T, 8)), torch.zeros((T, 256)), stream=0)
+    assert len(layer._shapes) == held
