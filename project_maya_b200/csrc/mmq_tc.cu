@@ -110,9 +110,6 @@ __host__ __device__ constexpr int64_t xq_tail(int64_t cols) { return ((cols / 32
 __host__ __device__ constexpr int64_t xq_ld(int64_t cols) { return cols + xq_tail(cols); }
 
 struct MmqArgs {
-    const uint8_t* w;            // the matrices (the i-quant path copies row windows itself; the others go through tm_w)
-    size_t expert_bytes;
-    int mat_rows;                // rows of one matrix (2 n_ff for the fused form)
     int w_rows, w_cols;          // rows of one output (n_ff for the fused form: gate rows, then up rows), K
     int n;                       // matrices of this product
     const int* expert_map;       // optional: matrix i owns the rows of bounds entry expert_map[i]
@@ -1195,7 +1192,6 @@ int run_product(const maya_mmq_product* p, bool glu, float limit, const Chain* c
     if (p->n <= 0 || p->total_rows <= 0) return MAYA_OK;
     const int64_t out_rows = glu ? p->w_rows / 2 : p->w_rows;
     MmqArgs A{};
-    A.w = (const uint8_t*) p->w; A.expert_bytes = p->expert_bytes; A.mat_rows = (int) p->w_rows;
     A.w_rows = (int) out_rows; A.w_cols = (int) p->w_cols; A.n = p->n; A.expert_map = p->expert_map; A.bounds = p->bounds;
     A.ids = p->ids; A.dst = p->dst; A.ld_dst = p->ld_dst; A.xq_out = glu ? (__half*) p->xq_out : nullptr; A.limit = limit;
     A.error = p->error;
