@@ -33,9 +33,10 @@
 // weights waiting 3000 cycles - the activation loader, one lane in a divergent branch, took 540 cycles a tile (every operand of a copy
 // crossed into a uniform register), longer than the expansion.  Now both loaders walk their loops as whole warps and an elected lane
 // copies, the role's number is warp-uniform to the compiler (an issuing warp's products 137 -> 47 cycles), the stages fill tensor
-// memory, and a stage is asked for before the expansion that goes there.  us a layer, before and after: 64 tokens of IQ3_S 463 / 385,
-// 777 of IQ2_S with a shared expert 1262 / 1165, 4096 of Q8_0 / Q4_K 3499 / 3190, 60 of Q8_0 236 / 200, 100 of Q4_K 265 / 245.  Then the
-// expansions themselves: Q4_K's header two sub-blocks at a time (100 of Q4_K 218), IQ2_S's codebook of byte selectors (777 of IQ2_S 1184 / 1108).
+// memory, and a stage is asked for before the expansion that goes there.  Then the
+// expansions themselves: Q4_K's header two sub-blocks at a time, IQ2_S's codebook of byte selectors.  us a layer, without and with all of
+// it, in turn on one board: 64 tokens of IQ3_S 437 / 367, 777 of IQ2_S with a shared expert 1309 / 1161, 4096 of Q8_0 / Q4_K 3580 / 3284,
+// 90 of Q8_0 with a shared expert 134 / 110, 363 of IQ3_S 2040 / 1667.
 //
 // Every mbarrier wait is bounded: a wait that runs out sets the error word, the roles stop, copies in
 // flight are waited for (bounded), tensor memory is freed and the block returns.
@@ -307,7 +308,7 @@ template<int T> __device__ __forceinline__ __half2 iq_scales(uint32_t word, int 
 // Sub-blocks J and J + 1 (J even): look-ups -> weights, in place; `mid` runs when the first is done.
 // IQ2_S (ggml dequantize_row_iq2_s): y = d (0.5 + ls) 0.25 * grid[qs | qh bits] * sign; the factor is f16(d (2 ls + 1) / 8), and the three
 // products by it are rounded once, as every weight's own would be.  (A selector's upper half is brought down by a dp2a: the byte permutes fill the integer pipe,
-// and with a shift there 3000 tokens of 4096 x 2048 took 1445 us, so 1416, with f16 entries 1561; 777 of 6144 x 2048 1138, 1108, 1184.)
+// and with a shift there 3000 tokens of 4096 x 2048 took 1.02 times, with f16 entries 1.10 times as long; 777 of 6144 x 2048 1.03 and 1.07 times.)
 template<int J, class Mid> __device__ __forceinline__ void iq_finish2(const IqFields<MAYA_IQ2_S>& F, uint32_t* o, Mid mid) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {

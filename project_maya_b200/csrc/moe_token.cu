@@ -74,8 +74,9 @@ bool token_better(int type, const FusedArgs& A, int sms) {
             // with a 512-wide one 1.09; 4096 x 2304, top 2 1.12; 6144 x 2048 67.1 / 55.4
             return (A.n_ff > 512 || (sh && A.n_embd > 6144)) &&
                    (A.n_embd > 3072 || (R >= 26 * MB && (!sh || A.n_embd > 2560)) || (R >= 20 * MB && sh && routed && A.n_embd > 2304));
-        default:                     // IQ2_S.  Its rows decode fastest: beside a shared expert's 8-bit rows they wait (6144 x 2048: 59.6 / 61.7, without
-            // one 69.6 / 58.0); 7168 x 512, top 8: 0.88 times as fast; 2560 x 1280, top 6 0.93; 3584 x 1024, top 5 1.00 and, out of HBM, 1.18
+        default:                     // IQ2_S.  Its rows decode fastest: beside a shared expert's 8-bit rows they wait (6144 x 2048, 2048 shared: 59.6 / 61.8,
+            // 7168 x 2048 68.9 / 70.5; narrower shared experts 0.98 to 1.04 times as fast; 6144 x 2048 without one 66.3 / 54.1); 7168 x 512, top 8: 0.88
+            // times as fast; 2560 x 1280, top 6 0.94; 3584 x 1024, top 5 0.99 and, out of HBM, 1.18
             return !sh && A.n_ff > 512 && ((R >= 40 * MB && A.n_embd > 2304) || (R >= 17 * MB && A.n_embd > 3072));
     }
 }
