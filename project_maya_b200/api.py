@@ -406,6 +406,7 @@ class MoeLayer:
                                  *((1, _ptr(sigmoid[0]), float(sigmoid[1]), int(bool(sigmoid[2]))) if sigmoid is not None else (0, None, 1.0, 0)),
                                  _ptr(cpu_part), _ptr(cpu_flag))
         self._keep = (sigmoid, cpu_part, cpu_flag)
+        self._ones = {experts.device: self._one(experts.device)}    # not at the first call: a graph's pool that held them would outlive the graph
         self._shapes = {}
         self.max_tokens = max_tokens
         nbytes = int(_lib.load().maya_moe_layer_scratch_bytes(C.byref(self.desc), max_tokens))
@@ -413,12 +414,16 @@ class MoeLayer:
             raise MayaError("moe_layer_scratch_bytes", -1)
         self.scratch = torch.zeros(nbytes, dtype=torch.uint8, device=experts.device)   # zeroed: holds a barrier counter
 
+    @staticmethod
+    def _one(device):
+        return torch.empty((), dtype=torch.int32, device=device), torch.empty((), dtype=torch.float32, device=device)
+
     def _like(self, T, device):
         """What a call's outputs look like (one value of memory each), on the logits' device: torch.empty_like of these takes 1.3 us,
         torch.empty of a shape, a type and a device 2.3."""
         like = self._shapes.get((T, device))
         if like is None:
-            i32, f32 = torch.empty((), dtype=torch.int32, device=device), torch.empty((), dtype=torch.float32, device=device)
+            i32, f32 = self._ones.get(device) or self._one(device)
             like = (i32.expand(T, self.cfg.k), f32.expand(T, self.cfg.k), f32.expand(T, self.cfg.n_embd))
             if T <= self.max_tokens:             # more are refused: nothing to keep
                 self._shapes[T, device] = like

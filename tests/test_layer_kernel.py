@@ -104,3 +104,36 @@ def test_a_layers_outputs_lie_where_its_logits_do(monkeypatch):
         with pytest.raises(api.MayaError):
             layer.forward(torch.zeros((T, 8)), torch.zeros((T, 256)), stream=0)
     assert len(layer._shapes) == held
+
+
+def test_a_layers_first_call_allocates_its_outputs_only(monkeypatch):
+    """What a MoeLayer keeps from call to call is allocated when it is made, on its experts' device: a first call under graph capture would
+    take it from the graph's own pool, which could then not be given back while the layer lives."""
+    import torch
+
+    from project_maya_b200 import _lib, api
+
+    class Fake:
+        maya_row_bytes = staticmethod(lambda t, n: 144 * (n // 256))
+        maya_moe_layer_scratch_bytes = staticmethod(lambda *a: 64)
+        maya_moe_layer_decode = staticmethod(lambda L, *a: 0)
+
+    monkeypatch.setattr(_lib, "load", lambda: Fake)
+    monkeypatch.setattr(api, "_ptr", lambda t: None)
+    cfg = api.MoeLayerConfig(256, 256, 8, 3, H.Q4_K, H.Q4_K)
+    layer = api.MoeLayer(cfg, torch.empty((8, cfg.blob_bytes), dtype=torch.uint8), max_tokens=4)
+    calls = [(torch.zeros((T, 8)), torch.zeros((T, 256))) for T in (1, 4)]
+    made = []
+
+    class Watch(torch.utils._python_dispatch.TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            if isinstance(out, torch.Tensor) and func.overloadpacket is not torch.ops.aten.expand:
+                made.append(out.shape)
+            return out
+
+    for logits, x in calls:
+        made.clear()
+        with Watch():
+            outs = layer.forward(logits, x, stream=0)
+        assert made == [o.shape for o in outs]
