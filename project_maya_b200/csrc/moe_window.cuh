@@ -288,10 +288,13 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
         const WKind& k = sh.kind[SH ? J.shared : 0];
         __syncwarp();                                            // every lane has read the stage's last bytes
         // Beside a shared expert which of two constants each: looked up, and with a division for the rows of a stage, they cost two-token windows
-        // 2 to 6 % (6144 x 2048 IQ2_S with 2048 shared 130.0 / 124.4 us).  Without one they are looked up: as constants 4 % slower on Q8_0.
+        // 2 to 6 % (6144 x 2048 IQ2_S with 2048 shared 130.0 / 124.4 us).  Without one they are looked up, each where it is used: as constants
+        // 4 % slower on Q8_0, looked up ahead of the branches below 1 % on IQ2_S (six tokens of 6400 x 3072 246.7 / 243.5 us): a register each.
         const bool js = SH && J.shared;
-        const int seg_bytes = SH ? (js ? GS::bytes : G::bytes) : k.bytes, pitch = SH ? (js ? GS::pitch : G::pitch) : k.pitch, split = js ? GS::split : 1;
-        const uint32_t at = (uint32_t) (ps * seg_bytes), len = min((uint32_t) seg_bytes, (uint32_t) k.rb - at);
+        auto seg_bytes = [&]() -> int { if constexpr (SH) return js ? GS::bytes : G::bytes; else return k.bytes; };
+        auto pitch = [&]() -> int { if constexpr (SH) return js ? GS::pitch : G::pitch; else return k.pitch; };
+        const int split = js ? GS::split : 1;
+        const uint32_t at = (uint32_t) (ps * seg_bytes()), len = min((uint32_t) seg_bytes(), (uint32_t) k.rb - at);
         const uint32_t pstage = asked & 1u, dst = ring + pstage * kStage;
         const int rows = js ? RW / GS::split : RW, first = js ? pq * rows : 0;      // the stage's rows
         if ((J.ptr & 15ull) == 0 && (!A.plain || js)) {
@@ -300,7 +303,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
                 const uint32_t off = (uint32_t) (uintptr_t) src & 15u, bytes = (off + len + 15u) & ~15u;
                 fence_proxy_async();
                 mbar_expect_tx(&sh.full[warp][pstage], bytes);
-                bulk_load(s_raw + dst + lane * pitch, src - off, bytes, &sh.full[warp][pstage]);
+                bulk_load(s_raw + dst + lane * pitch(), src - off, bytes, &sh.full[warp][pstage]);
             } else if (SH && lane < RW) {
                 mbar_arrive_one(&sh.full[warp][pstage]);
             }
@@ -308,7 +311,7 @@ __global__ void __launch_bounds__(WGeo<T>::threads, 1) window_kernel(const WArgs
             for (int r = 0; r < rows; ++r) {
                 const uint8_t* src = row_ptr(J.ptr, k, pc, first + r) + at;
                 const uint32_t off = (uint32_t) (uintptr_t) src & 15u;
-                for (uint32_t i = 2 * lane; i < len; i += 64) *(uint16_t*) (s_raw + dst + r * pitch + off + i) = *(const uint16_t*) (src + i);
+                for (uint32_t i = 2 * lane; i < len; i += 64) *(uint16_t*) (s_raw + dst + r * pitch() + off + i) = *(const uint16_t*) (src + i);
             }
             __syncwarp();
             if (lane < RW) mbar_arrive_one(&sh.full[warp][pstage]);
