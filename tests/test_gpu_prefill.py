@@ -259,6 +259,33 @@ def test_tall_groups_equal_short_groups_bitwise(T, api, t, rows):
 
 @pytest.mark.parametrize("t,cols", [(H.Q4_K, 256), (H.Q4_K, 1792), (H.Q4_K, 2304), (H.Q8_0, 256), (H.Q8_0, 768), (H.IQ2_S, 4096), (H.IQ3_S, 2048)])
 def test_tiles_of_every_height_one_after_another_bitwise(T, api, t, cols):
+    """A tile's rows decide how tensor memory and the activation ring are divided.  Blocks that take tiles of every division in turn
+    (heights at both edges of each, more tiles than SMs; K of less than a ring, and Q4_K chunks of 1, 7 and 8 + 1 blocks): the bits of
+    the same rows in groups of at most 16, which all have one division."""
+    w_rows, heights = 512, [1, 160, 33, 32, 129, 64, 97, 65, 128, 96, 16, 17] * 8
+    w1 = synth_matrices(T, api, t, 4, w_rows, cols, 61)
+    w = w1[T.arange(len(heights), device="cuda") % 4].contiguous()
+    total = sum(heights)
+    xq = api.mmq_quantize(dev(T, H.rng_for("heights", t, cols).standard_normal((total, cols)).astype(np.float32)), None, t)
+
+    def run(mats, counts):
+        out = T.full((total, w_rows), 7.0, dtype=T.float32, device="cuda")
+        err = T.zeros(1, dtype=T.int32, device="cuda")
+        bounds = dev(T, np.concatenate([[0], np.cumsum(counts)]).astype(np.int32))
+        api.mmq_run(api.mmq_product(mats, t, w_rows, cols, mats.shape[1], len(counts), xq, bounds, None, total, out, w_rows, error=err))
+        T.cuda.synchronize()
+        assert int(err.item()) == 0
+        return out
+
+    short = [(g % 4, min(16, h - at)) for g, h in enumerate(heights) for at in range(0, h, 16)]
+    want = run(w1[T.tensor([e for e, _ in short], device="cuda")].contiguous(), [n for _, n in short])
+    got = run(w, heights)
+    assert T.isfinite(got).all() and float(got.abs().max()) > 0.1
+    assert T.equal(got, want)
+
+
+@pytest.mark.parametrize("t,cols", [(H.Q4_K, 256), (H.Q4_K, 1792), (H.Q4_K, 2304), (H.Q8_0, 256), (H.Q8_0, 768), (H.IQ2_S, 4096), (H.IQ3_S, 2048)])
+def test_tiles_of_every_height_behind_every_other_bitwise(T, api, t, cols):
     """A tile's rows decide how tensor memory and the activation ring are divided.  Blocks that take ten tiles and more, every division behind
     every other (heights at both edges of each; K of less than a ring, and Q4_K chunks of 1, 7 and 8 + 1 blocks), plain and with
     SwiGLU and the rounding of h in the write-back: the bits of the same rows in groups of at most 16, which all have one division."""
@@ -330,7 +357,6 @@ def test_k_values_are_added_in_order(T, api, t, copies):
 @pytest.mark.parametrize("ta,tb,counts,n_ff", [
     (H.Q8_0, H.Q4_K, [1, 0, 161, 7, 320, 33], 256),                                       # fewer tiles than blocks, remainders of 160 rows
     (H.IQ2_S, H.IQ3_S, [5] * 24 + [0] * 3 + [170] * 3, 2048),                             # several rounds of tiles
-    (H.IQ3_S, H.Q4_K, [97, 1, 160, 33, 16, 129, 64, 32, 65, 128, 17, 96] * 4, 2048),      # ten tiles a block, of every division
     (H.Q4_K, H.Q8_0, [0] * 6, 256)])                                                      # no rows at all in one pair
 def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
     """Two pairs of gate/up and down products in one chain, each down tile starting when its own rows of h are there: the bits
@@ -356,7 +382,7 @@ def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
     for gu, dn, _, _ in want:
         api.mmq_run_glu(gu, 7.0)
         api.mmq_run(dn)
-    counters = T.zeros(max(4096, api._lib.load().maya_mmq_chain_bytes(sum(p["total"] for p in pairs), sum(p["n"] for p in pairs), 2)), dtype=T.uint8, device="cuda")
+    counters = T.zeros(4096, dtype=T.uint8, device="cuda")
     for _ in range(2):
         got = [products(p) for p in pairs]
         api.mmq_run_chain([g[0] for g in got], [g[1] for g in got], 7.0, counters)
@@ -367,6 +393,39 @@ def test_chain_equals_its_products_bitwise(T, api, ta, tb, counts, n_ff):
     assert want[1][3].abs().max() > 0.01
     with pytest.raises(api.MayaError):                                                    # the down product reads another h
         api.mmq_run_chain([want[0][0]], [got[0][1]], 7.0, counters)
+
+
+def test_chain_of_tiles_of_every_height_equals_its_products_bitwise(T, api):
+    """A chain's tiles are taken as blocks get to them: ten a block and more, every division of tensor memory behind others, i-quants in one pair
+    and Q4_K in the other.  The bits of the four products run one after another; the counters end at zero."""
+    cols, n_ff, counts = 2048, 2048, [97, 1, 160, 33, 16, 129, 64, 32, 65, 128, 17, 96] * 4
+    n, total = len(counts), sum(counts)
+    assert 2 * n * (n_ff // 128 + 512 // 256) >= 10 * T.cuda.get_device_properties(0).multi_processor_count
+    err = T.zeros(1, dtype=T.int32, device="cuda")
+    pairs = []
+    for t, c in ((H.IQ3_S, counts), (H.Q4_K, counts[::-1])):
+        x = H.rng_for("chain heights", t).standard_normal((total, cols)).astype(np.float32)
+        pairs.append((t, synth_matrices(T, api, t, n, 2 * n_ff, cols, 31), synth_matrices(T, api, t, n, 512, n_ff, 37),
+                      api.mmq_quantize(dev(T, x), None, t), dev(T, np.concatenate([[0], np.cumsum(c)]).astype(np.int32))))
+
+    def products(t, w, wd, xq, bounds):
+        hq = T.zeros(api.mmq_q8_bytes(total, n_ff), dtype=T.uint8, device="cuda")
+        out = T.zeros((total, 512), dtype=T.float32, device="cuda")
+        return (api.mmq_product(w, t, 2 * n_ff, cols, w.shape[1], n, xq, bounds, None, total, None, n_ff, error=err, xq_out=hq),
+                api.mmq_product(wd, t, 512, n_ff, wd.shape[1], n, hq, bounds, None, total, out, 512, error=err), hq, out)
+
+    want = [products(*p) for p in pairs]
+    for gu, dn, _, _ in want:
+        api.mmq_run_glu(gu, 7.0)
+        api.mmq_run(dn)
+    counters = T.zeros(api._lib.load().maya_mmq_chain_bytes(2 * total, 2 * n, 2), dtype=T.uint8, device="cuda")
+    got = [products(*p) for p in pairs]
+    api.mmq_run_chain([g[0] for g in got], [g[1] for g in got], 7.0, counters)
+    T.cuda.synchronize()
+    assert int(err.item()) == 0 and not counters.any()
+    for a, b in zip(got, want):
+        assert T.equal(a[2], b[2]) and T.equal(a[3], b[3])
+    assert min(float(p[3].abs().max()) for p in want) > 0.01
 
 
 def test_refused_chain_launches_nothing_and_leaves_its_counters_alone(T, api, lib):
